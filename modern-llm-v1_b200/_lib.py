@@ -7,7 +7,9 @@ there), RuntimeError for CUDA / device failures (std::runtime_error there).
 """
 from __future__ import annotations
 
+import atexit
 import ctypes
+import importlib
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -27,13 +29,11 @@ BWD_STATIC_MAX_ROWS = 524288
 
 LAYOUT_BHTD = 0
 LAYOUT_BTHD = 1
-LAYOUTS = {"BHTD": LAYOUT_BHTD, "BTHD": LAYOUT_BTHD}
 DTYPE_BF16 = 0
 DTYPE_F32 = 1
 BWD_AUTO = 0
 BWD_TWO_PASS = 1
 BWD_ONE_PASS = 2
-BWD_MODES = {"auto": BWD_AUTO, "two_pass": BWD_TWO_PASS, "one_pass": BWD_ONE_PASS}
 
 # every symbol include/b200attn.h declares
 SYMBOLS = (
@@ -67,6 +67,25 @@ SYMBOLS = (
 )
 
 _lib = None
+_host = None
+
+
+def host():
+    """The native module behind the operators (csrc/host_binding.cc); raises RuntimeError if it has not been built."""
+    return _host or _load_host()
+
+
+def _load_host():
+    global _host
+    load()
+    try:
+        h = importlib.import_module(__package__ + "._host")
+    except ImportError as e:
+        raise RuntimeError(f"{os.path.join(HERE, '_host.so')} cannot be loaded ({e}): build it with "
+                           "`python -m modern_llm_v1_b200.build`") from e
+    atexit.register(h.release_scratch)
+    _host = h
+    return h
 
 
 def load() -> ctypes.CDLL:

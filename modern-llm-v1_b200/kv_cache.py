@@ -15,13 +15,10 @@ PyTorch fallback.
 """
 from __future__ import annotations
 
-import ctypes
-
 import torch
 
 from . import _lib
-from .flash_attn import _check_tensors, _stream_ptr, _workspace
-from .rope_norm import _x_dtype, make_rope_cache
+from .rope_norm import make_rope_cache
 
 
 class KVCache:
@@ -60,95 +57,19 @@ class KVCache:
         self.lengths = torch.tensor(host, dtype=torch.int32, device=self.device)
         self._lens_next = self.lengths + 1
 
-    def _layer(self, fn: str, layer: int) -> None:
-        if not 0 <= layer < self.n_layers:
-            raise ValueError(f"{fn}: layer {layer} out of range")
-
     def append(self, layer: int, xq, xk, xv, gamma_q, gamma_k, q_out) -> None:
         """xq [B, n_new, Hq, D], xk / xv [B, n_new, Hkv, D] (the projection outputs, FP32 or BF16, all the
         same type) are the n_new tokens after the `length` cached ones.  Writes q_out [B, Hq, n_new, D] BF16
         (rotated, normalised, times gamma_q) and the tokens' rows of this layer's K (same chain with gamma_k)
         and V (converted to BF16)."""
-        fn = "KVCache.append"
-        self._layer(fn, layer)
-        xd = _x_dtype(fn, xq)
-        f32 = torch.float32
-        _check_tensors(fn, [(xq, "xq", xq.dtype), (xk, "xk", xq.dtype), (xv, "xv", xq.dtype),
-                            (q_out, "q_out", torch.bfloat16), (gamma_q, "gamma_q", f32), (gamma_k, "gamma_k", f32)])
-        B, Hq, Hkv, D = self.B, self.Hq, self.Hkv, self.D
-        if xq.dim() != 4 or xq.shape[0] != B or xq.shape[2] != Hq or xq.shape[3] != D:
-            raise ValueError(f"{fn}: xq must be [B, n_new, Hq, D]")
-        n_new = int(xq.shape[1])
-        if n_new <= 0:
-            raise ValueError(f"{fn}: no tokens")
-        if tuple(xk.shape) != (B, n_new, Hkv, D) or tuple(xv.shape) != (B, n_new, Hkv, D):
-            raise ValueError(f"{fn}: xk and xv must be [B, n_new, Hkv, D]")
-        if q_out.numel() != xq.numel():
-            raise ValueError(f"{fn}: q_out numel mismatch")
-        if gamma_q.numel() != D or gamma_k.numel() != D:
-            raise ValueError(f"{fn}: gamma_q and gamma_k must have d_h elements")
-        if self.length + n_new > self.L_cap:
-            raise ValueError(f"{fn}: {self.length} + {n_new} tokens exceed the capacity {self.L_cap}")
-        lib = _lib.load()
-        if self.lengths is not None:
-            if n_new != 1:
-                raise ValueError(f"{fn}: one token per sequence once the lengths differ")
-            with torch.cuda.device(self.device):
-                rc = lib.b200attn_kv_append_at(xq.data_ptr(), xk.data_ptr(), xv.data_ptr(), xd, q_out.data_ptr(),
-                                               self.k[layer].data_ptr(), self.v[layer].data_ptr(), gamma_q.data_ptr(),
-                                               gamma_k.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(),
-                                               self.lengths.data_ptr(), B, 1, self.L_cap, Hq, Hkv, D,
-                                               ctypes.c_float(self.eps), _stream_ptr())
-            _lib.check(rc, fn)
-            return
-        with torch.cuda.device(self.device):
-            rc = lib.b200attn_kv_append(xq.data_ptr(), xk.data_ptr(), xv.data_ptr(), xd, q_out.data_ptr(),
-                                        self.k[layer].data_ptr(), self.v[layer].data_ptr(), gamma_q.data_ptr(),
-                                        gamma_k.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), B, n_new,
-                                        self.length, self.L_cap, Hq, Hkv, D, ctypes.c_float(self.eps), _stream_ptr())
-        _lib.check(rc, fn)
+        _lib.host().kv_append(self, layer, xq, xk, xv, gamma_q, gamma_k, q_out)
 
     def attend(self, layer: int, q, ctx, lse, n_new: int = 1, softmax_scale=None) -> None:
         """Attention of the n_new appended tokens over the length + n_new cached ones.  q, ctx: [B, Hq, n_new, D]
         BF16; lse: [B, Hq, n_new] FP32 (may be None for n_new == 1).  n_new == 1 is the split-KV decode kernel;
         n_new > 1 is the causal forward of the new tokens over the cache: a whole prompt into an empty cache, or a
         further chunk of it behind the tokens already cached (chunked prefill; lock-step sequences only)."""
-        fn = "KVCache.attend"
-        self._layer(fn, layer)
-        bf = torch.bfloat16
-        items = [(q, "q", bf), (ctx, "ctx", bf)]
-        if lse is not None:
-            items.append((lse, "lse", torch.float32))
-        _check_tensors(fn, items)
-        B, Hq, Hkv, D = self.B, self.Hq, self.Hkv, self.D
-        if n_new <= 0 or self.length + n_new > self.L_cap:
-            raise ValueError(f"{fn}: n_new out of range")
-        if q.numel() != B * Hq * n_new * D or ctx.numel() != q.numel():
-            raise ValueError(f"{fn}: q and ctx must be [B, Hq, n_new, D]")
-        if lse is not None and lse.numel() != B * Hq * n_new:
-            raise ValueError(f"{fn}: lse must be [B, Hq, n_new]")
-        lib = _lib.load()
-        scale = float(softmax_scale or 0.0)
-        kc, vc = self.k[layer], self.v[layer]
-        with torch.cuda.device(self.device):
-            if n_new == 1:
-                L = self.length + 1
-                nbytes = int(lib.b200attn_decode_workspace_bytes(B, L, Hq, Hkv, D, 0))
-                ws = _workspace("decode", nbytes, self.device)
-                rc = lib.b200attn_decode_ragged(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), ctx.data_ptr(),
-                                                lse.data_ptr() if lse is not None else None,
-                                                self._lens_next.data_ptr() if self.lengths is not None else None, B, L,
-                                                self.L_cap, Hq, Hkv, D, scale, 0, ws.data_ptr(), ws.numel(),
-                                                _stream_ptr())
-            else:
-                if self.lengths is not None:
-                    raise ValueError(f"{fn}: several tokens at once only while the sequences advance in lock step")
-                if lse is None:
-                    raise ValueError(f"{fn}: lse is required for n_new > 1")
-                rc = lib.b200attn_fwd_kvcache_at(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), ctx.data_ptr(),
-                                                 lse.data_ptr(), B, n_new, self.length, self.L_cap, Hq, Hkv, D,
-                                                 _lib.LAYOUTS["BHTD"], scale, _stream_ptr())
-        _lib.check(rc, fn)
+        _lib.host().kv_attend(self, layer, q, ctx, lse, n_new, softmax_scale)
 
     def advance(self, n_new: int = 1) -> None:
         """Call once per step, after every layer has appended and attended."""
