@@ -533,7 +533,7 @@ def run_decode(m, cfg, args, rank, world, device, peaks, warmup, steps, barrier)
             "dtype": "bf16", "data": "synthetic",
             "config": {"workload": cfg.name, "B_per_gpu": cfg.B, "cache_len": cfg.T, "Hq": cfg.Hq, "Hkv": cfg.Hkv,
                        "D": cfg.D, "l2": f"cache of {nbytes / 1e6:.0f} MB > 126 MB L2"},
-            "clocks": clocks, "gpu_launches": 2 * steps,
+            "clocks": clocks, "gpu_launches": steps,
             "e2e": {"value": world * nbytes / (ms_e2e * 1e-3) / 1e9, "unit": "GB/s", "ms_per_step": ms_e2e,
                     "h2d_bytes_per_step": q.numel() * 2, "d2h_bytes_per_step": q.numel() * 2,
                     "note": "q from pinned host memory, o read back, a stream synchronise per step; the cache stays "
@@ -542,7 +542,7 @@ def run_decode(m, cfg, args, rank, world, device, peaks, warmup, steps, barrier)
                          "unit": "GB/s", "frac": gbs / world / peak,
                          "traffic": 273341184 if cfg.name == "c5_decode" else None,  # profiles/attn_decode_c5_decode.md
                          "peak_source": f"hbm_gbs of {peaks['_source']}", "bytes_per_launch": nbytes,
-                         "note": "time includes the combine kernel (2 launches per step)"},
+                         "note": "1 launch per step"},
         }), flush=True)
 
 
@@ -755,16 +755,16 @@ def run_decode_step(m, cfg, args, rank, world, device, peaks, warmup, steps, bar
         "config": {"workload": cfg.name + "_step", "B_per_gpu": B, "cache_len": L, "Hq": Hq, "Hkv": Hkv, "D": D,
                    "io": "new token's q, k, v FP32 [B,1,H,D] in; caches BF16 [B,Hkv,L,D]; o BF16 out",
                    "l2": f"cache of {cfg.decode_bytes() / 1e6:.0f} MB > 126 MB L2"},
-        "clocks": clocks, "gpu_launches": 3 * steps,
+        "clocks": clocks, "gpu_launches": 2 * steps,
         "e2e": {"value": world * nbytes / (ms_e2e * 1e-3) / 1e9, "unit": "GB/s", "ms_per_step": ms_e2e,
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "note": "the new token's rows from pinned host memory, o read back, a stream synchronise per step"},
         "roofline": {"bound": "hbm", "kernel": "attn_decode_kernel", "achieved": gbs / world, "peak": peak,
                      "unit": "GB/s", "frac": gbs / world / peak,
-                     # the three kernels of a step, profiles/kv_append_decode_step_c5_decode.md
+                     # the kernels of a step, profiles/kv_append_decode_step_c5_decode.md
                      "traffic": 272819456 if cfg.name == "c5_decode" else None,
                      "peak_source": f"hbm_gbs of {peaks['_source']}", "bytes_per_step": nbytes,
-                     "note": "3 launches per step: kv_append_kernel, attn_decode_kernel, attn_decode_combine_kernel"},
+                     "note": "2 launches per step: kv_append_kernel, attn_decode_kernel"},
     }
     if rank == 0 and not args.no_cpu_baseline:
         from oracle import attn_oracle as ao

@@ -3,15 +3,33 @@
 // llm/apps/infer_modern_gpt.cu:253-255); the math is row L-1 of its causal attention
 // (llm/src/model/flash_attn.cu:28-131) with T = L.
 //
-// The kernel is bound by HBM: every K and V byte of the cache is read exactly once.
-// A CTA owns one (batch, KV head, split of the cache length) and serves ALL query heads of
-// the group from the same K/V tile, which is the whole bandwidth win of GQA.  K/V tiles
-// (128 keys) stream through a 3-stage shared-memory ring filled by TMA (128-byte swizzle,
-// which also makes the row-per-thread reads bank-conflict free).
+// Large caches are bound by HBM (every K and V byte is read exactly once), small ones by latency.  A unit is one
+// (batch, KV head, chunk of at most 16 query heads of the group): all its query heads are served from the same K/V tile,
+// which is the bandwidth win of GQA.  One launch does everything; it deals the units' tiles in one of two ways
+// (decode_plan in b200attn_api.cu chooses):
+//  * clusters: a unit's tiles are split over the CTAs of a cluster (1, 2, 4 or 8), which exchange their partial results
+//    through distributed shared memory, each CTA finishing a slice of the outputs.
+//  * ranges: the tiles of all units are numbered through and CTA c of n takes tiles [c total / n, (c + 1) total / n), the
+//    same number for every CTA (to one) whatever the units' lengths are.  A range falls into pieces at unit boundaries; a
+//    piece that is a whole unit is written at once, the pieces of a unit that several CTAs share are left un-normalised
+//    (m, l, O) in the workspace, and the CTA that finishes last (a counter per shared unit) adds them up in the order of
+//    the tiles, so the result does not depend on who was last.
 //
-// Roles (160 threads): warps 0-3 compute with warp-level BF16 MMAs (m16n8k16: the 16 rows are
-// the query heads of the group), each warp on its own 32 keys of a tile; warp 4 = TMA producer.
-// Each split writes an un-normalised partial (m, l, O); a small combine kernel merges them.
+// K/V tiles stream through a 96 KB shared-memory ring filled by TMA (128-byte swizzle, which also makes the row-per-thread
+// reads bank-conflict free); the ring runs on across pieces.  Two CTAs share an SM: one streams while the other is at the end
+// of a piece.
+//
+// Roles (192 threads): warps 0-3 compute with warp-level BF16 MMAs (m16n8k16), each on its own quarter of a tile's keys.  Keys
+// and head dimension are the rows and the unit's query heads the columns, S^T = K Q^T and O^T = V^T P^T, eight heads at a time
+// (NH = 1 or 2): with the heads as rows the usual four of sixteen would be used, at twice the instructions.  Warp 4 = TMA
+// producer (converged, one elected lane issues: from a diverged lane a TMA instruction cost 160 clocks).  Warp 5 counts the
+// shared piece that a range begins with, so that the compute warps go on to the next piece at once (fence, counter and
+// addition are a chain of 3 us through L2).
+//
+// Measured on B200 against one CTA per (unit, split), heads as MMA rows and a second kernel for the partial results, us per
+// call back to back: B=1 L=110 6/2 D=64 4.1 -> 2.9; B=1 L=1500 16/4 D=128 8.5 -> 5.5; B=1 L=8192 16/4 D=128 23.8 -> 11.1;
+// B=48 L=300 16/4 D=64 7.9 -> 5.3; B=300 L=200 8/8 D=64 39.3 -> 24.6; B=64 L=4096 16/4 D=64 45.2 -> 42.1 (6.39 TB/s).
+// Eight compute warps in one CTA per SM, taking tiles in two groups, were slower at every piece's end (B=300: 42.8).
 #pragma once
 
 #include "ptx.cuh"
@@ -20,34 +38,48 @@ namespace b200attn {
 
 struct DecodeParams {
     int B, L, Hq, Hkv, group;
-    int G;         // query heads served per CTA (a divisor of group, <= 16)
+    int G;         // query heads per unit (a divisor of group, <= 16)
     int n_chunks;  // group / G
-    int n_splits;
-    int tiles_per_split;
+    int units_per_seq;  // Hkv * n_chunks
+    FastDiv div_units, div_chunks, div_cluster, div_tiles, div_slice;  // by units_per_seq, n_chunks, cluster, tiles of L, output pairs per CTA of a cluster
+    int cluster;        // CTAs per unit (clusters), or 0: ranges
+    int whole;          // ranges: they begin and end at unit boundaries (all sequences have length L)
+    int slot_mode;      // where a shared unit's pieces lie in the workspace, see decode_slot
     float scale, scale_log2;
     const int* lens;    // [B] cache length per sequence (1 <= lens[b]; clamped to L), or nullptr: every sequence has L
     const uint16_t* q;  // [B, Hq, D]
-    float* part_o;      // [B, Hq, n_splits, D]
-    float* part_m;      // [B, Hq, n_splits]   row maximum, raw score units
-    float* part_l;      // [B, Hq, n_splits]   sum of exp2((s - m) * scale_log2)
+    uint16_t* o;        // [B, Hq, D]
+    float* lse;         // [B, Hq] or nullptr
+    float* part_o;      // [slot][G][D]  un-normalised
+    float* part_m;      // [slot][G]     row maximum, raw score units
+    float* part_l;      // [slot][G]     sum of exp2((s - m) * scale_log2)
+    int* counters;      // one per CTA, zero between launches: pieces finished of the shared unit that begins in that CTA
     int* status;
 };
 
+constexpr int kDecodeMaxCtas = 320, kDecodeMaxCluster = 8, kDecodeThreads = 192;
+// Workspace slot of CTA c's piece of a shared unit.  The workspace has (units x splits) slots: one per tile when every
+// split is one tile (mode 0), one per CTA when the CTAs' ranges begin at unit boundaries (mode 1), else two per CTA
+// (mode 2: a range may end one shared unit and begin another).
+enum { kDecodeSlotTile = 0, kDecodeSlotCta = 1, kDecodeSlotTwo = 2 };
+
 template <int D>
 struct DecodeCfg {
+    static constexpr int kKeys = D == 64 ? 128 : 64;  // per tile
+    static constexpr int kTileBytes = kKeys * D * 2;  // 16 KB
     static constexpr int kStages = 3;
-    static constexpr int kTileKeys = 128;
-    static constexpr int kTileBytes = kTileKeys * D * 2;
-    static constexpr int kBoxBytes = 128 * 64 * 2;
+    static constexpr int kBoxBytes = kKeys * 64 * 2;
     static constexpr int kBoxes = D / 64;
-    static constexpr int kMaxG = 16;                    // query heads per CTA = rows of the m16n8k16 MMA
-    static constexpr int kQBytes = 16 * D * 2;          // q rows as BF16, zero padded to 16 rows, swizzled
-    // the end-of-kernel merge scratch (per warp 16 rows x (O row, m, l) as FP32) re-uses the K ring
-    static constexpr int kSmemBytes = 2 * kStages * kTileBytes + kQBytes + 256 + 1024;
+    static constexpr int kQRow = D * 2;
+    static constexpr int kQBytes = 16 * kQRow;          // rows >= G stay zero
+    static constexpr int kMlBytes = 4 * 16 * 8;         // (m, l) of the four warps' heads
+    static constexpr int kXBytes = 16 * D * 4 + kDecodeMaxCluster * 16 * 8;  // from the cluster: O slices, (m, l) rows
+    static_assert(4 * 16 * D * 4 <= 2 * kTileBytes, "the warps' O rows are merged in one K/V stage");
+    static constexpr int kSmemBytes = 2 * kStages * kTileBytes + 2 * kQBytes + kMlBytes + kXBytes + 256 + 1024;
 };
 
-// ---- warp-level tensor-core pieces (mma.sync is enough here: the kernel is bound by HBM, and the
-// ---- 16-row MMA shape matches "all query heads of a KV group against one key tile")
+// ---- warp-level tensor-core pieces (mma.sync is enough here: the kernel is bound by HBM and latency, and a unit has
+// ---- at most sixteen query heads, an eighth of a tcgen05 tile)
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
@@ -64,276 +96,615 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
+    uint32_t y;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+    return y;
+}
 // Byte offset of the 16-byte chunk `chunk` (8 BF16 of the head dimension) of row `r` inside a tile of
 // [rows][64]-boxes written by TMA with the 128-byte swizzle.
 __device__ __forceinline__ uint32_t swz_off(int r, int chunk, int box_bytes) {
     return uint32_t((chunk >> 3) * box_bytes + r * 128 + (((chunk & 7) ^ (r & 7)) << 4));
 }
 
-// One CTA = (split of the cache, KV head x head chunk, batch).  Warps 0-3 compute, each on its own
-// 32 keys of every 128-key tile and with its own running (m, l, O), so there is no CTA-wide
-// synchronisation inside the loop; the four states are merged once at the end.  Warp 4 is the TMA
-// producer.  S = Q K^T and O += P V run as m16n8k16 BF16 MMAs whose 16 rows are the G <= 16 query
-// heads that share this KV head (rows >= G are zero padding).
-template <int D>
-__global__ void __launch_bounds__(160)
+// Walks one CTA's pieces.  Executed by each warp on its own (all lanes alike); every warp sees the same pieces.
+struct DecodeWalk {
+    int t, t_end;        // next tile and end of this CTA's range, in the numbering over all units
+    int b, u, j0;        // unit at t: sequence, unit within the sequence, tile within the unit
+    int len, n_tiles;    // length and tiles per unit of sequence b
+    int total, n_ctas;   // tiles of all units, CTAs that share them
+};
+
+__device__ __forceinline__ int decode_len(const DecodeParams& p, int b) {
+    return p.lens ? max(1, min(__ldg(p.lens + b), p.L)) : p.L;
+}
+// First tile of CTA c's range, and the CTA whose range holds tile t.
+__device__ __forceinline__ int decode_range(const DecodeWalk& w, int c) {
+    const unsigned n = unsigned(w.n_ctas), q = unsigned(w.total) / n;
+    return int(unsigned(c) * q + unsigned(c) * (unsigned(w.total) - q * n) / n);
+}
+__device__ __forceinline__ int decode_cta_of(const DecodeWalk& w, int t) {
+    return int(((unsigned long long)(unsigned)(t + 1) * (unsigned)w.n_ctas - 1) / (unsigned)w.total);
+}
+
+template <int KEYS>
+__device__ __forceinline__ DecodeWalk decode_walk_start(const DecodeParams& p, int cta, int n_ctas, int lane) {
+    DecodeWalk w;
+    if (p.cluster) {  // one piece: this CTA's share of its unit's tiles, possibly none
+        const int unit = int(fastdiv(cta, p.div_cluster)), rank = cta - unit * p.cluster;
+        w.b = int(fastdiv(unit, p.div_units));
+        w.u = unit - w.b * p.units_per_seq;
+        w.len = decode_len(p, w.b);
+        w.n_tiles = (w.len + KEYS - 1) / KEYS;
+        w.total = w.n_tiles;
+        w.n_ctas = p.cluster;
+        w.t = w.j0 = int(fastdiv(w.n_tiles * rank, p.div_cluster));
+        w.t_end = int(fastdiv(w.n_tiles * (rank + 1), p.div_cluster));
+        return w;
+    }
+    if (!p.lens) {
+        w.len = p.L;
+        w.n_tiles = (p.L + KEYS - 1) / KEYS;
+        w.total = p.B * p.units_per_seq * w.n_tiles;
+    } else {
+        int sum = 0;
+        for (int b = lane; b < p.B; b += 32) sum += (decode_len(p, b) + KEYS - 1) / KEYS;
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        w.total = sum * p.units_per_seq;
+    }
+    w.n_ctas = min(n_ctas, w.total);
+    w.t = cta < w.n_ctas ? decode_range(w, cta) : 0;
+    w.t_end = cta < w.n_ctas ? decode_range(w, cta + 1) : 0;
+    if (p.whole) {  // (rounding the ends of all ranges down alike; at least one unit per CTA)
+        w.t -= w.t % w.n_tiles;
+        w.t_end -= w.t_end % w.n_tiles;
+    }
+    if (!p.lens) {
+        const int unit = int(fastdiv(w.t, p.div_tiles));
+        w.j0 = w.t - unit * w.n_tiles;
+        w.b = int(fastdiv(unit, p.div_units));
+        w.u = unit - w.b * p.units_per_seq;
+    } else {
+        // the sequence that holds tile t: 32 sequences at a time
+        const int target = int(fastdiv(w.t, p.div_units));  // in tiles of one unit per sequence
+        int before = 0;
+        w.b = p.B - 1, w.len = 1, w.n_tiles = 1, w.u = 0, w.j0 = 0;
+        for (int b0 = 0; b0 < p.B; b0 += 32) {
+            const int len = b0 + lane < p.B ? decode_len(p, b0 + lane) : 0;
+            const int n = (len + KEYS - 1) / KEYS;
+            int incl = n;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += up;
+            }
+            const unsigned hit = __ballot_sync(0xffffffffu, before + incl > target);
+            if (hit) {
+                const int src = __ffs(hit) - 1;
+                w.b = b0 + src;
+                w.len = __shfl_sync(0xffffffffu, len, src);
+                w.n_tiles = __shfl_sync(0xffffffffu, n, src);
+                const int start = (before + __shfl_sync(0xffffffffu, incl, src) - w.n_tiles) * p.units_per_seq;
+                w.u = (w.t - start) / w.n_tiles;
+                w.j0 = w.t - start - w.u * w.n_tiles;
+                break;
+            }
+            before += __shfl_sync(0xffffffffu, incl, 31);
+        }
+    }
+    return w;
+}
+// Tiles of the piece at w.t
+__device__ __forceinline__ int decode_piece(const DecodeWalk& w) { return min(w.t_end - w.t, w.n_tiles - w.j0); }
+template <int KEYS>
+__device__ __forceinline__ void decode_walk_next(const DecodeParams& p, DecodeWalk& w, int n) {
+    w.t += n;
+    w.j0 = 0;  // the piece ended at its unit's end, or the range is over
+    if (w.t < w.t_end && ++w.u == p.units_per_seq) {
+        w.u = 0;
+        ++w.b;
+        w.len = decode_len(p, w.b);
+        w.n_tiles = (w.len + KEYS - 1) / KEYS;
+    }
+}
+__device__ __forceinline__ int decode_slot(const DecodeParams& p, const DecodeWalk& w, int c, int first_cta, int unit_start) {
+    if (p.slot_mode == kDecodeSlotTile) return max(unit_start, decode_range(w, c));
+    if (p.slot_mode == kDecodeSlotCta) return c;
+    return 2 * c + (c == first_cta ? 1 : 0);
+}
+
+// One state of the online softmax over the unit's outputs, in the MMA's register layout (see the kernel): this lane's heads
+// are nh * 8 + (lane % 4) * 2 + {0, 1}, its head-dim rows of tile mt mt * 16 + lane / 4 + {0, 8}.  m is the same in the eight
+// lanes that share a head, l is each lane's share of the sum.
+template <int D, int NH>
+struct DecodeState {
+    float m[NH][2], l[NH][2];
+    float o[D / 16][NH][4];  // {row, head}: 0 {0, 0}, 1 {0, 1}, 2 {8, 0}, 3 {8, 1}
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int nh = 0; nh < NH; ++nh) {
+            m[nh][0] = m[nh][1] = -INFINITY;
+            l[nh][0] = l[nh][1] = 0.f;
+#pragma unroll
+            for (int mt = 0; mt < D / 16; ++mt) o[mt][nh][0] = o[mt][nh][1] = o[mt][nh][2] = o[mt][nh][3] = 0.f;
+        }
+    }
+};
+
+// barrier over the four compute warps that also tells every thread whether any of them has given up
+__device__ __forceinline__ bool decode_bar_ok(bool ok) {
+    uint32_t bad;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "setp.eq.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.or.pred q, 1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t"
+        "}\n"
+        : "=r"(bad)
+        : "r"(uint32_t(ok))
+        : "memory");
+    return bad == 0;
+}
+// Column swizzle of the merge scratch [warp][16 heads][D] FP32: the four heads a warp writes at once would share a bank
+__device__ __forceinline__ int decode_merge_col(int head, int col) { return col ^ (((head >> 1) & 3) << 3); }
+
+// The warps' states -> one, through shared memory; `use(g, d, acc0, acc1, m, l)` is called once per pair of output elements.
+template <int D, int NH, typename Use>
+__device__ __forceinline__ void decode_merge(DecodeState<D, NH>& s, float* sO, float2* sMl, int warp, int lane, int tid, int G,
+                                             float scale_log2, Use use) {
+    {
+        const int r = lane >> 2, c = (lane & 3) * 2;
+        float* mine = sO + warp * 16 * D;
+#pragma unroll
+        for (int nh = 0; nh < NH; ++nh)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float l = s.l[nh][e];
+                l += __shfl_xor_sync(0xffffffffu, l, 4);
+                l += __shfl_xor_sync(0xffffffffu, l, 8);
+                l += __shfl_xor_sync(0xffffffffu, l, 16);
+                const int g = nh * 8 + c + e;
+                if (g >= G) continue;
+#pragma unroll
+                for (int mt = 0; mt < D / 16; ++mt) {
+                    mine[g * D + decode_merge_col(g, mt * 16 + r)] = s.o[mt][nh][e];
+                    mine[g * D + decode_merge_col(g, mt * 16 + r + 8)] = s.o[mt][nh][e + 2];
+                }
+                if (r == 0) sMl[warp * 16 + g] = make_float2(s.m[nh][e], l);
+            }
+    }
+    named_bar_sync(1, 128);
+    for (int i = tid; i < G * (D / 2); i += 128) {
+        const int g = i / (D / 2), d = (i % (D / 2)) * 2;
+        float2 ml[4], v[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            ml[w] = sMl[w * 16 + g];
+            v[w] = *reinterpret_cast<const float2*>(sO + (w * 16 + g) * D + decode_merge_col(g, d));
+        }
+        const float m = fmaxf(fmaxf(ml[0].x, ml[1].x), fmaxf(ml[2].x, ml[3].x));
+        float a0 = 0.f, a1 = 0.f, l = 0.f;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const float f = (ml[w].x == -INFINITY) ? 0.f : ex2_approx((ml[w].x - m) * scale_log2);
+            a0 += f * v[w].x;
+            a1 += f * v[w].y;
+            l += f * ml[w].y;
+        }
+        use(g, d, a0, a1, m, l);
+    }
+}
+
+// One pair of output elements of a shared unit from its pieces in the workspace, in the order of the tiles.  `own`: the CTA
+// whose piece is passed in registers instead (the same values it would have stored), or -1.
+template <int D, typename Write>
+__device__ __forceinline__ void decode_add_pieces(const DecodeParams& p, const DecodeWalk& w, int first, int last, int unit_start, int g,
+                                                  int d, int own, float own0, float own1, float own_m, float own_l, Write write) {
+    float m = -INFINITY, l = 0.f, a0 = 0.f, a1 = 0.f;
+    for (int c0 = first; c0 <= last; c0 += 4) {
+        float pm[4], pl[4];
+        float2 po[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int c = c0 + k;
+            pm[k] = own_m, pl[k] = own_l, po[k] = make_float2(own0, own1);
+            if (c <= last && c != own) {
+                const size_t row = size_t(decode_slot(p, w, c, first, unit_start)) * p.G + g;
+                pm[k] = __ldcg(p.part_m + row);
+                pl[k] = __ldcg(p.part_l + row);
+                po[k] = __ldcg(reinterpret_cast<const float2*>(p.part_o + row * D + d));
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (c0 + k > last) break;
+            const float mn = fmaxf(m, pm[k]);  // finite: every piece has a key
+            const float fa = ex2_approx((m - mn) * p.scale_log2), fb = ex2_approx((pm[k] - mn) * p.scale_log2);
+            m = mn;
+            l = l * fa + fb * pl[k];
+            a0 = a0 * fa + fb * po[k].x;
+            a1 = a1 * fa + fb * po[k].y;
+        }
+    }
+    write(g, d, a0, a1, m, l);
+}
+__device__ __forceinline__ int decode_ld_acquire(const int* a) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(a) : "memory");
+    return v;
+}
+
+// ---- thread-block cluster
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_store_f2(const void* local, int rank, float2 v) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(rank));
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
+}
+
+template <int D, int NH>
+__global__ void __launch_bounds__(kDecodeThreads, 2)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                    const DecodeParams p) {
     using Cfg = DecodeCfg<D>;
+    constexpr int KEYS = Cfg::kKeys;
     constexpr int NST = Cfg::kStages;
-    constexpr int KS = D / 16;  // k-steps of Q K^T
-    constexpr int DT = D / 8;   // 8-column output tiles of P V
+    constexpr int KS = D / 16;     // k-steps of Q K^T
+    constexpr int MT = D / 16;     // 16-row output tiles of V^T P^T
+    constexpr int KT = KEYS / 64;  // 16-key tiles per warp
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* sK = smem;
-    uint8_t* sV = sK + NST * Cfg::kTileBytes;
-    uint8_t* sQ = sV + NST * Cfg::kTileBytes;                        // [16 rows][D] BF16, swizzled like a tile
-    float* sRed = reinterpret_cast<float*>(sK);  // [4 warps][16 rows][D + 2], used after the last tile only
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sQ + Cfg::kQBytes);
-    uint64_t* bar_full = bars;        // [NST]
-    uint64_t* bar_free = bars + NST;  // [NST]
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * NST);
+    uint8_t* sKV = smem;                                                 // [NST] K tile, V tile
+    uint8_t* sQ = sKV + NST * 2 * Cfg::kTileBytes;                       // [2][16 rows]
+    float2* sMl = reinterpret_cast<float2*>(sQ + 2 * Cfg::kQBytes);      // [4 warps][16 heads]
+    float2* sX = sMl + 4 * 16;                                           // [CTA of the cluster][slice of the output pairs]
+    float2* sXMl = sX + 16 * D / 2;                                      // [CTA of the cluster][16 rows]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sQ + 2 * Cfg::kQBytes + Cfg::kMlBytes + Cfg::kXBytes);
+    uint64_t* bar_full = bars;              // [NST]
+    uint64_t* bar_free = bars + NST;        // [NST]
+    uint64_t* bar_q = bars + 2 * NST;       // [2] the q rows of a piece have landed   (phase: piece / 2)
+    uint64_t* bar_q_free = bar_q + 2;       // [2] they are in registers               (phase: piece / 2)
+    uint64_t* bar_part = bar_q_free + 2;    // the shared piece at the range's beginning has been stored
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_part + 1);
+    volatile int* last_flag = abort_flag + 1;
+    volatile int* fail_flag = abort_flag + 2;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = p.G;
-    const int split = blockIdx.x;
-    const int hk = int(blockIdx.y) / p.n_chunks;
-    const int chunk = int(blockIdx.y) % p.n_chunks;
-    const int b = blockIdx.z;
-    const int h0 = hk * p.group + chunk * G;  // first query head served here
-    const int tile0 = split * p.tiles_per_split;
 
-    if (tid == 0) {
-        for (int s = 0; s < NST; ++s) {
-            mbar_init(&bar_full[s], 1);
-            mbar_init(&bar_free[s], 128);
-        }
-        fence_mbar_init();
-        tma_prefetch_desc(&tmK);
-        tma_prefetch_desc(&tmV);
-    }
-    // launched with programmatic stream serialization: everything above overlaps the previous kernel's end (the
-    // cache append that wrote q and the newest K / V row); nothing in global memory is touched before this wait
-    grid_dep_wait();
-    if (tid == 0) *abort_flag = *reinterpret_cast<volatile int*>(p.status);
-    __syncthreads();
-    if (*abort_flag != 0) return;
-    // this sequence's length: a split that lies beyond it writes an empty partial (m = -inf, l = 0)
-    const int L = p.lens ? max(1, min(__ldg(p.lens + b), p.L)) : p.L;
-    const int n_all = (L + 127) / 128;
-    const int n_tiles = max(0, min(p.tiles_per_split, n_all - tile0));
-    // q rows of the G heads -> shared memory (BF16, 16-byte chunks, swizzled); rows >= G are zero
-    for (int i = tid; i < 16 * (D / 8); i += blockDim.x) {
-        const int r = i / (D / 8), c = i % (D / 8);
-        uint4 val = make_uint4(0u, 0u, 0u, 0u);
-        if (r < G) val = *reinterpret_cast<const uint4*>(p.q + (size_t(b) * p.Hq + h0 + r) * D + c * 8);
-        *reinterpret_cast<uint4*>(sQ + swz_off(r, c, 16 * 128)) = val;
-    }
-    __syncthreads();
-
+    // All CTAs of a launch are resident at once, so the next kernel of the stream may be brought in at once too: its
+    // set-up then runs under this kernel, and it waits for this kernel's end before it touches global memory.
+    grid_dep_launch();
+    if (p.cluster > 1) cluster_arrive();  // waited for in front of the first access to another CTA's shared memory
     if (warp == 4) {
-        if (lane == 0) {
-            for (int j = 0; j < n_tiles; ++j) {
+        // ------------------------------------------------------------------ producer
+        if (elect_one()) {
+            tma_prefetch_desc(&tmK);
+            tma_prefetch_desc(&tmV);
+            *abort_flag = 0;
+        }
+        if (lane < 2 * NST + 5) {  // in the order of `bars`: full, free, q, q_free, part
+            mbar_init(bars + lane, lane < NST ? 1 : lane < 2 * NST ? 128 : lane < 2 * NST + 2 ? 1 : 128);
+            fence_mbar_init();
+        }
+        __syncwarp();
+        // everything above overlaps the previous kernel's end (the cache append that wrote q and the newest K / V row)
+        grid_dep_wait();
+        DecodeWalk w = decode_walk_start<KEYS>(p, int(blockIdx.x), int(gridDim.x), lane);
+        int j = 0;  // tiles issued so far (ring position)
+        bool synced = false, ok = true;
+        for (int n = 0; w.t < w.t_end && ok; ++n) {
+            const int tiles = decode_piece(w);
+            const int hk = int(fastdiv(w.u, p.div_chunks)), h0 = hk * p.group + (w.u - hk * p.n_chunks) * G;
+            for (int i = 0; i < tiles; ++i, ++j) {
                 const int s = j % NST;
-                if (j >= NST &&
-                    !mbar_wait(&bar_free[s], ((j / NST) - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE))
-                    break;
-                mbar_arrive_expect_tx(&bar_full[s], 2 * Cfg::kTileBytes);
+                if (j >= NST) {
+                    if (!synced) __syncthreads(), synced = true;  // the other warps have started
+                    ok = mbar_wait_warp(&bar_free[s], ((j / NST) - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
+                    if (!ok) break;
+                }
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&bar_full[s], 2 * Cfg::kTileBytes);
+                    uint8_t* k = sKV + s * 2 * Cfg::kTileBytes;
 #pragma unroll
-                for (int bx = 0; bx < Cfg::kBoxes; ++bx) {
-                    tma_load_4d(sK + s * Cfg::kTileBytes + bx * Cfg::kBoxBytes, &tmK, &bar_full[s], bx * 64,
-                                (tile0 + j) * 128, hk, b);
-                    tma_load_4d(sV + s * Cfg::kTileBytes + bx * Cfg::kBoxBytes, &tmV, &bar_full[s], bx * 64,
-                                (tile0 + j) * 128, hk, b);
+                    for (int bx = 0; bx < Cfg::kBoxes; ++bx) {
+                        tma_load_4d(k + bx * Cfg::kBoxBytes, &tmK, &bar_full[s], bx * 64, (w.j0 + i) * KEYS, hk, w.b);
+                        tma_load_4d(k + Cfg::kTileBytes + bx * Cfg::kBoxBytes, &tmV, &bar_full[s], bx * 64, (w.j0 + i) * KEYS, hk, w.b);
+                    }
+                }
+                __syncwarp();
+                if (i == 0) {  // behind the first tile's requests: the piece's q rows
+                    if (n >= 2) {
+                        if (!synced) __syncthreads(), synced = true;
+                        ok = mbar_wait_warp(&bar_q_free[n & 1], ((n >> 1) - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
+                        if (!ok) break;
+                    }
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(&bar_q[n & 1], G * D * 2);
+                        bulk_load_1d(sQ + (n & 1) * Cfg::kQBytes, p.q + (size_t(w.b) * p.Hq + h0) * D, G * D * 2, &bar_q[n & 1]);
+                    }
+                    __syncwarp();
                 }
             }
+            decode_walk_next<KEYS>(p, w, tiles);
         }
+        if (!synced) __syncthreads();
+        return;
+    }
+
+    auto write_rows_of = [&](const DecodeWalk& w) {  // final rows of the unit at w
+        const int hk = int(fastdiv(w.u, p.div_chunks));
+        const size_t row0 = size_t(w.b) * p.Hq + hk * p.group + (w.u - hk * p.n_chunks) * G;
+        return [&p, row0](int g, int d, float a0, float a1, float m, float l) {
+            const float inv = 1.f / l;
+            reinterpret_cast<uint32_t*>(p.o)[(row0 + g) * (D / 2) + d / 2] = pack_bf16x2(a0 * inv, a1 * inv);
+            if (p.lse && d == 0) p.lse[row0 + g] = m * p.scale + logf(l);
+        };
+    };
+    if (warp == 5) {
+        // ------------------------------------------------------------------ counter of the range's first piece
+        grid_dep_wait();
+        const DecodeWalk w = decode_walk_start<KEYS>(p, int(blockIdx.x), int(gridDim.x), lane);
+        __syncthreads();
+        if (p.cluster || *fail_flag != 0 || w.t >= w.t_end) return;
+        const int tiles = decode_piece(w);
+        if (tiles == w.n_tiles || w.t + tiles == w.t_end) return;
+        if (!mbar_wait_warp(bar_part, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX)) return;
+        const int unit_start = w.t - w.j0;
+        const int first = decode_cta_of(w, unit_start), last = decode_cta_of(w, unit_start + w.n_tiles - 1);
+        int is_last = 0;
+        if (lane == 0) {
+            __threadfence();
+            is_last = atomicAdd(p.counters + first, 1) == last - first;
+            if (is_last) p.counters[first] = 0;  // for the next launch that uses it
+            __threadfence();
+        }
+        if (!__shfl_sync(0xffffffffu, is_last, 0)) return;
+        const auto write = write_rows_of(w);
+        for (int i = lane; i < G * (D / 2); i += 32)
+            decode_add_pieces<D>(p, w, first, last, unit_start, i / (D / 2), (i % (D / 2)) * 2, -1, 0.f, 0.f, 0.f, 0.f, write);
         return;
     }
 
     // ---------------------------------------------------------------------- compute warps
-    // A fragments of Q (rows = heads): one ldmatrix.x4 per k-step
-    uint32_t aq[KS][4];
-    {
-        const uint32_t q_base = smem_u32(sQ);
-        const int r = (lane & 7) + ((lane >> 3) & 1) * 8;  // matrices 0,2: rows 0-7; 1,3: rows 8-15
-#pragma unroll
-        for (int ks = 0; ks < KS; ++ks) {
-            const int c = ks * 2 + (lane >> 4);  // matrices 0,1: k 0-7; 2,3: k 8-15
-            ldsm_x4(q_base + swz_off(r, c, 16 * 128), aq[ks][0], aq[ks][1], aq[ks][2], aq[ks][3]);
-        }
+    for (int i = tid; i < 2 * (16 - G) * (D / 8); i += 128) {  // rows >= G of both q buffers
+        const int buf = i / ((16 - G) * (D / 8)), r = i % ((16 - G) * (D / 8));
+        *reinterpret_cast<uint4*>(sQ + buf * Cfg::kQBytes + (G + r / (D / 8)) * Cfg::kQRow + (r % (D / 8)) * 16) = make_uint4(0u, 0u, 0u, 0u);
     }
-    // this thread holds rows r0 = lane / 4 and r1 = r0 + 8 (query heads), key / head-dim columns (lane % 4) * 2 + {0, 1}
-    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
-    float o[DT][4];
-#pragma unroll
-    for (int dt = 0; dt < DT; ++dt) o[dt][0] = o[dt][1] = o[dt][2] = o[dt][3] = 0.f;
-    const int kw = warp * 32;  // this warp's keys inside a tile
+    grid_dep_wait();
+    // (a launch behind a failure writes nothing; its loads are harmless, but shared memory has to outlive them)
+    if (tid == 0) *fail_flag = *reinterpret_cast<volatile int*>(p.status);
+    DecodeWalk w = decode_walk_start<KEYS>(p, int(blockIdx.x), int(gridDim.x), lane);
+    __syncthreads();
+    const bool failed = *fail_flag != 0;
     bool ok = true;
-    for (int j = 0; j < n_tiles; ++j) {
-        const int s = j % NST;
-        ok = mbar_wait_warp(&bar_full[s], (j / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+    const int rank = p.cluster > 1 ? int(blockIdx.x) % p.cluster : 0;
+    bool sent = false;
+    int j = 0;  // tiles before this piece (ring position)
+    for (int n = 0; w.t < w.t_end; ++n) {
+        const int tiles = decode_piece(w);
+        DecodeState<D, NH> st;
+        st.clear();
+        uint32_t bq[KS][NH][2];  // B fragments of Q^T (columns = heads)
+        if (ok) ok = mbar_wait_warp(&bar_q[n & 1], (n >> 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+        {
+            const uint32_t q_base = smem_u32(sQ + (n & 1) * Cfg::kQBytes);
+#pragma unroll
+            for (int nh = 0; nh < NH; ++nh)
+#pragma unroll
+                for (int ks = 0; ks < KS; ks += 2)  // matrices 0-3: head-dim chunks 2ks .. 2ks+3 of heads nh * 8 .. + 8
+                    ldsm_x4(q_base + (nh * 8 + (lane & 7)) * Cfg::kQRow + (ks * 2 + (lane >> 3)) * 16, bq[ks][nh][0], bq[ks][nh][1],
+                            bq[ks + 1][nh][0], bq[ks + 1][nh][1]);
+            fence_proxy_async_smem();
+            mbar_arrive(&bar_q_free[n & 1]);
+        }
+        const int kw = warp * (KEYS / 4);  // this warp's keys inside a tile
+        for (int i = 0; i < tiles; ++i, ++j) {
+            const int s = j % NST;
+            ok = ok && mbar_wait_warp(&bar_full[s], (j / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+            if (!ok) break;
+            const uint32_t k_base = smem_u32(sKV + s * 2 * Cfg::kTileBytes);
+            const uint32_t v_base = k_base + Cfg::kTileBytes;
+            // ---- S^T[keys x heads] = K Q^T, the keys of this warp in tiles of 16
+            float sc[KT][NH][4];  // {key, head}: 0 {0, 0}, 1 {0, 1}, 2 {8, 0}, 3 {8, 1} of key lane / 4, head (lane % 4) * 2
+#pragma unroll
+            for (int kt = 0; kt < KT; ++kt) {
+                float odd[NH][4];  // a second accumulator: half the chain of dependent products
+#pragma unroll
+                for (int nh = 0; nh < NH; ++nh)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) sc[kt][nh][e] = odd[nh][e] = 0.f;
+                const int key = kw + kt * 16 + (lane & 15);
+#pragma unroll
+                for (int ks = 0; ks < KS; ++ks) {
+                    uint32_t a[4];
+                    ldsm_x4(k_base + swz_off(key, ks * 2 + (lane >> 4), Cfg::kBoxBytes), a[0], a[1], a[2], a[3]);
+#pragma unroll
+                    for (int nh = 0; nh < NH; ++nh) mma_bf16_16816((ks & 1) ? odd[nh] : sc[kt][nh], a, bq[ks][nh][0], bq[ks][nh][1]);
+                }
+#pragma unroll
+                for (int nh = 0; nh < NH; ++nh)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) sc[kt][nh][e] += odd[nh][e];
+            }
+            // ---- mask keys beyond the cache length (a unit's last tile only)
+            const int tile_key = (w.j0 + i) * KEYS;
+            if (tile_key + KEYS > w.len) {
+#pragma unroll
+                for (int kt = 0; kt < KT; ++kt) {
+                    const int key = tile_key + kw + kt * 16 + (lane >> 2);
+#pragma unroll
+                    for (int nh = 0; nh < NH; ++nh) {
+                        if (key >= w.len) sc[kt][nh][0] = sc[kt][nh][1] = -INFINITY;
+                        if (key + 8 >= w.len) sc[kt][nh][2] = sc[kt][nh][3] = -INFINITY;
+                    }
+                }
+            }
+            // ---- online softmax per head over this warp's keys; P^T becomes the B operand of the second product: rows and
+            // columns of its 8 x 8 blocks change places (movmatrix)
+            uint32_t bp[KT][NH][2];
+#pragma unroll
+            for (int nh = 0; nh < NH; ++nh) {
+                float alpha[2], nb[2];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    float mx = -INFINITY;
+#pragma unroll
+                    for (int kt = 0; kt < KT; ++kt) mx = fmaxf(mx, fmaxf(sc[kt][nh][e], sc[kt][nh][e + 2]));
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+                    const float mn = fmaxf(st.m[nh][e], mx);
+                    // a warp whose keys are all beyond the cache has mn = -inf: keep its state neutral
+                    alpha[e] = (mn == -INFINITY) ? 1.f : ex2_approx((st.m[nh][e] - mn) * p.scale_log2);
+                    nb[e] = (mn == -INFINITY) ? 0.f : -mn * p.scale_log2;
+                    st.m[nh][e] = mn;
+                    st.l[nh][e] *= alpha[e];
+                }
+#pragma unroll
+                for (int kt = 0; kt < KT; ++kt) {
+                    const float p0 = ex2_approx(fmaf(sc[kt][nh][0], p.scale_log2, nb[0]));
+                    const float p1 = ex2_approx(fmaf(sc[kt][nh][1], p.scale_log2, nb[1]));
+                    const float p2 = ex2_approx(fmaf(sc[kt][nh][2], p.scale_log2, nb[0]));
+                    const float p3 = ex2_approx(fmaf(sc[kt][nh][3], p.scale_log2, nb[1]));
+                    st.l[nh][0] += p0 + p2;
+                    st.l[nh][1] += p1 + p3;
+                    bp[kt][nh][0] = movmatrix_trans(pack_bf16x2(p0, p1));
+                    bp[kt][nh][1] = movmatrix_trans(pack_bf16x2(p2, p3));
+                }
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) {
+                    st.o[mt][nh][0] *= alpha[0];
+                    st.o[mt][nh][1] *= alpha[1];
+                    st.o[mt][nh][2] *= alpha[0];
+                    st.o[mt][nh][3] *= alpha[1];
+                }
+            }
+            // ---- O^T[D x heads] += V^T P^T
+#pragma unroll
+            for (int kt = 0; kt < KT; ++kt) {
+                const int key = kw + kt * 16 + (lane & 7) + ((lane >> 4) << 3);  // matrices 0,1: keys 0-7; 2,3: 8-15
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) {
+                    uint32_t a[4];  // matrices 0,2: head-dim rows 0-7; 1,3: 8-15
+                    ldsm_x4_trans(v_base + swz_off(key, mt * 2 + ((lane >> 3) & 1), Cfg::kBoxBytes), a[0], a[1], a[2], a[3]);
+#pragma unroll
+                    for (int nh = 0; nh < NH; ++nh) mma_bf16_16816(st.o[mt][nh], a, bp[kt][nh][0], bp[kt][nh][1]);
+                }
+            }
+            if (i + 1 < tiles) {
+                // ordinary (ldmatrix) reads of a stage that TMA will overwrite: ordered before the async proxy's write
+                fence_proxy_async_smem();
+                mbar_arrive(&bar_free[s]);
+            }
+        }
+        // ---- end of the piece.  Its last stage stays with the compute warps as scratch until the piece is written.
+        ok = decode_bar_ok(ok);
         if (!ok) break;
-        const uint32_t k_base = smem_u32(sK + s * Cfg::kTileBytes);
-        const uint32_t v_base = smem_u32(sV + s * Cfg::kTileBytes);
-        // ---- S[16 heads x 32 keys] = Q K^T
-        float sc[4][4];
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f;
-            const int key = kw + nt * 8 + (lane & 7);
-#pragma unroll
-            for (int kk = 0; kk < KS / 2; ++kk) {
-                uint32_t b0, b1, b2, b3;  // chunks 4kk .. 4kk+3 of the key rows: two k-steps
-                ldsm_x4(k_base + swz_off(key, kk * 4 + (lane >> 3), Cfg::kBoxBytes), b0, b1, b2, b3);
-                mma_bf16_16816(sc[nt], aq[2 * kk], b0, b1);
-                mma_bf16_16816(sc[nt], aq[2 * kk + 1], b2, b3);
+        const int s_last = (j - 1) % NST;
+        if (failed && p.cluster <= 1) {
+            // every piece's loads are waited for, nothing is written
+            fence_proxy_async_smem();
+            mbar_arrive(&bar_free[s_last]);
+            decode_walk_next<KEYS>(p, w, tiles);
+            continue;
+        }
+        float* sO = reinterpret_cast<float*>(sKV + s_last * 2 * Cfg::kTileBytes);
+        const auto write_rows = write_rows_of(w);
+        if (p.cluster > 1) {
+            // output pair e belongs to CTA e / slice of the cluster; every CTA needs everyone's (m, l)
+            const int slice = int(p.div_slice.d);
+            cluster_wait();
+            decode_merge<D, NH>(st, sO, sMl, warp, lane, tid, G, p.scale_log2, [&](int g, int d, float a0, float a1, float m, float l) {
+                const int e = g * (D / 2) + d / 2, to = int(fastdiv(e, p.div_slice));
+                cluster_store_f2(&sX[rank * slice + e - to * slice], to, make_float2(a0, a1));
+                if (d == 0)
+                    for (int c = 0; c < p.cluster; ++c) cluster_store_f2(&sXMl[rank * 16 + g], c, make_float2(m, l));
+            });
+            sent = true;
+            break;
+        } else if (tiles == w.n_tiles) {
+            decode_merge<D, NH>(st, sO, sMl, warp, lane, tid, G, p.scale_log2, write_rows);
+        } else {
+            const int cta = int(blockIdx.x);
+            const int unit_start = w.t - w.j0;
+            const int first = decode_cta_of(w, unit_start), last = decode_cta_of(w, unit_start + w.n_tiles - 1);
+            const size_t slot = decode_slot(p, w, cta, first, unit_start);
+            const bool ends_range = w.t + tiles == w.t_end;
+            // At the range's end nothing is left to hide latency behind.  Usually all other pieces have been stored by then
+            // (they lie at the beginning of their CTAs' ranges): one look at the counter instead of store, fence and count.
+            if (tid == 0) *last_flag = ends_range && decode_ld_acquire(p.counters + first) == last - first;
+            decode_merge<D, NH>(st, sO, sMl, warp, lane, tid, G, p.scale_log2, [&](int g, int d, float a0, float a1, float m, float l) {
+                if (*last_flag) {
+                    decode_add_pieces<D>(p, w, first, last, unit_start, g, d, cta, a0, a1, m, l, write_rows);
+                    return;
+                }
+                *reinterpret_cast<float2*>(p.part_o + (slot * G + g) * D + d) = make_float2(a0, a1);
+                if (d == 0) {
+                    p.part_m[slot * G + g] = m;
+                    p.part_l[slot * G + g] = l;
+                }
+            });
+            if (!ends_range) {
+                mbar_arrive(bar_part);
+            } else if (*last_flag) {
+                if (tid == 0) p.counters[first] = 0;  // for the next launch that uses it
+            } else {
+                __threadfence();
+                named_bar_sync(1, 128);
+                if (tid == 0) {
+                    const int is_last = atomicAdd(p.counters + first, 1) == last - first;
+                    if (is_last) p.counters[first] = 0;
+                    *last_flag = is_last;
+                    __threadfence();
+                }
+                named_bar_sync(1, 128);
+                if (*last_flag)
+                    for (int i = tid; i < G * (D / 2); i += 128)
+                        decode_add_pieces<D>(p, w, first, last, unit_start, i / (D / 2), (i % (D / 2)) * 2, -1, 0.f, 0.f, 0.f, 0.f, write_rows);
             }
         }
-        // ---- mask keys beyond the cache length (last tile only)
-        const int key0 = (tile0 + j) * 128 + kw + (lane & 3) * 2;
-        if ((tile0 + j) * 128 + 128 > L) {
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                if (key0 + nt * 8 >= L) sc[nt][0] = sc[nt][2] = -INFINITY;
-                if (key0 + nt * 8 + 1 >= L) sc[nt][1] = sc[nt][3] = -INFINITY;
-            }
-        }
-        // ---- online softmax per head row (rows r0 and r1), over this warp's 32 keys
-        float mx0 = fmaxf(fmaxf(sc[0][0], sc[0][1]), fmaxf(sc[1][0], sc[1][1]));
-        float mx1 = fmaxf(fmaxf(sc[0][2], sc[0][3]), fmaxf(sc[1][2], sc[1][3]));
-        mx0 = fmaxf(mx0, fmaxf(fmaxf(sc[2][0], sc[2][1]), fmaxf(sc[3][0], sc[3][1])));
-        mx1 = fmaxf(mx1, fmaxf(fmaxf(sc[2][2], sc[2][3]), fmaxf(sc[3][2], sc[3][3])));
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-        const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
-        // a warp whose 32 keys are all beyond the cache has mn = -inf: keep its state neutral
-        const float a0 = (mn0 == -INFINITY) ? 1.f : ex2_approx((m0 - mn0) * p.scale_log2);
-        const float a1 = (mn1 == -INFINITY) ? 1.f : ex2_approx((m1 - mn1) * p.scale_log2);
-        const float nb0 = (mn0 == -INFINITY) ? 0.f : -mn0 * p.scale_log2;
-        const float nb1 = (mn1 == -INFINITY) ? 0.f : -mn1 * p.scale_log2;
-        m0 = mn0;
-        m1 = mn1;
-        float rs0 = 0.f, rs1 = 0.f;
-        uint32_t ap[2][4];  // P as A fragments: k-step kk covers keys 16 kk .. 16 kk + 15
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            const float p0 = ex2_approx(fmaf(sc[nt][0], p.scale_log2, nb0));
-            const float p1 = ex2_approx(fmaf(sc[nt][1], p.scale_log2, nb0));
-            const float p2 = ex2_approx(fmaf(sc[nt][2], p.scale_log2, nb1));
-            const float p3 = ex2_approx(fmaf(sc[nt][3], p.scale_log2, nb1));
-            rs0 += p0 + p1;
-            rs1 += p2 + p3;
-            ap[nt >> 1][(nt & 1) * 2 + 0] = pack_bf16x2(p0, p1);
-            ap[nt >> 1][(nt & 1) * 2 + 1] = pack_bf16x2(p2, p3);
-        }
-        l0 = l0 * a0 + rs0;
-        l1 = l1 * a1 + rs1;
-        // ---- O[16 x D] = alpha O + P V
-#pragma unroll
-        for (int dt = 0; dt < DT; ++dt) {
-            o[dt][0] *= a0;
-            o[dt][1] *= a0;
-            o[dt][2] *= a1;
-            o[dt][3] *= a1;
-        }
-#pragma unroll
-        for (int kk = 0; kk < 2; ++kk) {
-            const int key = kw + kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;  // matrices 0,2: keys 0-7; 1,3: 8-15
-#pragma unroll
-            for (int dp = 0; dp < DT / 2; ++dp) {
-                uint32_t b0, b1, b2, b3;  // head-dim chunks 2dp (matrices 0,1) and 2dp+1 (matrices 2,3)
-                ldsm_x4_trans(v_base + swz_off(key, dp * 2 + (lane >> 4), Cfg::kBoxBytes), b0, b1, b2, b3);
-                mma_bf16_16816(o[2 * dp], ap[kk], b0, b1);
-                mma_bf16_16816(o[2 * dp + 1], ap[kk], b2, b3);
-            }
-        }
-        // ordinary (ldmatrix) reads of a stage that TMA will overwrite: ordered before the async proxy's write
+        // the scratch was written and read with ordinary accesses; the stage goes back to TMA
         fence_proxy_async_smem();
-        mbar_arrive(&bar_free[s]);
+        mbar_arrive(&bar_free[s_last]);
+        named_bar_sync(1, 128);  // sMl and the flag are rewritten at the next piece's end
+        decode_walk_next<KEYS>(p, w, tiles);
     }
-    // ---- merge the four warps' states and write the split's partial (un-normalised O, m, l)
-    named_bar_sync(1, 128);  // every compute thread, also after a wait that gave up
-    if (*abort_flag != 0) return;
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-    constexpr int RS = D + 2;  // row stride of the scratch: O row, then m, then l
-    float* mine = sRed + warp * 16 * RS;
-    const int r0 = lane >> 2, r1 = r0 + 8, cq = (lane & 3) * 2;
-#pragma unroll
-    for (int dt = 0; dt < DT; ++dt) {
-        mine[r0 * RS + dt * 8 + cq] = o[dt][0];
-        mine[r0 * RS + dt * 8 + cq + 1] = o[dt][1];
-        mine[r1 * RS + dt * 8 + cq] = o[dt][2];
-        mine[r1 * RS + dt * 8 + cq + 1] = o[dt][3];
+    if (p.cluster <= 1) return;
+    // ---- the cluster's partial results: this CTA finishes its slice of the outputs.  A CTA without tiles (or one that has
+    // given up) sends weight zero; nobody leaves before everybody's stores have landed.
+    if (!sent) {
+        cluster_wait();
+        for (int i = tid; i < G * p.cluster; i += 128) cluster_store_f2(&sXMl[rank * 16 + i / p.cluster], i % p.cluster, make_float2(-INFINITY, 0.f));
     }
-    if ((lane & 3) == 0) {
-        mine[r0 * RS + D] = m0;
-        mine[r0 * RS + D + 1] = l0;
-        mine[r1 * RS + D] = m1;
-        mine[r1 * RS + D + 1] = l1;
-    }
-    named_bar_sync(1, 128);
-    for (int i = tid; i < G * D; i += 128) {
-        const int g = i / D, d = i % D;
-        float m = -INFINITY;
+    cluster_arrive();
+    cluster_wait();
+    if (failed || !ok) return;
+    const int slice = int(p.div_slice.d);
+    const auto write_rows = write_rows_of(w);
+    for (int i = tid; i < slice; i += 128) {
+        const int e = rank * slice + i, g = e / (D / 2), d2 = e - g * (D / 2);
+        float2 ml[kDecodeMaxCluster], v[kDecodeMaxCluster];
 #pragma unroll
-        for (int w = 0; w < 4; ++w) m = fmaxf(m, sRed[(w * 16 + g) * RS + D]);
-        float acc = 0.f, l = 0.f;
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            const float mw = sRed[(w * 16 + g) * RS + D];
-            const float f = (mw == -INFINITY) ? 0.f : ex2_approx((mw - m) * p.scale_log2);
-            acc += f * sRed[(w * 16 + g) * RS + d];
-            l += f * sRed[(w * 16 + g) * RS + D + 1];
+        for (int c = 0; c < kDecodeMaxCluster; ++c) {
+            ml[c] = c < p.cluster ? sXMl[c * 16 + g] : make_float2(-INFINITY, 0.f);
+            v[c] = c < p.cluster ? sX[c * slice + i] : make_float2(0.f, 0.f);
         }
-        const size_t idx = (size_t(b) * p.Hq + h0 + g) * p.n_splits + split;
-        p.part_o[idx * D + d] = acc;
-        if (d == 0) {
-            p.part_m[idx] = m;
-            p.part_l[idx] = l;
+        float m = ml[0].x;
+#pragma unroll
+        for (int c = 1; c < kDecodeMaxCluster; ++c) m = fmaxf(m, ml[c].x);
+        float a0 = 0.f, a1 = 0.f, l = 0.f;
+#pragma unroll
+        for (int c = 0; c < kDecodeMaxCluster; ++c) {
+            if (ml[c].x == -INFINITY) continue;  // no tiles: its slots hold nothing
+            const float f = ex2_approx((ml[c].x - m) * p.scale_log2);
+            a0 += f * v[c].x;
+            a1 += f * v[c].y;
+            l += f * ml[c].y;
         }
+        write_rows(g, d2 * 2, a0, a1, m, l);
     }
-}
-
-// Merges the per-split partials: one warp per (batch, query head).
-template <int D>
-__global__ void __launch_bounds__(128)
-attn_decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_m,
-                           const float* __restrict__ part_l, uint16_t* __restrict__ o, float* __restrict__ lse,
-                           int n_rows, int n_splits, float scale, float scale_log2) {
-    const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    grid_dep_wait();  // the partials come from the kernel before this one
-    if (row >= n_rows) return;
-    float m = -INFINITY;
-    for (int s = 0; s < n_splits; ++s) m = fmaxf(m, part_m[(size_t)row * n_splits + s]);
-    constexpr int DPT = D / 32;
-    float acc[DPT];
-#pragma unroll
-    for (int e = 0; e < DPT; ++e) acc[e] = 0.f;
-    float l = 0.f;
-    for (int s = 0; s < n_splits; ++s) {
-        const float ms = part_m[(size_t)row * n_splits + s];
-        const float w = (ms == -INFINITY) ? 0.f : ex2_approx((ms - m) * scale_log2);  // empty split
-        l += w * part_l[(size_t)row * n_splits + s];
-#pragma unroll
-        for (int e = 0; e < DPT; ++e) acc[e] += w * part_o[((size_t)row * n_splits + s) * D + lane * DPT + e];
-    }
-    const float inv = 1.f / l;
-    if (DPT == 2) {
-        reinterpret_cast<uint32_t*>(o)[(size_t)row * (D / 2) + lane] = pack_bf16x2(acc[0] * inv, acc[1] * inv);
-    } else {
-        uint2 w;
-        w.x = pack_bf16x2(acc[0] * inv, acc[1] * inv);
-        w.y = pack_bf16x2(acc[2] * inv, acc[3] * inv);
-        reinterpret_cast<uint2*>(o)[(size_t)row * (D / 4) + lane] = w;
-    }
-    if (lse && lane == 0) lse[row] = m * scale + logf(l);
 }
 
 }  // namespace b200attn

@@ -46,6 +46,12 @@ __device__ int g_sched_words[2 * kSchedSlots];
 int* g_sched_ptr[kMaxDevices] = {nullptr};
 std::atomic<unsigned> g_sched_seq{0};
 
+// Counters of the decode kernel's shared units, the same way: a set per launch, zero again when the launch ends.
+constexpr int kDecodeSlots = 64;
+__device__ int g_decode_counters[kDecodeSlots * kDecodeMaxCtas];
+int* g_decode_ptr[kMaxDevices] = {nullptr};
+std::atomic<unsigned> g_decode_seq{0};
+
 // Returns the device address of the status word of the current device (resolved once per device).
 int* status_ptr(int* err) {
     int dev = 0;
@@ -71,6 +77,13 @@ int* status_ptr(int* err) {
             *err = B200ATTN_ERR_NO_DEVICE;
             return nullptr;
         }
+        void* dp = nullptr;
+        if (cudaGetSymbolAddress(&dp, g_decode_counters) != cudaSuccess) {
+            cudaGetLastError();
+            *err = B200ATTN_ERR_NO_DEVICE;
+            return nullptr;
+        }
+        g_decode_ptr[dev] = static_cast<int*>(dp);
         g_sched_ptr[dev] = static_cast<int*>(sp);
         g_status_ptr[dev] = static_cast<int*>(p);
     }
@@ -91,6 +104,12 @@ int* next_sched_pair(long long n_items, unsigned n_ctas) {
     int dev = 0;
     cudaGetDevice(&dev);
     return g_sched_ptr[dev] + 2 * (g_sched_seq.fetch_add(1, std::memory_order_relaxed) % kSchedSlots);
+}
+
+int* next_decode_counters() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return g_decode_ptr[dev] + kDecodeMaxCtas * (g_decode_seq.fetch_add(1, std::memory_order_relaxed) % kDecodeSlots);
 }
 
 // The static deal of the forward and the dQ pass (two CTAs per SM) as a table: items (ids are heaviest first;
@@ -199,20 +218,28 @@ int check_common(int B, int T, int Hq, int Hkv, int D, int layout) {
 
 // Launch with programmatic stream serialization: the kernel may become resident while the
 // previous kernel of the stream drains; it calls griddepcontrol.wait before touching global memory.
+// cluster > 1: in thread-block clusters of that many blocks.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, unsigned block, size_t smem, cudaStream_t st,
-                       Args&&... args) {
+cudaError_t launch_cluster(void (*kernel)(KArgs...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, int cluster,
+                           Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(block, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, Args&&... args) {
+    return launch_cluster(kernel, grid, block, smem, st, 1, args...);
 }
 
 template <int D>
@@ -799,30 +826,75 @@ inline int decode_heads_per_cta(int group) {
     return 1;
 }
 
-inline int decode_pick_splits(int B, int L, int Hq, int Hkv, int n_splits) {
-    const int n_all = (L + 127) / 128;
-    if (n_splits <= 0) {
-        const int group = Hq / Hkv;
-        const long long units = (long long)B * Hkv * (group / decode_heads_per_cta(group));
-        // two CTAs fit on an SM: fill the 2 x 148 slots of the part once, and do not split further
-        // (every extra split costs a partial write, a combine read and a shorter stream per CTA)
-        long long want = (2 * 148) / units;
-        n_splits = (int)(want < 1 ? 1 : want);
+inline int decode_tile_keys(int D) { return D == 64 ? DecodeCfg<64>::kKeys : DecodeCfg<128>::kKeys; }
+inline int decode_max_ctas() { return std::min(2 * sm_count(), kDecodeMaxCtas); }  // two fit an SM: all are resident at once
+
+struct DecodePlan {
+    int G, n_chunks;
+    int splits;   // workspace slots per unit
+    int cluster;  // CTAs per unit, or 0: ranges of tiles
+    bool whole;   // ranges of whole units
+    int n_ctas, slot_mode;
+};
+
+// The deal (see attn_decode.cuh).
+//
+// Ranges cost about 3 us at the end (partial results through memory, a counter, the last CTA's additions), clusters
+// about 1 us, whole units nothing.  So units stay whole or in clusters unless that leaves the memory system idle for longer
+// than that: some 60 SMs saturate HBM, so what counts is how many CTAs the last round has (all, where the units are fewer
+// than the SMs) and how long a unit is, and, for sequences of different lengths, how much memory there is to read at all.
+// kRangesBytes is what HBM delivers in those 3 us.
+//
+// A cluster is the smallest that leaves a CTA at most two tiles, as far as that is one CTA per SM: more of them saturate
+// HBM by themselves.
+//
+// n_splits > 0 asks for that many splits per unit: clusters of the next power of two below.
+constexpr long long kRangesBytes = 16ll << 20;
+constexpr int kSaturatingCtas = 60;
+
+DecodePlan decode_plan(int B, int L, int Hq, int Hkv, int D, int n_splits, bool ragged) {
+    DecodePlan d;
+    const int group = Hq / Hkv, cap = decode_max_ctas();
+    d.G = decode_heads_per_cta(group);
+    d.n_chunks = group / d.G;
+    const long long units = (long long)B * Hkv * d.n_chunks;
+    const int keys = decode_tile_keys(D), n_all = (L + keys - 1) / keys, n_128 = (L + 127) / 128;
+    const long long unit_bytes = 4ll * L * D, tiles = units * n_all;
+    d.cluster = 1;
+    d.whole = false;
+    d.slot_mode = kDecodeSlotTile;
+    if (n_splits > 0) {
+        const int want = std::min(std::min(n_splits, n_128), 64), per = (n_128 + want - 1) / want;
+        d.splits = (n_128 + per - 1) / per;  // no split is empty
+        while (d.cluster * 2 <= std::min(d.splits, kDecodeMaxCluster)) d.cluster *= 2;
+    } else {
+        d.splits = (int)std::min<long long>(n_all, (2 * cap + units - 1) / units);
+        while (d.cluster < kDecodeMaxCluster && units * d.cluster * 2 <= sm_count() && n_all > 2 * d.cluster) d.cluster *= 2;
+        const long long ctas = units * d.cluster, last = ctas % cap ? ctas % cap : cap;
+        const long long idle = last < kSaturatingCtas ? unit_bytes / d.cluster * (kSaturatingCtas - last) : 0;
+        if (tiles > d.cluster * units && (idle > kRangesBytes || (ragged && units * unit_bytes > kRangesBytes))) {
+            d.cluster = 0;
+            d.n_ctas = (int)std::min<long long>(tiles, cap);
+            d.slot_mode = d.splits == n_all ? kDecodeSlotTile : kDecodeSlotTwo;
+            return d;
+        }
     }
-    if (n_splits > n_all) n_splits = n_all;
-    if (n_splits > 64) n_splits = 64;
-    const int tps = (n_all + n_splits - 1) / n_splits;
-    return (n_all + tps - 1) / tps;  // drop splits that would be empty
+    d.n_ctas = (int)std::min<long long>(units * d.cluster, 1ll << 30);
+    if (d.cluster == 1 && units > cap && !ragged) {  // the ring of a CTA then runs on from unit to unit
+        d.cluster = 0;
+        d.whole = true;
+        d.n_ctas = cap;
+    }
+    return d;
 }
 
-template <int D>
-int launch_decode(const CUtensorMap& tk, const CUtensorMap& tv, const DecodeParams& p, cudaStream_t st) {
+template <int D, int NH>
+int launch_decode(const CUtensorMap& tk, const CUtensorMap& tv, const DecodeParams& p, int n_ctas, cudaStream_t st) {
     using Cfg = DecodeCfg<D>;
     static bool set[kMaxDevices] = {false};
-    int rc = set_smem_once(attn_decode_kernel<D>, Cfg::kSmemBytes, set);
+    int rc = set_smem_once(attn_decode_kernel<D, NH>, Cfg::kSmemBytes, set);
     if (rc) return rc;
-    if (launch_pdl(attn_decode_kernel<D>, dim3(p.n_splits, p.Hkv * p.n_chunks, p.B), 160, Cfg::kSmemBytes, st, tk, tv,
-                   p) != cudaSuccess) {
+    if (launch_cluster(attn_decode_kernel<D, NH>, dim3(n_ctas), kDecodeThreads, Cfg::kSmemBytes, st, p.cluster, tk, tv, p) != cudaSuccess) {
         cudaGetLastError();
         return B200ATTN_ERR_CUDA;
     }
@@ -832,14 +904,13 @@ int launch_decode(const CUtensorMap& tk, const CUtensorMap& tv, const DecodePara
 }  // namespace
 
 extern "C" int b200attn_decode_default_splits(int B, int L, int Hq, int Hkv, int D) {
-    (void)D;
     if (B <= 0 || L <= 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv != 0) return 0;
-    return decode_pick_splits(B, L, Hq, Hkv, 0);
+    return decode_plan(B, L, Hq, Hkv, D, 0, false).splits;
 }
 
 extern "C" size_t b200attn_decode_workspace_bytes(int B, int L, int Hq, int Hkv, int D, int n_splits) {
     if (B <= 0 || L <= 0 || Hq <= 0 || Hkv <= 0 || D <= 0 || Hq % Hkv != 0) return 0;
-    const int s = decode_pick_splits(B, L, Hq, Hkv, n_splits);
+    const int s = decode_plan(B, L, Hq, Hkv, D, n_splits, false).splits;
     return (size_t)B * Hq * s * (size_t)(D + 2) * sizeof(float);
 }
 
@@ -871,11 +942,12 @@ extern "C" int b200attn_decode_ragged(const void* q, const void* kcache, const v
         return B200ATTN_ERR_WORKSPACE;
     int* status = status_ptr(&rc);
     if (!status) return rc;
+    const DecodePlan d = decode_plan(B, L, Hq, Hkv, D, n_splits, lens != nullptr);
     // the maps end at row L of every (batch, head): rows of the cache beyond it are never read (TMA fills zeros)
     const Strides sk = strides_for(B200ATTN_LAYOUT_BHTD, Hkv, L_cap, D);
     CUtensorMap tk, tv;
-    if (!make_tmap_bf16_4d(&tk, kcache, D, L, Hkv, B, sk.t, sk.h, sk.b, 128) ||
-        !make_tmap_bf16_4d(&tv, vcache, D, L, Hkv, B, sk.t, sk.h, sk.b, 128))
+    if (!make_tmap_bf16_4d(&tk, kcache, D, L, Hkv, B, sk.t, sk.h, sk.b, decode_tile_keys(D)) ||
+        !make_tmap_bf16_4d(&tv, vcache, D, L, Hkv, B, sk.t, sk.h, sk.b, decode_tile_keys(D)))
         return B200ATTN_ERR_TENSOR_MAP;
     DecodeParams p;
     p.B = B;
@@ -883,38 +955,32 @@ extern "C" int b200attn_decode_ragged(const void* q, const void* kcache, const v
     p.Hq = Hq;
     p.Hkv = Hkv;
     p.group = Hq / Hkv;
-    p.G = decode_heads_per_cta(p.group);
-    p.n_chunks = p.group / p.G;
-    p.n_splits = decode_pick_splits(B, L, Hq, Hkv, n_splits);
-    p.tiles_per_split = ((L + 127) / 128 + p.n_splits - 1) / p.n_splits;
+    p.G = d.G;
+    p.n_chunks = d.n_chunks;
+    p.units_per_seq = Hkv * d.n_chunks;
+    p.div_units = fastdiv_make((unsigned)p.units_per_seq);
+    p.div_chunks = fastdiv_make((unsigned)d.n_chunks);
+    p.div_cluster = fastdiv_make((unsigned)std::max(d.cluster, 1));
+    p.div_tiles = fastdiv_make((unsigned)((L + decode_tile_keys(D) - 1) / decode_tile_keys(D)));
+    p.div_slice = fastdiv_make((unsigned)(d.G * (D / 2) / std::max(d.cluster, 1)));
+    p.cluster = d.cluster;
+    p.whole = d.whole;
+    p.slot_mode = d.slot_mode;
     p.scale = softmax_scale > 0.f ? softmax_scale : 1.f / sqrtf((float)D);
     p.scale_log2 = p.scale * 1.4426950408889634f;
-    p.q = static_cast<const uint16_t*>(q);
     p.lens = lens;
-    float* ws = static_cast<float*>(workspace);
-    const size_t rows = (size_t)B * Hq;
-    p.part_o = ws;
-    p.part_m = ws + rows * p.n_splits * D;
-    p.part_l = p.part_m + rows * p.n_splits;
+    p.q = static_cast<const uint16_t*>(q);
+    p.o = static_cast<uint16_t*>(o);
+    p.lse = lse;
+    const size_t rows = (size_t)B * Hq * d.splits;  // slots x heads per slot
+    p.part_o = static_cast<float*>(workspace);
+    p.part_m = p.part_o + rows * D;
+    p.part_l = p.part_m + rows;
+    p.counters = next_decode_counters();
     p.status = status;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    rc = D == 64 ? launch_decode<64>(tk, tv, p, st) : launch_decode<128>(tk, tv, p, st);
-    if (rc) return rc;
-    const dim3 blocks((unsigned)((rows + 3) / 4), 1, 1);
-    const float* po = p.part_o;
-    const float* pm = p.part_m;
-    const float* pl = p.part_l;
-    uint16_t* o16 = static_cast<uint16_t*>(o);
-    const cudaError_t e =
-        D == 64 ? launch_pdl(attn_decode_combine_kernel<64>, blocks, 128, 0, st, po, pm, pl, o16, lse, (int)rows,
-                             p.n_splits, p.scale, p.scale_log2)
-                : launch_pdl(attn_decode_combine_kernel<128>, blocks, 128, 0, st, po, pm, pl, o16, lse, (int)rows,
-                             p.n_splits, p.scale, p.scale_log2);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return B200ATTN_ERR_CUDA;
-    }
-    return B200ATTN_OK;
+    if (D == 64) return d.G <= 8 ? launch_decode<64, 1>(tk, tv, p, d.n_ctas, st) : launch_decode<64, 2>(tk, tv, p, d.n_ctas, st);
+    return d.G <= 8 ? launch_decode<128, 1>(tk, tv, p, d.n_ctas, st) : launch_decode<128, 2>(tk, tv, p, d.n_ctas, st);
 }
 
 namespace {
@@ -1036,6 +1102,7 @@ extern "C" int b200attn_last_device_status(void* stream) {
         cudaGetDevice(&dev);
         cudaDeviceSynchronize();
         cudaMemset(g_sched_ptr[dev], 0, sizeof(int) * 2 * kSchedSlots);
+        cudaMemset(g_decode_ptr[dev], 0, sizeof(int) * kDecodeSlots * kDecodeMaxCtas);
         cudaMemset(status, 0, sizeof(int));
         return host;
     }

@@ -70,3 +70,40 @@ def test_decode_is_bit_repeatable():
     for _ in range(100):
         o, lse = _decode(q, kc, vc)
         assert torch.equal(o, first[0]) and torch.equal(lse, first[1])
+
+
+@pytest.mark.parametrize("B,L,Hq,Hkv,D", [
+    (1, 1025, 4, 2, 64),      # a cluster of eight over nine tiles: one CTA has two
+    (1, 449, 24, 2, 128),     # a cluster, twelve heads per unit (two column tiles of the MMA)
+    (120, 130, 6, 3, 64),     # more units than CTAs: ranges of whole units
+    (1, 70001, 2, 1, 64),     # few long units: one unit shared by every CTA, 547 tiles
+    (3, 30001, 16, 1, 128),   # sixteen heads per unit, ranges that end one unit and begin another
+])
+def test_every_deal_of_the_tiles_matches_the_oracle(B, L, Hq, Hkv, D):
+    q, kc, vc = randn_bf16((B, Hq, D), 11), randn_bf16((B, Hkv, L, D), 12), randn_bf16((B, Hkv, L, D), 13)
+    o, lse = _decode(q, kc, vc)
+    o2, lse2 = _decode(q, kc, vc)
+    assert torch.equal(o, o2) and torch.equal(lse, lse2)  # whoever finishes a shared unit
+    for b in sorted({0, B // 2, B - 1}):
+        wo, wl = ao.decode_c(np32(q[b:b + 1]), np32(kc[b:b + 1]), np32(vc[b:b + 1]))
+        assert_close("O", o[b:b + 1], wo)
+        assert_close("LSE", lse[b:b + 1], wl, max_abs=TOL_LSE, rel_l2=1.0)
+
+
+@pytest.mark.parametrize("B,L,Hq,Hkv,D", [(40, 3000, 6, 2, 64), (70, 1500, 8, 2, 128)])
+def test_ranges_over_sequences_of_different_lengths(B, L, Hq, Hkv, D):
+    # lengths from a single token to L, more than a warp's worth of sequences
+    lens = torch.tensor([1 + (L - 1) * ((i * 37) % B) // (B - 1) for i in range(B)], dtype=torch.int32)
+    q, kc, vc = randn_bf16((B, Hq, D), 21), randn_bf16((B, Hkv, L, D), 22), randn_bf16((B, Hkv, L, D), 23)
+    cache = m.KVCache(1, B, Hq, Hkv, D, L)
+    cache.k[0].copy_(kc)
+    cache.v[0].copy_(vc)
+    cache.set_lengths((lens - 1).tolist())
+    o, lse = torch.full_like(q, float("nan")), torch.full((B, Hq), float("nan"), device="cuda")
+    cache.attend(0, q, o, lse)
+    m.device_status()
+    for b in (int(lens.argmin()), int(lens.argmax()), 1, 33, B - 1):
+        n = int(lens[b])
+        wo, wl = ao.decode_c(np32(q[b:b + 1]), np32(kc[b:b + 1, :, :n]), np32(vc[b:b + 1, :, :n]))
+        assert_close(f"O[{b}]", o[b:b + 1], wo)
+        assert_close(f"LSE[{b}]", lse[b:b + 1], wl, max_abs=TOL_LSE, rel_l2=1.0)
