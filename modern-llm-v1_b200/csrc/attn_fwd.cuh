@@ -5,7 +5,7 @@
 //
 // Persistent CTAs, two per SM.  A CTA walks a static list of work items (item = one 128-row
 // query tile of one (batch, query head); items are ordered heaviest first and dealt by a host-built
-// table, see ItemTable) and, per item, the 64-key tiles of K/V up to the diagonal (tiles above it are
+// table, see ItemTable) and, per item, the key tiles of K/V up to the diagonal (tiles above it are
 // never loaded).  Every pipeline keeps running across item boundaries: the K/V ring prefetches
 // the next item's tiles and the MMA warp issues the next item's first Q K^T products while the
 // softmax warps write the previous item's output rows.  GQA is an index: the K/V tensor maps are
@@ -17,16 +17,16 @@
 //   warp  4    TMA producer (converged warp, one elected lane issues)
 //   warp  5    TMEM allocation and tcgen05.mma issue (converged warp, one elected lane issues)
 //   warps 6-7  idle (they only donate registers)
-// TMEM (256 columns): two S buffers of 64 FP32 columns, each re-used as P (BF16 pairs, 32 columns); the O
-//   accumulator (FP32, D columns) behind them; for D = 64 two Q buffers of 32 columns behind that.
-// Q in tensor memory (D = 64): every D = 64 kernel here is bound by the shared-memory data path (an SS product
-//   M128 N64 K16 fetches 4 KB of A and 2 KB of B for 32 clocks of math), and Q is the same for all key tiles of an
-//   item.  The softmax warps therefore copy an item's Q tile once from shared memory into tensor memory (the
-//   128 bytes of row r are the 32 BF16-pair columns of lane r as they stand) and Q K^T is issued with the A
-//   operand in tensor memory, like P V: per key tile the products then read 16 KB of shared memory instead of 32.
-// The MMA warp's work is a chain softmax(g) -> P V(g) -> Q K^T(g + buffers) -> softmax(g + buffers);
-// with several S buffers the products Q K^T run that many tiles ahead of the softmax, and P V of
-// tile g runs under the softmax of tile g+1.
+// TMEM (256 columns):
+//   D = 64   S (128 FP32 columns), O (64), P (BF16 pairs, 64).  Tiles of 128 keys.  The softmax warps take a tile's scores
+//            into registers in one go and hand S back, so the next tile's Q K^T runs under this tile's exponentials; P V of a
+//            tile runs under the next tile's.
+//   D = 128  two S buffers of 64 columns, each re-used as P, and O (128).  Tiles of 64 keys; Q K^T runs two tiles ahead of P V.
+// What bounds it: at D = 128 the tensor pipe (Q K^T with both operands in shared memory); at D = 64 the chain of a tile in the
+// softmax warps (scores out of tensor memory, maximum, exponentials at 16 a clock, P back, three barriers of about 100 clocks
+// each), two such chains per scheduler.  Hence 128 keys a tile at D = 64, packed FP32 arithmetic, and no commit whose completion
+// another barrier implies.  Measured against 64-key tiles with P over S and Q in tensor memory, us: B=2 T=128 6/2 D=64
+// 6.0 -> 5.4, B=32 T=512 6/2 21.9 -> 20.6, B=16 T=1024 16/4 74.3 -> 69.2, B=8 T=2000 16/4 122.0 -> 115.1.
 #pragma once
 
 #include "ptx.cuh"
@@ -50,21 +50,23 @@ struct FwdParams {
 
 template <int D>
 struct FwdCfg {
-    static constexpr int kKeys = 64;                  // keys per K/V tile
-    static constexpr int kStages = (D == 64) ? 4 : 2;
+    static constexpr bool kSepP = (D == 64);          // P has its own columns (else it overwrites S)
+    static constexpr int kKeys = kSepP ? 128 : 64;    // keys per K/V tile
+    static constexpr int kStages = 2;
     static constexpr int kQBufs = (D == 64) ? 2 : 1;  // Q tiles in shared memory (the next item's Q is prefetched)
     static constexpr int kQTileBytes = 128 * D * 2;
     static constexpr int kQBoxBytes = 128 * 64 * 2;   // Q TMA box: 128 rows x 64 bf16
     static constexpr int kKVTileBytes = kKeys * D * 2;
-    static constexpr int kKVBoxBytes = kKeys * 64 * 2;  // K/V TMA box: 64 rows x 64 bf16
+    static constexpr int kKVBoxBytes = kKeys * 64 * 2;  // K/V TMA box: kKeys rows x 64 bf16
     static constexpr int kBoxes = D / 64;
     static constexpr int kBarBytes = 384;
-    static constexpr bool kQInTmem = (D == 64);
     static constexpr int kSmemBytes = kQBufs * kQTileBytes + 2 * kStages * kKVTileBytes + kBarBytes + 1024;
     static constexpr int kTmemCols = 256;
-    static constexpr int kSBufs = 2;
-    static constexpr int kColO = kSBufs * 64;
-    static constexpr int kColQ = kColO + D;  // D = 64 only: [192, 224) and [224, 256)
+    static constexpr int kSBufs = kSepP ? 1 : 2;
+    static constexpr int kColO = 128;
+    static constexpr int kColP = kColO + D;  // kSepP only
+    // registers per thread of the softmax warpgroup and of the other one: together the launch's 256 x 128
+    static constexpr int kRegsSoftmax = kSepP ? 192 : 168, kRegsOther = 256 - kRegsSoftmax;
     __host__ __device__ static constexpr int col_s(int buf) { return buf * 64; }
 };
 
@@ -90,17 +92,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     uint64_t* bar_q_free = bars + 2;   // [2] per Q buffer: every Q K^T product of the item done (phase: item / NQB)
     uint64_t* bar_s_full = bars + 4;   // [NSB] per S buffer                                      (phase: tile / NSB)
     uint64_t* bar_p_full = bars + 7;   // [NSB] per S buffer: P written, O rescaled               (phase: tile / NSB)
-    uint64_t* bar_pv_done = bars + 10; // P V of a tile is complete                               (phase: tile)
     uint64_t* bar_o_done = bars + 11;  // O of an item is complete                                (phase: item)
     uint64_t* bar_o_free = bars + 12;  // O has been read by the epilogue                         (phase: item)
     uint64_t* bar_k_full = bars + 13;            // [NST]
-    uint64_t* bar_k_free = bars + 13 + NST;      // [NST]
+    uint64_t* bar_k_free = bars + 13 + NST;      // [NST] Q K^T of the tile is complete (a softmax thread that has seen it says so)
     uint64_t* bar_v_full = bars + 13 + 2 * NST;  // [NST]
-    uint64_t* bar_v_free = bars + 13 + 3 * NST;  // [NST]
+    uint64_t* bar_v_free = bars + 13 + 3 * NST;  // [NST] P V of the tile is complete
     uint64_t* bar_item = bars + 32;    // [kItemRing] item ids handed out by the producer
     volatile int* item_ring = reinterpret_cast<volatile int*>(bars + 32 + kItemRing);
-    uint64_t* bar_qs_free = bars + 44;  // [2] per Q buffer: the tile in shared memory has been copied (phase: item / NQB)
-    uint64_t* bar_qt_full = bars + 46;  // [2] per Q buffer: Q of an item is in tensor memory          (phase: item / NQB)
+    uint64_t* bar_s_loaded = bars + 44; // kSepP: S is in registers                              (phase: tile)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 30);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 31);
 
@@ -128,14 +128,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bar_q[i], 1);
             mbar_init(&bar_q_free[i], 1);
-            mbar_init(&bar_qs_free[i], 128);
-            mbar_init(&bar_qt_full[i], 128);
         }
         for (int i = 0; i < NSB; ++i) {
             mbar_init(&bar_s_full[i], 1);
             mbar_init(&bar_p_full[i], 128);
         }
-        mbar_init(bar_pv_done, 1);
+        mbar_init(bar_s_loaded, 128);
         mbar_init(bar_o_done, 1);
         mbar_init(bar_o_free, 128);
         for (int s = 0; s < NST; ++s) {
@@ -162,10 +160,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (*abort_flag != 0) {
         // an earlier CTA already failed: fall through to the teardown
     } else if (warp >= 6) {
-        reg_dealloc<88>();  // idle warps
+        reg_dealloc<Cfg::kRegsOther>();  // idle warps
     } else if (warp == 4) {
         // ------------------------------------------------------------------ producer
-        reg_dealloc<88>();
+        reg_dealloc<Cfg::kRegsOther>();
         int g = 0;  // key tiles issued so far by this CTA (ring position)
         bool ok = true;
         int id_next = 0;  // lane 0: the id fetched for the item after the next Q load
@@ -173,8 +171,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         auto load_q = [&](int n, int id) {
             const int qb = n % NQB;
             if (n >= NQB)
-                ok = mbar_wait_warp(Cfg::kQInTmem ? &bar_qs_free[qb] : &bar_q_free[qb], uint32_t(n / NQB - 1) & 1, abort_flag,
-                                    p.status, DEV_WAIT_TIMEOUT_FREE);
+                ok = mbar_wait_warp(&bar_q_free[qb], uint32_t(n / NQB - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
             if (!ok) return;
             if (elect_one()) {
                 mbar_arrive_expect_tx(&bar_q[qb], Cfg::kQTileBytes);
@@ -240,7 +237,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (ok && lane == 0) sched_finish(p.sched, int(gridDim.x));
     } else if (warp == 5) {
         // ------------------------------------------------------------------ MMA issuer
-        reg_dealloc<88>();
+        reg_dealloc<Cfg::kRegsOther>();
         constexpr uint32_t idesc_s = make_idesc_bf16(128, Cfg::kKeys, 0, 0);
         constexpr uint32_t idesc_o = make_idesc_bf16(128, D, 0, 1);
         // This CTA's key tiles are numbered g = 0, 1, ... across all its items: ring stage g % NST,
@@ -252,33 +249,24 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         Cursor sc{get_item(0), 0, 0, 0, 0};
         if (sc.id >= 0) sc.n_kv = item_nkv(sc.id);
         bool ok = true;
-        auto issue_next_s = [&]() {
+        // Waits for what S(cursor) reads: its Q (first tile of an item) and K.  (The S buffer is free once the products before
+        // it in the pipe have run.)
+        auto wait_s = [&]() {
             if (sc.id < 0) return;
             const int s = sc.g % NST, qb = sc.n % NQB;
             if (sc.j == 0)
-                ok = mbar_wait_warp(Cfg::kQInTmem ? &bar_qt_full[qb] : &bar_q[qb], uint32_t(sc.n / NQB) & 1, abort_flag, p.status,
-                                    DEV_WAIT_TIMEOUT_LOAD);
+                ok = mbar_wait_warp(&bar_q[qb], uint32_t(sc.n / NQB) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
             if (ok) ok = mbar_wait_warp(&bar_k_full[s], uint32_t(sc.g / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
-            if (!ok) return;
-            tc_fence_after_sync();
-            const uint64_t q_desc = make_sdesc_sw128(smem_u32(sQ + qb * Cfg::kQTileBytes), 16, 1024);
-            const uint64_t k_desc = make_sdesc_sw128(smem_u32(sK + s * Cfg::kKVTileBytes), 16, 1024);
-            const bool last = sc.j + 1 == sc.n_kv;  // no later MMA reads this item's Q
-            if (elect_one()) {
+        };
+        // one thread: S(cursor) = Q K^T
+        auto issue_s = [&](uint32_t s_col, uint64_t q_desc, uint64_t k_desc, int qb, uint64_t* full, bool last) {
 #pragma unroll
-                for (int ks = 0; ks < D / 16; ++ks) {
-                    if constexpr (Cfg::kQInTmem)
-                        umma_ts(tmem + Cfg::col_s(sc.g % NSB), tmem + Cfg::kColQ + qb * 32 + ks * 8,
-                                k_desc + kmajor_step(ks, Cfg::kKVBoxBytes), idesc_s, ks > 0);
-                    else
-                        umma_ss(tmem + Cfg::col_s(sc.g % NSB), q_desc + kmajor_step(ks, Cfg::kQBoxBytes),
-                                k_desc + kmajor_step(ks, Cfg::kKVBoxBytes), idesc_s, ks > 0);
-                }
-                umma_commit(&bar_s_full[sc.g % NSB]);
-                umma_commit(&bar_k_free[s]);
-                if (last) umma_commit(&bar_q_free[qb]);
-            }
-            __syncwarp();
+            for (int ks = 0; ks < D / 16; ++ks)
+                umma_ss(tmem + s_col, q_desc + kmajor_step(ks, Cfg::kQBoxBytes), k_desc + kmajor_step(ks, Cfg::kKVBoxBytes), idesc_s, ks > 0);
+            umma_commit(full);
+            if (last) umma_commit(&bar_q_free[qb]);  // no later product reads this item's Q
+        };
+        auto next_s = [&]() {
             ++sc.g;
             if (++sc.j == sc.n_kv) {
                 sc.id = get_item(++sc.n);
@@ -286,51 +274,85 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 sc.n_kv = sc.id >= 0 ? item_nkv(sc.id) : 0;
             }
         };
-        for (int i = 0; i < NSB && ok; ++i) issue_next_s();
+        const uint32_t sq_addr = smem_u32(sQ), sk_addr = smem_u32(sK), sv_addr = smem_u32(sV);
+        for (int i = 0; i < NSB && ok && sc.id >= 0; ++i) {
+            wait_s();
+            if (!ok) break;
+            tc_fence_after_sync();
+            if (elect_one())
+                issue_s(Cfg::col_s(sc.g % NSB), make_sdesc_sw128(sq_addr + (sc.n % NQB) * Cfg::kQTileBytes, 16, 1024),
+                        make_sdesc_sw128(sk_addr + (sc.g % NST) * Cfg::kKVTileBytes, 16, 1024), sc.n % NQB, &bar_s_full[sc.g % NSB],
+                        sc.j + 1 == sc.n_kv);
+            __syncwarp();
+            next_s();
+        }
         int g = 0, n = 0;
         // (this warp has already waited for the ring entry of item n: the cursor above is never behind)
         for (int id; ok && (id = item_ring[n % kItemRing]) >= 0; ++n) {
             const int n_kv = item_nkv(id);
-            for (int j = 0; j < n_kv && ok; ++j, ++g) {
+            for (int j = 0; j < n_kv; ++j, ++g) {
+                // What P V needs besides P is waited for first: a wait costs 100 clocks even when the barrier is complete.
                 const int s = g % NST;
+                if constexpr (Cfg::kSepP) {
+                    // S(g + 1) as soon as S(g) is in registers: it runs under the exponentials of tile g
+                    if (sc.id >= 0) {
+                        wait_s();
+                        if (ok) ok = mbar_wait_warp(bar_s_loaded, uint32_t(g) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
+                        if (!ok) break;
+                        tc_fence_after_sync();
+                        if (elect_one())
+                            issue_s(Cfg::col_s(0), make_sdesc_sw128(sq_addr + (sc.n % NQB) * Cfg::kQTileBytes, 16, 1024),
+                                    make_sdesc_sw128(sk_addr + (sc.g % NST) * Cfg::kKVTileBytes, 16, 1024), sc.n % NQB, &bar_s_full[0],
+                                    sc.j + 1 == sc.n_kv);
+                        __syncwarp();
+                        next_s();
+                    }
+                }
+                if (ok) ok = mbar_wait_warp(&bar_v_full[s], uint32_t(g / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+                // the accumulator belongs to the previous item's epilogue until it has been read
+                if (ok && j == 0 && n > 0) ok = mbar_wait_warp(bar_o_free, uint32_t(n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
+                if (!ok) break;
+                const bool more = !Cfg::kSepP && sc.id >= 0, s_last = sc.j + 1 == sc.n_kv, o_last = j + 1 == n_kv;
+                const int qb = sc.n % NQB;
+                const uint64_t v_desc = make_sdesc_sw128(sv_addr + s * Cfg::kKVTileBytes, Cfg::kKVBoxBytes, 1024);
+                const uint64_t q_desc = make_sdesc_sw128(sq_addr + qb * Cfg::kQTileBytes, 16, 1024);
+                const uint64_t k_desc = make_sdesc_sw128(sk_addr + (sc.g % NST) * Cfg::kKVTileBytes, 16, 1024);
+                const uint32_t col = Cfg::kSepP ? Cfg::kColP : Cfg::col_s(g % NSB);  // of P(g), and without kSepP of S(g + NSB)
                 ok = mbar_wait_warp(&bar_p_full[g % NSB], uint32_t(g / NSB) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
                 if (!ok) break;
                 B200ATTN_STAMP(lane == 0, 16 + 8 * g + 4);
-                // the accumulator belongs to the previous item's epilogue until it has been read
-                if (j == 0 && n > 0) {
-                    ok = mbar_wait_warp(bar_o_free, uint32_t(n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
-                    if (!ok) break;
-                }
-                ok = mbar_wait_warp(&bar_v_full[s], uint32_t(g / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
-                if (!ok) break;
                 tc_fence_after_sync();
-                const uint64_t v_desc = make_sdesc_sw128(smem_u32(sV + s * Cfg::kKVTileBytes), Cfg::kKVBoxBytes, 1024);
                 if (elect_one()) {
-                    // O += P V : 64 keys = 4 K steps; P lives in the first 32 columns of its S buffer
+                    // O += P V : 16 keys per K step, 8 columns of BF16 pairs each
 #pragma unroll
                     for (int ks = 0; ks < Cfg::kKeys / 16; ++ks)
-                        umma_ts(tmem + Cfg::kColO, tmem + Cfg::col_s(g % NSB) + ks * 8,
-                                v_desc + uint64_t(ks * 128), idesc_o, (j > 0) || (ks > 0));
-                    umma_commit(bar_pv_done);
+                        umma_ts(tmem + Cfg::kColO, tmem + col + ks * 8, v_desc + uint64_t(ks * 128), idesc_o, (j > 0) || (ks > 0));
                     umma_commit(&bar_v_free[s]);
-                    if (j + 1 == n_kv) umma_commit(bar_o_done);
+                    if (o_last) umma_commit(bar_o_done);
                 }
                 __syncwarp();
-                B200ATTN_STAMP(lane == 0, 16 + 8 * g + 5);
-                issue_next_s();  // tile g + NSB: its S buffer was read by the P V just issued
+                if (more) {
+                    // S of tile g + NSB into the buffer that the products just issued read.  (With two K/V stages its K is
+                    // requested late: P V must not wait for it.)
+                    wait_s();
+                    if (!ok) break;
+                    if (elect_one()) issue_s(col, q_desc, k_desc, qb, &bar_s_full[g % NSB], s_last);
+                    __syncwarp();
+                }
                 B200ATTN_STAMP(lane == 0, 16 + 8 * g + 6);
+                if (more) next_s();
             }
         }
         // nothing may be in flight when TMEM is freed: the last commit covers every MMA issued above
         if (ok && n > 0) mbar_wait_warp(bar_o_done, uint32_t(n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
     } else {
         // ------------------------------------------------------------------ softmax + epilogue
-        reg_alloc<168>();
+        reg_alloc<Cfg::kRegsSoftmax>();
         const int row = tid;                                   // query row inside the tile == TMEM lane
         const uint32_t lane_base = uint32_t(warp * 32) << 16;  // this warp's TMEM lane quadrant
         const uint32_t t_o = tmem + lane_base + Cfg::kColO;
         bool ok = true;
-        // Epilogue of one item: O / l -> BF16 -> global memory, logsumexp.  (bar_pv_done cannot be used for
+        // Epilogue of one item: O / l -> BF16 -> global memory, logsumexp.  (bar_v_free cannot be used for
         // "O is complete": P V of the last TWO tiles may still be in flight, and a parity wait is only
         // unambiguous when the waiter is at most one phase behind; bar_o_done completes once per item.)
         auto epilogue = [&](int n_item, int id, float m_ref, float l) -> bool {
@@ -373,33 +395,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             B200ATTN_STAMP(tid == 0, 400 + 4 * n_item + 2);
             return true;
         };
-        // D = 64: Q of this CTA's n-th item from shared memory into Q buffer n % NQB of tensor memory.  The buffer
-        // held Q of item n - NQB, whose last Q K^T product must have completed.
-        auto copy_q = [&](int n_item) -> bool {
-            const int qb = n_item % NQB;
-            if (!mbar_wait_warp(&bar_q[qb], uint32_t(n_item / NQB) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD)) return false;
-            if (n_item >= NQB &&
-                !mbar_wait_warp(&bar_q_free[qb], uint32_t(n_item / NQB - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE))
-                return false;
-            tc_fence_after_sync();
-            uint32_t qw[32];
-            const uint8_t* qrow = sQ + qb * Cfg::kQTileBytes + row * 128;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const uint4 w = *reinterpret_cast<const uint4*>(qrow + ((c ^ (row & 7)) << 4));
-                qw[4 * c] = w.x, qw[4 * c + 1] = w.y, qw[4 * c + 2] = w.z, qw[4 * c + 3] = w.w;
-            }
-            tmem_st_x32(tmem + lane_base + Cfg::kColQ + qb * 32, qw);
-            fence_proxy_async_smem();  // ordinary reads before the async proxy (TMA) overwrites the tile
-            mbar_arrive(&bar_qs_free[qb]);  // the values are in registers: the tile in shared memory may be reloaded
-            tmem_wait_st();
-            tc_fence_before_sync();
-            mbar_arrive(&bar_qt_full[qb]);
-            return true;
-        };
-        if constexpr (Cfg::kQInTmem) {
-            if (get_item(0) >= 0) ok = copy_q(0);
-        }
         // The epilogue of an item is deferred until the softmax of the next item's first tile has been handed
         // to the MMA warp: the wait for the item's last P V then overlaps useful work.
         bool pending = false;
@@ -412,74 +407,91 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             float m_ref = -INFINITY;  // exponent reference (a past row maximum), raw score units
             float l = 0.f;            // running sum of exp2((s - m_ref) * scale_log2)
             for (int j = 0; j < n_kv; ++j, ++g) {
-                if constexpr (Cfg::kQInTmem) {
-                    // the next item's Q, a few tiles before the MMA warp wants it for that item's first products
-                    if (j == max(0, n_kv - 3) && get_item(n + 1) >= 0) {
-                        ok = copy_q(n + 1);
-                        if (!ok) break;
-                    }
-                }
                 const uint32_t t_s = tmem + lane_base + Cfg::col_s(g % NSB);
                 ok = mbar_wait_warp(&bar_s_full[g % NSB], uint32_t(g / NSB) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
                 if (!ok) break;
                 B200ATTN_STAMP(tid == 0, 16 + 8 * g + 0);
+                if (tid == 0) mbar_arrive(&bar_k_free[g % NST]);
                 tc_fence_after_sync();
-                uint32_t sr[64];
-                tmem_ld_x32(t_s, &sr[0]);
-                tmem_ld_x32(t_s + 32, &sr[32]);
+                constexpr int KEYS = Cfg::kKeys;
+                uint32_t sr[KEYS];
+#pragma unroll
+                for (int c = 0; c < KEYS; c += 32) tmem_ld_x32(t_s + c, &sr[c]);
                 tmem_wait_ld();
-                const int kbase = j * Cfg::kKeys;  // first key of this tile
-                if (kbase + Cfg::kKeys - 1 > q0 + p.kv_off) {
+                if constexpr (Cfg::kSepP) {
+                    tc_fence_before_sync();
+                    mbar_arrive(bar_s_loaded);  // the buffer goes back to the MMA warp at once
+                }
+                const int kbase = j * KEYS;  // first key of this tile
+                if (kbase + KEYS - 1 > q0 + p.kv_off) {
                     // tile touches the diagonal: key kbase + c is visible to query q0 + row iff it is <= the query's
                     // own position kv_off + q0 + row
                     const int lim = p.kv_off + q0 + row - kbase;  // columns c <= lim are visible
 #pragma unroll
-                    for (int c = 0; c < 64; ++c)
+                    for (int c = 0; c < KEYS; ++c)
                         if (c > lim) sr[c] = 0xff800000u;  // -inf
                 }
-                float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-                for (int c = 0; c < 64; c += 4) {
-                    mx0 = fmaxf(mx0, __uint_as_float(sr[c + 0]));
-                    mx1 = fmaxf(mx1, __uint_as_float(sr[c + 1]));
-                    mx2 = fmaxf(mx2, __uint_as_float(sr[c + 2]));
-                    mx3 = fmaxf(mx3, __uint_as_float(sr[c + 3]));
-                }
-                const float m_new = fmaxf(fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)), m_ref);
+                for (int c = 0; c < KEYS; c += 8)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        mx[k] = fmaxf(mx[k], fmaxf(__uint_as_float(sr[c + 2 * k]), __uint_as_float(sr[c + 2 * k + 1])));
+                const float m_new = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])), m_ref);
                 float alpha = 1.f;
                 if ((m_new - m_ref) * p.scale_log2 > kRescaleThresholdLog2) {  // also true for m_ref == -inf
                     alpha = ex2_approx((m_ref - m_new) * p.scale_log2);
                     m_ref = m_new;
                 }
                 const float neg_m = -m_ref * p.scale_log2;
-                float sum0 = 0.f, sum1 = 0.f, sum2 = 0.f, sum3 = 0.f;
+                const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), neg2 = pack_f32x2(neg_m, neg_m);
+                uint64_t sum2[2] = {0ull, 0ull};
+                // 32 columns at a time: exponentials, sums and BF16 pairs
+                auto chunk = [&](int c, uint32_t (&pk)[16]) {
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    uint32_t pk[16];
-#pragma unroll
-                    for (int i = 0; i < 16; i += 2) {
-                        const float p0 = ex2_approx(fmaf(__uint_as_float(sr[c * 32 + 2 * i + 0]), p.scale_log2, neg_m));
-                        const float p1 = ex2_approx(fmaf(__uint_as_float(sr[c * 32 + 2 * i + 1]), p.scale_log2, neg_m));
-                        const float p2 = ex2_approx(fmaf(__uint_as_float(sr[c * 32 + 2 * i + 2]), p.scale_log2, neg_m));
-                        const float p3 = ex2_approx(fmaf(__uint_as_float(sr[c * 32 + 2 * i + 3]), p.scale_log2, neg_m));
-                        sum0 += p0;
-                        sum1 += p1;
-                        sum2 += p2;
-                        sum3 += p3;
-                        pk[i + 0] = pack_bf16x2(p0, p1);
-                        pk[i + 1] = pack_bf16x2(p2, p3);
+                    for (int i = 0; i < 16; ++i) {
+                        float a0, a1;
+                        unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sr[c + 2 * i]), __uint_as_float(sr[c + 2 * i + 1])), scale2, neg2), a0, a1);
+                        a0 = ex2_approx(a0);
+                        a1 = ex2_approx(a1);
+                        sum2[i & 1] = add_f32x2(sum2[i & 1], pack_f32x2(a0, a1));
+                        pk[i] = pack_bf16x2(a0, a1);
                     }
-                    tmem_st_x16(t_s + c * 16, pk);
-                }
-                l = l * alpha + ((sum0 + sum1) + (sum2 + sum3));
-                B200ATTN_STAMP(tid == 0, 16 + 8 * g + 1);
-                if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-                    // O must hold P V of the previous tile before it is rescaled.  (At most one phase of
-                    // this barrier is outstanding here: P V of this tile cannot start before this
-                    // warp has arrived on bar_p_full below.)
-                    ok = mbar_wait_warp(bar_pv_done, uint32_t(g - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+                };
+                // P V of the previous tile: it reads the columns P goes to (kSepP) and adds to O, which may have to be rescaled.
+                // (At most one phase of this barrier is outstanding here: P V of this tile cannot start before this warp has
+                // arrived on bar_p_full below.)
+                uint64_t* bar_pv = &bar_v_free[(g - 1) % NST];
+                const uint32_t pv_par = uint32_t((g - 1) / NST) & 1;
+                const bool pv_seen = Cfg::kSepP && (g == 0 || mbar_try_wait(bar_pv, pv_par));  // (looked at again below)
+                auto wait_pv = [&]() {
+                    if (!__all_sync(0xffffffffu, pv_seen)) ok = mbar_wait_warp(bar_pv, pv_par, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+                    if (ok) tc_fence_after_sync();
+                };
+                const bool rescale = j > 0 && __any_sync(0xffffffffu, alpha != 1.f);
+                const uint32_t t_p = Cfg::kSepP ? tmem + lane_base + Cfg::kColP : t_s;
+                {
+                    uint32_t pk[16];
+                    chunk(0, pk);
+                    if (Cfg::kSepP) wait_pv();
                     if (!ok) break;
-                    tc_fence_after_sync();
+                    tmem_st_x16(t_p, pk);
+                }
+#pragma unroll
+                for (int c = 1; c < KEYS / 32; ++c) {
+                    uint32_t pk[16];
+                    chunk(c * 32, pk);
+                    tmem_st_x16(t_p + c * 16, pk);
+                }
+                {
+                    float s0, s1;
+                    unpack_f32x2(add_f32x2(sum2[0], sum2[1]), s0, s1);
+                    l = l * alpha + (s0 + s1);
+                }
+                B200ATTN_STAMP(tid == 0, 16 + 8 * g + 1);
+                if (rescale) {
+                    if (!Cfg::kSepP) wait_pv();
+                    if (!ok) break;
 #pragma unroll
                     for (int c = 0; c < D / 32; ++c) {
                         uint32_t orr[32];

@@ -288,10 +288,11 @@ int fwd_run(const void* q, const void* k, const void* v, void* o, float* lse, in
     int* status = status_ptr(&rc);
     if (!status) return rc;
     const Strides sq = strides_for(layout, Hq, T, D);
+    const int keys = D == 64 ? FwdCfg<64>::kKeys : FwdCfg<128>::kKeys;
     CUtensorMap tq, tk, tv;
     if (!make_tmap_bf16_4d(&tq, q, D, T, Hq, B, sq.t, sq.h, sq.b, 128) ||
-        !make_tmap_bf16_4d(&tk, k, D, kv_off + T, Hkv, B, sk.t, sk.h, sk.b, 64) ||
-        !make_tmap_bf16_4d(&tv, v, D, kv_off + T, Hkv, B, sk.t, sk.h, sk.b, 64))
+        !make_tmap_bf16_4d(&tk, k, D, kv_off + T, Hkv, B, sk.t, sk.h, sk.b, keys) ||
+        !make_tmap_bf16_4d(&tv, v, D, kv_off + T, Hkv, B, sk.t, sk.h, sk.b, keys))
         return B200ATTN_ERR_TENSOR_MAP;
     FwdParams p;
     p.B = B;

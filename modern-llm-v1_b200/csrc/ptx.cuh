@@ -214,9 +214,11 @@ __device__ __forceinline__ bool elect_one() {
     return pred != 0;
 }
 
-// Bounded wait executed by a whole warp; the result is made warp-uniform.
+// Bounded wait executed by a whole warp; the result is made warp-uniform.  The first probe is voted on before anything
+// branches, so that a barrier that is complete already costs no divergence handling.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
                                                int code) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code));
 }
 
@@ -415,6 +417,29 @@ __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+// Two FP32 operations per instruction (each half rounds like the scalar one).
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
 
 // Register re-balancing between warpgroups (each executed by all four warps of a group).
