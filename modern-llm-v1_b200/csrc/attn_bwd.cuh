@@ -11,22 +11,19 @@
 // the query heads of its group and keeps one accumulator, which replaces
 // accumulate_kv_grads (llm/src/model/attention.cu:412-429,510-543).
 //
-// Roles in the dK/dV pass (576 threads; the dQ pass is described at its kernel):
-//   warps 0-15  compute: thread owns TMEM lane (warp % 4) * 32 + lane and the 32 score
-//               columns of its part (warp / 4); four warps per scheduler hide the TMEM and
-//               MUFU latencies of one another
+// Roles in the dK/dV pass (640 threads; the dQ pass is described at its kernel):
+//   warps 0-15  compute: thread owns TMEM lane (warp % 4) * 32 + lane and 32 of the 128 score columns (warp / 4); four warps
+//               per scheduler hide the TMEM and MUFU latencies of one another
 //   warp  16    TMA producer (converged warp, one elected lane issues)
-//   warp  17    TMEM allocation and tcgen05.mma issue (converged warp, one elected lane issues)
-// TMEM (512 columns), D = 64:  S buffer 0 [0,128), S buffer 1 [128,256), dP [256,384),
-//   accumulators [384,448) and [448,512).  With two S buffers the next tile's QK^T product
-//   is issued while the compute warps still work on the current tile.
-//   D = 128: one S buffer [0,128), dP [128,256), accumulators [256,384) and [384,512).
+//   warp  17    TMEM allocation and the products S^T (converged warp, one elected lane issues)
+//   warp  18    the other products
+//   warp  19    D = 64: the row vectors as MMA operands (see there); else idle
+// TMEM (512 columns): S [0,128), dP blocks of 128 columns (two at D = 64, one at D = 128), then the dV and dK accumulators.
+//   The compute warps take a unit's scores into registers in one go and hand the S buffer back at once, so the next S^T runs
+//   under this unit's exponentials; P^T and dS^T go over the unit's dP block.
 // The compute step has two phases so that it can start on S before dP has arrived:
-//   A: P = exp2(S * scale*log2e - L*log2e)   (kept in registers; the dK/dV pass also stores it)
-//   B: dS = P * (dP - D)                      (stored over dP as BF16)
-// The BF16 operands of the second-stage MMAs overwrite the FP32 values they were computed
-// from: part q of a 128-wide block keeps its 32 BF16 values in the first 16 columns of its
-// own 32-column range.
+//   A: P = exp2(S * scale*log2e - L*log2e)   (kept in registers)
+//   B: dS = P * (dP - D)                      (stored over dP as BF16, in the dK/dV pass beside P)
 #pragma once
 
 #include "ptx.cuh"
@@ -56,27 +53,32 @@ struct BwdParams {
 
 template <int D>
 struct BwdCfg {
-    static constexpr bool kDoubleS = (D == 64);
-    static constexpr int kStages = kDoubleS ? 3 : 2;  // streamed operand pairs in shared memory
+    static constexpr int kStages = D == 64 ? 4 : 2;   // streamed operand pairs (Q, dO) in shared memory
     static constexpr int kTileBytes = 128 * D * 2;
     static constexpr int kBoxBytes = 128 * 64 * 2;
     static constexpr int kBoxes = D / 64;
     static constexpr int kVecBytes = kStages * 2 * 512;  // per stage (lse2, dvec) of 128 rows
     static constexpr int kBarBytes = 512;
-    static constexpr int kKvBufs = kDoubleS ? 2 : 1;       // K/V tile pairs in shared memory (the next item's are prefetched)
-    static constexpr int kOutTiles = kDoubleS ? 2 : 0;     // staging tiles for dV, dK (D = 128 has no room: direct stores)
-    static constexpr int kParts = 4;                       // compute warpgroups: each owns 128 / kParts score columns
-    static constexpr int kPartCols = 128 / kParts;         // 32
-    static constexpr int kComputeThreads = 128 * kParts;   // 512
-    static constexpr int kThreads = kComputeThreads + 64;  // + producer warp + MMA warp
-    static constexpr int kSmemBytes = (2 * kKvBufs + 2 * kStages + kOutTiles) * kTileBytes + kVecBytes + kBarBytes + 1024;
+    static constexpr int kKvBufs = D == 64 ? 2 : 1;      // K/V tile pairs in shared memory (the next item's are prefetched)
+    static constexpr int kPartCols = 16;                 // score columns whose P^T and dS^T lie side by side
+    static constexpr int kCols = 32;                     // score columns per compute thread
+    static constexpr int kComputeThreads = 512;
+    static constexpr int kThreads = kComputeThreads + 128;
+    // registers per thread of the compute warps and of the others: together the launch's kThreads x 96
+    static constexpr int kRegsCompute = 104, kRegsOther = 64;
+    static_assert(kRegsCompute * kComputeThreads + kRegsOther * 128 <= 96 * kThreads, "more registers than the launch has");
+    static constexpr bool kVecOps = D == 64;             // the row vectors enter the products (see the row-vector warp)
+    static constexpr int kOpBytes = 128 * 16;            // a row vector as MMA operand: 8 BF16 per row
+    static constexpr int kOpsBytes = kVecOps ? (2 * kStages + 2) * kOpBytes : 0;  // two per stage, ones, zeros
+    static constexpr int kSmemBytes = (2 * kKvBufs + 2 * kStages) * kTileBytes + kVecBytes + kOpsBytes + kBarBytes + 1024;
+    static_assert(kSmemBytes <= 232448, "shared memory of an SM");
     static constexpr int kTmemCols = 512;
-    static constexpr int kColS0 = 0;
-    static constexpr int kColS1 = kDoubleS ? 128 : 0;
-    static constexpr int kColDP = kDoubleS ? 256 : 128;
-    static constexpr int kColAcc0 = kDoubleS ? 384 : 256;
-    static constexpr int kColAcc1 = kDoubleS ? 448 : 384;
-    __host__ __device__ static constexpr int col_s(int buf) { return buf ? kColS1 : kColS0; }
+    static constexpr int kDpBufs = D == 64 ? 2 : 1;
+    static constexpr int kColS = 0;
+    static constexpr int kColAcc0 = 128 + 128 * kDpBufs;  // dV
+    static constexpr int kColAcc1 = kColAcc0 + D;         // dK
+    static_assert(kColAcc1 + D <= kTmemCols, "tensor memory");
+    __host__ __device__ static constexpr int col_dp(int buf) { return 128 + 128 * buf; }
 };
 
 // D[tmem] = A[smem, K-major] * B[smem, K-major]^T over the head dimension; a_desc / b_desc
@@ -91,17 +93,13 @@ __device__ __forceinline__ void issue_ss_over_headdim(uint32_t d_tmem, uint64_t 
 }
 
 // D[tmem] (+)= A[tmem, BF16 pairs] * B[smem, MN-major] over 128 rows of B (b_desc describes
-// rows 0..15).  The A operand lives in kParts pieces: part q keeps its kPartCols BF16 values in
-// the first kPartCols / 2 columns of its own FP32 column range, which starts at a_col + q * kPartCols.
+// rows 0..15).  The A operand lies in pieces of 16 values (8 columns) that are kPartCols columns apart.
 template <int D>
 __device__ __forceinline__ void issue_ts_over_rows(uint32_t d_tmem, uint32_t a_col, uint64_t b_desc, uint32_t idesc,
                                                    bool accumulate) {
-    constexpr int kStepsPerPart = BwdCfg<D>::kPartCols / 16;  // K steps (16 rows of B) per part
 #pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
-        const uint32_t a = a_col + (ks / kStepsPerPart) * BwdCfg<D>::kPartCols + (ks % kStepsPerPart) * 8;
-        umma_ts(d_tmem, a, b_desc + uint64_t(ks * 128), idesc, accumulate || ks > 0);
-    }
+    for (int ks = 0; ks < 8; ++ks)
+        umma_ts(d_tmem, a_col + ks * BwdCfg<D>::kPartCols, b_desc + uint64_t(ks * 128), idesc, accumulate || ks > 0);
 }
 
 template <int D>
@@ -879,47 +877,53 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 // handed out as described in ptx.cuh.  All pipelines run across item boundaries: the next item's K and V
 // tiles (second buffer, D = 64) and its first Q / dO tiles are loaded, and its first S^T and dP^T
 // products issued, while the compute warps still drain the accumulators of the previous item.
+// What bounds it: D = 128 the tensor pipe (two products with both operands in shared memory, two with one in tensor memory);
+// D = 64 a unit's chain, scores -> exponentials -> dP -> dS -> products, of which S^T and dP^T of the following units are off
+// the chain because there is one more dP block than units in work and S goes back as soon as it is in registers.  Measured
+// against two S buffers (P^T and dS^T over the scores), one dP block, one MMA warp and row vectors read by the compute warps,
+// us: B=16 T=1024 16/4 D=64 94.7 -> 84.5, B=8 T=2000 16/4 D=64 171 -> 148, B=4 T=4096 16/4 D=128 496 -> 468.  Two groups of eight
+// warps on alternate units (64 columns a thread) were slower: 93 to 117 at the first of these, they spill.
 // ---------------------------------------------------------------------------------------
 template <int D>
 __global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                     const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
-                     const __grid_constant__ CUtensorMap tmdK, const __grid_constant__ CUtensorMap tmdV,
-                     const BwdParams p) {
+                     const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO, const BwdParams p) {
     using Cfg = BwdCfg<D>;
     constexpr int NST = Cfg::kStages;
     constexpr int NKV = Cfg::kKvBufs;
-    constexpr bool DBL = Cfg::kDoubleS;
+    constexpr int NDP = Cfg::kDpBufs;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sK = smem;                         // [NKV]
     uint8_t* sV = sK + NKV * Cfg::kTileBytes;   // [NKV]
     uint8_t* sQ = sV + NKV * Cfg::kTileBytes;   // [NST]
     uint8_t* sdO = sQ + NST * Cfg::kTileBytes;  // [NST]
-    uint8_t* sOut = sdO + NST * Cfg::kTileBytes;  // [2] staging of dV and dK for the TMA store (D = 64 only)
-    float* sLse = reinterpret_cast<float*>(sOut + Cfg::kOutTiles * Cfg::kTileBytes);  // [NST][128]
-    float* sDv = sLse + NST * 128;                                         // [NST][128]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + Cfg::kOutTiles * Cfg::kTileBytes + Cfg::kVecBytes);
+    float* sLse = reinterpret_cast<float*>(sdO + NST * Cfg::kTileBytes);  // [NST][128]
+    float* sDv = sLse + NST * 128;                                        // [NST][128]
+    uint8_t* sOps = reinterpret_cast<uint8_t*>(sLse) + Cfg::kVecBytes;    // kVecOps: [NST] L and D operands; ones; zeros
+    uint8_t* sOnes = sOps + 2 * NST * Cfg::kOpBytes;
+    uint8_t* sZero = sOnes + Cfg::kOpBytes;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sOps + Cfg::kOpsBytes);
     uint64_t* bar_kv = bars + 0;        // [2] per K/V buffer: K, V of an item have landed      (phase: item / NKV)
     uint64_t* bar_kv_free = bars + 2;   // [2] per K/V buffer: every MMA reading them is done   (phase: item / NKV)
-    uint64_t* bar_s_full = bars + 4;    // [2] per S buffer                                      (phase: unit / 2 or unit)
-    uint64_t* bar_dp_full = bars + 6;   //                                                       (phase: unit)
-    uint64_t* bar_dp_free = bars + 7;   // dP^T has been read into registers                     (phase: unit)
+    uint64_t* bar_s_full = bars + 4;    //                                                       (phase: unit)
+    uint64_t* bar_s_loaded = bars + 5;  // S^T is in registers, the buffer is free               (phase: unit)
+    uint64_t* bar_dp_full = bars + 6;   // [2] by unit parity                                    (phase: unit / 2)
     uint64_t* bar_pds_full = bars + 8;  // [2] by unit parity: P^T and dS^T written              (phase: unit / 2)
     uint64_t* bar_acc = bars + 10;      // accumulators of an item complete                      (phase: item)
     uint64_t* bar_acc_free = bars + 11; // accumulators read by the epilogue                     (phase: item)
-    uint64_t* bar_full = bars + 12;        // [NST] Q, dO and the two row vectors of a unit have landed
-    uint64_t* bar_free = bars + 12 + NST;  // [NST]
-    uint64_t* bar_s_loaded = bars + 22;  // one S buffer (D = 128): S^T is in registers, the buffer is free (phase: unit)
-    uint64_t* bar_out_free = bars + 20;  // the TMA store of the previous item has read the staging tiles (phase: item)
-    uint64_t* bar_out_full = bars + 21;  // every compute thread has staged its part of dV / dK        (phase: item)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 19);
+    uint64_t* bar_full = bars + 12;     // [4] per stage: Q, dO and the two row vectors of a unit have landed (phase: unit / NST)
+    uint64_t* bar_free = bars + 16;     // [4] per stage                                         (phase: unit / NST)
+    uint64_t* bar_vec = bars + 20;      // [4] per stage, kVecOps: the row vectors are there as operands (phase: unit / NST)
     uint64_t* bar_item = bars + 24;     // [kItemRing] item ids handed out by the producer
     volatile int* item_ring = reinterpret_cast<volatile int*>(bars + 24 + kItemRing);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 40);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 41);
+    static_assert(NST <= 4, "the barriers are laid out for four stages");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr int kProducerWarp = Cfg::kParts * 4, kMmaWarp = Cfg::kParts * 4 + 1;
+    constexpr int kProducerWarp = Cfg::kComputeThreads / 32, kMmaSWarp = kProducerWarp + 1, kMmaWarp = kProducerWarp + 2,
+                  kVecWarp = kProducerWarp + 3;
     // item id -> (key tile, KV head, batch); ids are ordered by work: key tile 0 has the most query tiles below it
     const int n_bh = p.B * p.Hkv;
     const int n_items = p.n_tiles * n_bh;
@@ -936,24 +940,20 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         tma_prefetch_desc(&tmV);
         tma_prefetch_desc(&tmQ);
         tma_prefetch_desc(&tmdO);
-        tma_prefetch_desc(&tmdK);
-        tma_prefetch_desc(&tmdV);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bar_kv[i], 1);
-            mbar_init(&bar_kv_free[i], 1);
-            mbar_init(&bar_s_full[i], 1);
+            mbar_init(&bar_kv_free[i], 2);  // each of the MMA warps reads K or V
+            mbar_init(&bar_dp_full[i], 1);
             mbar_init(&bar_pds_full[i], Cfg::kComputeThreads);
         }
-        mbar_init(bar_dp_full, 1);
-        mbar_init(bar_dp_free, Cfg::kComputeThreads);
+        mbar_init(bar_s_full, 1);
+        mbar_init(bar_s_loaded, Cfg::kComputeThreads);
         mbar_init(bar_acc, 1);
         mbar_init(bar_acc_free, Cfg::kComputeThreads);
-        mbar_init(bar_out_free, 1);
-        mbar_init(bar_out_full, Cfg::kComputeThreads);
-        mbar_init(bar_s_loaded, Cfg::kComputeThreads);
         for (int s = 0; s < NST; ++s) {
             mbar_init(&bar_full[s], 1);
             mbar_init(&bar_free[s], 1);
+            mbar_init(&bar_vec[s], 32);
         }
         for (int i = 0; i < kItemRing; ++i) mbar_init(&bar_item[i], 1);
         fence_mbar_init();
@@ -962,7 +962,14 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         grid_dep_wait();
         *abort_flag = *reinterpret_cast<volatile int*>(p.status);
     }
-    if (warp == kMmaWarp) {
+    if (Cfg::kVecOps && warp == kVecWarp) {  // ones: 1, 1, 1, 0, ... per row; zeros
+        for (int r = lane; r < 128; r += 32) {
+            reinterpret_cast<uint4*>(sOnes)[r] = make_uint4(0x3f803f80u, 0x3f80u, 0u, 0u);
+            reinterpret_cast<uint4*>(sZero)[r] = make_uint4(0u, 0u, 0u, 0u);
+        }
+        fence_proxy_async_smem();
+    }
+    if (warp == kMmaSWarp) {
         tmem_alloc(tmem_slot, Cfg::kTmemCols);
         tmem_relinquish();
     }
@@ -976,6 +983,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         // an earlier CTA already failed: fall through to the teardown
     } else if (warp == kProducerWarp) {
         // ------------------------------------------------------------------ producer (whole warp, one lane issues)
+        reg_dealloc<Cfg::kRegsOther>();
         int u = 0;  // units issued so far by this CTA (ring position)
         bool ok = true;
         int id = blockIdx.x;  // the first item needs no fetch
@@ -1035,149 +1043,150 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             id = id_new;
         }
         if (ok && lane == 0) sched_finish(p.sched2, int(gridDim.x));
-    } else if (warp == kMmaWarp) {
-        // ------------------------------------------------------------------ MMA issuer (whole warp, one lane issues)
+    } else if (warp == kVecWarp) {
+        // ------------------------------------------------------------------ row vectors
+        // L and D are the same for a whole column of S^T and dP^T, so reading them costs the compute warps 32 shared-memory
+        // loads per unit and warp, in the pipe that the products' operands come through: 10 % of the kernel at D = 64.  There
+        // they enter the products as one more K step instead, ones[128 keys x 16] times the vector, split into three BF16 terms
+        // (24 bits), so that S^T arrives as s - L / scale and dP^T as dP - D.  This warp turns a unit's two vectors into such
+        // operands.  (At D = 128 the tensor pipe sets the pace: two more K steps per unit cost 10 %.)
+        reg_dealloc<Cfg::kRegsOther>();
+        if constexpr (Cfg::kVecOps) {
+            const float to_scores = -1.f / p.scale_log2;
+            auto split = [](float v) {
+                const float hi = __bfloat162float(__float2bfloat16_rn(v)), r = v - hi;
+                const float mid = __bfloat162float(__float2bfloat16_rn(r));
+                return make_uint4(pack_bf16x2(hi, mid), pack_bf16x2(r - mid, 0.f), 0u, 0u);
+            };
+            int u = 0;
+            bool ok = true;
+            for (int n = 0, id; ok && (id = get_item(n)) >= 0; ++n) {
+                for (int it = item_units(id); it > 0; --it, ++u) {
+                    const int s = u % NST;
+                    ok = mbar_wait_warp(&bar_full[s], uint32_t(u / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+                    if (!ok) break;
+                    uint4* op_l = reinterpret_cast<uint4*>(sOps + 2 * s * Cfg::kOpBytes);
+                    uint4* op_d = op_l + 128;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int r = i * 32 + lane;
+                        // padding rows have L = inf: a large finite number keeps the split free of NaN, and P is 0 just the same
+                        op_l[r] = split(fmaxf(sLse[s * 128 + r] * to_scores, -1.7014118e38f));
+                        op_d[r] = split(-sDv[s * 128 + r]);
+                    }
+                    fence_proxy_async_smem();  // ordinary accesses before the products' reads and the next loads' writes
+                    mbar_arrive(&bar_vec[s]);
+                }
+            }
+        }
+    } else if (warp == kMmaSWarp || warp == kMmaWarp) {
+        // ------------------------------------------------------------------ MMA issuers (whole warps, one lane issues)
+        // Two warps share the products: the first issues S^T, the second dV, dK and, into the block whose operands these have
+        // read, dP^T of the unit kDpBufs ahead.  (Between two products a warp spends 100 clocks on every wait and every commit.)
+        reg_dealloc<Cfg::kRegsOther>();
         constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
         constexpr uint32_t idesc_acc = make_idesc_bf16(128, D, 0, 1);
-        // This CTA's units are numbered u = 0, 1, ... across all its items: ring stage u % NST, S buffer u & 1
-        // (two S buffers).  Three cursors walk that sequence: S^T = K Q^T runs two units ahead (one with a
-        // single S buffer) and dP^T = V dO^T one unit ahead of the products into the accumulators.
+        // This CTA's units are numbered u = 0, 1, ... across all its items: ring stage u % NST, dP block u % NDP.
         struct Cursor {
             int n, it, n_it, u;  // items before this one on this CTA, unit in item, units of item (0: list ended), unit number
         };
         bool ok = true;
-        // `wait`: the first cursor to reach an item waits for its id; the others find it in the ring
-        auto cursor_start = [&](bool wait) {
-            const int id = wait ? get_item(0) : item_ring[0];
+        auto cursor_start = [&]() {
+            const int id = get_item(0);
             return Cursor{0, 0, id >= 0 ? item_units(id) : 0, 0};
         };
-        auto cursor_next = [&](Cursor& c, bool wait) {
+        auto cursor_next = [&](Cursor& c) {
             ++c.u;
             if (++c.it == c.n_it) {
                 ++c.n;
                 c.it = 0;
-                const int id = wait ? get_item(c.n) : item_ring[c.n % kItemRing];
+                const int id = get_item(c.n);
                 c.n_it = id >= 0 ? item_units(id) : 0;
             }
         };
-        auto issue_s = [&](const Cursor& c) {  // S^T(u) = K Q^T
+        // Q, dO and the row vectors of the unit (and K and V of its item) have landed
+        auto wait_loaded = [&](const Cursor& c) {
             const int s = c.u % NST, kb = c.n % NKV;
-            // one S buffer: it still holds S^T of the unit before until the compute warps have read it into registers
-            if (!DBL && c.u > 0) ok = mbar_wait_warp(bar_s_loaded, uint32_t(c.u - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
-            if (ok && c.it == 0) ok = mbar_wait_warp(&bar_kv[kb], uint32_t(c.n / NKV) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
-            if (ok) ok = mbar_wait_warp(&bar_full[s], uint32_t(c.u / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
-            if (!ok) return;
+            if (c.it == 0) ok = mbar_wait_warp(&bar_kv[kb], uint32_t(c.n / NKV) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+            if (ok)
+                ok = mbar_wait_warp(Cfg::kVecOps ? &bar_vec[s] : &bar_full[s], uint32_t(c.u / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+        };
+        // One thread: D[tmem] = A B^T over the head dimension, plus the row vector `which` of stage s (0 L, 1 D; kVecOps).  After
+        // the item's last unit this warp's products read its K or V no more.
+        const uint64_t ones_desc = make_sdesc_plain(smem_u32(sOnes), uint32_t(sZero - sOnes), 128);
+        auto issue_block = [&](uint32_t d_tmem, const uint8_t* key_tile, const uint8_t* query_tile, const Cursor& c, int which, uint64_t* full) {
             tc_fence_after_sync();
-            const int buf = DBL ? (c.u & 1) : 0;
             if (elect_one()) {
-                issue_ss_over_headdim<D>(tmem + Cfg::col_s(buf), kmajor_desc<D>(sK + kb * Cfg::kTileBytes),
-                                         kmajor_desc<D>(sQ + s * Cfg::kTileBytes), idesc_s);
-                umma_commit(&bar_s_full[buf]);
+                issue_ss_over_headdim<D>(d_tmem, kmajor_desc<D>(key_tile), kmajor_desc<D>(query_tile), idesc_s);
+                if constexpr (Cfg::kVecOps) {
+                    const uint8_t* op = sOps + (2 * (c.u % NST) + which) * Cfg::kOpBytes;
+                    umma_ss(d_tmem, ones_desc, make_sdesc_plain(smem_u32(op), uint32_t(sZero - op), 128), idesc_s, 1);  // (second half of the K step: zeros)
+                }
+                umma_commit(full);
+                if (c.it + 1 == c.n_it) umma_commit(&bar_kv_free[c.n % NKV]);
             }
             __syncwarp();
         };
-        // dP^T(u) = V dO^T; the loads of the unit are known to be complete (S^T of the unit was issued before).
-        // After the item's last unit no MMA reads its K and V any more.
-        auto issue_dp = [&](const Cursor& c) {
-            const int s = c.u % NST, kb = c.n % NKV;
-            if (elect_one()) {
-                issue_ss_over_headdim<D>(tmem + Cfg::kColDP, kmajor_desc<D>(sV + kb * Cfg::kTileBytes),
-                                         kmajor_desc<D>(sdO + s * Cfg::kTileBytes), idesc_s);
-                umma_commit(bar_dp_full);
-                if (c.it + 1 == c.n_it) umma_commit(&bar_kv_free[kb]);
-            }
-            __syncwarp();
-        };
-        Cursor cs = cursor_start(true);
-        Cursor cd = cs, ca = cs;
-        if (cs.n_it > 0) {
-            issue_s(cs);
-            cursor_next(cs, true);
-            if (ok) {
-                issue_dp(cd);
-                cursor_next(cd, false);
-            }
-            if (ok && DBL && cs.n_it > 0) {
-                issue_s(cs);
-                cursor_next(cs, true);
-            }
-        }
-        int n_done = 0;  // items whose accumulators have been completed
-        while (ok && ca.n_it > 0) {
-            const int s = ca.u % NST;
-            const int buf = DBL ? (ca.u & 1) : 0;
-            // dP^T of the next unit as soon as the compute warps have read this one into registers
-            // (dS^T is written next to P^T inside the S buffer, so the dP block is free): the MMA round trip
-            // runs under their arithmetic.  (With a single S buffer, D = 128, the loads of the next unit
-            // may still be in flight: there dP^T follows S^T below instead.)
-            if (!DBL && cs.n_it > 0 && cs.it != 0) {
-                // one S buffer (D = 128): S^T of the next unit as soon as this unit's scores are in registers, so that
-                // it runs under this unit's exponentials.  (Not across an item boundary: the next item's K and V are
-                // only loaded once this item's last dP^T product has run; that S^T follows the products below.)
-                issue_s(cs);
-                cursor_next(cs, true);
+        if (warp == kMmaSWarp) {
+            for (Cursor c = cursor_start(); ok && c.n_it > 0; cursor_next(c)) {
+                wait_loaded(c);
+                // the buffer holds S^T of the unit before until the compute warps have read it into registers
+                if (ok && c.u > 0) ok = mbar_wait_warp(bar_s_loaded, uint32_t(c.u - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
                 if (!ok) break;
+                issue_block(tmem + Cfg::kColS, sK + (c.n % NKV) * Cfg::kTileBytes, sQ + (c.u % NST) * Cfg::kTileBytes, c, 0, bar_s_full);
             }
-            if (DBL && cd.n_it > 0) {
-                ok = mbar_wait_warp(bar_dp_free, uint32_t(ca.u) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
+        } else {
+            Cursor ca = cursor_start(), cd = ca;
+            auto next_dp = [&]() {
+                wait_loaded(cd);
+                if (!ok) return;
+                issue_block(tmem + Cfg::col_dp(cd.u % NDP), sV + (cd.n % NKV) * Cfg::kTileBytes, sdO + (cd.u % NST) * Cfg::kTileBytes, cd, 1,
+                            &bar_dp_full[cd.u & 1]);
+                cursor_next(cd);
+            };
+            for (int i = 0; i < NDP && ok && cd.n_it > 0; ++i) next_dp();
+            int n_done = 0;  // items whose accumulators have been completed
+            while (ok && ca.n_it > 0) {
+                const int s = ca.u % NST;
+                ok = mbar_wait_warp(&bar_pds_full[ca.u & 1], uint32_t(ca.u >> 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
+                // the accumulators belong to the previous item's epilogue until it has read them
+                if (ok && ca.it == 0 && ca.n > 0)
+                    ok = mbar_wait_warp(bar_acc_free, uint32_t(ca.n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
                 if (!ok) break;
+                B200ATTN_STAMP(lane == 0, 16 + 8 * ca.u + 4);
                 tc_fence_after_sync();
-                issue_dp(cd);
-                cursor_next(cd, false);
+                if (elect_one()) {
+                    // dV += P^T dO ; dK += dS^T Q   (P^T and dS^T sit side by side over the unit's dP block)
+                    const uint32_t a_pds = tmem + Cfg::col_dp(ca.u % NDP);
+                    issue_ts_over_rows<D>(tmem + Cfg::kColAcc0, a_pds, mnmajor_desc<D>(sdO + s * Cfg::kTileBytes), idesc_acc, ca.it > 0);
+                    issue_ts_over_rows<D>(tmem + Cfg::kColAcc1, a_pds + Cfg::kPartCols / 2, mnmajor_desc<D>(sQ + s * Cfg::kTileBytes),
+                                          idesc_acc, ca.it > 0);
+                    umma_commit(&bar_free[s]);
+                    if (ca.it + 1 == ca.n_it) umma_commit(bar_acc);
+                }
+                __syncwarp();
+                B200ATTN_STAMP(lane == 0, 16 + 8 * ca.u + 5);
+                if (ca.it + 1 == ca.n_it) ++n_done;
+                if (cd.n_it > 0) next_dp();  // overwrites this unit's P^T and dS^T: behind the two products just issued
+                cursor_next(ca);
             }
-            ok = mbar_wait_warp(&bar_pds_full[ca.u & 1], uint32_t(ca.u >> 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
-            if (!ok) break;
-            B200ATTN_STAMP(lane == 0, 16 + 8 * ca.u + 4);
-            // the accumulators belong to the previous item's epilogue until it has read them
-            if (ca.it == 0 && ca.n > 0) {
-                ok = mbar_wait_warp(bar_acc_free, uint32_t(ca.n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
-                if (!ok) break;
-            }
-            tc_fence_after_sync();
-            if (elect_one()) {
-                // dV += P^T dO ; dK += dS^T Q   (P^T and dS^T sit side by side: in S buffer `buf`, or, with one S
-                // buffer, over the dP block, which the compute warps have read by then)
-                const uint32_t a_pds = tmem + (DBL ? Cfg::col_s(buf) : Cfg::kColDP);
-                issue_ts_over_rows<D>(tmem + Cfg::kColAcc0, a_pds, mnmajor_desc<D>(sdO + s * Cfg::kTileBytes), idesc_acc, ca.it > 0);
-                issue_ts_over_rows<D>(tmem + Cfg::kColAcc1, a_pds + Cfg::kPartCols / 2, mnmajor_desc<D>(sQ + s * Cfg::kTileBytes),
-                                      idesc_acc, ca.it > 0);
-                umma_commit(&bar_free[s]);
-                if (ca.it + 1 == ca.n_it) umma_commit(bar_acc);
-            }
-            __syncwarp();
-            B200ATTN_STAMP(lane == 0, 16 + 8 * ca.u + 5);
-            if (ca.it + 1 == ca.n_it) ++n_done;
-            if (!DBL && cs.n_it > 0 && cs.u == ca.u + 1) {  // S^T of the next unit is still to come (item boundary)
-                issue_s(cs);
-                cursor_next(cs, true);
-                if (!ok) break;
-            }
-            if (!DBL && cd.n_it > 0) {
-                // dP^T of the next unit overwrites P^T and dS^T of this one: behind the two products just issued
-                issue_dp(cd);
-                cursor_next(cd, false);
-            }
-            if (DBL && cs.n_it > 0) {
-                issue_s(cs);
-                cursor_next(cs, true);
-            }
-            B200ATTN_STAMP(lane == 0, 16 + 8 * ca.u + 6);
-            cursor_next(ca, false);
+            // nothing may be in flight when TMEM is freed: the last commit covers every product issued here, and the other warp's
+            // were waited for by the compute warps
+            if (ok && n_done > 0) mbar_wait_warp(bar_acc, uint32_t(n_done - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
         }
-        // nothing may be in flight when TMEM is freed: the last commit covers every MMA issued above
-        if (ok && n_done > 0) mbar_wait_warp(bar_acc, uint32_t(n_done - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
     } else {
         // ------------------------------------------------------------------ compute
+        reg_alloc<Cfg::kRegsCompute>();
         const int w4 = warp & 3, part = warp >> 2;
         const int row = w4 * 32 + lane;  // key row in the tile == TMEM lane
         const uint32_t lane_base = uint32_t(w4 * 32) << 16;
-        const int c0 = part * Cfg::kPartCols;  // first query column of this thread's part
+        constexpr int NC = Cfg::kCols;
+        const int c0 = part * NC;  // first query column of this thread
         bool ok = true;
         // Epilogue of an item.  It is deferred until the first unit of the next item has been handed to the MMA
-        // warp, so that the wait for the item's last products overlaps that unit's arithmetic.
+        // warp, so that the wait for the item's last products overlaps that unit's arithmetic.  Parts 0, 1 write dV, parts 2, 3
+        // dK (times scale); each takes D / 2 columns of its key row, which are contiguous in global memory.
         auto epilogue = [&](int n_item, int id_item) -> bool {
-            // epilogue of the item: parts 0,1 write dV, parts 2,3 write dK (times scale); each part takes D / 2
-            // of the accumulator's columns of its key row, which is contiguous in global memory
             B200ATTN_STAMP(tid == 0, 460 + 4 * n_item + 0);
             ok = mbar_wait_warp(bar_acc, uint32_t(n_item) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
             if (!ok) return false;
@@ -1187,77 +1196,40 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             // compute them ahead of the unit loop and keep them in registers there)
             int part_e = part, id_e = id_item;
             asm volatile("" : "+r"(part_e), "+r"(id_e));
-            constexpr int kHalfParts = Cfg::kParts / 2;
-            constexpr int kColsPerPart = D / kHalfParts;
-            const bool is_dk = part_e >= kHalfParts;
+            constexpr int kCols = D / 2;
+            const bool is_dk = part_e >= 2;
             const uint32_t acc = is_dk ? Cfg::kColAcc1 : Cfg::kColAcc0;
             const float mul = is_dk ? p.scale : 1.f;
-            const int col0 = (part_e % kHalfParts) * kColsPerPart;
+            const int col0 = (part_e & 1) * kCols;
             const int k0 = item_kt(id_e) * 128;
-            if constexpr (Cfg::kOutTiles > 0) {
-                // through shared memory and a TMA store, so that no compute thread waits on the memory system:
-                // the previous item's store must have read the staging tiles before they are rewritten
-                // (mbarriers with bounded waits rather than bar.sync: a warp that has given up never arrives)
-                if (tid == 0) {
-                    tma_store_wait_read0();
-                    mbar_arrive(bar_out_free);
-                }
-                ok = mbar_wait_warp(bar_out_free, uint32_t(n_item) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
-                if (!ok) return false;
+            const bool in_range = k0 + row < p.T;
+            uint16_t* out = (is_dk ? p.dk : p.dv) + size_t(item_b(id_e)) * p.k_sb + size_t(item_hk(id_e)) * p.k_sh +
+                            size_t(k0 + row) * p.k_st + col0;
 #pragma unroll
-                for (int c = 0; c < kColsPerPart / 32; ++c) {
-                    uint32_t v[32];
-                    tmem_ld_x32(tmem + lane_base + acc + col0 + c * 32, v);
-                    tmem_wait_ld();
-                    if (c + 1 == kColsPerPart / 32) {
-                        tc_fence_before_sync();
-                        mbar_arrive(bar_acc_free);  // the MMA warp may start the next item's accumulation
-                    }
-                    stage_row_chunk<D>(sOut + (is_dk ? Cfg::kTileBytes : 0), row, col0 + c * 32, v, mul);
+            for (int c = 0; c < kCols / 32; ++c) {
+                uint32_t v[32];
+                tmem_ld_x32(tmem + lane_base + acc + col0 + c * 32, v);
+                tmem_wait_ld();
+                if (c + 1 == kCols / 32) {
+                    tc_fence_before_sync();
+                    mbar_arrive(bar_acc_free);  // the MMA warp may start the next item's accumulation
                 }
-                fence_proxy_async_smem();
-                mbar_arrive(bar_out_full);
-                if (warp == 0) {
-                    ok = mbar_wait_warp(bar_out_full, uint32_t(n_item) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
-                    if (!ok) return false;
-                }
-                if (tid == 0) {
+                if (in_range) {
 #pragma unroll
-                    for (int bx = 0; bx < Cfg::kBoxes; ++bx) {
-                        tma_store_4d(&tmdV, sOut + bx * Cfg::kBoxBytes, bx * 64, k0, item_hk(id_e), item_b(id_e));
-                        tma_store_4d(&tmdK, sOut + Cfg::kTileBytes + bx * Cfg::kBoxBytes, bx * 64, k0, item_hk(id_e), item_b(id_e));
-                    }
-                    tma_store_commit();
-                }
-            } else {
-                const bool in_range = k0 + row < p.T;
-                uint16_t* out = (is_dk ? p.dk : p.dv) + size_t(item_b(id_e)) * p.k_sb + size_t(item_hk(id_e)) * p.k_sh +
-                                size_t(k0 + row) * p.k_st + col0;
-#pragma unroll
-                for (int c = 0; c < kColsPerPart / 32; ++c) {
-                    uint32_t v[32];
-                    tmem_ld_x32(tmem + lane_base + acc + col0 + c * 32, v);
-                    tmem_wait_ld();
-                    if (c + 1 == kColsPerPart / 32) {
-                        tc_fence_before_sync();
-                        mbar_arrive(bar_acc_free);  // the MMA warp may start the next item's accumulation
-                    }
-                    if (in_range) {
-#pragma unroll
-                        for (int g = 0; g < 4; ++g) {
-                            uint4 w;
-                            w.x = pack_bf16x2(__uint_as_float(v[g * 8 + 0]) * mul, __uint_as_float(v[g * 8 + 1]) * mul);
-                            w.y = pack_bf16x2(__uint_as_float(v[g * 8 + 2]) * mul, __uint_as_float(v[g * 8 + 3]) * mul);
-                            w.z = pack_bf16x2(__uint_as_float(v[g * 8 + 4]) * mul, __uint_as_float(v[g * 8 + 5]) * mul);
-                            w.w = pack_bf16x2(__uint_as_float(v[g * 8 + 6]) * mul, __uint_as_float(v[g * 8 + 7]) * mul);
-                            *reinterpret_cast<uint4*>(out + c * 32 + g * 8) = w;
-                        }
+                    for (int g = 0; g < 4; ++g) {
+                        uint4 w;
+                        w.x = pack_bf16x2(__uint_as_float(v[g * 8 + 0]) * mul, __uint_as_float(v[g * 8 + 1]) * mul);
+                        w.y = pack_bf16x2(__uint_as_float(v[g * 8 + 2]) * mul, __uint_as_float(v[g * 8 + 3]) * mul);
+                        w.z = pack_bf16x2(__uint_as_float(v[g * 8 + 4]) * mul, __uint_as_float(v[g * 8 + 5]) * mul);
+                        w.w = pack_bf16x2(__uint_as_float(v[g * 8 + 6]) * mul, __uint_as_float(v[g * 8 + 7]) * mul);
+                        *reinterpret_cast<uint4*>(out + c * 32 + g * 8) = w;
                     }
                 }
             }
             B200ATTN_STAMP(tid == 0, 460 + 4 * n_item + 2);
             return true;
         };
+        const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2);
         bool pending = false;
         int pend_id = 0;
         int u = 0, n = 0;
@@ -1266,129 +1238,80 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             // units of the item: for each query head of the group, the query tiles from the diagonal down
             for (int it = p.group * n_i, i_in = 0; it > 0; --it, ++u, i_in = (i_in + 1 == n_i ? 0 : i_in + 1)) {
                 const int s = u % NST;
-                const int buf = DBL ? (u & 1) : 0;
-                const uint32_t s_par = DBL ? ((u >> 1) & 1) : (u & 1);
                 const bool diag = i_in == 0;
-                ok = mbar_wait_warp(&bar_s_full[buf], s_par, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+                ok = mbar_wait_warp(bar_s_full, uint32_t(u) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
                 if (!ok) break;
                 B200ATTN_STAMP(tid == 0, 16 + 8 * u + 0);
                 tc_fence_after_sync();
                 const float4* lse4 = reinterpret_cast<const float4*>(sLse + s * 128 + c0);
                 const float4* dv4 = reinterpret_cast<const float4*>(sDv + s * 128 + c0);
-                float pr[32];
-                if constexpr (DBL) {
-                // phase A: P^T from S^T (kept in registers and stored over S^T as BF16), 16 columns at a time
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    uint32_t sv[16], pk[8];
-                    tmem_ld_x16(tmem + lane_base + Cfg::col_s(buf) + c0 + hh * 16, sv);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int g = 0; g < 4; ++g) {
-                        const float4 l4 = lse4[hh * 4 + g];
-                        float* q = &pr[hh * 16 + g * 4];
-                        q[0] = ex2_approx(fmaf(__uint_as_float(sv[g * 4 + 0]), p.scale_log2, -l4.x));
-                        q[1] = ex2_approx(fmaf(__uint_as_float(sv[g * 4 + 1]), p.scale_log2, -l4.y));
-                        q[2] = ex2_approx(fmaf(__uint_as_float(sv[g * 4 + 2]), p.scale_log2, -l4.z));
-                        q[3] = ex2_approx(fmaf(__uint_as_float(sv[g * 4 + 3]), p.scale_log2, -l4.w));
-                    }
-                    if (diag) {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            if (c0 + hh * 16 + i < row) pr[hh * 16 + i] = 0.f;  // query above the key: masked
-                    }
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) pk[i] = pack_bf16x2(pr[hh * 16 + 2 * i], pr[hh * 16 + 2 * i + 1]);
-                    tmem_st_x8(tmem + lane_base + Cfg::col_s(buf) + c0 + hh * 8, pk);
-                }
-                } else {
-                // phase A with one S buffer: the scores leave tensor memory in one go and the buffer goes back to the
-                // MMA warp at once; P^T stays in registers until phase B
+                const uint32_t t_dp = tmem + lane_base + Cfg::col_dp(u % NDP) + c0;
+                // phase A: the scores leave tensor memory in one go and the buffer goes back to the MMA warp at once; P^T stays
+                // in registers until phase B
+                float pr[NC];
                 {
-                    uint32_t sv[32];
-                    tmem_ld_x16(tmem + lane_base + Cfg::kColS0 + c0, sv);
-                    tmem_ld_x16(tmem + lane_base + Cfg::kColS0 + c0 + 16, sv + 16);
+                    uint32_t sv[NC];
+                    tmem_ld_x32(tmem + lane_base + Cfg::kColS + c0, sv);
                     tmem_wait_ld();
                     tc_fence_before_sync();
                     mbar_arrive(bar_s_loaded);
 #pragma unroll
-                    for (int g = 0; g < 8; ++g) {
-                        const float4 l4 = lse4[g];
-                        float* q = &pr[g * 4];
-                        q[0] = ex2_approx(fmaf(__uint_as_float(sv[g * 4 + 0]), p.scale_log2, -l4.x));
-                        q[1] = ex2_approx(fmaf(__uint_as_float(sv[g * 4 + 1]), p.scale_log2, -l4.y));
-                        q[2] = ex2_approx(fmaf(__uint_as_float(sv[g * 4 + 2]), p.scale_log2, -l4.z));
-                        q[3] = ex2_approx(fmaf(__uint_as_float(sv[g * 4 + 3]), p.scale_log2, -l4.w));
+                    for (int i = 0; i < NC; i += 2) {
+                        uint64_t x = pack_f32x2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1]));
+                        float x0, x1;
+                        if constexpr (Cfg::kVecOps) {
+                            unpack_f32x2(mul_f32x2(x, scale2), x0, x1);
+                        } else {
+                            const float4 l4 = lse4[i / 4];
+                            unpack_f32x2(fma_f32x2(x, scale2, i % 4 ? pack_f32x2(-l4.z, -l4.w) : pack_f32x2(-l4.x, -l4.y)), x0, x1);
+                        }
+                        pr[i] = ex2_approx(x0);
+                        pr[i + 1] = ex2_approx(x1);
                     }
                 }
                 if (diag) {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i)
+                    for (int i = 0; i < NC; ++i)
                         if (c0 + i < row) pr[i] = 0.f;  // query above the key: masked
                 }
-                }
                 B200ATTN_STAMP(tid == 0, 16 + 8 * u + 1);
-                ok = mbar_wait_warp(bar_dp_full, uint32_t(u) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+                ok = mbar_wait_warp(&bar_dp_full[u & 1], uint32_t(u >> 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
                 if (!ok) break;
                 B200ATTN_STAMP(tid == 0, 16 + 8 * u + 2);
                 tc_fence_after_sync();
-                if constexpr (DBL) {
-                // phase B: dS^T = P^T (dP^T - D), stored as BF16 next to P^T in the S buffer
+                // phase B: 16 columns of dP^T at a time into registers, then P^T and dS^T = P^T (dP^T - D) as BF16 side by side
+                // over those columns (P^T in the first 8, dS^T in the second 8)
 #pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
+                for (int h = 0; h < NC / 16; ++h) {
                     uint32_t dp[16], pk[8];
-                    tmem_ld_x16(tmem + lane_base + Cfg::kColDP + c0 + hh * 16, dp);
-                    tmem_wait_ld();
-                    if (hh == 1) {
-                        tc_fence_before_sync();
-                        mbar_arrive(bar_dp_free);  // dP^T is in registers: the next product may overwrite the block
-                    }
-#pragma unroll
-                    for (int g = 0; g < 4; ++g) {
-                        const float4 d4 = dv4[hh * 4 + g];
-                        const float* q = &pr[hh * 16 + g * 4];
-                        pk[g * 2 + 0] = pack_bf16x2(q[0] * (__uint_as_float(dp[g * 4 + 0]) - d4.x),
-                                                    q[1] * (__uint_as_float(dp[g * 4 + 1]) - d4.y));
-                        pk[g * 2 + 1] = pack_bf16x2(q[2] * (__uint_as_float(dp[g * 4 + 2]) - d4.z),
-                                                    q[3] * (__uint_as_float(dp[g * 4 + 3]) - d4.w));
-                    }
-                    tmem_st_x8(tmem + lane_base + Cfg::col_s(buf) + c0 + Cfg::kPartCols / 2 + hh * 8, pk);
-                }
-                } else {
-                // phase B with one S buffer: all of this thread's dP^T into registers, then P^T and dS^T as BF16 side by
-                // side over the part's own 32 columns of the dP block (P^T in the first 16, dS^T in the second 16)
-                {
-                    uint32_t dp[32], pp[16], pd[16];
-                    const uint32_t t_dp = tmem + lane_base + Cfg::kColDP + c0;
-                    tmem_ld_x16(t_dp, dp);
-                    tmem_ld_x16(t_dp + 16, dp + 16);
+                    tmem_ld_x16(t_dp + h * 16, dp);
                     tmem_wait_ld();
 #pragma unroll
-                    for (int g = 0; g < 8; ++g) {
-                        const float4 d4 = dv4[g];
-                        const float* q = &pr[g * 4];
-                        pp[g * 2 + 0] = pack_bf16x2(q[0], q[1]);
-                        pp[g * 2 + 1] = pack_bf16x2(q[2], q[3]);
-                        pd[g * 2 + 0] = pack_bf16x2(q[0] * (__uint_as_float(dp[g * 4 + 0]) - d4.x),
-                                                    q[1] * (__uint_as_float(dp[g * 4 + 1]) - d4.y));
-                        pd[g * 2 + 1] = pack_bf16x2(q[2] * (__uint_as_float(dp[g * 4 + 2]) - d4.z),
-                                                    q[3] * (__uint_as_float(dp[g * 4 + 3]) - d4.w));
+                    for (int i = 0; i < 16; i += 2) {
+                        uint64_t d = pack_f32x2(__uint_as_float(dp[i]), __uint_as_float(dp[i + 1]));
+                        if constexpr (!Cfg::kVecOps) {
+                            const float4 d4 = dv4[h * 4 + i / 4];
+                            d = add_f32x2(d, i % 4 ? pack_f32x2(-d4.z, -d4.w) : pack_f32x2(-d4.x, -d4.y));
+                        }
+                        float y0, y1;
+                        unpack_f32x2(mul_f32x2(pack_f32x2(pr[h * 16 + i], pr[h * 16 + i + 1]), d), y0, y1);
+                        pk[i / 2] = pack_bf16x2(y0, y1);
                     }
-                    tmem_st_x16(t_dp, pp);
-                    tmem_st_x16(t_dp + 16, pd);
-                }
+                    tmem_st_x8(t_dp + h * 16 + 8, pk);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) pk[i] = pack_bf16x2(pr[h * 16 + 2 * i], pr[h * 16 + 2 * i + 1]);
+                    tmem_st_x8(t_dp + h * 16, pk);
                 }
                 tmem_wait_st();
                 tc_fence_before_sync();
-                // the unit's two row vectors were read from shared memory with ordinary loads; the stage goes back
-                // to TMA (async proxy) through the products this arrival lets go
-                fence_proxy_async_smem();
+                // the unit's row vectors were read from shared memory with ordinary loads; the stage goes back to TMA (async
+                // proxy) through the products this arrival lets go
+                if constexpr (!Cfg::kVecOps) fence_proxy_async_smem();
                 mbar_arrive(&bar_pds_full[u & 1]);
                 B200ATTN_STAMP(tid == 0, 16 + 8 * u + 3);
                 if (pending) {  // first unit of this item: now the previous item's epilogue
                     pending = false;
-                    ok = epilogue(n - 1, pend_id);
-                    if (!ok) break;
+                    if (!epilogue(n - 1, pend_id)) break;
                 }
             }
             if (!ok) break;
@@ -1396,13 +1319,11 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             pend_id = id;
         }
         if (ok && pending) epilogue(n - 1, pend_id);
-        // the staging tiles must outlive the last store's reads
-        if (Cfg::kOutTiles > 0 && tid == 0) tma_store_wait_read0();
     }
 
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == kMmaWarp) {
+    if (warp == kMmaSWarp) {
         tc_fence_after_sync();
         tmem_dealloc(tmem, Cfg::kTmemCols);
     }

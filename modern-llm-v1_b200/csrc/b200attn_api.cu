@@ -417,7 +417,7 @@ int launch_bwd_onepass(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
 template <int D>
 int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk64, const CUtensorMap& tv64, const CUtensorMap& tk,
                const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& to, const CUtensorMap& tdq,
-               const CUtensorMap& tdk, const CUtensorMap& tdv, const BwdParams& p, cudaStream_t st) {
+               const BwdParams& p, cudaStream_t st) {
     static bool dq_set[kMaxDevices] = {false}, dkdv_set[kMaxDevices] = {false};
     // D = 64: 64-key tiles, two CTAs per SM.  D = 128: 128-key tiles, one CTA per SM (tensor-pipe bound).
     constexpr bool kWide = (D == 128);
@@ -452,7 +452,7 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk64, const CUtensorMap
     BwdParams pk = p;
     pk.sched2 = next_sched_pair(kv_items, kv_grid);
     if (launch_pdl(attn_bwd_dkdv_kernel<D>, kv_grid, BwdCfg<D>::kThreads, BwdCfg<D>::kSmemBytes, st, tk, tv, tq, tdo,
-                   tdk, tdv, pk) != cudaSuccess) {
+                   pk) != cudaSuccess) {
         cudaGetLastError();
         return B200ATTN_ERR_CUDA;
     }
@@ -714,7 +714,7 @@ extern "C" int b200attn_bwd_mode(const void* q, const void* k, const void* v, co
     int* status = status_ptr(&rc);
     if (!status) return rc;
     const Strides sq = strides_for(layout, Hq, T, D), sk = strides_for(layout, Hkv, T, D);
-    CUtensorMap tq, tk, tv, tk64, tv64, tdo, to, tdq, tdk, tdv;
+    CUtensorMap tq, tk, tv, tk64, tv64, tdo, to, tdq;
     if (!make_tmap_bf16_4d(&tq, q, D, T, Hq, B, sq.t, sq.h, sq.b, 128) ||
         !make_tmap_bf16_4d(&tk, k, D, T, Hkv, B, sk.t, sk.h, sk.b, 128) ||
         !make_tmap_bf16_4d(&tv, v, D, T, Hkv, B, sk.t, sk.h, sk.b, 128) ||
@@ -722,9 +722,7 @@ extern "C" int b200attn_bwd_mode(const void* q, const void* k, const void* v, co
         !make_tmap_bf16_4d(&tv64, v, D, T, Hkv, B, sk.t, sk.h, sk.b, 64) ||
         !make_tmap_bf16_4d(&tdo, dout, D, T, Hq, B, sq.t, sq.h, sq.b, 128) ||
         !make_tmap_bf16_4d(&to, o, D, T, Hq, B, sq.t, sq.h, sq.b, 128) ||
-        !make_tmap_bf16_4d(&tdq, dq, D, T, Hq, B, sq.t, sq.h, sq.b, 128) ||
-        !make_tmap_bf16_4d(&tdk, dk, D, T, Hkv, B, sk.t, sk.h, sk.b, 128) ||
-        !make_tmap_bf16_4d(&tdv, dv, D, T, Hkv, B, sk.t, sk.h, sk.b, 128))
+        !make_tmap_bf16_4d(&tdq, dq, D, T, Hq, B, sq.t, sq.h, sq.b, 128))
         return B200ATTN_ERR_TENSOR_MAP;
     float* ws = static_cast<float*>(workspace);
     const size_t nvec = bwd_vec_elems(B, T, Hq);
@@ -767,8 +765,8 @@ extern "C" int b200attn_bwd_mode(const void* q, const void* k, const void* v, co
         float* dq_acc = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + bwd_vec_bytes_padded(B, T, Hq));
         return launch_bwd_onepass(tq, tk, tv, tdo, p, dq_acc, st);
     }
-    return D == 64 ? launch_bwd<64>(tq, tk64, tv64, tk, tv, tdo, to, tdq, tdk, tdv, p, st)
-                   : launch_bwd<128>(tq, tk64, tv64, tk, tv, tdo, to, tdq, tdk, tdv, p, st);
+    return D == 64 ? launch_bwd<64>(tq, tk64, tv64, tk, tv, tdo, to, tdq, p, st)
+                   : launch_bwd<128>(tq, tk64, tv64, tk, tv, tdo, to, tdq, p, st);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -185,6 +185,12 @@ __device__ __forceinline__ uint64_t make_sdesc_sw128(uint32_t smem_addr, uint32_
     return d;
 }
 
+// The same without a swizzle, K-major: the operand is made of 8-row x 16-byte core matrices (128 bytes each, rows 16 bytes
+// apart); lbo = stride between core matrices along K, sbo = stride between 8-row groups.
+__device__ __forceinline__ uint64_t make_sdesc_plain(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+    return make_sdesc_sw128(smem_addr, lbo_bytes, sbo_bytes) & ~(uint64_t(7) << 61);
+}
+
 // Programmatic dependent launch: a kernel launched with the programmatic-stream-serialization
 // attribute may become resident while the previous kernel of the stream is still draining.
 // grid_dep_launch() lets the NEXT kernel start its own set-up early; grid_dep_wait() blocks
