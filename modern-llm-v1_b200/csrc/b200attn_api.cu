@@ -467,7 +467,8 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk64, const CUtensorMap
 // ---------------------------------------------------------------------------------------
 namespace {
 
-constexpr int kRopeNormMaxCtasPerSm = 8;  // 2048 threads per SM / 256
+constexpr int kRopeNormMaxCtasPerSm = 8;  // of the backward, as far as its workspace goes
+static_assert(kRopeNormBwdBlocks <= kRopeNormMaxCtasPerSm, "a partial sum per CTA");
 
 int rope_norm_check(int B, int T, int H, int D, int x_dtype, int x_layout, int y_layout) {
     if (B <= 0 || T <= 0 || H <= 0 || D <= 0) return B200ATTN_ERR_INVALID_ARG;
@@ -479,49 +480,43 @@ int rope_norm_check(int B, int T, int H, int D, int x_dtype, int x_layout, int y
     return B200ATTN_OK;
 }
 
-// grid: as many CTAs as the device keeps resident at once (asked of the runtime once per kernel and device), never
-// more than the rows need
-template <typename K>
-unsigned rope_norm_grid(K kernel, long long rows, int rows_per_cta_iter, int* cached_occ, int dyn_smem = 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= kMaxDevices) dev = 0;
-    if (cached_occ[dev] == 0) {
-        int occ = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kRopeNormThreads, dyn_smem) != cudaSuccess || occ <= 0) {
-            cudaGetLastError();
-            occ = 1;
-        }
-        cached_occ[dev] = occ;
+// Heads per item: eight of them share a token's cosines and sines and addresses, fewer when that leaves less than four items
+// for a resident warp (one eighth of a wave is then the most that the last round can waste).
+void rope_norm_plan(RopeNormParams* p, int n_tensors, int D, unsigned warps) {
+    int chunk = 8;
+    auto items = [&](const RopeNormParams& q) { return (long long)((q.n_tokens + 256u / D - 1) / (256u / D)) * ((q.H + chunk - 1) / chunk); };
+    auto all = [&] { return items(p[0]) + (n_tensors > 1 ? items(p[1]) : 0); };
+    while (chunk > 1 && all() < (chunk > 4 ? 4LL : 1LL) * warps) chunk /= 2;
+    for (int i = 0; i < n_tensors; ++i) {
+        p[i].chunk = chunk;
+        p[i].n_items = (unsigned)items(p[i]);
+        p[i].div_chunks = fastdiv_make((unsigned)((p[i].H + chunk - 1) / chunk));
     }
-    const long long need = (rows + rows_per_cta_iter - 1) / rows_per_cta_iter;
-    const long long cap = (long long)cached_occ[dev] * sm_count();
-    return (unsigned)std::max<long long>(1, std::min(need, cap));
+}
+
+// CTAs that the device keeps resident at once, never more than the items need
+inline unsigned rope_norm_grid(const RopeNormParams* p, int n_tensors, int blocks) {
+    const long long items = (long long)p[0].n_items + (n_tensors > 1 ? p[1].n_items : 0);
+    const long long need = (items + kRopeNormThreads / 32 - 1) / (kRopeNormThreads / 32);
+    return (unsigned)std::min<long long>(need, (long long)blocks * sm_count());
 }
 
 template <int D, bool F32>
-void rope_norm_launch_fwd(const RopeNormParams& p0, const RopeNormParams& p1, int n_tensors, long long rows,
-                          cudaStream_t st) {
-    static int occ[kMaxDevices] = {0};
-    const unsigned grid = rope_norm_grid(rope_norm_fwd_kernel<D, F32>, rows, (kRopeNormThreads / 32) * kFwdSteps * (256 / D), occ);
-    launch_pdl(rope_norm_fwd_kernel<D, F32>, dim3(grid, 1, 1), kRopeNormThreads, 0, st, p0, p1, n_tensors);
+void rope_norm_launch_fwd(RopeNormParams* p, int n_tensors, cudaStream_t st) {
+    rope_norm_plan(p, n_tensors, D, (unsigned)(kRopeNormFwdBlocks * (kRopeNormThreads / 32) * sm_count()));
+    launch_pdl(rope_norm_fwd_kernel<D, F32>, dim3(rope_norm_grid(p, n_tensors, kRopeNormFwdBlocks)), kRopeNormThreads, 0, st, p[0], p[1], n_tensors);
 }
 template <int D, bool F32>
-void rope_norm_launch_bwd(RopeNormParams p0, RopeNormParams p1, int n_tensors, long long rows, float* workspace,
-                          cudaStream_t st) {
-    static int occ[kMaxDevices] = {0};
-    static bool smem_set[kMaxDevices] = {false};
-    constexpr int kSmem = kRopeNormBwdSmemBytes<F32>;
-    if (set_smem_once(rope_norm_bwd_kernel<D, F32>, kSmem, smem_set) != B200ATTN_OK) return;
-    unsigned grid = rope_norm_grid(rope_norm_bwd_kernel<D, F32>, rows, (kRopeNormThreads / 32) * kBwdSteps * (256 / D), occ, kSmem);
-    grid = std::min(grid, (unsigned)(kRopeNormMaxCtasPerSm * sm_count()));  // the workspace holds that many partial sums
-    p0.partial = workspace;
-    p1.partial = workspace + (size_t)kRopeNormMaxCtasPerSm * sm_count() * D;
-    launch_pdl(rope_norm_bwd_kernel<D, F32>, dim3(grid, 1, 1), kRopeNormThreads, kSmem, st, p0, p1, n_tensors);
-    const float* part0 = p0.partial;
-    const float* part1 = p1.partial;
-    launch_pdl(rope_norm_dgamma_kernel<D>, dim3(n_tensors * D, 1, 1), 32, 0, st, part0, p0.d_gamma, part1, p1.d_gamma,
-               (int)grid);
+void rope_norm_launch_bwd(RopeNormParams* p, int n_tensors, float* workspace, cudaStream_t st) {
+    rope_norm_plan(p, n_tensors, D, (unsigned)(kRopeNormBwdBlocks * (kRopeNormThreads / 32) * sm_count()));
+    const unsigned grid = rope_norm_grid(p, n_tensors, kRopeNormBwdBlocks);
+    p[0].partial = workspace;
+    p[1].partial = workspace + (size_t)kRopeNormMaxCtasPerSm * sm_count() * D;
+    launch_pdl(rope_norm_bwd_kernel<D, F32>, dim3(grid), kRopeNormThreads, 0, st, p[0], p[1], n_tensors);
+    const float* part0 = p[0].partial;
+    const float* part1 = p[1].partial;
+    launch_pdl(rope_norm_dgamma_kernel<D>, dim3(n_tensors * (D / 8)), kDgammaThreads, 0, st, part0, p[0].d_gamma, part1,
+               p[1].d_gamma, (int)grid);
 }
 
 void rope_norm_fill(RopeNormParams& p, int B, int T, int H, int D, int x_layout, int y_layout) {
@@ -529,9 +524,9 @@ void rope_norm_fill(RopeNormParams& p, int B, int T, int H, int D, int x_layout,
     p.B = B;
     p.T = T;
     p.H = H;
+    p.n_tokens = (unsigned)B * (unsigned)T;
     p.x_st = sx.t, p.x_sh = sx.h, p.x_sb = sx.b;
     p.y_st = sy.t, p.y_sh = sy.h, p.y_sb = sy.b;
-    p.div_h = fastdiv_make((unsigned)H);
     p.div_t = fastdiv_make((unsigned)T);
 }
 
@@ -549,7 +544,6 @@ int rope_norm_run(bool backward, const RopeNormTensor* t, int n_tensors, int x_d
                   const float* cos_t, const float* sin_t, int B, int T, int D, float eps, void* workspace,
                   size_t workspace_bytes, void* stream) {
     RopeNormParams p[2] = {};
-    long long rows = 0;
     for (int i = 0; i < n_tensors; ++i) {
         int rc = rope_norm_check(B, T, t[i].H, D, x_dtype, x_layout, y_layout);
         if (rc) return rc;
@@ -557,8 +551,6 @@ int rope_norm_run(bool backward, const RopeNormTensor* t, int n_tensors, int x_d
             return B200ATTN_ERR_INVALID_ARG;
         if (!aligned16(t[i].x) || !aligned16(t[i].y) || (backward && !aligned16(t[i].dy))) return B200ATTN_ERR_ALIGNMENT;
         rope_norm_fill(p[i], B, T, t[i].H, D, x_layout, y_layout);
-        // rows are walked in the order of the tensor that is written (y forward, d_x backward): dense stores
-        p[i].walk_bthd = (backward ? x_layout : y_layout) == B200ATTN_LAYOUT_BTHD;
         p[i].x = t[i].x;
         p[i].y = t[i].y;
         p[i].dy = static_cast<const uint16_t*>(t[i].dy);
@@ -568,7 +560,6 @@ int rope_norm_run(bool backward, const RopeNormTensor* t, int n_tensors, int x_d
         p[i].cos_t = cos_t;
         p[i].sin_t = sin_t;
         p[i].eps = eps;
-        rows = std::max(rows, (long long)B * T * t[i].H);
     }
     if (!cos_t || !sin_t) return B200ATTN_ERR_INVALID_ARG;
     if (backward && (!workspace || workspace_bytes < b200attn_rope_norm_bwd_workspace_bytes(D) ||
@@ -579,19 +570,19 @@ int rope_norm_run(bool backward, const RopeNormTensor* t, int n_tensors, int x_d
     float* ws = static_cast<float*>(workspace);
     if (!backward) {
         if (D == 64) {
-            if (f32) rope_norm_launch_fwd<64, true>(p[0], p[1], n_tensors, rows, st);
-            else rope_norm_launch_fwd<64, false>(p[0], p[1], n_tensors, rows, st);
+            if (f32) rope_norm_launch_fwd<64, true>(p, n_tensors, st);
+            else rope_norm_launch_fwd<64, false>(p, n_tensors, st);
         } else {
-            if (f32) rope_norm_launch_fwd<128, true>(p[0], p[1], n_tensors, rows, st);
-            else rope_norm_launch_fwd<128, false>(p[0], p[1], n_tensors, rows, st);
+            if (f32) rope_norm_launch_fwd<128, true>(p, n_tensors, st);
+            else rope_norm_launch_fwd<128, false>(p, n_tensors, st);
         }
     } else {
         if (D == 64) {
-            if (f32) rope_norm_launch_bwd<64, true>(p[0], p[1], n_tensors, rows, ws, st);
-            else rope_norm_launch_bwd<64, false>(p[0], p[1], n_tensors, rows, ws, st);
+            if (f32) rope_norm_launch_bwd<64, true>(p, n_tensors, ws, st);
+            else rope_norm_launch_bwd<64, false>(p, n_tensors, ws, st);
         } else {
-            if (f32) rope_norm_launch_bwd<128, true>(p[0], p[1], n_tensors, rows, ws, st);
-            else rope_norm_launch_bwd<128, false>(p[0], p[1], n_tensors, rows, ws, st);
+            if (f32) rope_norm_launch_bwd<128, true>(p, n_tensors, ws, st);
+            else rope_norm_launch_bwd<128, false>(p, n_tensors, ws, st);
         }
     }
     if (cudaGetLastError() != cudaSuccess) return B200ATTN_ERR_CUDA;

@@ -15,10 +15,15 @@
 //   dx[2i]  = dr[2i] cos + dr[2i+1] sin                     dx[2i+1] = -dr[2i] sin + dr[2i+1] cos
 //   d_gamma[d] += sum over rows of dy[d] r[d] rstd
 //
-// The work is bound by HBM bandwidth (one read and one write of the tensor), so the kernels are built for
-// coalescing and for bytes in flight: a lane owns 8 consecutive elements of a row (one 16-byte access for BF16,
-// two for FP32), so a row takes D / 8 lanes and a warp covers 32 / (D / 8) rows per access; kStepsPerIter
-// such accesses are issued before the first use, and the grid is a multiple of the SM count.
+// The work is bound by HBM bandwidth (one read and one write of the tensors).  A lane owns 8 consecutive elements of a row
+// (16-byte accesses), so a row takes D / 8 lanes and a warp works on 32 / (D / 8) consecutive tokens at a time.  A warp's
+// item is such a group of tokens and a chunk of heads: the cosines and sines of its tokens are loaded once and stay in
+// registers for all heads of the chunk, and so do the token's addresses.  (Loaded per row they were as many bytes through
+// L2 as x and y together, and the row's decoding as many instructions as its arithmetic.)  kUnroll rows are loaded
+// before the first is used; together with 24 warps per SM that is enough in flight.
+// Measured on B200 against rows walked one by one with staged loads, q and k together: FP32 B=16 T=1024 16/4 D=128
+// 69.6 -> 42.4 us forward (5.97 TB/s), 92.7 -> 72.6 us backward (5.80 TB/s); BF16 B=4 T=8192 16/4 D=128 82.8 -> 65.0 and
+// 107.8 -> 97.3; BF16 B=32 T=512 6/2 D=64 11.0 -> 9.6 and 16.7 -> 16.5, of which some 4 us each are launch and latency.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -39,23 +44,17 @@ struct RopeNormParams {
     float* partial;      // backward: [gridDim.x, D] partial d_gamma sums
     float* d_gamma;      // backward: [D], accumulated into by rope_norm_dgamma_kernel
     int B, T, H;
-    FastDiv div_h, div_t;  // division by H and by T as multiply + shift
-    int walk_bthd;       // rows are walked in [B, T, H] order (else [B, H, T]): the order of the tensor that is WRITTEN
-                         // (y in the forward, d_x in the backward), so that all stores are dense
+    unsigned n_tokens;   // B * T
+    unsigned n_items;    // groups of tokens x chunks of heads
+    int chunk;           // heads per item
+    FastDiv div_t, div_chunks;  // division by T and by the number of chunks
     long long x_st, x_sh, x_sb;  // element strides of x (and of d_x): token, head, batch
     long long y_st, y_sh, y_sb;  // element strides of y (and of dy)
     float eps;
 };
 
 constexpr int kRopeNormThreads = 256;  // 8 warps
-#ifndef RN_FWD_STEPS
-#define RN_FWD_STEPS 1
-#define RN_FWD_BLOCKS 4
-#define RN_BWD_STEPS 1
-#define RN_BWD_BLOCKS 3
-#endif
-constexpr int kFwdSteps = RN_FWD_STEPS;  // row groups per loop iteration (all their loads are issued first)
-constexpr int kBwdSteps = RN_BWD_STEPS;
+constexpr int kRopeNormFwdBlocks = 3, kRopeNormBwdBlocks = 3;  // CTAs per SM that the register budgets are made for
 
 __device__ __forceinline__ float rn_bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float rn_bf16_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
@@ -75,21 +74,6 @@ __device__ __forceinline__ float rn_row_sum(float v) {
 #pragma unroll
     for (int o = LPR / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
-}
-
-// Row r of the walk -> (batch, token, head)
-__device__ __forceinline__ void rn_decode_row(const RopeNormParams& p, unsigned r, int& b, int& t, int& h) {
-    if (p.walk_bthd) {
-        const unsigned bt = fastdiv(r, p.div_h);
-        h = int(r - bt * unsigned(p.H));
-        b = int(fastdiv(bt, p.div_t));
-        t = int(bt - unsigned(b) * unsigned(p.T));
-    } else {
-        const unsigned bh = fastdiv(r, p.div_t);
-        t = int(r - bh * unsigned(p.T));
-        b = int(fastdiv(bh, p.div_h));
-        h = int(bh - unsigned(b) * unsigned(p.H));
-    }
 }
 
 // 8 consecutive elements starting at element offset `off`
@@ -142,236 +126,171 @@ __device__ __forceinline__ void rn_scale8(const float (&rot)[8], float rstd, con
     for (int e = 0; e < 8; ++e) out[e] = rot[e] * rstd * gm[e];
 }
 
-// 16-byte asynchronous copy global -> shared (LDGSTS): the data does not pass through registers, so a lane can keep
-// several iterations' worth of loads in flight at no register cost.
-__device__ __forceinline__ void rn_cp_async16(void* smem_dst, const void* gsrc) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void rn_cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void rn_cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// iterations in flight per lane in the forward (their loads are staged in shared memory: 48 KB per CTA either way)
+// 8 elements as they lie in memory, and as numbers
 template <bool F32>
-constexpr int kFwdDepth = F32 ? 3 : 4;
-
-// Shared memory of one forward stage: per thread 16 bytes each of cos and sin and 16 (BF16 x) or 32 (FP32 x) bytes
-// of x, laid out [piece][thread] so that a warp's accesses are contiguous.
-template <bool F32>
-struct RnFwdStage {
-    uint4 cs[kRopeNormThreads], sn[kRopeNormThreads], x0[kRopeNormThreads], x1[kRopeNormThreads];
-};
-template <>
-struct RnFwdStage<false> {
-    uint4 cs[kRopeNormThreads], sn[kRopeNormThreads], x0[kRopeNormThreads];
+struct RnRaw {
+    uint4 w[F32 ? 2 : 1];
+    __device__ __forceinline__ void load(const void* base, long long off) {
+        const uint4* ptr = F32 ? reinterpret_cast<const uint4*>(static_cast<const float*>(base) + off)
+                               : reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(base) + off);
+        w[0] = __ldcs(ptr);
+        if (F32) w[F32 ? 1 : 0] = __ldcs(ptr + 1);
+    }
+    __device__ __forceinline__ void clear() { w[0] = w[F32 ? 1 : 0] = make_uint4(0u, 0u, 0u, 0u); }
+    __device__ __forceinline__ void get(float (&v)[8]) const {
+        if (F32) {
+            const uint4 a = w[0], c = w[F32 ? 1 : 0];
+            v[0] = __uint_as_float(a.x), v[1] = __uint_as_float(a.y), v[2] = __uint_as_float(a.z), v[3] = __uint_as_float(a.w);
+            v[4] = __uint_as_float(c.x), v[5] = __uint_as_float(c.y), v[6] = __uint_as_float(c.z), v[7] = __uint_as_float(c.w);
+        } else {
+            const uint4 a = w[0];
+            v[0] = rn_bf16_lo(a.x), v[1] = rn_bf16_hi(a.x), v[2] = rn_bf16_lo(a.y), v[3] = rn_bf16_hi(a.y);
+            v[4] = rn_bf16_lo(a.z), v[5] = rn_bf16_hi(a.z), v[6] = rn_bf16_lo(a.w), v[7] = rn_bf16_hi(a.w);
+        }
+    }
 };
 
-// One tensor's forward.  (A function of its own, called once per tensor with the kernel parameter itself, so that
-// every field stays a constant-bank operand; selecting the struct at run time would move it to local memory.)
-// A lane works on one row piece per iteration; the loads of the next few iterations (x, cos, sin) are
-// already on their way into this lane's own slots of the stage ring, so no barrier is needed: a lane only ever
-// reads what it has copied itself, after cp.async.wait_group.
+// A warp's item: D / 8 lanes per token; lane's token, and the heads [h0, h1) that are the item's
+template <int D>
+struct RnItem {
+    bool live;  // the lane has a token
+    int b, t, h0, h1;
+    __device__ __forceinline__ RnItem(const RopeNormParams& p, unsigned item, int sub) {
+        const unsigned group = fastdiv(item, p.div_chunks);
+        h0 = int(item - group * p.div_chunks.d) * p.chunk;
+        h1 = min(h0 + p.chunk, p.H);
+        unsigned token = group * (256u / D) + unsigned(sub);
+        live = token < p.n_tokens;
+        if (!live) token = 0;
+        b = int(fastdiv(token, p.div_t));
+        t = int(token - unsigned(b) * unsigned(p.T));
+    }
+};
+
+// One tensor's forward: the items `item`, item + n_warps, ... of this warp; returns how far the last step went beyond the
+// tensor's items, which is where the warp begins in the next tensor.  (A function of its own, called once per tensor with
+// the kernel parameter itself, so that every field stays a constant-bank operand; selecting the struct at run time would
+// move it to local memory.)
 template <int D, bool F32>
-__device__ __forceinline__ void rope_norm_fwd_tensor(const RopeNormParams& p, RnFwdStage<F32>* ring) {
-    constexpr int LPR = D / 8;      // lanes per row
-    constexpr int RPS = 32 / LPR;   // rows per warp and iteration
+__device__ __forceinline__ unsigned rope_norm_fwd_tensor(const RopeNormParams& p, unsigned item, unsigned n_warps) {
+    constexpr int LPR = D / 8;  // lanes per row
+    constexpr int kUnroll = 4;
     const int lane = threadIdx.x & 31;
-    const int sub = lane / LPR, li = lane % LPR;  // row within the iteration, position within the row
-    const unsigned warp0 = (blockIdx.x * kRopeNormThreads + threadIdx.x) >> 5;
-    const unsigned n_warps = (gridDim.x * kRopeNormThreads) >> 5;
-    const unsigned n_rows = unsigned(p.B) * unsigned(p.T) * unsigned(p.H);
+    const int sub = lane / LPR, li = lane % LPR;  // token within the group, position within the row
     float gm[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) gm[e] = p.gamma[li * 8 + e];
-    const unsigned long long stride = static_cast<unsigned long long>(n_warps) * RPS;
-    const unsigned long long first = static_cast<unsigned long long>(warp0) * RPS + sub;
-
-    // requests the loads of this lane's iteration `it` (row first + it * stride) into ring slot it % depth
-    auto request = [&](unsigned it) {
-        const unsigned long long r = first + it * stride;
-        if (r < n_rows) {
-            int b, t, h;
-            rn_decode_row(p, unsigned(r), b, t, h);
-            RnFwdStage<F32>& st = ring[it % kFwdDepth<F32>];
-            const long long off = b * p.x_sb + t * p.x_st + h * p.x_sh + li * 8;
-            if constexpr (F32) {
-                rn_cp_async16(&st.x0[threadIdx.x], static_cast<const float*>(p.x) + off);
-                rn_cp_async16(&st.x1[threadIdx.x], static_cast<const float*>(p.x) + off + 4);
-            } else {
-                rn_cp_async16(&st.x0[threadIdx.x], static_cast<const uint16_t*>(p.x) + off);
-            }
-            rn_cp_async16(&st.cs[threadIdx.x], p.cos_t + static_cast<long long>(t) * (D / 2) + li * 4);
-            rn_cp_async16(&st.sn[threadIdx.x], p.sin_t + static_cast<long long>(t) * (D / 2) + li * 4);
-        }
-        rn_cp_async_commit();  // one group per iteration, also when it is empty
-    };
+    for (; item < p.n_items; item += n_warps) {
+        const RnItem<D> it(p, item, sub);
+        const float4 cs = *reinterpret_cast<const float4*>(p.cos_t + static_cast<long long>(it.t) * (D / 2) + li * 4);
+        const float4 sn = *reinterpret_cast<const float4*>(p.sin_t + static_cast<long long>(it.t) * (D / 2) + li * 4);
+        const long long x_off = it.b * p.x_sb + it.t * p.x_st + li * 8, y_off = it.b * p.y_sb + it.t * p.y_st + li * 8;
+        float* rstd_t = p.rstd + static_cast<long long>(it.b) * p.H * p.T + it.t;
+        for (int h = it.h0; h < it.h1; h += kUnroll) {
+            RnRaw<F32> raw[kUnroll];
 #pragma unroll
-    for (int i = 0; i < kFwdDepth<F32> - 1; ++i) request(i);
-    for (unsigned it = 0; first + it * stride - sub < n_rows; ++it) {  // (all lanes of a warp run the same iterations)
-        request(it + kFwdDepth<F32> - 1);
-        rn_cp_async_wait<kFwdDepth<F32> - 1>();  // everything but the newest kFwdDepth - 1 groups has landed: iteration `it`
-        const unsigned long long r = first + it * stride;
-        const bool live = r < n_rows;
-        float rot[8];
-        float ss = 0.f;
-        int b = 0, t = 0, h = 0;
-        if (live) {
-            const RnFwdStage<F32>& st = ring[it % kFwdDepth<F32>];
-            float v[8];
-            if constexpr (F32) {
-                const uint4 a = st.x0[threadIdx.x], c = st.x1[threadIdx.x];
-                v[0] = __uint_as_float(a.x), v[1] = __uint_as_float(a.y), v[2] = __uint_as_float(a.z), v[3] = __uint_as_float(a.w);
-                v[4] = __uint_as_float(c.x), v[5] = __uint_as_float(c.y), v[6] = __uint_as_float(c.z), v[7] = __uint_as_float(c.w);
-            } else {
-                const uint4 a = st.x0[threadIdx.x];
-                v[0] = rn_bf16_lo(a.x), v[1] = rn_bf16_hi(a.x), v[2] = rn_bf16_lo(a.y), v[3] = rn_bf16_hi(a.y);
-                v[4] = rn_bf16_lo(a.z), v[5] = rn_bf16_hi(a.z), v[6] = rn_bf16_lo(a.w), v[7] = rn_bf16_hi(a.w);
+            for (int k = 0; k < kUnroll; ++k) {
+                raw[k].clear();
+                if (it.live && h + k < it.h1) raw[k].load(p.x, x_off + (h + k) * p.x_sh);
             }
-            const uint4 cw = st.cs[threadIdx.x], sw = st.sn[threadIdx.x];
-            const float4 cs = make_float4(__uint_as_float(cw.x), __uint_as_float(cw.y), __uint_as_float(cw.z), __uint_as_float(cw.w));
-            const float4 sn = make_float4(__uint_as_float(sw.x), __uint_as_float(sw.y), __uint_as_float(sw.z), __uint_as_float(sw.w));
-            ss = rn_rotate8(v, cs, sn, rot);
-            rn_decode_row(p, unsigned(r), b, t, h);
-        }
-        ss = rn_row_sum<LPR>(ss);  // every lane takes part in the shuffles
-        if (live) {
-            const float rstd = rn_rstd<D>(ss, p.eps);
-            float out[8];
-            rn_scale8(rot, rstd, gm, out);
-            rn_store8<false>(p.y, static_cast<long long>(r) * D + li * 8, out);  // y is dense in walk order
-            if (li == 0) p.rstd[(static_cast<long long>(b) * p.H + h) * p.T + t] = rstd;
+#pragma unroll
+            for (int k = 0; k < kUnroll; ++k) {
+                if (h + k >= it.h1) break;
+                float v[8], rot[8], out[8];
+                raw[k].get(v);
+                const float ss = rn_row_sum<LPR>(rn_rotate8(v, cs, sn, rot));  // every lane takes part in the shuffles
+                const float rstd = rn_rstd<D>(ss, p.eps);
+                rn_scale8(rot, rstd, gm, out);
+                if (it.live) {
+                    rn_store8<false>(p.y, y_off + (h + k) * p.y_sh, out);
+                    if (li == 0) rstd_t[static_cast<long long>(h + k) * p.T] = rstd;
+                }
+            }
         }
     }
-    rn_cp_async_wait<0>();
+    return item - p.n_items;
 }
 
 // one launch takes q and k (n_tensors = 2), one after the other
 template <int D, bool F32>
-__global__ void __launch_bounds__(kRopeNormThreads, RN_FWD_BLOCKS)
+__global__ void __launch_bounds__(kRopeNormThreads, kRopeNormFwdBlocks)
 rope_norm_fwd_kernel(const __grid_constant__ RopeNormParams p0, const __grid_constant__ RopeNormParams p1,
                      const int n_tensors) {
-    __shared__ RnFwdStage<F32> ring[kFwdDepth<F32>];
+    const unsigned warp = (blockIdx.x * kRopeNormThreads + threadIdx.x) >> 5, n_warps = (gridDim.x * kRopeNormThreads) >> 5;
     grid_dep_wait();  // launched with programmatic stream serialization: the inputs come from the kernel before
-    rope_norm_fwd_tensor<D, F32>(p0, ring);
-    if (n_tensors > 1) rope_norm_fwd_tensor<D, F32>(p1, ring);
+    const unsigned next = rope_norm_fwd_tensor<D, F32>(p0, warp, n_warps);
+    if (n_tensors > 1) rope_norm_fwd_tensor<D, F32>(p1, next, n_warps);
 }
 
-// Shared memory of one backward stage, per thread: cos, sin, x (16 or 32 bytes), dy (16 bytes) and the row's rstd.
-template <bool F32>
-struct RnBwdStage {
-    uint4 cs[kRopeNormThreads], sn[kRopeNormThreads], x0[kRopeNormThreads], x1[kRopeNormThreads], dy[kRopeNormThreads];
-    float rstd[kRopeNormThreads];
-};
-template <>
-struct RnBwdStage<false> {
-    uint4 cs[kRopeNormThreads], sn[kRopeNormThreads], x0[kRopeNormThreads], dy[kRopeNormThreads];
-    float rstd[kRopeNormThreads];
-};
-constexpr int kBwdDepth = 3;  // iterations in flight per lane in the backward
-template <bool F32>
-constexpr int kRopeNormBwdSmemBytes = kBwdDepth * int(sizeof(RnBwdStage<F32>));
-
-__device__ __forceinline__ void rn_cp_async4(void* smem_dst, const void* gsrc) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
-}
-
-// One tensor's backward; the loads are staged like the forward's (see rope_norm_fwd_tensor).
+// One tensor's backward, in the same manner; leaves this CTA's d_gamma sums in p.partial.
 template <int D, bool F32>
-__device__ __forceinline__ void rope_norm_bwd_tensor(const RopeNormParams& p, float (*s_part)[D], RnBwdStage<F32>* ring) {
+__device__ __forceinline__ unsigned rope_norm_bwd_tensor(const RopeNormParams& p, unsigned item, unsigned n_warps, float (*s_part)[D]) {
     constexpr int LPR = D / 8;
-    constexpr int RPS = 32 / LPR;
+    constexpr int kUnroll = 2;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = lane / LPR, li = lane % LPR;
-    const unsigned warp0 = (blockIdx.x * kRopeNormThreads + threadIdx.x) >> 5;
-    const unsigned n_warps = (gridDim.x * kRopeNormThreads) >> 5;
-    const unsigned n_rows = unsigned(p.B) * unsigned(p.T) * unsigned(p.H);
     float gm[8], dg[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
         gm[e] = p.gamma[li * 8 + e];
         dg[e] = 0.f;
     }
-    const unsigned long long stride = static_cast<unsigned long long>(n_warps) * RPS;
-    const unsigned long long first = static_cast<unsigned long long>(warp0) * RPS + sub;
-    auto request = [&](unsigned it) {
-        const unsigned long long r = first + it * stride;
-        if (r < n_rows) {
-            int b, t, h;
-            rn_decode_row(p, unsigned(r), b, t, h);
-            RnBwdStage<F32>& st = ring[it % kBwdDepth];
-            const long long xoff = static_cast<long long>(r) * D + li * 8;  // x is dense in walk order
-            if constexpr (F32) {
-                rn_cp_async16(&st.x0[threadIdx.x], static_cast<const float*>(p.x) + xoff);
-                rn_cp_async16(&st.x1[threadIdx.x], static_cast<const float*>(p.x) + xoff + 4);
-            } else {
-                rn_cp_async16(&st.x0[threadIdx.x], static_cast<const uint16_t*>(p.x) + xoff);
-            }
-            rn_cp_async16(&st.dy[threadIdx.x], p.dy + (b * p.y_sb + t * p.y_st + h * p.y_sh + li * 8));
-            rn_cp_async4(&st.rstd[threadIdx.x], p.rstd + ((static_cast<long long>(b) * p.H + h) * p.T + t));
-            rn_cp_async16(&st.cs[threadIdx.x], p.cos_t + static_cast<long long>(t) * (D / 2) + li * 4);
-            rn_cp_async16(&st.sn[threadIdx.x], p.sin_t + static_cast<long long>(t) * (D / 2) + li * 4);
-        }
-        rn_cp_async_commit();
-    };
+    for (; item < p.n_items; item += n_warps) {
+        const RnItem<D> it(p, item, sub);
+        const float4 cs = *reinterpret_cast<const float4*>(p.cos_t + static_cast<long long>(it.t) * (D / 2) + li * 4);
+        const float4 sn = *reinterpret_cast<const float4*>(p.sin_t + static_cast<long long>(it.t) * (D / 2) + li * 4);
+        const float c[4] = {cs.x, cs.y, cs.z, cs.w}, sv[4] = {sn.x, sn.y, sn.z, sn.w};
+        const long long x_off = it.b * p.x_sb + it.t * p.x_st + li * 8, y_off = it.b * p.y_sb + it.t * p.y_st + li * 8;
+        const float* rstd_t = p.rstd + static_cast<long long>(it.b) * p.H * p.T + it.t;
+        for (int h = it.h0; h < it.h1; h += kUnroll) {
+            RnRaw<F32> raw_x[kUnroll];
+            RnRaw<false> raw_dy[kUnroll];
+            float rstd[kUnroll];
 #pragma unroll
-    for (int i = 0; i < kBwdDepth - 1; ++i) request(i);
-    for (unsigned it = 0; first + it * stride - sub < n_rows; ++it) {
-        request(it + kBwdDepth - 1);
-        rn_cp_async_wait<kBwdDepth - 1>();
-        const unsigned long long r = first + it * stride;
-        const bool live = r < n_rows;
-        float rot[8], g[8];
-        float s = 0.f, rs = 0.f;
-        float c[4] = {0.f, 0.f, 0.f, 0.f}, sv[4] = {0.f, 0.f, 0.f, 0.f};
-        if (live) {
-            const RnBwdStage<F32>& st = ring[it % kBwdDepth];
-            float v[8], dyv[8];
-            if constexpr (F32) {
-                const uint4 a = st.x0[threadIdx.x], q = st.x1[threadIdx.x];
-                v[0] = __uint_as_float(a.x), v[1] = __uint_as_float(a.y), v[2] = __uint_as_float(a.z), v[3] = __uint_as_float(a.w);
-                v[4] = __uint_as_float(q.x), v[5] = __uint_as_float(q.y), v[6] = __uint_as_float(q.z), v[7] = __uint_as_float(q.w);
-            } else {
-                const uint4 a = st.x0[threadIdx.x];
-                v[0] = rn_bf16_lo(a.x), v[1] = rn_bf16_hi(a.x), v[2] = rn_bf16_lo(a.y), v[3] = rn_bf16_hi(a.y);
-                v[4] = rn_bf16_lo(a.z), v[5] = rn_bf16_hi(a.z), v[6] = rn_bf16_lo(a.w), v[7] = rn_bf16_hi(a.w);
-            }
-            const uint4 d = st.dy[threadIdx.x];
-            dyv[0] = rn_bf16_lo(d.x), dyv[1] = rn_bf16_hi(d.x), dyv[2] = rn_bf16_lo(d.y), dyv[3] = rn_bf16_hi(d.y);
-            dyv[4] = rn_bf16_lo(d.z), dyv[5] = rn_bf16_hi(d.z), dyv[6] = rn_bf16_lo(d.w), dyv[7] = rn_bf16_hi(d.w);
-            const uint4 cw = st.cs[threadIdx.x], sw = st.sn[threadIdx.x];
-            c[0] = __uint_as_float(cw.x), c[1] = __uint_as_float(cw.y), c[2] = __uint_as_float(cw.z), c[3] = __uint_as_float(cw.w);
-            sv[0] = __uint_as_float(sw.x), sv[1] = __uint_as_float(sw.y), sv[2] = __uint_as_float(sw.z), sv[3] = __uint_as_float(sw.w);
-            rs = st.rstd[threadIdx.x];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float x0 = v[2 * i], x1 = v[2 * i + 1];
-                rot[2 * i] = x0 * c[i] - x1 * sv[i];
-                rot[2 * i + 1] = x0 * sv[i] + x1 * c[i];
+            for (int k = 0; k < kUnroll; ++k) {
+                raw_x[k].clear();
+                raw_dy[k].clear();
+                rstd[k] = 0.f;
+                if (it.live && h + k < it.h1) {
+                    raw_x[k].load(p.x, x_off + (h + k) * p.x_sh);
+                    raw_dy[k].load(p.dy, y_off + (h + k) * p.y_sh);
+                    rstd[k] = rstd_t[static_cast<long long>(h + k) * p.T];
+                }
             }
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                g[e] = dyv[e] * gm[e];
-                s += g[e] * rot[e];
-                dg[e] += dyv[e] * rot[e] * rs;
-            }
-        }
-        s = rn_row_sum<LPR>(s);
-        if (live) {
-            const float coeff = rs * rs * rs * (1.f / float(D)) * s;
-            float dx[8];
+            for (int k = 0; k < kUnroll; ++k) {
+                if (h + k >= it.h1) break;
+                float v[8], dyv[8], rot[8], g[8];
+                raw_x[k].get(v);
+                raw_dy[k].get(dyv);
+                const float rs = rstd[k];
+                float s = 0.f;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float d0 = rs * g[2 * i] - coeff * rot[2 * i];
-                const float d1 = rs * g[2 * i + 1] - coeff * rot[2 * i + 1];
-                dx[2 * i] = d0 * c[i] + d1 * sv[i];
-                dx[2 * i + 1] = -d0 * sv[i] + d1 * c[i];
+                for (int i = 0; i < 4; ++i) {
+                    const float x0 = v[2 * i], x1 = v[2 * i + 1];
+                    rot[2 * i] = x0 * c[i] - x1 * sv[i];
+                    rot[2 * i + 1] = x0 * sv[i] + x1 * c[i];
+                }
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    g[e] = dyv[e] * gm[e];
+                    s += g[e] * rot[e];
+                    dg[e] += dyv[e] * rot[e] * rs;
+                }
+                s = rn_row_sum<LPR>(s);
+                const float coeff = rs * rs * rs * (1.f / float(D)) * s;
+                float dx[8];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float d0 = rs * g[2 * i] - coeff * rot[2 * i];
+                    const float d1 = rs * g[2 * i + 1] - coeff * rot[2 * i + 1];
+                    dx[2 * i] = d0 * c[i] + d1 * sv[i];
+                    dx[2 * i + 1] = -d0 * sv[i] + d1 * c[i];
+                }
+                if (it.live) rn_store8<F32>(p.y, x_off + (h + k) * p.x_sh, dx);
             }
-            rn_store8<F32>(p.y, static_cast<long long>(r) * D + li * 8, dx);
         }
     }
-    rn_cp_async_wait<0>();
     // d_gamma: a lane holds sums for its 8 columns over its rows.  Add the lanes that own the same columns
     // (they differ in `sub`), then the warps of the CTA, both in a fixed order.
 #pragma unroll
@@ -390,38 +309,45 @@ __device__ __forceinline__ void rope_norm_bwd_tensor(const RopeNormParams& p, fl
         for (int w = 0; w < kRopeNormThreads / 32; ++w) acc += s_part[w][d];
         p.partial[static_cast<long long>(blockIdx.x) * D + d] = acc;
     }
-    __syncthreads();  // s_part is rewritten for the next tensor
+    return item - p.n_items;
 }
 
 template <int D, bool F32>
-__global__ void __launch_bounds__(kRopeNormThreads, RN_BWD_BLOCKS)
+__global__ void __launch_bounds__(kRopeNormThreads, kRopeNormBwdBlocks)
 rope_norm_bwd_kernel(const __grid_constant__ RopeNormParams p0, const __grid_constant__ RopeNormParams p1,
                      const int n_tensors) {
-    __shared__ float s_part[kRopeNormThreads / 32][D];
-    extern __shared__ uint4 rn_dyn_smem[];
-    RnBwdStage<F32>* ring = reinterpret_cast<RnBwdStage<F32>*>(rn_dyn_smem);
+    __shared__ float s_part[2][kRopeNormThreads / 32][D];
+    const unsigned warp = (blockIdx.x * kRopeNormThreads + threadIdx.x) >> 5, n_warps = (gridDim.x * kRopeNormThreads) >> 5;
     grid_dep_wait();
-    rope_norm_bwd_tensor<D, F32>(p0, s_part, ring);
-    if (n_tensors > 1) rope_norm_bwd_tensor<D, F32>(p1, s_part, ring);
+    const unsigned next = rope_norm_bwd_tensor<D, F32>(p0, warp, n_warps, s_part[0]);
+    if (n_tensors > 1) rope_norm_bwd_tensor<D, F32>(p1, next, n_warps, s_part[1]);
 }
 
-// d_gamma[d] += sum of the CTAs' partial sums, for one or two tensors.  One warp per column (CTA c takes column
-// c % D of tensor c / D): lane l adds parts l, l + 32, ... in order, then the 32 lane sums are added in a fixed
-// tree, so the result is bit-reproducible; the loads of a lane are independent, which keeps this tail kernel at a
-// microsecond or two.  (Done by the last CTA of the backward kernel instead, the same sums took 25 us: one CTA
-// cannot keep enough loads in flight.)
+// d_gamma[d] += sum of the CTAs' partial sums, for one or two tensors.  A CTA takes 8 columns (one 32-byte sector of every
+// part): thread (r, c) adds parts r, r + 32, ... of column c in order, then the 32 sums of a column are added in order, so
+// the result is bit-reproducible and all loads are in flight at once.  (Done by the last CTA of the backward kernel
+// instead, the same sums took 25 us: one CTA cannot keep enough loads in flight.)
+constexpr int kDgammaThreads = 256;
 template <int D>
-__global__ void __launch_bounds__(32) rope_norm_dgamma_kernel(const float* __restrict__ partial0, float* __restrict__ d_gamma0,
-                                                              const float* __restrict__ partial1, float* __restrict__ d_gamma1,
-                                                              int n_parts) {
-    const int ts = blockIdx.x / D, d = blockIdx.x % D, lane = threadIdx.x;
+__global__ void __launch_bounds__(kDgammaThreads) rope_norm_dgamma_kernel(const float* __restrict__ partial0, float* __restrict__ d_gamma0,
+                                                                          const float* __restrict__ partial1, float* __restrict__ d_gamma1,
+                                                                          int n_parts) {
+    __shared__ float s_sum[32][9];
+    const int ts = blockIdx.x / (D / 8), c = threadIdx.x & 7, r = threadIdx.x >> 3, d = (blockIdx.x % (D / 8)) * 8 + c;
     const float* partial = ts ? partial1 : partial0;
     float* d_gamma = ts ? d_gamma1 : d_gamma0;
     float acc = 0.f;
     grid_dep_wait();  // the partial sums come from the kernel before this one
-    for (int i = lane; i < n_parts; i += 32) acc += partial[static_cast<long long>(i) * D + d];
-    acc = rn_warp_sum(acc);
-    if (lane == 0) d_gamma[d] += acc;
+#pragma unroll 8
+    for (int i = r; i < n_parts; i += 32) acc += partial[static_cast<long long>(i) * D + d];
+    s_sum[r][c] = acc;
+    __syncthreads();
+    if (r == 0) {
+        acc = 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) acc += s_sum[i][c];
+        d_gamma[d] += acc;
+    }
 }
 
 }  // namespace b200attn

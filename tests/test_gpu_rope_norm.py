@@ -56,6 +56,16 @@ def test_matches_oracle(B, T, H, D, x_dtype, x_layout, y_layout):
     assert_close("d_gamma", got[3], want[3], max_abs=1e-2 * max(1.0, float(np.abs(want[3]).max())), rel_l2=1e-4)
 
 
+@pytest.mark.parametrize("B,T,H,D,x_dtype", [(5, 1999, 11, 64, torch.bfloat16), (3, 1333, 9, 128, torch.float32), (8, 4001, 12, 64, torch.bfloat16)])
+def test_chunks_of_heads_with_a_remainder(B, T, H, D, x_dtype):
+    # four and eight heads per item, the last chunk shorter; token groups that cross a sequence's end
+    got, want = _case(B, T, H, D, x_dtype, "BTHD", "BHTD")
+    assert_close("y", got[0], want[0])
+    assert_close("rstd", got[1], want[1], max_abs=1e-4, rel_l2=1e-5)
+    assert_close("d_x", got[2], want[2])
+    assert_close("d_gamma", got[3], want[3], max_abs=1e-2 * max(1.0, float(np.abs(want[3]).max())), rel_l2=1e-4)
+
+
 def test_full_size_bit_reproducible_and_accumulating():
     # q of the 50M training shape; d_gamma is summed without atomics and accumulated into
     B, T, H, D = 32, 512, 6, 64
