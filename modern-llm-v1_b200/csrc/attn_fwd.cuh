@@ -38,6 +38,8 @@ struct FwdParams {
     int n_qtiles;
     int kv_off;        // keys in front of the first query row: query row t sees keys 0 .. kv_off + t (0 when q and k
                        // cover the same tokens; the cached tokens' count when a chunk of new tokens attends over a KV cache)
+    int split;         // CTAs (a cluster) that share an item's key tiles; 1 except in the split kernel
+    FastDiv div_split;
     float scale;       // softmax scale
     float scale_log2;  // scale * log2(e)
     float* lse;        // [B, Hq, T]
@@ -74,7 +76,12 @@ struct FwdCfg {
 // sum are rescaled; below it the stale maximum stays the exponent reference.
 constexpr float kRescaleThresholdLog2 = 8.0f;
 
-template <int D>
+// SPLIT: few, long items (a chunk of new tokens behind a long cache, a single long sequence).  A CTA walks a share of ONE
+// item's key tiles, and the CTAs of a cluster add up their (m, l, O) through distributed shared memory, each finishing
+// 128 / split of the rows.  Measured on B200: 15 tokens behind 6000, B=1 6/2
+// D=64 (6 items, 8 CTAs each) 57.2 -> 15.0 us; 720 behind 4000, B=1 8/1 D=64 (48 items, 4) 47.7 -> 26.8; 500 behind 3000,
+// B=2 16/4 D=128 (128 items, 2) 47.4 -> 40.8.
+template <int D, bool SPLIT>
 __global__ void __launch_bounds__(256, 2)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const FwdParams p, const __grid_constant__ ItemTable tab) {
@@ -116,7 +123,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     auto item_qt = [&](int id) { return p.n_qtiles - 1 - int(fastdiv(unsigned(id), p.div_bh)); };
     auto item_b = [&](int id) { return int(fastdiv(unsigned(item_rest(id)), p.div_h)); };
     auto item_h = [&](int id) { return item_rest(id) - item_b(id) * p.Hq; };
-    auto item_nkv = [&](int id) { return (p.kv_off + min(p.T, item_qt(id) * 128 + 128) + Cfg::kKeys - 1) / Cfg::kKeys; };
+    auto item_all = [&](int id) { return (p.kv_off + min(p.T, item_qt(id) * 128 + 128) + Cfg::kKeys - 1) / Cfg::kKeys; };
+    const int split_id = SPLIT ? int(fastdiv(blockIdx.x, p.div_split)) : 0, rank = SPLIT ? int(blockIdx.x) - split_id * p.split : 0;
+    // key tiles of an item that are this CTA's: [j_first, j_first + item_nkv)
+    const int j_first = SPLIT ? int(fastdiv(unsigned(item_all(split_id) * rank), p.div_split)) : 0;
+    auto item_nkv = [&](int id) {
+        return SPLIT ? int(fastdiv(unsigned(item_all(id) * (rank + 1)), p.div_split)) - j_first : item_all(id);
+    };
+    float split_m = -INFINITY, split_l = 0.f;  // SPLIT: this thread's row
 
     B200ATTN_TRACE_BEGIN(0);
     // Set-up with one CTA-wide barrier: one lane of the producer warp initialises every mbarrier while
@@ -182,13 +196,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             }
             __syncwarp();
         };
-        int id = sched_first(tab, p.sched, int(blockIdx.x));  // the first item needs no fetch
+        int id = SPLIT ? split_id : sched_first(tab, p.sched, int(blockIdx.x));  // the first item needs no fetch
+        const bool any = !SPLIT || item_nkv(id) > 0;
         if (lane == 0) {
-            item_publish(bar_item, item_ring, 0, id);
-            id_next = sched_fetch(tab, p.sched, 1, int(blockIdx.x), int(gridDim.x));
+            item_publish(bar_item, item_ring, 0, any ? id : -1);
+            id_next = SPLIT ? n_items : sched_fetch(tab, p.sched, 1, int(blockIdx.x), int(gridDim.x));
         }
         __syncwarp();
-        load_q(0, id);
+        if (any) load_q(0, id);
+        else ok = false;
         for (int n = 0; ok; ++n) {
             const int h = item_h(id), b = item_b(id), hk = int(fastdiv(unsigned(h), p.div_group)), n_kv = item_nkv(id);
             // The next item is taken, announced and its Q requested a few tiles before this item's loads end
@@ -206,7 +222,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
                     for (int bx = 0; bx < Cfg::kBoxes; ++bx)
                         tma_load_4d(sK + s * Cfg::kKVTileBytes + bx * Cfg::kKVBoxBytes, &tmK, &bar_k_full[s], bx * 64,
-                                    j * Cfg::kKeys, hk, b);
+                                    (j_first + j) * Cfg::kKeys, hk, b);
                 }
                 __syncwarp();
                 if (g >= NST) ok = mbar_wait_warp(&bar_v_free[s], (use - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
@@ -216,7 +232,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
                     for (int bx = 0; bx < Cfg::kBoxes; ++bx)
                         tma_load_4d(sV + s * Cfg::kKVTileBytes + bx * Cfg::kKVBoxBytes, &tmV, &bar_v_full[s], bx * 64,
-                                    j * Cfg::kKeys, hk, b);
+                                    (j_first + j) * Cfg::kKeys, hk, b);
                 }
                 __syncwarp();
                 if (j == j_next) {
@@ -234,7 +250,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             if (!ok || id_new >= n_items) break;
             id = id_new;
         }
-        if (ok && lane == 0) sched_finish(p.sched, int(gridDim.x));
+        if (!SPLIT && ok && lane == 0) sched_finish(p.sched, int(gridDim.x));
     } else if (warp == 5) {
         // ------------------------------------------------------------------ MMA issuer
         reg_dealloc<Cfg::kRegsOther>();
@@ -422,7 +438,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     tc_fence_before_sync();
                     mbar_arrive(bar_s_loaded);  // the buffer goes back to the MMA warp at once
                 }
-                const int kbase = j * KEYS;  // first key of this tile
+                const int kbase = (j_first + j) * KEYS;  // first key of this tile
                 if (kbase + KEYS - 1 > q0 + p.kv_off) {
                     // tile touches the diagonal: key kbase + c is visible to query q0 + row iff it is <= the query's
                     // own position kv_off + q0 + row
@@ -443,7 +459,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     alpha = ex2_approx((m_ref - m_new) * p.scale_log2);
                     m_ref = m_new;
                 }
-                const float neg_m = -m_ref * p.scale_log2;
+                // (a share of an item may hold no key that a row sees: its exponentials are 0 then, not NaN)
+                const float neg_m = SPLIT && m_ref == -INFINITY ? 0.f : -m_ref * p.scale_log2;
                 const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), neg2 = pack_f32x2(neg_m, neg_m);
                 uint64_t sum2[2] = {0ull, 0ull};
                 // 32 columns at a time: exponentials, sums and BF16 pairs
@@ -516,10 +533,91 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             pending = true;
             pend_id = id, pend_m = m_ref, pend_l = l;
         }
-        if (ok && pending) epilogue(n - 1, pend_id, pend_m, pend_l);
+        if constexpr (SPLIT) {
+            if (ok && pending) ok = mbar_wait_warp(bar_o_done, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+            if (ok && pending) split_m = pend_m, split_l = pend_l;
+        } else if (ok && pending) {
+            epilogue(n - 1, pend_id, pend_m, pend_l);
+        }
         tc_fence_before_sync();
     }
 
+    if constexpr (SPLIT) {
+        // Every role comes here, also after a wait that gave up.  Row r is finished by CTA r / rows of the cluster; the K/V ring
+        // holds the arrivals, so all CTAs must be through with theirs first.
+        const int rows = 128 / p.split;
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        if (tid < 128) {
+            tc_fence_after_sync();
+            const int to = (tid * p.split) >> 7, r = tid - to * rows;
+            uint8_t* own = sK + (rank * rows + r) * D * 4;
+            const uint32_t dst = cluster_addr(own, to);
+#pragma unroll
+            for (int c = 0; c < D / 32; ++c) {
+                uint32_t v[32];
+                tmem_ld_x32(tmem + (uint32_t(warp * 32) << 16) + Cfg::kColO + c * 32, v);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {  // 16-byte pieces swizzled by the row: the rows of a warp would share a bank
+                    const int at = ((c * 8 + i) ^ (r & 7)) << 4;
+                    if (to == rank)
+                        *reinterpret_cast<uint4*>(own + at) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                    else
+                        cluster_store_4(dst + at, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                }
+            }
+            cluster_store_f2(sQ + (rank * rows + r) * 8, to, make_float2(split_m, split_l));
+            tc_fence_before_sync();
+        }
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        if (tid < 128) {
+            const float2* ml = reinterpret_cast<const float2*>(sQ);
+            const int q0 = item_qt(split_id) * 128 + rank * rows, b = item_b(split_id), h = item_h(split_id);
+            // `split` threads per row, each with D / split columns, 16 at a time (8 when there are no more)
+            const int r = fastdiv(unsigned(tid), p.div_split), part = tid - r * p.split, cols = fastdiv(unsigned(D), p.div_split);
+            if (q0 + r < p.T) {
+                float m = -INFINITY, l = 0.f;
+                for (int k = 0; k < p.split; ++k) m = fmaxf(m, ml[k * rows + r].x);
+                for (int k = 0; k < p.split; ++k) {
+                    const float2 s = ml[k * rows + r];
+                    l += s.x == -INFINITY ? 0.f : ex2_approx((s.x - m) * p.scale_log2) * s.y;
+                }
+                const float inv_l = 1.f / l;
+                uint16_t* orow = p.o + size_t(b) * p.o_sb + size_t(h) * p.o_sh + size_t(q0 + r) * p.o_st + part * cols;
+                for (int c = 0; c < cols; c += 16) {
+                    const bool two = c + 8 < cols;
+                    float acc[16] = {};
+                    for (int k = 0; k < p.split; ++k) {
+                        const float mk = ml[k * rows + r].x;
+                        if (mk == -INFINITY) continue;  // no key of the row (or no tile at all: nothing valid was sent)
+                        const float f = ex2_approx((mk - m) * p.scale_log2) * inv_l;
+                        const uint8_t* row = sK + (k * rows + r) * D * 4;
+                        float4 v[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (e < 2 || two) v[e] = *reinterpret_cast<const float4*>(row + ((((part * cols + c) / 4 + e) ^ (r & 7)) << 4));
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (e < 2 || two) {
+                                acc[e * 4 + 0] += f * v[e].x, acc[e * 4 + 1] += f * v[e].y;
+                                acc[e * 4 + 2] += f * v[e].z, acc[e * 4 + 3] += f * v[e].w;
+                            }
+                    }
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        if (e == 0 || two)
+                            *reinterpret_cast<uint4*>(orow + c + e * 8) =
+                                make_uint4(pack_bf16x2(acc[e * 8], acc[e * 8 + 1]), pack_bf16x2(acc[e * 8 + 2], acc[e * 8 + 3]),
+                                           pack_bf16x2(acc[e * 8 + 4], acc[e * 8 + 5]), pack_bf16x2(acc[e * 8 + 6], acc[e * 8 + 7]));
+                }
+                if (part == 0) p.lse[(size_t(b) * p.Hq + h) * p.T + q0 + r] = m * p.scale + logf(l);
+            }
+        }
+    }
     // teardown: every role falls through to here, also after a wait that gave up
     tc_fence_before_sync();
     __syncthreads();

@@ -242,31 +242,59 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, unsigned block, size
     return launch_cluster(kernel, grid, block, smem, st, 1, args...);
 }
 
+template <typename K>
+int set_smem_once(K kernel, int bytes, bool* done) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!done[dev]) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return B200ATTN_ERR_CUDA;
+        }
+        done[dev] = true;
+    }
+    return B200ATTN_OK;
+}
+
+// CTAs that share an item's key tiles in the forward.  1 unless the items leave CTA slots free (two per SM) and are long: the
+// exchange at the end costs 2 to 3 us, which is what some 300 keys take, and about twice that where a second CTA on the SM
+// slows both down.  Clusters of more than two CTAs do not always fill the last SMs of a GPC, so these are held to 256 CTAs.
+int fwd_split(long long items, int keys) {
+    const int sms = sm_count();
+    for (int split = 1;; split *= 2) {
+        const long long ctas = items * split * 2;
+        if (split == 8 || ctas > (split == 1 ? 2 * sms : std::min(2 * sms, 256)) || keys < 2 * split * (ctas > sms ? 768 : 384)) return split;
+    }
+}
+
 template <int D>
 int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p,
                cudaStream_t st) {
     using Cfg = FwdCfg<D>;
-    static bool attr_set[kMaxDevices] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!attr_set[dev]) {
-        if (cudaFuncSetAttribute(attn_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) !=
-            cudaSuccess) {
-            cudaGetLastError();
-            return B200ATTN_ERR_CUDA;
-        }
-        attr_set[dev] = true;
-    }
-    // persistent CTAs, two per SM, each walking a heaviest-first list of (query tile, head, batch) items
     const long long items = (long long)p.n_qtiles * p.Hq * p.B;
-    const unsigned grid = (unsigned)std::min<long long>(items, 2LL * sm_count());
     FwdParams pl = p;
-    pl.sched = next_sched_pair(items, grid);
     pl.div_bh = fastdiv_make((unsigned)(p.B * p.Hq));
     pl.div_h = fastdiv_make((unsigned)p.Hq);
     pl.div_group = fastdiv_make((unsigned)p.group);
-    const ItemTable& tab = item_table_for(pl.sched ? -1 : items, grid, p.B * p.Hq, p.n_qtiles, p.T, 1);
-    if (launch_pdl(attn_fwd_kernel<D>, grid, 256, Cfg::kSmemBytes, st, tq, tk, tv, pl, tab) != cudaSuccess) {
+    pl.split = fwd_split(items, p.kv_off + p.T);
+    pl.div_split = fastdiv_make((unsigned)pl.split);
+    cudaError_t e;
+    if (pl.split > 1) {
+        static bool set[kMaxDevices] = {false};
+        if (int rc = set_smem_once(attn_fwd_kernel<D, true>, Cfg::kSmemBytes, set)) return rc;
+        pl.sched = nullptr;
+        e = launch_cluster(attn_fwd_kernel<D, true>, dim3((unsigned)(items * pl.split)), 256, Cfg::kSmemBytes, st, pl.split, tq, tk, tv, pl,
+                           item_table_for(-1, 1, 1, 1, 1, 1));
+    } else {
+        static bool set[kMaxDevices] = {false};
+        if (int rc = set_smem_once(attn_fwd_kernel<D, false>, Cfg::kSmemBytes, set)) return rc;
+        // persistent CTAs, two per SM, each walking a heaviest-first list of (query tile, head, batch) items
+        const unsigned grid = (unsigned)std::min<long long>(items, 2LL * sm_count());
+        pl.sched = next_sched_pair(items, grid);
+        const ItemTable& tab = item_table_for(pl.sched ? -1 : items, grid, p.B * p.Hq, p.n_qtiles, p.T, 1);
+        e = launch_pdl(attn_fwd_kernel<D, false>, grid, 256, Cfg::kSmemBytes, st, tq, tk, tv, pl, tab);
+    }
+    if (e != cudaSuccess) {
         cudaGetLastError();
         return B200ATTN_ERR_CUDA;
     }
@@ -340,20 +368,6 @@ extern "C" int b200attn_fwd_kvcache_at(const void* q, const void* kcache, const 
 namespace {
 
 inline size_t bwd_vec_elems(int B, int T, int Hq) { return (size_t)B * Hq * (size_t)((T + 127) / 128 * 128); }
-
-template <typename K>
-int set_smem_once(K kernel, int bytes, bool* done) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!done[dev]) {
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
-            cudaGetLastError();
-            return B200ATTN_ERR_CUDA;
-        }
-        done[dev] = true;
-    }
-    return B200ATTN_OK;
-}
 
 cudaEvent_t g_bwd_events[4] = {nullptr, nullptr, nullptr, nullptr};
 

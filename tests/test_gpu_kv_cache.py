@@ -102,6 +102,8 @@ def test_prefill_over_the_cache_equals_the_forward_on_dense_tensors(B, T, Hq, Hk
     (2, 6, 2, 64, (200, 1, 130, 57, 300), 700),     # prompt in chunks of uneven size, one of a single token
     (1, 8, 2, 128, (129, 128, 64), 400),
     (3, 4, 4, 64, (64, 64, 64, 64), 256),           # chunk boundaries on the 64-key tile boundaries
+    (1, 6, 2, 64, (3100, 15), 3200),                # items split over 4 and 8 CTAs, shares without a key for some rows
+    (1, 4, 2, 128, (1500, 129, 2), 1700),           # 2 to 4 CTAs, a last tile of two query rows
 ])
 def test_chunked_prefill_equals_the_rows_of_the_whole_forward(B, Hq, Hkv, D, chunks, L_cap):
     # several new tokens against a non-empty cache: every chunk's rows must be the rows of one causal forward over
