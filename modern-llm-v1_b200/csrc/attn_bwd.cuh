@@ -543,16 +543,21 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 }
 
 // ---------------------------------------------------------------------------------------
-// dQ pass for D = 128: one CTA per item (128-row query tile of one (batch, query head)), 128-key tiles, eight
-// compute warps (thread owns a row and 64 of the 128 score columns), one CTA per SM.  As in the D = 64 kernel, Q
-// and dO are copied once from shared memory into tensor memory, so that S = Q K^T, dP = dO V^T and dQ += dS K all
-// take their A operand from there (a 128-wide product with A in shared memory fetches 4 KB of A and 4 KB of B per
-// K step), and the one S buffer is handed back as soon as the scores are in registers: the next tile's Q K^T runs
-// under this tile's exponentials, and the next dP product follows the dQ product that consumes dS out of the dP
-// block.
+// dQ pass for D = 128: one CTA per item (128-row query tile of one (batch, query head)), one CTA per SM, 128-key tiles loaded
+// by TMA and worked on as two halves of 64 keys.  As in the D = 64 kernel, Q and dO are copied once from shared memory into
+// tensor memory, so that S = Q K^T, dP = dO V^T and dQ += dS K all take their A operand from there (a 128-wide product with
+// A in shared memory fetches 4 KB of A and 4 KB of B per K step).
+// The halves are two streams with their own barriers: S of the next tile's half follows as soon as this one's scores are in
+// registers, and dP of the next tile's half as soon as dQ has read dS out of its block, so one half's products run under the
+// other half's arithmetic.  (With whole tiles and one dP block, dS, dQ and the next dP followed one another: 3900 clocks per
+// 128 x 128 block for 1800 of tensor-pipe time.  There is no room for a second dP block beside S, dQ, Q and dO.)
+// The halves' dQ products are issued by one warp in a fixed order, so dQ is bit-reproducible.
+//
+// Roles (608 threads): warps 0-15 compute (thread owns row (warp % 4) * 32 + lane and 32 of the half's 64 columns: half
+// warp / 8, part (warp / 4) % 2), warp 16 TMA producer, warp 17 TMEM allocation and S, warp 18 dQ and dP.
 // Shared memory: the Q and dO staging tiles (64 KB; re-used as the third K/V ring stage once they have been copied
 // into tensor memory, and at the very end as the staging tile of the dQ store) and two more K/V stages.
-// TMEM (512 columns): S [0,128), dP [128,256) (dS as BF16 over the first 32 columns of each half's range), dQ
+// TMEM (512 columns): S [0,128), dP [128,256) (dS as BF16 over the first 16 columns of each part's range), dQ
 // accumulator [256,384), Q [384,448), dO [448,512).
 // ---------------------------------------------------------------------------------------
 template <int D>
@@ -561,27 +566,14 @@ struct DqWideCfg {
     static constexpr int kTileBytes = 128 * D * 2;
     static constexpr int kBoxBytes = 128 * 64 * 2;
     static constexpr int kBoxes = D / 64;
-    static constexpr int kSmemBytes = 2 * kStages * kTileBytes + 256 + 1024;
+    static constexpr int kComputeThreads = 512, kStreamThreads = 256, kThreads = kComputeThreads + 96;
+    static constexpr int kSmemBytes = 2 * kStages * kTileBytes + 512 + 256 + 1024;
     static constexpr int kTmemCols = 512;
     static constexpr int kColS = 0, kColDP = 128, kColAcc = 256, kColQ = 384, kColDO = 448;
 };
 
-// D[tmem] = A[tmem, BF16 pairs] * B[smem, K-major]^T over the head dimension (b_desc describes K step 0)
 template <int D>
-__device__ __forceinline__ void wide_ts_headdim(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc) {
-#pragma unroll
-    for (int ks = 0; ks < D / 16; ++ks) umma_ts(d_tmem, a_tmem + ks * 8, b_desc + kmajor_step(ks, 16384), idesc, ks > 0);
-}
-// A in two 32-column pieces at a_col and a_col + 64 (one per column half)
-template <int D>
-__device__ __forceinline__ void wide_ts(uint32_t d_tmem, uint32_t a_col, uint64_t b_desc, uint32_t idesc, bool accumulate) {
-#pragma unroll
-    for (int ks = 0; ks < 8; ++ks)
-        umma_ts(d_tmem, a_col + (ks < 4 ? ks * 8 : 64 + (ks - 4) * 8), b_desc + uint64_t(ks * 128), idesc,
-                accumulate || ks > 0);
-}
-template <int D>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(DqWideCfg<D>::kThreads, 1)
 attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                    const __grid_constant__ CUtensorMap tmdQ, const BwdParams p) {
@@ -597,67 +589,69 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     // ring stage 2 re-uses the two tiles Q and dO were staged in (free once they are in tensor memory)
     auto stage_k = [&](int st) { return st < 2 ? sK01 + st * Cfg::kTileBytes : sQ; };
     auto stage_v = [&](int st) { return st < 2 ? sV01 + st * Cfg::kTileBytes : sdO; };
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sV01 + 2 * Cfg::kTileBytes);
+    float* sD = reinterpret_cast<float*>(sV01 + 2 * Cfg::kTileBytes);  // [128] rowsum(O * dO)
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sD + 128);
     uint64_t* bar_q = bars + 0;         // Q and dO have landed in shared memory
     uint64_t* bar_qt_full = bars + 1;   // Q and dO are in tensor memory
-    uint64_t* bar_s_full = bars + 2;    //                                                     (phase: tile)
-    uint64_t* bar_s_loaded = bars + 3;  // S is in registers: the buffer may be overwritten   (phase: tile)
-    uint64_t* bar_dp_full = bars + 4;   //                                                     (phase: tile)
-    uint64_t* bar_ds_full = bars + 5;   // dS written over dP                                  (phase: tile)
-    uint64_t* bar_acc = bars + 6;
-    uint64_t* bar_kv_full = bars + 7;          // [NST]
-    uint64_t* bar_kv_free = bars + 7 + NST;    // [NST]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 17);
+    uint64_t* bar_acc = bars + 2;
+    uint64_t* bar_s_full = bars + 3;    // [2] per half                                        (phase: tile)
+    uint64_t* bar_s_loaded = bars + 5;  // [2] S is in registers: the half may be overwritten  (phase: tile)
+    uint64_t* bar_dp_full = bars + 7;   // [2]                                                 (phase: tile)
+    uint64_t* bar_ds_full = bars + 9;   // [2] dS written over dP                              (phase: tile)
+    uint64_t* bar_kv_full = bars + 11;          // [NST]
+    uint64_t* bar_kv_free = bars + 11 + NST;    // [NST]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 19);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    constexpr int kProducerWarp = Cfg::kComputeThreads / 32, kMmaSWarp = kProducerWarp + 1;
     const int n_bh = p.B * p.Hq;
-    const int qt = p.n_tiles - 1 - int(blockIdx.x) / n_bh;
-    const int h = (int(blockIdx.x) % n_bh) % p.Hq, b = (int(blockIdx.x) % n_bh) / p.Hq;
-    const int hk = h / p.group;
+    const int item_hi = int(fastdiv(blockIdx.x, p.div_bhq));  // ids are ordered by work, heaviest query tile first
+    const int qt = p.n_tiles - 1 - item_hi, rest = int(blockIdx.x) - item_hi * n_bh;
+    const int b = int(fastdiv(unsigned(rest), p.div_hq)), h = rest - b * p.Hq;
+    const int hk = int(fastdiv(unsigned(h), p.div_group));
     const int q0 = qt * 128;
     const int n_kv = qt + 1;
 
     B200ATTN_TRACE_BEGIN(1);
-    // launched with programmatic stream serialization: wait for the previous kernel before any global access
     grid_dep_launch();
-    grid_dep_wait();
-    if (tid == 0) *abort_flag = *reinterpret_cast<volatile int*>(p.status);
-    __syncthreads();
-    if (*abort_flag != 0) return;
-    __syncthreads();
-
-    if (tid == 0) {
-        mbar_init(bar_q, 1);
-        mbar_init(bar_qt_full, 256);
-        mbar_init(bar_s_full, 1);
-        mbar_init(bar_s_loaded, 256);
-        mbar_init(bar_dp_full, 1);
-        mbar_init(bar_ds_full, 256);
-        mbar_init(bar_acc, 1);
-        for (int s = 0; s < NST; ++s) {
-            mbar_init(&bar_kv_full[s], 1);
-            mbar_init(&bar_kv_free[s], 1);
-        }
-        fence_mbar_init();
-    }
-    if (warp == 9) {
-        tmem_alloc(tmem_slot, Cfg::kTmemCols);
-        tmem_relinquish();
-    }
-    if (warp == 8 && lane == 0) {
+    if (warp == kProducerWarp && lane == 0) {
         tma_prefetch_desc(&tmQ);
         tma_prefetch_desc(&tmK);
         tma_prefetch_desc(&tmV);
         tma_prefetch_desc(&tmdO);
         tma_prefetch_desc(&tmdQ);
+        mbar_init(bar_q, 1);
+        mbar_init(bar_qt_full, Cfg::kComputeThreads);
+        mbar_init(bar_acc, 1);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&bar_s_full[i], 1);
+            mbar_init(&bar_s_loaded[i], Cfg::kStreamThreads);
+            mbar_init(&bar_dp_full[i], 1);
+            mbar_init(&bar_ds_full[i], Cfg::kStreamThreads);
+        }
+        for (int s = 0; s < NST; ++s) {
+            mbar_init(&bar_kv_full[s], 1);
+            mbar_init(&bar_kv_free[s], 1);
+        }
+        fence_mbar_init();
+        // launched with programmatic stream serialization: wait for the previous kernel before any global access
+        grid_dep_wait();
+        *abort_flag = *reinterpret_cast<volatile int*>(p.status);
     }
+    if (warp == kMmaSWarp) {
+        tmem_alloc(tmem_slot, Cfg::kTmemCols);
+        tmem_relinquish();
+    }
+    grid_dep_wait();
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
 
-    if (warp == 8) {
+    if (*abort_flag != 0) {
+        // an earlier CTA already failed: fall through to the teardown
+    } else if (warp == kProducerWarp) {
         // ------------------------------------------------------------------ producer (whole warp, one lane issues)
         if (elect_one()) {
             mbar_arrive_expect_tx(bar_q, 2 * Cfg::kTileBytes);
@@ -685,74 +679,84 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
             }
             __syncwarp();
         }
-    } else if (warp == 9) {
-        // ------------------------------------------------------------------ MMA issuer (whole warp, one lane issues)
-        constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);   // A in TMEM, B (K or V tile) K-major
+    } else if (warp >= kMmaSWarp) {
+        // ------------------------------------------------------------------ MMA issuers (whole warps, one lane issues)
+        constexpr uint32_t idesc_s = make_idesc_bf16(128, 64, 0, 0);    // A in TMEM, B (64 rows of the K or V tile) K-major
         constexpr uint32_t idesc_acc = make_idesc_bf16(128, D, 0, 1);   // A in TMEM, B (K tile) MN-major
         bool ok = mbar_wait_warp(bar_qt_full, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
-        // S(j) = Q K_j^T; the buffer still holds S(j - 1) until it has been read into registers
-        auto issue_s = [&](int j) -> bool {
-            const int s = j % NST;
-            if (j > 0 && !mbar_wait_warp(bar_s_loaded, uint32_t(j - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX))
-                return false;
-            if (!mbar_wait_warp(&bar_kv_full[s], (j / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD)) return false;
-            tc_fence_after_sync();
+        // D[tmem, 64 columns] = A[tmem] * (rows 64 half .. + 64 of the tile)^T
+        auto issue_half = [&](uint32_t d_col, uint32_t a_col, const uint8_t* tile, int half, uint64_t* full) {
+            const uint64_t desc = kmajor_desc<D>(tile + half * 64 * 128);
             if (elect_one()) {
-                wide_ts_headdim<D>(tmem + Cfg::kColS, tmem + Cfg::kColQ, kmajor_desc<D>(stage_k(s)), idesc_s);
-                umma_commit(bar_s_full);
-            }
-            __syncwarp();
-            return true;
-        };
-        // dP(j) = dO V_j^T; the tile's loads are known to be complete (S(j) was issued), and the product that read
-        // dS(j - 1) out of this block was issued before
-        auto issue_dp = [&](int j) {
-            const int s = j % NST;
-            if (elect_one()) {
-                wide_ts_headdim<D>(tmem + Cfg::kColDP, tmem + Cfg::kColDO, kmajor_desc<D>(stage_v(s)), idesc_s);
-                umma_commit(bar_dp_full);
+#pragma unroll
+                for (int ks = 0; ks < D / 16; ++ks)
+                    umma_ts(tmem + d_col + half * 64, tmem + a_col + ks * 8, desc + kmajor_step(ks, Cfg::kBoxBytes), idesc_s, ks > 0);
+                umma_commit(full);
             }
             __syncwarp();
         };
-        if (ok) ok = issue_s(0);
-        if (ok) issue_dp(0);
-        for (int j = 0; j < n_kv && ok; ++j) {
-            const int s = j % NST;
-            if (j + 1 < n_kv) {
-                ok = issue_s(j + 1);  // as soon as S(j) is in registers
-                if (!ok) break;
+        if (warp == kMmaSWarp) {
+            for (int j = 0; j < n_kv && ok; ++j) {
+                const int s = j % NST;
+                ok = mbar_wait_warp(&bar_kv_full[s], (j / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+                for (int half = 0; half < 2 && ok; ++half) {
+                    if (j > 0) ok = mbar_wait_warp(&bar_s_loaded[half], uint32_t(j - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    issue_half(Cfg::kColS, Cfg::kColQ, stage_k(s), half, &bar_s_full[half]);
+                }
             }
-            ok = mbar_wait_warp(bar_ds_full, uint32_t(j) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
-            if (!ok) break;
-            tc_fence_after_sync();
-            if (elect_one()) {
-                // dQ += dS K_j
-                wide_ts<D>(tmem + Cfg::kColAcc, tmem + Cfg::kColDP, mnmajor_desc<D>(stage_k(s)), idesc_acc, j > 0);
-                umma_commit(&bar_kv_free[s]);
+        } else {
+            if (ok) ok = mbar_wait_warp(&bar_kv_full[0], 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+            if (ok) {
+                tc_fence_after_sync();
+                for (int half = 0; half < 2; ++half) issue_half(Cfg::kColDP, Cfg::kColDO, stage_v(0), half, &bar_dp_full[half]);
             }
+            for (int j = 0; j < n_kv && ok; ++j) {
+                const int s = j % NST, s1 = (j + 1) % NST;
+                const uint64_t k_desc = mnmajor_desc<D>(stage_k(s));
+                if (j + 1 < n_kv) ok = mbar_wait_warp(&bar_kv_full[s1], ((j + 1) / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+                for (int half = 0; half < 2 && ok; ++half) {
+                    ok = mbar_wait_warp(&bar_ds_full[half], uint32_t(j) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    if (elect_one()) {
+                        // dQ += dS K over the half's 64 keys: 4 K steps, two per part
+#pragma unroll
+                        for (int ks = 0; ks < 4; ++ks)
+                            umma_ts(tmem + Cfg::kColAcc, tmem + Cfg::kColDP + half * 64 + (ks >> 1) * 32 + (ks & 1) * 8,
+                                    k_desc + uint64_t((half * 4 + ks) * 128), idesc_acc, j > 0 || half > 0 || ks > 0);
+                        if (half == 1) umma_commit(&bar_kv_free[s]);
+                    }
+                    __syncwarp();
+                    // behind the product that reads dS out of the block
+                    if (j + 1 < n_kv) issue_half(Cfg::kColDP, Cfg::kColDO, stage_v(s1), half, &bar_dp_full[half]);
+                }
+            }
+            if (elect_one()) umma_commit(bar_acc);
             __syncwarp();
-            if (j + 1 < n_kv) issue_dp(j + 1);
+            // nothing may be in flight when TMEM is freed (the compute warps have waited for the other warp's products)
+            if (ok) mbar_wait_warp(bar_acc, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
         }
-        if (elect_one()) umma_commit(bar_acc);
-        __syncwarp();
     } else {
         // ------------------------------------------------------------------ compute
-        const int w4 = warp & 3, half = warp >> 2;
+        const int w4 = warp & 3, part = (warp >> 2) & 1, half = warp >> 3;
         const int row = w4 * 32 + lane;  // query row in the tile == TMEM lane
         const uint32_t lane_base = uint32_t(w4 * 32) << 16;
-        const int c0 = half * 64;  // first key column of this thread's half
-        const size_t vrow = (size_t(b) * p.Hq + h) * p.Tpad + q0 + row;
-        // preprocess for the warp's 32 rows (both halves compute it, half 0 stores it for the dK/dV pass)
+        const int c0 = half * 64 + part * 32;  // first key column of this thread
         float lse2 = INFINITY, dv = 0.f;
         {
+            // preprocess D = rowsum(O * dO): the four warps that share 32 rows take 8 each
             constexpr int LPR = D / 8, RPP = 32 / LPR;
             const size_t tile_off = size_t(b) * p.q_sb + size_t(h) * p.q_sh;
+            const int r0 = w4 * 32 + (warp >> 2) * 8;
+            const float lse_raw = q0 + row < p.T ? p.lse[(size_t(b) * p.Hq + h) * p.T + q0 + row] : INFINITY;
 #pragma unroll
-            for (int i = 0; i < LPR; ++i) {
-                const int r = q0 + w4 * 32 + i * RPP + lane / LPR;
+            for (int i = 0; i < 8 / RPP; ++i) {
+                const int r = r0 + i * RPP + lane / LPR;
                 float acc = 0.f;
-                if (r < p.T) {
-                    const size_t off = tile_off + size_t(r) * p.q_st + (lane % LPR) * 8;
+                if (q0 + r < p.T) {
+                    const size_t off = tile_off + size_t(q0 + r) * p.q_st + (lane % LPR) * 8;
                     const uint4 a = *reinterpret_cast<const uint4*>(p.o + off);
                     const uint4 g = *reinterpret_cast<const uint4*>(p.dout + off);
                     const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
@@ -765,30 +769,29 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
                 }
 #pragma unroll
                 for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                const float v = __shfl_sync(0xffffffffu, acc, (lane % RPP) * LPR);
-                if (lane / RPP == i) dv = v;
+                if (lane % LPR == 0) sD[r] = acc;
             }
-            if (q0 + row < p.T) lse2 = p.lse[(size_t(b) * p.Hq + h) * p.T + q0 + row] * 1.4426950408889634f;
-            if (half == 0) {
+            lse2 = lse_raw * 1.4426950408889634f;
+            named_bar_sync(1, Cfg::kComputeThreads);
+            dv = sD[row];
+            if (warp < 4) {
+                const size_t vrow = (size_t(b) * p.Hq + h) * p.Tpad + q0 + row;
                 p.lse2_w[vrow] = lse2;
                 p.dvec_w[vrow] = dv;
             }
         }
-        // this row of Q (half 0) or dO (half 1) from the swizzled tile in shared memory into tensor memory: the 256
-        // bytes of the row are the 64 BF16-pair columns of lane `row` as they stand
+        // 64 elements (box `part`) of this row of Q (half 0) or dO (half 1) from the swizzled tile in shared memory into tensor
+        // memory: its 128 bytes are 32 BF16-pair columns of lane `row` as they stand
         bool ok = mbar_wait_warp(bar_q, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
         if (ok) {
-            const uint8_t* tile = half == 0 ? sQ : sdO;
+            const uint8_t* tile = (half == 0 ? sQ : sdO) + part * Cfg::kBoxBytes + row * 128;
+            uint32_t tw[32];
 #pragma unroll
-            for (int bx = 0; bx < Cfg::kBoxes; ++bx) {
-                uint32_t tw[32];
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const uint4 w = *reinterpret_cast<const uint4*>(tile + bx * Cfg::kBoxBytes + row * 128 + ((c ^ (row & 7)) << 4));
-                    tw[4 * c] = w.x, tw[4 * c + 1] = w.y, tw[4 * c + 2] = w.z, tw[4 * c + 3] = w.w;
-                }
-                tmem_st_x32(tmem + lane_base + (half == 0 ? Cfg::kColQ : Cfg::kColDO) + bx * 32, tw);
+            for (int c = 0; c < 8; ++c) {
+                const uint4 w = *reinterpret_cast<const uint4*>(tile + ((c ^ (row & 7)) << 4));
+                tw[4 * c] = w.x, tw[4 * c + 1] = w.y, tw[4 * c + 2] = w.z, tw[4 * c + 3] = w.w;
             }
+            tmem_st_x32(tmem + lane_base + (half == 0 ? Cfg::kColQ : Cfg::kColDO) + part * 32, tw);
             tmem_wait_st();
             tc_fence_before_sync();
             // the producer re-uses the two tiles as a K/V stage once this barrier completes: the ordinary reads
@@ -796,62 +799,65 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
             fence_proxy_async_smem();
             mbar_arrive(bar_qt_full);
         }
+        const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), neg_l2 = pack_f32x2(-lse2, -lse2), neg_d2 = pack_f32x2(-dv, -dv);
         for (int j = 0; j < n_kv && ok; ++j) {
-            ok = mbar_wait_warp(bar_s_full, uint32_t(j) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+            ok = mbar_wait_warp(&bar_s_full[half], uint32_t(j) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
             if (!ok) break;
             tc_fence_after_sync();
             // phase A: P from S (the scores leave tensor memory in one go)
-            float pr[64];
+            float pr[32];
             {
-                uint32_t sv[64];
+                uint32_t sv[32];
                 tmem_ld_x32(tmem + lane_base + Cfg::kColS + c0, sv);
-                tmem_ld_x32(tmem + lane_base + Cfg::kColS + c0 + 32, sv + 32);
                 tmem_wait_ld();
                 tc_fence_before_sync();
-                mbar_arrive(bar_s_loaded);
+                mbar_arrive(&bar_s_loaded[half]);
 #pragma unroll
-                for (int i = 0; i < 64; ++i) pr[i] = ex2_approx(fmaf(__uint_as_float(sv[i]), p.scale_log2, -lse2));
+                for (int i = 0; i < 32; i += 2) {
+                    float x0, x1;
+                    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), scale2, neg_l2), x0, x1);
+                    pr[i] = ex2_approx(x0);
+                    pr[i + 1] = ex2_approx(x1);
+                }
             }
             if (j == qt) {
 #pragma unroll
-                for (int i = 0; i < 64; ++i)
+                for (int i = 0; i < 32; ++i)
                     if (c0 + i > row) pr[i] = 0.f;  // key above the diagonal
             }
-            ok = mbar_wait_warp(bar_dp_full, uint32_t(j) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+            ok = mbar_wait_warp(&bar_dp_full[half], uint32_t(j) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
             if (!ok) break;
             tc_fence_after_sync();
-            // phase B: dS = P (dP - D), written over dP as BF16
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
+            // phase B: dS = P (dP - D), written as BF16 over the first 16 of the thread's dP columns
+            {
                 uint32_t dp[32], pk[16];
-                tmem_ld_x32(tmem + lane_base + Cfg::kColDP + c0 + c * 32, dp);
+                const uint32_t t_dp = tmem + lane_base + Cfg::kColDP + c0;
+                tmem_ld_x32(t_dp, dp);
                 tmem_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    pk[i] = pack_bf16x2(pr[c * 32 + 2 * i] * (__uint_as_float(dp[2 * i]) - dv),
-                                        pr[c * 32 + 2 * i + 1] * (__uint_as_float(dp[2 * i + 1]) - dv));
-                tmem_st_x16(tmem + lane_base + Cfg::kColDP + c0 + c * 16, pk);
+                for (int i = 0; i < 32; i += 2) {
+                    float y0, y1;
+                    unpack_f32x2(mul_f32x2(pack_f32x2(pr[i], pr[i + 1]),
+                                           add_f32x2(pack_f32x2(__uint_as_float(dp[i]), __uint_as_float(dp[i + 1])), neg_d2)), y0, y1);
+                    pk[i / 2] = pack_bf16x2(y0, y1);
+                }
+                tmem_st_x16(t_dp, pk);
             }
             tmem_wait_st();
             tc_fence_before_sync();
-            mbar_arrive(bar_ds_full);
+            mbar_arrive(&bar_ds_full[half]);
         }
-        if (ok) ok = mbar_wait(bar_acc, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
-        ok = __all_sync(0xffffffffu, ok);
+        if (ok) ok = mbar_wait_warp(bar_acc, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
         if (ok) {
             tc_fence_after_sync();
-#pragma unroll
-            for (int c = 0; c < D / 64; ++c) {
-                uint32_t v[32];
-                const int col = half * (D / 2) + c * 32;
-                tmem_ld_x32(tmem + lane_base + Cfg::kColAcc + col, v);
-                tmem_wait_ld();
-                stage_row_chunk<D>(sQ, row, col, v, p.scale);
-            }
+            uint32_t v[32];
+            tmem_ld_x32(tmem + lane_base + Cfg::kColAcc + c0, v);
+            tmem_wait_ld();
+            stage_row_chunk<D>(sQ, row, c0, v, p.scale);
             fence_proxy_async_smem();
         }
         tc_fence_before_sync();
-        named_bar_sync(1, 256);
+        named_bar_sync(1, Cfg::kComputeThreads);
         if (ok && tid == 0) {
 #pragma unroll
             for (int bx = 0; bx < Cfg::kBoxes; ++bx) tma_store_4d(&tmdQ, sQ + bx * Cfg::kBoxBytes, bx * 64, q0, h, b);
@@ -862,7 +868,7 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 9) {
+    if (warp == kMmaSWarp) {
         tc_fence_after_sync();
         tmem_dealloc(tmem, Cfg::kTmemCols);
     }

@@ -446,7 +446,7 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk64, const CUtensorMap
     const unsigned dq_items = (unsigned)(p.n_tiles * p.Hq * p.B);
     cudaError_t e;
     if constexpr (kWide) {
-        e = launch_pdl(attn_bwd_dq_wide_kernel<D>, dq_items, 320, DqWideCfg<D>::kSmemBytes, st, tq, tk, tv, tdo, tdq, p);
+        e = launch_pdl(attn_bwd_dq_wide_kernel<D>, dq_items, DqWideCfg<D>::kThreads, DqWideCfg<D>::kSmemBytes, st, tq, tk, tv, tdo, tdq, p);
     } else {
         // the D = 64 kernel is persistent: two CTAs per SM walk the item list
         const unsigned dq_grid = std::min(dq_items, 2u * (unsigned)sm_count());
