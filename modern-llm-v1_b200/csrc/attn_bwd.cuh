@@ -443,6 +443,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             mbar_arrive(bar_qt_full);
             return true;
         };
+        const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2);
         int g0 = 0, n = 0;
         int id = get_item(0);
         if (id >= 0) ok = item_head(0, id);
@@ -464,7 +465,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                     tc_fence_before_sync();
                     mbar_arrive(bar_s_loaded);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) pr[i] = ex2_approx(fmaf(__uint_as_float(sv[i]), p.scale_log2, -lse2));
+                    for (int i = 0; i < 32; i += 2) {
+                        float x0, x1;
+                        unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), scale2, pack_f32x2(-lse2, -lse2)), x0, x1);
+                        pr[i] = ex2_approx(x0);
+                        pr[i + 1] = ex2_approx(x1);
+                    }
                 }
                 const int kbase = j * Cfg::kKeys;
                 if (kbase + Cfg::kKeys - 1 > q0) {
@@ -485,9 +491,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                     tmem_ld_x32(t_dp, dp);
                     tmem_wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        pk[i] = pack_bf16x2(pr[2 * i] * (__uint_as_float(dp[2 * i]) - dv),
-                                            pr[2 * i + 1] * (__uint_as_float(dp[2 * i + 1]) - dv));
+                    for (int i = 0; i < 32; i += 2) {
+                        float y0, y1;
+                        unpack_f32x2(mul_f32x2(pack_f32x2(pr[i], pr[i + 1]),
+                                               add_f32x2(pack_f32x2(__uint_as_float(dp[i]), __uint_as_float(dp[i + 1])), pack_f32x2(-dv, -dv))), y0, y1);
+                        pk[i / 2] = pack_bf16x2(y0, y1);
+                    }
                     tmem_st_x16(t_dp, pk);
                 }
                 tmem_wait_st();
