@@ -48,6 +48,8 @@ struct BwdParams {
     long long k_st, k_sh, k_sb;  // element strides of the k layout: token, head, batch
     int* sched;   // two words of the device-wide item counter of the persistent dQ pass (see ptx.cuh), or nullptr
     int* sched2;  // the same for the dK/dV pass
+    int split;    // dK/dV pass: CTAs (a cluster) that share an item's units; 1 except in the split kernel
+    FastDiv div_split;
     FastDiv div_bhq, div_hq, div_bhkv, div_hkv, div_group;  // division by B * Hq, Hq, B * Hkv, Hkv and the group size
 };
 
@@ -899,7 +901,10 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 // us: B=16 T=1024 16/4 D=64 94.7 -> 84.5, B=8 T=2000 16/4 D=64 171 -> 148, B=4 T=4096 16/4 D=128 496 -> 468.  Two groups of eight
 // warps on alternate units (64 columns a thread) were slower: 93 to 117 at the first of these, they spill.
 // ---------------------------------------------------------------------------------------
-template <int D>
+// SPLIT: few, long items (few sequences and key/value heads).  A CTA works on a share of ONE item's units, and the CTAs of a
+// cluster add up their accumulators through distributed shared memory in the order of the units, each finishing
+// 128 / split of the key rows.
+template <int D, bool SPLIT>
 __global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                      const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO, const BwdParams p) {
@@ -946,7 +951,12 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     auto item_rest = [&](int id) { return id - item_kt(id) * n_bh; };  // b * Hkv + hk
     auto item_b = [&](int id) { return int(fastdiv(unsigned(item_rest(id)), p.div_hkv)); };
     auto item_hk = [&](int id) { return item_rest(id) - item_b(id) * p.Hkv; };
-    auto item_units = [&](int id) { return p.group * (p.n_tiles - item_kt(id)); };
+    // units of an item that are this CTA's: [u_first, u_first + item_units); SPLIT: of cluster CTA r, [units r / split, ...)
+    const int split_id = SPLIT ? int(fastdiv(blockIdx.x, p.div_split)) : 0, rank = SPLIT ? int(blockIdx.x) - split_id * p.split : 0;
+    auto item_all = [&](int id) { return p.group * (p.n_tiles - item_kt(id)); };
+    auto share_begin = [&](int r) { return int(fastdiv(unsigned(item_all(split_id) * r), p.div_split)); };
+    const int u_first = SPLIT ? share_begin(rank) : 0;
+    auto item_units = [&](int id) { return SPLIT ? share_begin(rank + 1) - u_first : item_all(id); };
     auto get_item = [&](int n) { return item_get(bar_item, item_ring, n, abort_flag, p.status); };
 
     B200ATTN_TRACE_BEGIN(2);
@@ -1001,16 +1011,17 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         reg_dealloc<Cfg::kRegsOther>();
         int u = 0;  // units issued so far by this CTA (ring position)
         bool ok = true;
-        int id = blockIdx.x;  // the first item needs no fetch
+        int id = SPLIT ? split_id : blockIdx.x;  // the first item needs no fetch
         int id_next = 0;      // lane 0: the id fetched for the next item
+        if (SPLIT && item_units(id) == 0) ok = false;
         if (lane == 0) {
-            item_publish(bar_item, item_ring, 0, id);
-            id_next = sched_fetch(p.sched2, 1, int(blockIdx.x), int(gridDim.x));
+            item_publish(bar_item, item_ring, 0, ok ? id : -1);
+            id_next = SPLIT ? n_items : sched_fetch(p.sched2, 1, int(blockIdx.x), int(gridDim.x));
         }
         __syncwarp();
         for (int n = 0; ok; ++n) {
             const int kt = item_kt(id), hk = item_hk(id), b = item_b(id), k0 = kt * 128;
-            const int n_i = p.n_tiles - kt, n_it = p.group * n_i;
+            const int n_it = item_units(id), n_i = p.n_tiles - kt, h_skip = SPLIT ? u_first / n_i : 0;
             const int kb = n % NKV;
             if (n >= NKV) ok = mbar_wait_warp(&bar_kv_free[kb], uint32_t(n / NKV - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
             if (!ok) break;
@@ -1027,7 +1038,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             // ring has been filled for this item
             const int j_next = max(min(n_it, NST) - 1, n_it - 2);
             int id_new = n_items;
-            for (int it = 0, h = hk * p.group, i = kt; it < n_it; ++it, ++u, i = (i + 1 == p.n_tiles ? kt : i + 1), h += (i == kt)) {
+            for (int it = 0, h = hk * p.group + h_skip, i = kt + u_first - h_skip * n_i; it < n_it; ++it, ++u, i = (i + 1 == p.n_tiles ? kt : i + 1), h += (i == kt)) {
                 const int s = u % NST;
                 if (u >= NST) ok = mbar_wait_warp(&bar_free[s], uint32_t(u / NST - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
                 if (!ok) break;
@@ -1057,7 +1068,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             if (!ok || id_new >= n_items) break;
             id = id_new;
         }
-        if (ok && lane == 0) sched_finish(p.sched2, int(gridDim.x));
+        if (!SPLIT && ok && lane == 0) sched_finish(p.sched2, int(gridDim.x));
     } else if (warp == kVecWarp) {
         // ------------------------------------------------------------------ row vectors
         // L and D are the same for a whole column of S^T and dP^T, so reading them costs the compute warps 32 shared-memory
@@ -1251,7 +1262,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         for (int id; ok && (id = get_item(n)) >= 0; ++n) {
             const int n_i = p.n_tiles - item_kt(id);
             // units of the item: for each query head of the group, the query tiles from the diagonal down
-            for (int it = p.group * n_i, i_in = 0; it > 0; --it, ++u, i_in = (i_in + 1 == n_i ? 0 : i_in + 1)) {
+            for (int it = item_units(id), i_in = SPLIT ? u_first % n_i : 0; it > 0; --it, ++u, i_in = (i_in + 1 == n_i ? 0 : i_in + 1)) {
                 const int s = u % NST;
                 const bool diag = i_in == 0;
                 ok = mbar_wait_warp(bar_s_full, uint32_t(u) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
@@ -1333,9 +1344,69 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             pending = true;
             pend_id = id;
         }
-        if (ok && pending) epilogue(n - 1, pend_id);
+        if constexpr (SPLIT) {
+            if (ok && pending) mbar_wait_warp(bar_acc, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+        } else if (ok && pending) {
+            epilogue(n - 1, pend_id);
+        }
     }
 
+    if constexpr (SPLIT) {
+        // Every role comes here, also after a wait that gave up.  Key row r is finished by CTA r / rows of the cluster; the
+        // tiles in shared memory make room for the arrivals, so all CTAs must be through with theirs first.
+        const int rows = 128 / p.split;
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        if (tid < Cfg::kComputeThreads && item_units(split_id) > 0) {
+            tc_fence_after_sync();
+            const int row = (warp & 3) * 32 + lane, part = warp >> 2, to = (row * p.split) >> 7, r = row - to * rows;
+            // [source CTA][row][dV: D, dK: D] FP32, 16-byte pieces swizzled by the row: the rows of a warp would share a bank
+            uint8_t* own = smem + (rank * rows + r) * D * 8;
+            const uint32_t dst = cluster_addr(own, to);
+            const uint32_t t_acc = tmem + (uint32_t((warp & 3) * 32) << 16) + (part < 2 ? Cfg::kColAcc0 : Cfg::kColAcc1) + (part & 1) * (D / 2);
+#pragma unroll
+            for (int c = 0; c < D / 64; ++c) {
+                uint32_t v[32];
+                tmem_ld_x32(t_acc + c * 32, v);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int at = ((part * (D / 8) + c * 8 + i) ^ (r & 7)) << 4;
+                    if (to == rank)
+                        *reinterpret_cast<uint4*>(own + at) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                    else
+                        cluster_store_4(dst + at, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                }
+            }
+            tc_fence_before_sync();
+        }
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        if (tid < Cfg::kComputeThreads) {
+            const int k0 = item_kt(split_id) * 128 + rank * rows, b = item_b(split_id), hk = item_hk(split_id);
+            for (int i = tid; i < rows * (D / 4); i += Cfg::kComputeThreads) {  // eight columns each: dV, then dK
+                const int r = i / (D / 4), c8 = i % (D / 4);
+                if (k0 + r >= p.T) break;
+                float acc[8] = {};
+#pragma unroll 2
+                for (int k = 0; k < p.split; ++k) {
+                    if (share_begin(k + 1) == share_begin(k)) continue;  // nothing was sent
+                    const uint8_t* src = smem + (k * rows + r) * D * 8;
+                    const float4 v0 = *reinterpret_cast<const float4*>(src + (((c8 * 2) ^ (r & 7)) << 4));
+                    const float4 v1 = *reinterpret_cast<const float4*>(src + (((c8 * 2 + 1) ^ (r & 7)) << 4));
+                    acc[0] += v0.x, acc[1] += v0.y, acc[2] += v0.z, acc[3] += v0.w;
+                    acc[4] += v1.x, acc[5] += v1.y, acc[6] += v1.z, acc[7] += v1.w;
+                }
+                const bool is_dk = c8 >= D / 8;
+                const float mul = is_dk ? p.scale : 1.f;
+                uint16_t* out = (is_dk ? p.dk : p.dv) + size_t(b) * p.k_sb + size_t(hk) * p.k_sh + size_t(k0 + r) * p.k_st + (c8 % (D / 8)) * 8;
+                *reinterpret_cast<uint4*>(out) = make_uint4(pack_bf16x2(acc[0] * mul, acc[1] * mul), pack_bf16x2(acc[2] * mul, acc[3] * mul),
+                                                            pack_bf16x2(acc[4] * mul, acc[5] * mul), pack_bf16x2(acc[6] * mul, acc[7] * mul));
+            }
+        }
+    }
     tc_fence_before_sync();
     __syncthreads();
     if (warp == kMmaSWarp) {

@@ -428,6 +428,15 @@ int launch_bwd_onepass(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
     return B200ATTN_OK;
 }
 
+// CTAs that share an item's units in the dK/dV pass.  1 unless the items leave SMs idle (one CTA per SM) and the longest has
+// units enough: a unit takes about 1.4 us at D = 64 and 1.9 at D = 128, the exchange at the end 2 to 3 us.  Clusters of more
+// than two CTAs do not fill the last SMs of a GPC, so these are held to 128 CTAs.
+int dkdv_split(long long items, int longest) {
+    int split = 1;
+    while (split < 8 && items * split * 2 <= (split == 1 ? sm_count() : std::min(sm_count(), 128)) && longest >= 6 * split) split *= 2;
+    return split;
+}
+
 template <int D>
 int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk64, const CUtensorMap& tv64, const CUtensorMap& tk,
                const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& to, const CUtensorMap& tdq,
@@ -439,7 +448,7 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk64, const CUtensorMap
     if constexpr (kWide) rc = set_smem_once(attn_bwd_dq_wide_kernel<D>, DqWideCfg<D>::kSmemBytes, dq_set);
     else rc = set_smem_once(attn_bwd_dq_kernel<D>, DqCfg<D>::kSmemBytes, dq_set);
     if (rc) return rc;
-    rc = set_smem_once(attn_bwd_dkdv_kernel<D>, BwdCfg<D>::kSmemBytes, dkdv_set);
+    rc = set_smem_once(attn_bwd_dkdv_kernel<D, false>, BwdCfg<D>::kSmemBytes, dkdv_set);
     if (rc) return rc;
     record_bwd_event(0, st);
     // the dQ pass also writes the two per-row vectors the dK/dV pass reads
@@ -462,11 +471,20 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk64, const CUtensorMap
     record_bwd_event(1, st);
     // the dK/dV pass is persistent too: one CTA per SM walks the list of (key tile, KV head, batch) items
     const unsigned kv_items = (unsigned)(p.n_tiles * p.Hkv * p.B);
-    const unsigned kv_grid = std::min(kv_items, (unsigned)sm_count());
     BwdParams pk = p;
-    pk.sched2 = next_sched_pair(kv_items, kv_grid);
-    if (launch_pdl(attn_bwd_dkdv_kernel<D>, kv_grid, BwdCfg<D>::kThreads, BwdCfg<D>::kSmemBytes, st, tk, tv, tq, tdo,
-                   pk) != cudaSuccess) {
+    pk.split = dkdv_split(kv_items, p.group * p.n_tiles);
+    pk.div_split = fastdiv_make((unsigned)pk.split);
+    if (pk.split > 1) {
+        static bool set[kMaxDevices] = {false};
+        if ((rc = set_smem_once(attn_bwd_dkdv_kernel<D, true>, BwdCfg<D>::kSmemBytes, set))) return rc;
+        e = launch_cluster(attn_bwd_dkdv_kernel<D, true>, dim3(kv_items * (unsigned)pk.split), BwdCfg<D>::kThreads, BwdCfg<D>::kSmemBytes, st,
+                           pk.split, tk, tv, tq, tdo, pk);
+    } else {
+        const unsigned kv_grid = std::min(kv_items, (unsigned)sm_count());
+        pk.sched2 = next_sched_pair(kv_items, kv_grid);
+        e = launch_pdl(attn_bwd_dkdv_kernel<D, false>, kv_grid, BwdCfg<D>::kThreads, BwdCfg<D>::kSmemBytes, st, tk, tv, tq, tdo, pk);
+    }
+    if (e != cudaSuccess) {
         cudaGetLastError();
         return B200ATTN_ERR_CUDA;
     }
