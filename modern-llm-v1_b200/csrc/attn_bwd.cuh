@@ -72,7 +72,8 @@ struct BwdCfg {
     static constexpr bool kVecOps = D == 64;             // the row vectors enter the products (see the row-vector warp)
     static constexpr int kOpBytes = 128 * 16;            // a row vector as MMA operand: 8 BF16 per row
     static constexpr int kOpsBytes = kVecOps ? (2 * kStages + 2) * kOpBytes : 0;  // two per stage, ones, zeros
-    static constexpr int kSmemBytes = (2 * kKvBufs + 2 * kStages) * kTileBytes + kVecBytes + kOpsBytes + kBarBytes + 1024;
+    static constexpr int kOutBytes = D == 64 ? 0 : (kComputeThreads / 32) * kRowStageBytes;  // D = 64: in the item's own K/V tiles
+    static constexpr int kSmemBytes = (2 * kKvBufs + 2 * kStages) * kTileBytes + kOutBytes + kVecBytes + kOpsBytes + kBarBytes;
     static_assert(kSmemBytes <= 232448, "shared memory of an SM");
     static constexpr int kTmemCols = 512;
     static constexpr int kDpBufs = D == 64 ? 2 : 1;
@@ -163,7 +164,9 @@ struct DqCfg {
     static constexpr int kKVTileBytes = kKeys * D * 2;
     static constexpr int kKVBoxBytes = kKeys * 64 * 2;
     static constexpr int kBoxes = D / 64;
-    static constexpr int kSmemBytes = 3 * kQTileBytes + 2 * kStages * kKVTileBytes + 512 + 1024;  // Q, dO, O + ring + barriers
+    static constexpr int kOutBytes = 8 * kRowStageBytes;  // per compute warp: its output rows on their way to global memory
+    static constexpr int kSmemBytes = 3 * kQTileBytes + 2 * kStages * kKVTileBytes + kOutBytes + 512;  // Q, dO, O + ring + barriers
+    static_assert(2 * (kSmemBytes + 1024) <= 228 * 1024, "two CTAs per SM");
     static constexpr int kTmemCols = 256;
     static constexpr int kCtasPerSm = 2;
     static constexpr int kColS = 0, kColDP = 64, kColAcc = 128, kColQ = 192, kColDO = 224;
@@ -182,14 +185,14 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     static_assert(D == 64, "the persistent dQ pass keeps Q and dO in 64 tensor-memory columns: D = 64 only");
     using Cfg = DqCfg<D>;
     constexpr int NST = Cfg::kStages;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sQ = smem;
     uint8_t* sdO = sQ + Cfg::kQTileBytes;
     uint8_t* sO = sdO + Cfg::kQTileBytes;
     uint8_t* sK = sO + Cfg::kQTileBytes;         // [NST]
     uint8_t* sV = sK + NST * Cfg::kKVTileBytes;  // [NST]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + NST * Cfg::kKVTileBytes);
+    uint8_t* sOut = sV + NST * Cfg::kKVTileBytes;  // [8 warps]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + Cfg::kOutBytes);
     uint64_t* bar_q = bars + 0;         // Q, dO, O of an item have landed in shared memory      (phase: item)
     uint64_t* bar_qs_free = bars + 1;   // the compute warps have read those three tiles          (phase: item)
     uint64_t* bar_qt_full = bars + 2;   // Q and dO of an item are in tensor memory               (phase: item)
@@ -526,18 +529,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             tmem_wait_ld();
             tc_fence_before_sync();
             mbar_arrive(bar_acc_free);  // the MMA warp may start the next item's accumulation
-            if (q0 + row < p.T) {
-                uint16_t* dqrow = p.dq + size_t(b) * p.q_sb + size_t(h) * p.q_sh + size_t(q0 + row) * p.q_st + part * kCols;
+            uint32_t w[kCols / 2];
 #pragma unroll
-                for (int gq = 0; gq < kCols / 8; ++gq) {
-                    uint4 w;
-                    w.x = pack_bf16x2(__uint_as_float(v[gq * 8 + 0]) * p.scale, __uint_as_float(v[gq * 8 + 1]) * p.scale);
-                    w.y = pack_bf16x2(__uint_as_float(v[gq * 8 + 2]) * p.scale, __uint_as_float(v[gq * 8 + 3]) * p.scale);
-                    w.z = pack_bf16x2(__uint_as_float(v[gq * 8 + 4]) * p.scale, __uint_as_float(v[gq * 8 + 5]) * p.scale);
-                    w.w = pack_bf16x2(__uint_as_float(v[gq * 8 + 6]) * p.scale, __uint_as_float(v[gq * 8 + 7]) * p.scale);
-                    *reinterpret_cast<uint4*>(dqrow + gq * 8) = w;
-                }
-            }
+            for (int i = 0; i < kCols / 2; ++i) w[i] = pack_bf16x2(__uint_as_float(v[2 * i]) * p.scale, __uint_as_float(v[2 * i + 1]) * p.scale);
+            store_rows_64b(sOut + warp * kRowStageBytes, w, lane,
+                           p.dq + size_t(b) * p.q_sb + size_t(h) * p.q_sh + size_t(q0 + w4 * 32) * p.q_st + part * kCols, p.q_st,
+                           p.T - (q0 + w4 * 32));
             B200ATTN_STAMP(tid == 0, 400 + 4 * n + 3);
             id = id_next;
             ++n;
@@ -912,13 +909,13 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     constexpr int NST = Cfg::kStages;
     constexpr int NKV = Cfg::kKvBufs;
     constexpr int NDP = Cfg::kDpBufs;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sK = smem;                         // [NKV]
     uint8_t* sV = sK + NKV * Cfg::kTileBytes;   // [NKV]
     uint8_t* sQ = sV + NKV * Cfg::kTileBytes;   // [NST]
     uint8_t* sdO = sQ + NST * Cfg::kTileBytes;  // [NST]
-    float* sLse = reinterpret_cast<float*>(sdO + NST * Cfg::kTileBytes);  // [NST][128]
+    uint8_t* sOut = sdO + NST * Cfg::kTileBytes;  // per compute warp: a piece of its output rows (D = 128)
+    float* sLse = reinterpret_cast<float*>(sOut + Cfg::kOutBytes);        // [NST][128]
     float* sDv = sLse + NST * 128;                                        // [NST][128]
     uint8_t* sOps = reinterpret_cast<uint8_t*>(sLse) + Cfg::kVecBytes;    // kVecOps: [NST] L and D operands; ones; zeros
     uint8_t* sOnes = sOps + 2 * NST * Cfg::kOpBytes;
@@ -967,7 +964,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         tma_prefetch_desc(&tmdO);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bar_kv[i], 1);
-            mbar_init(&bar_kv_free[i], 2);  // each of the MMA warps reads K or V
+            // each of the MMA warps reads K or V; at D = 64 the epilogue stages its rows in the item's tiles
+            mbar_init(&bar_kv_free[i], 2 + (Cfg::kOutBytes == 0 && !SPLIT ? Cfg::kComputeThreads : 0));
             mbar_init(&bar_dp_full[i], 1);
             mbar_init(&bar_pds_full[i], Cfg::kComputeThreads);
         }
@@ -1228,29 +1226,26 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             const float mul = is_dk ? p.scale : 1.f;
             const int col0 = (part_e & 1) * kCols;
             const int k0 = item_kt(id_e) * 128;
-            const bool in_range = k0 + row < p.T;
+            uint8_t* stage = Cfg::kOutBytes > 0 ? sOut + warp * kRowStageBytes
+                                                : (is_dk ? sV : sK) + (n_item % NKV) * Cfg::kTileBytes + (warp & 7) * kRowStageBytes;
             uint16_t* out = (is_dk ? p.dk : p.dv) + size_t(item_b(id_e)) * p.k_sb + size_t(item_hk(id_e)) * p.k_sh +
-                            size_t(k0 + row) * p.k_st + col0;
+                            size_t(k0 + w4 * 32) * p.k_st + col0;
 #pragma unroll
             for (int c = 0; c < kCols / 32; ++c) {
-                uint32_t v[32];
+                uint32_t v[32], w[16];
                 tmem_ld_x32(tmem + lane_base + acc + col0 + c * 32, v);
                 tmem_wait_ld();
                 if (c + 1 == kCols / 32) {
                     tc_fence_before_sync();
                     mbar_arrive(bar_acc_free);  // the MMA warp may start the next item's accumulation
                 }
-                if (in_range) {
 #pragma unroll
-                    for (int g = 0; g < 4; ++g) {
-                        uint4 w;
-                        w.x = pack_bf16x2(__uint_as_float(v[g * 8 + 0]) * mul, __uint_as_float(v[g * 8 + 1]) * mul);
-                        w.y = pack_bf16x2(__uint_as_float(v[g * 8 + 2]) * mul, __uint_as_float(v[g * 8 + 3]) * mul);
-                        w.z = pack_bf16x2(__uint_as_float(v[g * 8 + 4]) * mul, __uint_as_float(v[g * 8 + 5]) * mul);
-                        w.w = pack_bf16x2(__uint_as_float(v[g * 8 + 6]) * mul, __uint_as_float(v[g * 8 + 7]) * mul);
-                        *reinterpret_cast<uint4*>(out + c * 32 + g * 8) = w;
-                    }
-                }
+                for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(__uint_as_float(v[2 * i]) * mul, __uint_as_float(v[2 * i + 1]) * mul);
+                store_rows_64b(stage, w, lane, out + c * 32, p.k_st, p.T - (k0 + w4 * 32));
+            }
+            if constexpr (Cfg::kOutBytes == 0) {
+                fence_proxy_async_smem();  // ordinary accesses before the next load (TMA) into the tiles
+                mbar_arrive(&bar_kv_free[n_item % NKV]);
             }
             B200ATTN_STAMP(tid == 0, 460 + 4 * n_item + 2);
             return true;

@@ -428,12 +428,13 @@ int launch_bwd_onepass(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
     return B200ATTN_OK;
 }
 
-// CTAs that share an item's units in the dK/dV pass.  1 unless the items leave SMs idle (one CTA per SM) and the longest has
-// units enough: a unit takes about 1.4 us at D = 64 and 1.9 at D = 128, the exchange at the end 2 to 3 us.  Clusters of more
-// than two CTAs do not fill the last SMs of a GPC, so these are held to 128 CTAs.
-int dkdv_split(long long items, int longest) {
+// CTAs that share an item's units in the dK/dV pass.  1 unless the items leave SMs idle (one CTA per SM) and twice the CTAs
+// save more than the exchange at the end costs: a unit takes about 1.4 us at D = 64 and 1.9 at D = 128, the exchange 3 and 7
+// (64 KB in and out of every CTA at D = 128, at the 13 bytes a clock of distributed shared memory).  Clusters of more than
+// two CTAs do not fill the last SMs of a GPC, so these are held to 128 CTAs.
+int dkdv_split(long long items, int longest, int D) {
     int split = 1;
-    while (split < 8 && items * split * 2 <= (split == 1 ? sm_count() : std::min(sm_count(), 128)) && longest >= 6 * split) split *= 2;
+    while (split < 8 && items * split * 2 <= (split == 1 ? sm_count() : std::min(sm_count(), 128)) && longest >= (D == 64 ? 5 : 8) * split) split *= 2;
     return split;
 }
 
@@ -472,7 +473,7 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk64, const CUtensorMap
     // the dK/dV pass is persistent too: one CTA per SM walks the list of (key tile, KV head, batch) items
     const unsigned kv_items = (unsigned)(p.n_tiles * p.Hkv * p.B);
     BwdParams pk = p;
-    pk.split = dkdv_split(kv_items, p.group * p.n_tiles);
+    pk.split = dkdv_split(kv_items, p.group * p.n_tiles, D);
     pk.div_split = fastdiv_make((unsigned)pk.split);
     if (pk.split > 1) {
         static bool set[kMaxDevices] = {false};

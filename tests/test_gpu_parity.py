@@ -44,6 +44,16 @@ def test_layouts_and_head_dims(D, layout):
     check_against_oracle(*_case(2, 300, 4, 2, D, seed=D), layout=layout)
 
 
+@pytest.mark.parametrize("B,T,Hq,Hkv,D", [
+    (1, 900, 6, 2, 64),    # dK/dV items split over 4 CTAs, shares that begin inside a query head
+    (1, 1100, 3, 1, 64),   # over 8
+    (2, 600, 8, 1, 128),   # over 8, uneven shares
+    (1, 1400, 2, 2, 128),  # one query head per KV head: the last items have fewer units than CTAs
+])
+def test_few_long_items_are_split(B, T, Hq, Hkv, D):
+    check_against_oracle(*_case(B, T, Hq, Hkv, D, seed=T))
+
+
 def test_reference_test_shapes_with_d64():
     # the D=64 shape of llm/tests/test_flash_attn.cu:72 ([B'=4, T=128, D=64], B' = batch x heads)
     # through the reference-shaped entry points
