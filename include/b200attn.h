@@ -21,6 +21,10 @@
  * replicated, which replaces repeat_kv_heads / accumulate_kv_grads
  * (llm/src/model/attention.cu:481-543).
  *
+ * A call gives the same bits whenever it is repeated.  The grouping of its FP32 sums depends on the sizes: a forward or
+ * dK/dV item may be shared by several CTAs when a problem has few or uneven items, so a batch and the same sequences one
+ * by one agree to FP32 rounding of those sums, not bit for bit.
+ *
  * Constraints (checked, B200ATTN_ERR_* otherwise): D in {64, 128}; Hq % Hkv == 0;
  * all sizes > 0; base pointers 16-byte aligned.
  */

@@ -73,9 +73,12 @@ struct DecodeCfg {
     static constexpr int kQRow = D * 2;
     static constexpr int kQBytes = 16 * kQRow;          // rows >= G stay zero
     static constexpr int kMlBytes = 4 * 16 * 8;         // (m, l) of the four warps' heads
-    static constexpr int kXBytes = 16 * D * 4 + kDecodeMaxCluster * 16 * 8;  // from the cluster: O slices, (m, l) rows
+    // from the cluster: O slices (over the second q buffer, which a CTA with one piece does not use) and (m, l) rows
+    static constexpr int kXBytes = 16 * D * 4, kXMlBytes = kDecodeMaxCluster * 16 * 8;
     static_assert(4 * 16 * D * 4 <= 2 * kTileBytes, "the warps' O rows are merged in one K/V stage");
-    static constexpr int kSmemBytes = 2 * kStages * kTileBytes + 2 * kQBytes + kMlBytes + kXBytes + 256 + 1024;
+    static constexpr int kSmemBytes = 2 * kStages * kTileBytes + kQBytes + kXBytes + kMlBytes + kXMlBytes + 256 + 1024;
+    static_assert(kXBytes >= kQBytes, "the second q buffer lies in the cluster's region");
+    static_assert(2 * (kSmemBytes + 1024) <= 228 * 1024, "two CTAs per SM");
 };
 
 // ---- warp-level tensor-core pieces (mma.sync is enough here: the kernel is bound by HBM and latency, and a unit has
@@ -348,10 +351,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sKV = smem;                                                 // [NST] K tile, V tile
     uint8_t* sQ = sKV + NST * 2 * Cfg::kTileBytes;                       // [2][16 rows]
-    float2* sMl = reinterpret_cast<float2*>(sQ + 2 * Cfg::kQBytes);      // [4 warps][16 heads]
-    float2* sX = sMl + 4 * 16;                                           // [CTA of the cluster][slice of the output pairs]
-    float2* sXMl = sX + 16 * D / 2;                                      // [CTA of the cluster][16 rows]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sQ + 2 * Cfg::kQBytes + Cfg::kMlBytes + Cfg::kXBytes);
+    float2* sX = reinterpret_cast<float2*>(sQ + Cfg::kQBytes);           // [CTA of the cluster][slice of the output pairs]
+    float2* sMl = reinterpret_cast<float2*>(sQ + Cfg::kQBytes + Cfg::kXBytes);  // [4 warps][16 heads]
+    float2* sXMl = sMl + 4 * 16;                                         // [CTA of the cluster][16 heads]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sXMl + kDecodeMaxCluster * 16);
     uint64_t* bar_full = bars;              // [NST]
     uint64_t* bar_free = bars + NST;        // [NST]
     uint64_t* bar_q = bars + 2 * NST;       // [2] the q rows of a piece have landed   (phase: piece / 2)
@@ -459,7 +462,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     }
 
     // ---------------------------------------------------------------------- compute warps
-    for (int i = tid; i < 2 * (16 - G) * (D / 8); i += 128) {  // rows >= G of both q buffers
+    for (int i = tid; i < (p.cluster > 1 ? 1 : 2) * (16 - G) * (D / 8); i += 128) {  // rows >= G of the q buffers
         const int buf = i / ((16 - G) * (D / 8)), r = i % ((16 - G) * (D / 8));
         *reinterpret_cast<uint4*>(sQ + buf * Cfg::kQBytes + (G + r / (D / 8)) * Cfg::kQRow + (r % (D / 8)) * 16) = make_uint4(0u, 0u, 0u, 0u);
     }

@@ -256,15 +256,37 @@ int set_smem_once(K kernel, int bytes, bool* done) {
     return B200ATTN_OK;
 }
 
-// CTAs that share an item's key tiles in the forward.  1 unless the items leave CTA slots free (two per SM) and are long: the
-// exchange at the end costs 2 to 3 us, which is what some 300 keys take, and about twice that where a second CTA on the SM
-// slows both down.  Clusters of more than two CTAs do not always fill the last SMs of a GPC, so these are held to 256 CTAs.
-int fwd_split(long long items, int keys) {
+// How many CTAs of a cluster share an item (forward: its key tiles, dK/dV pass: its units): the number with the smallest
+// estimate of the kernel's time, 1 unless another one is at least 5 % better.  Not only few items are split: 126 items of
+// 126 to 2 units on 148 SMs are bound by the longest one (dK/dV at B=1 T=8000 4/2 D=128: 229 -> 134 us).  The estimates were
+// held against measurements of some thirty shapes, most of which they meet within 15 %.
+struct SplitCosts {
+    int per_sm;                // CTAs of the kernel that fit an SM
+    float tile_one, tile_all;  // us per tile in a CTA that has the SM to itself, and with a second CTA beside it
+    float exchange, start;     // us: the exchange in a cluster of two, a CTA's start
+};
+int pick_split(long long items, int longest, double total, const SplitCosts& c) {
     const int sms = sm_count();
-    for (int split = 1;; split *= 2) {
-        const long long ctas = items * split * 2;
-        if (split == 8 || ctas > (split == 1 ? 2 * sms : std::min(2 * sms, 256)) || keys < 2 * split * (ctas > sms ? 768 : 384)) return split;
+    int best = 1;
+    double best_us = 1e30;
+    for (int split = 1; split <= 8; split *= 2) {
+        // clusters of four and eight do not fill the last SMs of a GPC: they get 132 and 120 of 148
+        const double slots = c.per_sm * (split <= 2 ? sms : split == 4 ? sms * 0.89 : sms * 0.81), ctas = (double)items * split;
+        const double shared = c.per_sm > 1 ? std::min(1.0, std::max(0.0, ctas / sms - 1)) : 0.0;  // SMs with two CTAs
+        const double share = (longest + split - 1) / split * (c.tile_one + (c.tile_all - c.tile_one) * shared);
+        const double all = total * c.tile_all / slots;
+        // in one round the longest share decides; in several the work, and what the last CTAs leave uneven
+        double us = split == 1 ? std::max(share, all) + c.start : (ctas <= slots ? share : all + 0.5 * share) + c.start * ceil(ctas / slots);
+        if (split > 1) us += c.exchange * (1 + shared) + (split == 4 ? 1.5 : split == 8 ? 4.0 : 0.0);
+        if (split == 1 || us < 0.95 * best_us) best = split, best_us = us;
+        if (ctas >= 4 * slots) break;
     }
+    return best;
+}
+// tiles of all items of a causal problem: query tiles of 128 rows behind kv_off keys, key tiles of `keys`
+double fwd_total_tiles(int n_qtiles, int kv_off, int T, int keys) {
+    const double last = (kv_off + T + keys - 1) / keys, first = (kv_off + std::min(T, 128) + keys - 1) / keys;
+    return n_qtiles * (first + last) / 2;
 }
 
 template <int D>
@@ -276,7 +298,8 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     pl.div_bh = fastdiv_make((unsigned)(p.B * p.Hq));
     pl.div_h = fastdiv_make((unsigned)p.Hq);
     pl.div_group = fastdiv_make((unsigned)p.group);
-    pl.split = fwd_split(items, p.kv_off + p.T);
+    constexpr SplitCosts kCosts = D == 64 ? SplitCosts{2, 1.25f, 1.95f, 2.f, 3.5f} : SplitCosts{2, 0.83f, 1.f, 3.5f, 3.5f};
+    pl.split = pick_split(items, (p.kv_off + p.T + Cfg::kKeys - 1) / Cfg::kKeys, (double)p.B * p.Hq * fwd_total_tiles(p.n_qtiles, p.kv_off, p.T, Cfg::kKeys), kCosts);
     pl.div_split = fastdiv_make((unsigned)pl.split);
     cudaError_t e;
     if (pl.split > 1) {
@@ -428,16 +451,6 @@ int launch_bwd_onepass(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
     return B200ATTN_OK;
 }
 
-// CTAs that share an item's units in the dK/dV pass.  1 unless the items leave SMs idle (one CTA per SM) and twice the CTAs
-// save more than the exchange at the end costs: a unit takes about 1.4 us at D = 64 and 1.9 at D = 128, the exchange 3 and 7
-// (64 KB in and out of every CTA at D = 128, at the 13 bytes a clock of distributed shared memory).  Clusters of more than
-// two CTAs do not fill the last SMs of a GPC, so these are held to 128 CTAs.
-int dkdv_split(long long items, int longest, int D) {
-    int split = 1;
-    while (split < 8 && items * split * 2 <= (split == 1 ? sm_count() : std::min(sm_count(), 128)) && longest >= (D == 64 ? 5 : 8) * split) split *= 2;
-    return split;
-}
-
 template <int D>
 int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk64, const CUtensorMap& tv64, const CUtensorMap& tk,
                const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& to, const CUtensorMap& tdq,
@@ -473,7 +486,9 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk64, const CUtensorMap
     // the dK/dV pass is persistent too: one CTA per SM walks the list of (key tile, KV head, batch) items
     const unsigned kv_items = (unsigned)(p.n_tiles * p.Hkv * p.B);
     BwdParams pk = p;
-    pk.split = dkdv_split(kv_items, p.group * p.n_tiles, D);
+    // (the exchange is 64 KB in and out of every CTA at D = 128, at the 13 bytes a clock of distributed shared memory)
+    constexpr SplitCosts kCosts = D == 64 ? SplitCosts{1, 1.4f, 1.4f, 3.f, 3.5f} : SplitCosts{1, 1.9f, 1.9f, 7.f, 3.5f};
+    pk.split = pick_split(kv_items, p.group * p.n_tiles, (double)p.B * p.Hq * p.n_tiles * (p.n_tiles + 1) / 2, kCosts);
     pk.div_split = fastdiv_make((unsigned)pk.split);
     if (pk.split > 1) {
         static bool set[kMaxDevices] = {false};
