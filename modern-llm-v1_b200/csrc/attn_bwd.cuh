@@ -250,6 +250,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tmem_relinquish();
     }
     grid_dep_wait();
+    grid_dep_launch();  // the dK/dV pass: only now, see there
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -622,7 +623,6 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     const int n_kv = qt + 1;
 
     B200ATTN_TRACE_BEGIN(1);
-    grid_dep_launch();
     if (warp == kProducerWarp && lane == 0) {
         tma_prefetch_desc(&tmQ);
         tma_prefetch_desc(&tmK);
@@ -652,6 +652,7 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         tmem_relinquish();
     }
     grid_dep_wait();
+    grid_dep_launch();  // the dK/dV pass: only now, see there
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -980,9 +981,6 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         }
         for (int i = 0; i < kItemRing; ++i) mbar_init(&bar_item[i], 1);
         fence_mbar_init();
-        // Everything above touched no global memory.  From here on the previous kernel of the stream
-        // (the dQ pass, which writes the two per-row vectors) must have completed.
-        grid_dep_wait();
         *abort_flag = *reinterpret_cast<volatile int*>(p.status);
     }
     if (Cfg::kVecOps && warp == kVecWarp) {  // ones: 1, 1, 1, 0, ... per row; zeros
@@ -996,7 +994,9 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         tmem_alloc(tmem_slot, Cfg::kTmemCols);
         tmem_relinquish();
     }
-    grid_dep_wait();
+    // No wait for the previous kernel of the stream here: it is the dQ pass, and that lets this grid in only when all its CTAs
+    // have passed their own wait, so everything before it is complete.  What it writes itself, the two row vectors, is waited
+    // for by the producer in front of their first load; K, V and the first Q and dO load meanwhile.
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -1049,6 +1049,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
                         tma_load_4d(sdO + s * Cfg::kTileBytes + bx * Cfg::kBoxBytes, &tmdO, &bar_full[s], bx * 64, i * 128,
                                     h, b);
                     }
+                    if (u == 0) grid_dep_wait();  // (the same lane issues all loads)
                     const size_t voff = (size_t(b) * p.Hq + h) * p.Tpad + size_t(i) * 128;
                     bulk_load_1d(sLse + s * 128, p.lse2 + voff, 512, &bar_full[s]);
                     bulk_load_1d(sDv + s * 128, p.dvec + voff, 512, &bar_full[s]);
