@@ -201,9 +201,10 @@ int b200attn_fwd_kvcache_at(const void* q, const void* kcache, const void* vcach
  * The same two calls for sequences of different lengths (a batch that does not advance in lock step).
  * b200attn_kv_append_at: pos [B] (device, int32) is the first position of each sequence's n_new tokens.  A
  * sequence whose pos[b] + n_new exceeds L_cap is skipped and sets the device status word to 105 (unless the word
- * already holds an earlier code).  While the status word is non-zero every kernel of this library on that device
- * returns at once without writing anything, although its launching call still returns B200ATTN_OK: check
- * b200attn_last_device_status (which reports the code and clears the word) before trusting later results.
+ * already holds an earlier code).  While the status word is non-zero every attention kernel of this library on that
+ * device (forward, backward, decode) returns at once without writing its outputs, although its launching call still
+ * returns B200ATTN_OK: check b200attn_last_device_status (which reports the code and clears the word) before trusting
+ * later results.  (The RoPE / QK-Norm and append kernels wait on nothing that can fail and run all the same.)
  * b200attn_decode_ragged: lens [B] (device, int32), 1 <= lens[b] <= L, is each sequence's cache length
  * (the newest token included); L is the host's upper bound on them: it sizes the grid, the splits and the
  * workspace (b200attn_decode_workspace_bytes with this L).  Rows lens[b] .. L-1 of a sequence's caches are

@@ -1348,13 +1348,18 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     }
 
     if constexpr (SPLIT) {
-        // Every role comes here, also after a wait that gave up.  Key row r is finished by CTA r / rows of the cluster; the
-        // tiles in shared memory make room for the arrivals, so all CTAs must be through with theirs first.
+        // Every role comes here, also after a wait that gave up and when the status word was set before the launch.  Key row r
+        // is finished by CTA r / rows of the cluster; the tiles in shared memory make room for the arrivals, so all CTAs must be
+        // through with theirs first.  Nobody writes an item of which a CTA has failed.
         const int rows = 128 / p.split;
+        volatile uint32_t* fail = reinterpret_cast<volatile uint32_t*>(sLse);  // [CTA of the cluster]
         __syncwarp();
         cluster_arrive();
         cluster_wait();
-        if (tid < Cfg::kComputeThreads && item_units(split_id) > 0) {
+        const bool failed = *abort_flag != 0;  // (final: every warp of the CTA has passed the barrier)
+        if (tid < p.split) cluster_store_1(const_cast<uint32_t*>(fail) + rank, tid, failed);
+        __syncwarp();
+        if (tid < Cfg::kComputeThreads && !failed && item_units(split_id) > 0) {
             tc_fence_after_sync();
             const int row = (warp & 3) * 32 + lane, part = warp >> 2, to = (row * p.split) >> 7, r = row - to * rows;
             // [source CTA][row][dV: D, dK: D] FP32, 16-byte pieces swizzled by the row: the rows of a warp would share a bank
@@ -1380,7 +1385,9 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         __syncwarp();
         cluster_arrive();
         cluster_wait();
-        if (tid < Cfg::kComputeThreads) {
+        bool good = true;
+        for (int k = 0; k < p.split; ++k) good = good && fail[k] == 0;
+        if (tid < Cfg::kComputeThreads && good) {
             const int k0 = item_kt(split_id) * 128 + rank * rows, b = item_b(split_id), hk = item_hk(split_id);
             for (int i = tid; i < rows * (D / 4); i += Cfg::kComputeThreads) {  // eight columns each: dV, then dK
                 const int r = i / (D / 4), c8 = i % (D / 4);

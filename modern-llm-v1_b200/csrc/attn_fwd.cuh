@@ -543,19 +543,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
 
     if constexpr (SPLIT) {
-        // Every role comes here, also after a wait that gave up.  Row r is finished by CTA r / rows of the cluster; the K/V ring
-        // holds the arrivals, so all CTAs must be through with theirs first.
+        // Every role comes here, also after a wait that gave up and when the status word was set before the launch.  Row r is
+        // finished by CTA r / rows of the cluster; the K/V ring holds the arrivals, so all CTAs must be through with theirs
+        // first.  A CTA that has failed sends a negative row sum instead of its share, and nobody writes the item.
         const int rows = 128 / p.split;
         __syncwarp();
         cluster_arrive();
         cluster_wait();
         if (tid < 128) {
+            const bool failed = *abort_flag != 0;  // (final: every warp of the CTA has passed the barrier)
             tc_fence_after_sync();
             const int to = (tid * p.split) >> 7, r = tid - to * rows;
             uint8_t* own = sK + (rank * rows + r) * D * 4;
             const uint32_t dst = cluster_addr(own, to);
 #pragma unroll
             for (int c = 0; c < D / 32; ++c) {
+                if (failed) break;
                 uint32_t v[32];
                 tmem_ld_x32(tmem + (uint32_t(warp * 32) << 16) + Cfg::kColO + c * 32, v);
                 tmem_wait_ld();
@@ -568,7 +571,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         cluster_store_4(dst + at, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
                 }
             }
-            cluster_store_f2(sQ + (rank * rows + r) * 8, to, make_float2(split_m, split_l));
+            cluster_store_f2(sQ + (rank * rows + r) * 8, to, failed ? make_float2(-INFINITY, -1.f) : make_float2(split_m, split_l));
             tc_fence_before_sync();
         }
         __syncwarp();
@@ -579,9 +582,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             const int q0 = item_qt(split_id) * 128 + rank * rows, b = item_b(split_id), h = item_h(split_id);
             // `split` threads per row, each with D / split columns, 16 at a time (8 when there are no more)
             const int r = fastdiv(unsigned(tid), p.div_split), part = tid - r * p.split, cols = fastdiv(unsigned(D), p.div_split);
-            if (q0 + r < p.T) {
-                float m = -INFINITY, l = 0.f;
-                for (int k = 0; k < p.split; ++k) m = fmaxf(m, ml[k * rows + r].x);
+            float m = -INFINITY;
+            bool good = q0 + r < p.T;
+            for (int k = 0; k < p.split; ++k) {
+                m = fmaxf(m, ml[k * rows + r].x);
+                if (ml[k * rows + r].y < 0.f) good = false;
+            }
+            if (good) {
+                float l = 0.f;
                 for (int k = 0; k < p.split; ++k) {
                     const float2 s = ml[k * rows + r];
                     l += s.x == -INFINITY ? 0.f : ex2_approx((s.x - m) * p.scale_log2) * s.y;

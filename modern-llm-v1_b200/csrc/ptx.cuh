@@ -547,6 +547,9 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* local, int rank) {
 __device__ __forceinline__ void cluster_store_f2(const void* local, int rank, float2 v) {
     asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(cluster_addr(local, rank)), "f"(v.x), "f"(v.y) : "memory");
 }
+__device__ __forceinline__ void cluster_store_1(const void* local, int rank, uint32_t v) {
+    asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(cluster_addr(local, rank)), "r"(v) : "memory");
+}
 __device__ __forceinline__ void cluster_store_4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }

@@ -1,0 +1,66 @@
+"""While the device status word is set, no attention kernel writes its outputs (include/b200attn.h).  The word is set here the
+way a program would meet it, by an append beyond a cache's capacity (code 105): no kernel waits for anything that never comes."""
+import pytest
+import torch
+
+import modern_llm_v1_b200 as m
+
+from gpu_util import randn_bf16
+
+pytestmark = pytest.mark.gpu
+
+
+def _full_cache():
+    """A cache whose device-side position says "full" behind the host's back; _overflow() then sets the status word."""
+    cache = m.KVCache(1, 1, 1, 1, 64, 4)
+    cache.set_lengths([3])
+    cache.lengths[0] = 4
+    x, g = torch.zeros((1, 1, 1, 64), device="cuda"), torch.ones(64, device="cuda")
+    return cache, x, g, torch.empty((1, 1, 1, 64), dtype=torch.bfloat16, device="cuda")
+
+
+def _overflow(c):
+    cache, x, g, q = c
+    cache.append(0, x, x, x, g, g, q)
+
+
+def _take_status():
+    with pytest.raises(RuntimeError, match="exceeds the cache capacity"):
+        m.device_status()
+    assert m.device_status() == 0
+
+
+def _nan_like(*ts):
+    return [torch.full_like(t, float("nan")) for t in ts]
+
+
+def _untouched(*ts):
+    return all(torch.isnan(t.float()).all().item() for t in ts)
+
+
+# an item of its own per CTA and items shared by 2, 4 or 8 CTAs (forward, dK/dV pass), at both head dimensions
+SHAPES = [(32, 512, 6, 2, 64), (1, 2000, 6, 2, 64), (1, 3000, 1, 1, 64), (1, 700, 8, 1, 64),
+          (8, 1001, 16, 4, 128), (1, 2000, 4, 2, 128), (1, 3000, 1, 1, 128)]
+
+
+@pytest.mark.parametrize("B,T,Hq,Hkv,D", SHAPES)
+def test_a_set_status_word_leaves_the_outputs_of_forward_and_backward_alone(B, T, Hq, Hkv, D):
+    q, k, v, do = (randn_bf16((B, h, T, D), s) for s, h in ((1, Hq), (2, Hkv), (3, Hkv), (4, Hq)))
+    o0, l0 = torch.empty_like(q), torch.empty((B, Hq, T), device="cuda")
+    m.flash_attn_forward_gqa(q, k, v, o0, l0, B, T, Hq, Hkv, D)
+    c = _full_cache()
+    m.device_status()
+    o, lse, dq, dk, dv = _nan_like(q, l0, q, k, v)
+    _overflow(c)
+    m.flash_attn_forward_gqa(q, k, v, o, lse, B, T, Hq, Hkv, D)
+    m.flash_attn_backward_gqa(q, k, v, o0, l0, do, dq, dk, dv, B, T, Hq, Hkv, D)
+    _take_status()
+    assert _untouched(o, lse), "the forward wrote"
+    assert _untouched(dq), "the dQ pass wrote"
+    assert _untouched(dk, dv), "the dK/dV pass wrote"
+    # and with the word cleared the same calls work
+    m.flash_attn_forward_gqa(q, k, v, o, lse, B, T, Hq, Hkv, D)
+    m.flash_attn_backward_gqa(q, k, v, o, lse, do, dq, dk, dv, B, T, Hq, Hkv, D)
+    m.device_status()
+    assert torch.equal(o, o0) and torch.equal(lse, l0)
+    assert all(torch.isfinite(x.float()).all().item() for x in (dq, dk, dv))
