@@ -930,7 +930,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     uint64_t* bar_pds_full = bars + 8;  // [2] by unit parity: P^T and dS^T written              (phase: unit / 2)
     uint64_t* bar_acc = bars + 10;      // accumulators of an item complete                      (phase: item)
     uint64_t* bar_acc_free = bars + 11; // accumulators read by the epilogue                     (phase: item)
-    uint64_t* bar_full = bars + 12;     // [4] per stage: Q, dO and the two row vectors of a unit have landed (phase: unit / NST)
+    uint64_t* bar_full = bars + 12;     // [4] per stage: Q, dO and the two row vectors of a unit have landed (phase: unit / NST;
+                                        // of the CTA's first unit: they may be used as soon as bar_kv[0] is complete too)
     uint64_t* bar_free = bars + 16;     // [4] per stage                                         (phase: unit / NST)
     uint64_t* bar_vec = bars + 20;      // [4] per stage, kVecOps: the row vectors are there as operands (phase: unit / NST)
     uint64_t* bar_item = bars + 24;     // [kItemRing] item ids handed out by the producer
@@ -996,14 +997,18 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     }
     // No wait for the previous kernel of the stream here: it is the dQ pass, and that lets this grid in only when all its CTAs
     // have passed their own wait, so everything before it is complete.  What it writes itself, the two row vectors, is waited
-    // for by the producer in front of their first load; K, V and the first Q and dO load meanwhile.
+    // for by the producer in front of their first load; K, V and the first Q and dO load meanwhile.  The status word is looked
+    // at twice: here, to leave at once behind an earlier failure, and by the producer behind that wait, because a dQ pass that
+    // gave up leaves row vectors of an earlier call.
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
 
     if (*abort_flag != 0) {
-        // an earlier CTA already failed: fall through to the teardown
+        // an earlier kernel failed: fall through to the teardown, but not ahead of the dQ pass (what follows this grid may
+        // start when it ends)
+        grid_dep_wait();
     } else if (warp == kProducerWarp) {
         // ------------------------------------------------------------------ producer (whole warp, one lane issues)
         reg_dealloc<Cfg::kRegsOther>();
@@ -1024,7 +1029,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             if (n >= NKV) ok = mbar_wait_warp(&bar_kv_free[kb], uint32_t(n / NKV - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
             if (!ok) break;
             if (elect_one()) {
-                mbar_arrive_expect_tx(&bar_kv[kb], 2 * Cfg::kTileBytes);
+                // (all loads of the CTA's first unit complete on this barrier: see there)
+                mbar_arrive_expect_tx(&bar_kv[kb], n == 0 ? 4 * Cfg::kTileBytes + 1024 : 2 * Cfg::kTileBytes);
 #pragma unroll
                 for (int bx = 0; bx < Cfg::kBoxes; ++bx) {
                     tma_load_4d(sK + kb * Cfg::kTileBytes + bx * Cfg::kBoxBytes, &tmK, &bar_kv[kb], bx * 64, k0, hk, b);
@@ -1040,21 +1046,34 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
                 const int s = u % NST;
                 if (u >= NST) ok = mbar_wait_warp(&bar_free[s], uint32_t(u / NST - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
                 if (!ok) break;
+                // The first unit's loads complete on bar_kv[0], which whoever needs them waits for too; bar_full[0] is arrived
+                // on once the dQ pass is complete and the status word, read under the loads' latency, is still clear.
+                uint64_t* full = u == 0 ? &bar_kv[0] : &bar_full[s];
+                int failed = 0;
                 if (elect_one()) {
-                    mbar_arrive_expect_tx(&bar_full[s], 2 * Cfg::kTileBytes + 1024);
+                    if (u > 0) mbar_arrive_expect_tx(full, 2 * Cfg::kTileBytes + 1024);
 #pragma unroll
                     for (int bx = 0; bx < Cfg::kBoxes; ++bx) {
-                        tma_load_4d(sQ + s * Cfg::kTileBytes + bx * Cfg::kBoxBytes, &tmQ, &bar_full[s], bx * 64, i * 128, h,
-                                    b);
-                        tma_load_4d(sdO + s * Cfg::kTileBytes + bx * Cfg::kBoxBytes, &tmdO, &bar_full[s], bx * 64, i * 128,
-                                    h, b);
+                        tma_load_4d(sQ + s * Cfg::kTileBytes + bx * Cfg::kBoxBytes, &tmQ, full, bx * 64, i * 128, h, b);
+                        tma_load_4d(sdO + s * Cfg::kTileBytes + bx * Cfg::kBoxBytes, &tmdO, full, bx * 64, i * 128, h, b);
                     }
                     if (u == 0) grid_dep_wait();  // (the same lane issues all loads)
                     const size_t voff = (size_t(b) * p.Hq + h) * p.Tpad + size_t(i) * 128;
-                    bulk_load_1d(sLse + s * 128, p.lse2 + voff, 512, &bar_full[s]);
-                    bulk_load_1d(sDv + s * 128, p.dvec + voff, 512, &bar_full[s]);
+                    bulk_load_1d(sLse + s * 128, p.lse2 + voff, 512, full);
+                    bulk_load_1d(sDv + s * 128, p.dvec + voff, 512, full);
+                    if (u == 0) {
+                        failed = *reinterpret_cast<volatile int*>(p.status);
+                        if (failed == 0) mbar_arrive(&bar_full[0]);
+                    }
                 }
                 __syncwarp();
+                if (u == 0 && __any_sync(0xffffffffu, failed != 0)) {
+                    // the other roles stand at bar_full[0]: they are sent home once the loads in flight have landed
+                    mbar_wait_warp(&bar_kv[0], 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+                    if (failed != 0) *abort_flag = failed;
+                    ok = false;
+                    break;
+                }
                 if (it == j_next) {
                     id_new = __shfl_sync(0xffffffffu, id_next, 0);
                     if (lane == 0) {
@@ -1089,6 +1108,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
                 for (int it = item_units(id); it > 0; --it, ++u) {
                     const int s = u % NST;
                     ok = mbar_wait_warp(&bar_full[s], uint32_t(u / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+                    if (ok && u == 0) ok = mbar_wait_warp(&bar_kv[0], 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
                     if (!ok) break;
                     uint4* op_l = reinterpret_cast<uint4*>(sOps + 2 * s * Cfg::kOpBytes);
                     uint4* op_d = op_l + 128;

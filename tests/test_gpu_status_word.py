@@ -64,3 +64,34 @@ def test_a_set_status_word_leaves_the_outputs_of_forward_and_backward_alone(B, T
     m.device_status()
     assert torch.equal(o, o0) and torch.equal(lse, l0)
     assert all(torch.isfinite(x.float()).all().item() for x in (dq, dk, dv))
+
+
+@pytest.mark.parametrize("T,D", [(16384, 64), (16384, 128)])
+def test_a_word_set_while_the_dq_pass_runs_keeps_the_dkdv_pass_from_writing(T, D):
+    # The dK/dV pass's CTAs get in under the dQ pass (which leaves SMs free here and runs for hundreds of microseconds) and
+    # read the word while it is clear.  Everything is enqueued behind one event, so the host's pace does not matter.
+    B, Hq, Hkv = 1, 1, 1
+    q, k, v, do = (randn_bf16((B, 1, T, D), s) for s in (1, 2, 3, 4))
+    o, lse = torch.empty_like(q), torch.empty((B, Hq, T), device="cuda")
+    m.flash_attn_forward_gqa(q, k, v, o, lse, B, T, Hq, Hkv, D)
+    dq, dk, dv = _nan_like(q, k, v)
+    # (of higher priority: its block must not queue behind the dK/dV pass's, which wait for SMs)
+    main, other, gate = torch.cuda.current_stream(), torch.cuda.Stream(priority=-1), torch.cuda.Stream()
+    c = _full_cache()
+    # (a backward allocates its scratch on its first call)
+    m.flash_attn_backward_gqa(q, k, v, o, lse, do, torch.empty_like(q), torch.empty_like(k), torch.empty_like(v), B, T, Hq, Hkv, D)
+    m.device_status()
+    go = torch.cuda.Event()
+    with torch.cuda.stream(gate):
+        torch.cuda._sleep(4_000_000)  # about 2 ms, for the host to enqueue what follows
+        go.record()
+    with torch.cuda.stream(other):
+        other.wait_event(go)
+        torch.cuda._sleep(60_000)  # about 30 us into the dQ pass
+        _overflow(c)
+    main.wait_event(go)
+    m.flash_attn_backward_gqa(q, k, v, o, lse, do, dq, dk, dv, B, T, Hq, Hkv, D)
+    main.wait_stream(other)
+    main.synchronize()
+    _take_status()
+    assert _untouched(dk, dv)
