@@ -122,6 +122,7 @@ __global__ void __launch_bounds__(128) attn_bwd_dq_convert_kernel(const BwdParam
     const int b = bh / p.Hq, h = bh % p.Hq;
     const int r = threadIdx.x, t = tile * 128 + r;
     grid_dep_wait();
+    if (*reinterpret_cast<volatile int*>(p.status) != 0) return;  // the fused kernel, or one before it, failed
     const float4* src = reinterpret_cast<const float4*>(dq_acc + size_t(blockIdx.x) * (128 * D)) + r;
     float4 v[D / 4];
 #pragma unroll

@@ -44,7 +44,10 @@ SHAPES = [(32, 512, 6, 2, 64), (1, 2000, 6, 2, 64), (1, 3000, 1, 1, 64), (1, 700
 
 
 @pytest.mark.parametrize("B,T,Hq,Hkv,D", SHAPES)
-def test_a_set_status_word_leaves_the_outputs_of_forward_and_backward_alone(B, T, Hq, Hkv, D):
+@pytest.mark.parametrize("mode", ["two_pass", "one_pass"])
+def test_a_set_status_word_leaves_the_outputs_of_forward_and_backward_alone(B, T, Hq, Hkv, D, mode):
+    if mode == "one_pass" and D != 64:
+        pytest.skip("the one-pass backward is a D = 64 kernel")
     q, k, v, do = (randn_bf16((B, h, T, D), s) for s, h in ((1, Hq), (2, Hkv), (3, Hkv), (4, Hq)))
     o0, l0 = torch.empty_like(q), torch.empty((B, Hq, T), device="cuda")
     m.flash_attn_forward_gqa(q, k, v, o0, l0, B, T, Hq, Hkv, D)
@@ -53,14 +56,14 @@ def test_a_set_status_word_leaves_the_outputs_of_forward_and_backward_alone(B, T
     o, lse, dq, dk, dv = _nan_like(q, l0, q, k, v)
     _overflow(c)
     m.flash_attn_forward_gqa(q, k, v, o, lse, B, T, Hq, Hkv, D)
-    m.flash_attn_backward_gqa(q, k, v, o0, l0, do, dq, dk, dv, B, T, Hq, Hkv, D)
+    m.flash_attn_backward_gqa(q, k, v, o0, l0, do, dq, dk, dv, B, T, Hq, Hkv, D, mode=mode)
     _take_status()
     assert _untouched(o, lse), "the forward wrote"
     assert _untouched(dq), "the dQ pass wrote"
     assert _untouched(dk, dv), "the dK/dV pass wrote"
     # and with the word cleared the same calls work
     m.flash_attn_forward_gqa(q, k, v, o, lse, B, T, Hq, Hkv, D)
-    m.flash_attn_backward_gqa(q, k, v, o, lse, do, dq, dk, dv, B, T, Hq, Hkv, D)
+    m.flash_attn_backward_gqa(q, k, v, o, lse, do, dq, dk, dv, B, T, Hq, Hkv, D, mode=mode)
     m.device_status()
     assert torch.equal(o, o0) and torch.equal(lse, l0)
     assert all(torch.isfinite(x.float()).all().item() for x in (dq, dk, dv))
