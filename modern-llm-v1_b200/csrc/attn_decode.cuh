@@ -597,8 +597,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         ok = decode_bar_ok(ok);
         if (!ok) break;
         const int s_last = (j - 1) % NST;
-        if (failed && p.cluster <= 1) {
+        if (failed) {
             // every piece's loads are waited for, nothing is written
+            if (p.cluster > 1) break;  // (one piece)
             fence_proxy_async_smem();
             mbar_arrive(&bar_free[s_last]);
             decode_walk_next<KEYS>(p, w, tiles);
@@ -666,15 +667,17 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         decode_walk_next<KEYS>(p, w, tiles);
     }
     if (p.cluster <= 1) return;
-    // ---- the cluster's partial results: this CTA finishes its slice of the outputs.  A CTA without tiles (or one that has
-    // given up) sends weight zero; nobody leaves before everybody's stores have landed.
+    // ---- the cluster's partial results: this CTA finishes its slice of the outputs.  A CTA without tiles sends weight zero, one
+    // that has failed a negative row sum, upon which nobody writes the unit; nobody leaves before everybody's stores have landed.
     if (!sent) {
         cluster_wait();
-        for (int i = tid; i < G * p.cluster; i += 128) cluster_store_f2(&sXMl[rank * 16 + i / p.cluster], i % p.cluster, make_float2(-INFINITY, 0.f));
+        for (int i = tid; i < G * p.cluster; i += 128)
+            cluster_store_f2(&sXMl[rank * 16 + i / p.cluster], i % p.cluster, make_float2(-INFINITY, failed || !ok ? -1.f : 0.f));
     }
     cluster_arrive();
     cluster_wait();
-    if (failed || !ok) return;
+    for (int c = 0; c < p.cluster; ++c)
+        if (sXMl[c * 16].y < 0.f) return;
     const int slice = int(p.div_slice.d);
     const auto write_rows = write_rows_of(w);
     for (int i = tid; i < slice; i += 128) {

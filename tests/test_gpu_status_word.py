@@ -69,6 +69,21 @@ def test_a_set_status_word_leaves_the_outputs_of_forward_and_backward_alone(B, T
     assert all(torch.isfinite(x.float()).all().item() for x in (dq, dk, dv))
 
 
+@pytest.mark.parametrize("B,L,Hq,Hkv,D", [(1, 1025, 4, 2, 64), (1, 1500, 16, 4, 128), (120, 130, 6, 3, 64), (1, 30001, 2, 1, 64)])
+def test_a_set_status_word_leaves_the_outputs_of_the_decode_alone(B, L, Hq, Hkv, D):
+    q, kc, vc = randn_bf16((B, Hq, D), 1), randn_bf16((B, Hkv, L, D), 2), randn_bf16((B, Hkv, L, D), 3)
+    c = _full_cache()
+    m.device_status()
+    o, lse = _nan_like(q, torch.empty((B, Hq), device="cuda"))
+    _overflow(c)
+    m.flash_attn_decode(q, kc, vc, o, lse, B, L, Hq, Hkv, D)
+    _take_status()
+    assert _untouched(o, lse)
+    m.flash_attn_decode(q, kc, vc, o, lse, B, L, Hq, Hkv, D)
+    m.device_status()
+    assert torch.isfinite(o.float()).all() and torch.isfinite(lse).all()
+
+
 @pytest.mark.parametrize("T,D", [(16384, 64), (16384, 128)])
 def test_a_word_set_while_the_dq_pass_runs_keeps_the_dkdv_pass_from_writing(T, D):
     # The dK/dV pass's CTAs get in under the dQ pass (which leaves SMs free here and runs for hundreds of microseconds) and
