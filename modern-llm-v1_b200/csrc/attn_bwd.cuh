@@ -1098,7 +1098,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         if constexpr (Cfg::kVecOps) {
             const float to_scores = -1.f / p.scale_log2;
             auto split = [](float v) {
-                const float hi = __bfloat162float(__float2bfloat16_rn(v)), r = v - hi;
+                const float hi = __bfloat162float(__float2bfloat16_rn(v)), r = fabsf(hi) == INFINITY ? 0.f : v - hi;  // (NaN stays NaN)
                 const float mid = __bfloat162float(__float2bfloat16_rn(r));
                 return make_uint4(pack_bf16x2(hi, mid), pack_bf16x2(r - mid, 0.f), 0u, 0u);
             };
@@ -1115,8 +1115,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const int r = i * 32 + lane;
-                        // padding rows have L = inf: a large finite number keeps the split free of NaN, and P is 0 just the same
-                        op_l[r] = split(fmaxf(sLse[s * 128 + r] * to_scores, -1.7014118e38f));
+                        op_l[r] = split(sLse[s * 128 + r] * to_scores);  // padding rows: L = inf, so S^T = -inf and P = 0
                         op_d[r] = split(-sDv[s * 128 + r]);
                     }
                     fence_proxy_async_smem();  // ordinary accesses before the products' reads and the next loads' writes

@@ -108,3 +108,24 @@ def test_shape_errors_raise_value_error_on_gpu_tensors():
     with pytest.raises(ValueError, match="unsupported head dimension"):
         m.flash_attn_forward(q32, q32, q32, q32.clone(), torch.empty(1, 128, device="cuda"), 1, 128, 32)
     assert m.device_status() == 0
+
+
+@pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 300, 4, 2), (16, 512, 8, 4)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_a_nan_key_reaches_every_value_gradient_of_its_head(B, T, Hq, Hkv, D):
+    # Key j of one head is NaN: the logsumexp of rows j .. T-1 is NaN, so P of those rows is NaN and with it dV of every key of
+    # the head (all of them are seen by row T-1).  Other heads and batches stay finite.  T is no multiple of the tile: the
+    # padding rows, whose logsumexp is +inf, must not bring a NaN of their own.
+    j, b, hk = 70, 0, 1
+    q, k, v, do = (randn_bf16((B, h, T, D), s) for s, h in ((1, Hq), (2, Hkv), (3, Hkv), (4, Hq)))
+    k[b, hk, j] = float("nan")
+    o, lse, dq, dk, dv = (x.float() for x in run_fwd_bwd(q, k, v, do))
+    group = Hq // Hkv
+    own = slice(hk * group, (hk + 1) * group)
+    assert torch.isnan(lse[b, own, j:]).all() and torch.isfinite(lse[b, own, :j]).all()
+    assert torch.isnan(o[b, own, j:]).all() and torch.isfinite(o[b, own, :j]).all()
+    assert torch.isnan(dv[b, hk]).all() and torch.isnan(dk[b, hk]).all() and torch.isnan(dq[b, own, j:]).all()
+    for x, mine in ((o, own), (lse, own), (dq, own), (dk, hk), (dv, hk)):
+        rest = x.clone()
+        rest[b, mine] = 0.0
+        assert torch.isfinite(rest).all()
