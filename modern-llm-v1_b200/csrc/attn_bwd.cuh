@@ -1107,8 +1107,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             for (int n = 0, id; ok && (id = get_item(n)) >= 0; ++n) {
                 for (int it = item_units(id); it > 0; --it, ++u) {
                     const int s = u % NST;
-                    ok = mbar_wait_warp(&bar_full[s], uint32_t(u / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
-                    if (ok && u == 0) ok = mbar_wait_warp(&bar_kv[0], 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+                    ok = mbar_wait_warp(u == 0 ? &bar_kv[0] : &bar_full[s], uint32_t(u / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
                     if (!ok) break;
                     uint4* op_l = reinterpret_cast<uint4*>(sOps + 2 * s * Cfg::kOpBytes);
                     uint4* op_d = op_l + 128;
@@ -1119,6 +1118,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
                         op_d[r] = split(-sDv[s * 128 + r]);
                     }
                     fence_proxy_async_smem();  // ordinary accesses before the products' reads and the next loads' writes
+                    if (u == 0) ok = mbar_wait_warp(&bar_full[0], 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);  // the status word
+                    if (!ok) break;
                     mbar_arrive(&bar_vec[s]);
                 }
             }

@@ -676,8 +676,6 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     }
     cluster_arrive();
     cluster_wait();
-    for (int c = 0; c < p.cluster; ++c)
-        if (sXMl[c * 16].y < 0.f) return;
     const int slice = int(p.div_slice.d);
     const auto write_rows = write_rows_of(w);
     for (int i = tid; i < slice; i += 128) {
@@ -689,8 +687,13 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
             v[c] = c < p.cluster ? sX[c * slice + i] : make_float2(0.f, 0.f);
         }
         float m = ml[0].x;
+        bool good = !(ml[0].y < 0.f);
 #pragma unroll
-        for (int c = 1; c < kDecodeMaxCluster; ++c) m = fmaxf(m, ml[c].x);
+        for (int c = 1; c < kDecodeMaxCluster; ++c) {
+            m = fmaxf(m, ml[c].x);
+            good = good && !(ml[c].y < 0.f);
+        }
+        if (!good) return;  // a CTA has failed (and said so for every head)
         float a0 = 0.f, a1 = 0.f, l = 0.f;
 #pragma unroll
         for (int c = 0; c < kDecodeMaxCluster; ++c) {
