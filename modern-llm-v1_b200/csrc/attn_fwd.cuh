@@ -592,16 +592,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 float l = 0.f;
                 for (int k = 0; k < p.split; ++k) {
                     const float2 s = ml[k * rows + r];
-                    l += s.x == -INFINITY ? 0.f : ex2_approx((s.x - m) * p.scale_log2) * s.y;
+                    // a share without a key for the row has l = 0, one whose scores are all NaN l = NaN: that must not get lost
+                    l += s.x == -INFINITY ? s.y : ex2_approx((s.x - m) * p.scale_log2) * s.y;
                 }
+                if (m == -INFINITY) l = __int_as_float(0x7fffffff);  // no score above -inf: NaN, as 0 / 0 is
                 const float inv_l = 1.f / l;
                 uint16_t* orow = p.o + size_t(b) * p.o_sb + size_t(h) * p.o_sh + size_t(q0 + r) * p.o_st + part * cols;
                 for (int c = 0; c < cols; c += 16) {
                     const bool two = c + 8 < cols;
-                    float acc[16] = {};
+                    float acc[16];
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) acc[e] = l != l ? l : 0.f;
                     for (int k = 0; k < p.split; ++k) {
                         const float mk = ml[k * rows + r].x;
-                        if (mk == -INFINITY) continue;  // no key of the row (or no tile at all: nothing valid was sent)
+                        if (mk == -INFINITY) continue;  // no key of the row, or no tile at all: nothing valid was sent
                         const float f = ex2_approx((mk - m) * p.scale_log2) * inv_l;
                         const uint8_t* row = sK + (k * rows + r) * D * 4;
                         float4 v[4];

@@ -129,3 +129,22 @@ def test_a_nan_key_reaches_every_value_gradient_of_its_head(B, T, Hq, Hkv, D):
         rest = x.clone()
         rest[b, mine] = 0.0
         assert torch.isfinite(rest).all()
+
+
+@pytest.mark.parametrize("B,T,Hq,Hkv,D", [(1, 2000, 6, 2, 64), (1, 3000, 1, 1, 64), (1, 2000, 4, 2, 128), (1, 3000, 1, 1, 128),
+                                          (16, 512, 8, 4, 64), (16, 512, 8, 4, 128)])
+def test_a_nan_score_stays_nan_however_an_item_is_shared(B, T, Hq, Hkv, D):
+    # one query row of NaN, and a NaN in all of the first keys of another head (whole shares of an item then have no other
+    # scores): exactly those rows of O and of the logsumexp are NaN
+    q, k, v = (randn_bf16((B, h, T, D), s) for s, h in ((1, Hq), (2, Hkv), (3, Hkv)))
+    q[0, 0, T - 1] = float("nan")
+    want = torch.zeros((B, Hq, T), dtype=torch.bool, device="cuda")
+    want[0, 0, T - 1] = True
+    if Hkv > 1:
+        k[0, 1, : T // 3, 5] = float("nan")
+        want[0, Hq // Hkv : 2 * (Hq // Hkv)] = True
+    o, lse = run_fwd(q, k, v)
+    m.device_status()
+    assert torch.equal(torch.isnan(lse), want)
+    assert torch.equal(torch.isnan(o), want[..., None].expand_as(o))
+    assert torch.isfinite(o[~want]).all() and torch.isfinite(lse[~want]).all()
