@@ -697,7 +697,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         float a0 = 0.f, a1 = 0.f, l = 0.f;
 #pragma unroll
         for (int c = 0; c < kDecodeMaxCluster; ++c) {
-            if (ml[c].x == -INFINITY) continue;  // no tiles: its slots hold nothing
+            if (ml[c].x == -INFINITY && ml[c].y == 0.f) continue;  // no tiles: its slots hold nothing (all scores NaN: l is NaN)
             const float f = ex2_approx((ml[c].x - m) * p.scale_log2);
             a0 += f * v[c].x;
             a1 += f * v[c].y;

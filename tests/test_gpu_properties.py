@@ -148,3 +148,18 @@ def test_a_nan_score_stays_nan_however_an_item_is_shared(B, T, Hq, Hkv, D):
     assert torch.equal(torch.isnan(lse), want)
     assert torch.equal(torch.isnan(o), want[..., None].expand_as(o))
     assert torch.isfinite(o[~want]).all() and torch.isfinite(lse[~want]).all()
+
+
+@pytest.mark.parametrize("B,L,Hq,Hkv,D", [(1, 1025, 4, 2, 64), (1, 1500, 16, 4, 128), (120, 130, 6, 3, 64), (2, 30001, 4, 2, 64)])
+def test_a_nan_score_stays_nan_however_a_cache_is_dealt(B, L, Hq, Hkv, D):
+    q, kc, vc = randn_bf16((B, Hq, D), 11), randn_bf16((B, Hkv, L, D), 12), randn_bf16((B, Hkv, L, D), 13)
+    q[0, 0] = float("nan")
+    kc[B - 1, 1, : 2 * L // 3, 5] = float("nan")
+    want = torch.zeros((B, Hq), dtype=torch.bool, device="cuda")
+    want[0, 0] = True
+    want[B - 1, Hq // Hkv : 2 * (Hq // Hkv)] = True
+    o, lse = torch.empty_like(q), torch.empty((B, Hq), device="cuda")
+    m.flash_attn_decode(q, kc, vc, o, lse, B, L, Hq, Hkv, D)
+    m.device_status()
+    assert torch.equal(torch.isnan(lse), want)
+    assert torch.equal(torch.isnan(o), want[..., None].expand_as(o))
