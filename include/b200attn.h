@@ -142,7 +142,8 @@ int b200attn_bwd_static(const void* q, const void* k, const void* v, const void*
  * (llm/apps/infer_modern_gpt.cu:253-255); this is the kernel its KV cache would call.
  * n_splits <= 0 lets the library choose how the cache is split over CTAs; n_splits > 0 asks for that many splits
  * per (batch, KV head) and gets the next power of two below, at most 8.  Results are bit-reproducible either
- * way.  workspace: at least b200attn_decode_workspace_bytes(...) bytes, 256-byte aligned.
+ * way.  workspace: at least b200attn_decode_workspace_bytes(...) bytes, 256-byte aligned; it needs no initialisation,
+ * and calls that may overlap (other streams, concurrently replayed graphs) need workspaces of their own.
  */
 int b200attn_decode(const void* q, const void* kcache, const void* vcache, void* o, float* lse, int B, int L, int Hq,
                     int Hkv, int D, float softmax_scale, int n_splits, void* workspace, size_t workspace_bytes,

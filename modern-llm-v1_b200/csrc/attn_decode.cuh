@@ -53,8 +53,9 @@ struct DecodeParams {
     float* part_o;      // [slot][G][D]  un-normalised
     float* part_m;      // [slot][G]     row maximum, raw score units
     float* part_l;      // [slot][G]     sum of exp2((s - m) * scale_log2)
-    int* counters;      // one per CTA, zero between launches: pieces finished of the shared unit that begins in that CTA
-    int* status;
+    unsigned long long* counters;  // one per CTA, see decode_count: pieces finished of the shared unit that begins in that CTA
+    unsigned long long tag;        // of this launch
+    int* status;                   // status word and epoch
 };
 
 constexpr int kDecodeMaxCtas = 320, kDecodeMaxCluster = 8, kDecodeThreads = 192;
@@ -331,10 +332,25 @@ __device__ __forceinline__ void decode_add_pieces(const DecodeParams& p, const D
     }
     write(g, d, a0, a1, m, l);
 }
-__device__ __forceinline__ int decode_ld_acquire(const int* a) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(a) : "memory");
+__device__ __forceinline__ unsigned long long decode_ld_acquire(const unsigned long long* a) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(a) : "memory");
     return v;
+}
+// The counters lie in the caller's workspace, so that launches which may overlap (other streams, other graphs) never share one,
+// and nobody clears them: a word is launch tag (40 bits), epoch (14 bits) and count (10 bits), and one with another tag or epoch,
+// whatever the workspace held before, counts as zero.  The last piece of a unit puts its count back to zero, so a captured
+// launch, which keeps its tag, can be replayed; what a launch that gave up leaves behind has the epoch before, which ends when
+// the host takes the error off the status word.  (Words that nobody has counted in: one in 2^54 would pass.)
+constexpr int kDecodeCountBits = 10, kDecodeEpochBits = 14;
+static_assert(kDecodeMaxCtas < (1 << kDecodeCountBits), "a count fits");
+// One more piece finished; returns how many there are now.  `seen`: what the word held at some point of this launch.
+__device__ __forceinline__ int decode_count(unsigned long long* word, unsigned long long tag, unsigned long long seen) {
+    if ((seen >> kDecodeCountBits) != (tag >> kDecodeCountBits)) {
+        if (atomicCAS(word, seen, tag + 1) == seen) return 1;
+        // another CTA of this launch has tagged it meanwhile
+    }
+    return int(atomicAdd(word, 1ull) - tag) + 1;
 }
 
 template <int D, int NH>
@@ -363,6 +379,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_part + 1);
     volatile int* last_flag = abort_flag + 1;
     volatile int* fail_flag = abort_flag + 2;
+    volatile int* epoch = abort_flag + 3;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = p.G;
@@ -444,14 +461,16 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         if (p.cluster || *fail_flag != 0 || w.t >= w.t_end) return;
         const int tiles = decode_piece(w);
         if (tiles == w.n_tiles || w.t + tiles == w.t_end) return;
-        if (!mbar_wait_warp(bar_part, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX)) return;
         const int unit_start = w.t - w.j0;
         const int first = decode_cta_of(w, unit_start), last = decode_cta_of(w, unit_start + w.n_tiles - 1);
+        const unsigned long long tag = p.tag + ((unsigned long long)*epoch << kDecodeCountBits);
+        const unsigned long long seen = decode_ld_acquire(p.counters + first);
+        if (!mbar_wait_warp(bar_part, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX)) return;
         int is_last = 0;
         if (lane == 0) {
             __threadfence();
-            is_last = atomicAdd(p.counters + first, 1) == last - first;
-            if (is_last) p.counters[first] = 0;  // for the next launch that uses it
+            is_last = decode_count(p.counters + first, tag, seen) == last - first + 1;
+            if (is_last) p.counters[first] = tag;
             __threadfence();
         }
         if (!__shfl_sync(0xffffffffu, is_last, 0)) return;
@@ -468,7 +487,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     }
     grid_dep_wait();
     // (a launch behind a failure writes nothing; its loads are harmless, but shared memory has to outlive them)
-    if (tid == 0) *fail_flag = *reinterpret_cast<volatile int*>(p.status);
+    if (tid == 0) {
+        *fail_flag = *reinterpret_cast<volatile int*>(p.status);
+        *epoch = *reinterpret_cast<volatile int*>(p.status + 1);
+    }
     DecodeWalk w = decode_walk_start<KEYS>(p, int(blockIdx.x), int(gridDim.x), lane);
     __syncthreads();
     const bool failed = *fail_flag != 0;
@@ -629,7 +651,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
             const bool ends_range = w.t + tiles == w.t_end;
             // At the range's end nothing is left to hide latency behind.  Usually all other pieces have been stored by then
             // (they lie at the beginning of their CTAs' ranges): one look at the counter instead of store, fence and count.
-            if (tid == 0) *last_flag = ends_range && decode_ld_acquire(p.counters + first) == last - first;
+            const unsigned long long tag = p.tag + ((unsigned long long)*epoch << kDecodeCountBits);
+            unsigned long long seen = 0;
+            if (tid == 0 && ends_range) seen = decode_ld_acquire(p.counters + first);
+            if (tid == 0) *last_flag = ends_range && seen == tag + (last - first);
             decode_merge<D, NH>(st, sO, sMl, warp, lane, tid, G, p.scale_log2, [&](int g, int d, float a0, float a1, float m, float l) {
                 if (*last_flag) {
                     decode_add_pieces<D>(p, w, first, last, unit_start, g, d, cta, a0, a1, m, l, write_rows);
@@ -644,13 +669,13 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
             if (!ends_range) {
                 mbar_arrive(bar_part);
             } else if (*last_flag) {
-                if (tid == 0) p.counters[first] = 0;  // for the next launch that uses it
+                if (tid == 0) p.counters[first] = tag;
             } else {
                 __threadfence();
                 named_bar_sync(1, 128);
                 if (tid == 0) {
-                    const int is_last = atomicAdd(p.counters + first, 1) == last - first;
-                    if (is_last) p.counters[first] = 0;
+                    const bool is_last = decode_count(p.counters + first, tag, seen) == last - first + 1;
+                    if (is_last) p.counters[first] = tag;
                     *last_flag = is_last;
                     __threadfence();
                 }

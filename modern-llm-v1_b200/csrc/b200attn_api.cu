@@ -7,6 +7,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <functional>
 #include <queue>
 #include <utility>
@@ -27,8 +28,9 @@ using namespace b200attn;
 
 namespace {
 
-// One status word per device, living in the library's device image.
-__device__ int g_status_word;
+// One status word per device, living in the library's device image, and behind it the epoch: how many errors have been taken
+// off the word (see decode_count).
+__device__ int g_status_word[2];
 
 constexpr int kMaxDevices = 64;
 int* g_status_ptr[kMaxDevices] = {nullptr};
@@ -46,11 +48,19 @@ __device__ int g_sched_words[2 * kSchedSlots];
 int* g_sched_ptr[kMaxDevices] = {nullptr};
 std::atomic<unsigned> g_sched_seq{0};
 
-// Counters of the decode kernel's shared units, the same way: a set per launch, zero again when the launch ends.
-constexpr int kDecodeSlots = 64;
-__device__ int g_decode_counters[kDecodeSlots * kDecodeMaxCtas];
-int* g_decode_ptr[kMaxDevices] = {nullptr};
-std::atomic<unsigned> g_decode_seq{0};
+// What tells a decode launch's counters from those of every other launch (see decode_count).  The sequence starts anywhere, so
+// that the counters of another process in recycled memory are as unlikely to pass as anything else.
+std::atomic<unsigned long long> g_decode_seq{0};
+unsigned long long next_decode_tag() {
+    static const unsigned long long start = [] {
+        unsigned long long x = (unsigned long long)std::chrono::steady_clock::now().time_since_epoch().count() +
+                               (unsigned long long)reinterpret_cast<uintptr_t>(&g_decode_seq);
+        x = (x ^ (x >> 30)) * 0xbf58476d1ce4e5b9ull;  // the finaliser of SplitMix64 (Steele, Lea and Flood)
+        x = (x ^ (x >> 27)) * 0x94d049bb133111ebull;
+        return x ^ (x >> 31);
+    }();
+    return (start + g_decode_seq.fetch_add(1, std::memory_order_relaxed)) << (kDecodeCountBits + kDecodeEpochBits);
+}
 
 // Returns the device address of the status word of the current device (resolved once per device).
 int* status_ptr(int* err) {
@@ -66,7 +76,7 @@ int* status_ptr(int* err) {
             *err = B200ATTN_ERR_NO_DEVICE;
             return nullptr;
         }
-        if (cudaMemset(p, 0, sizeof(int)) != cudaSuccess) {
+        if (cudaMemset(p, 0, sizeof(g_status_word)) != cudaSuccess) {
             cudaGetLastError();
             *err = B200ATTN_ERR_CUDA;
             return nullptr;
@@ -77,13 +87,6 @@ int* status_ptr(int* err) {
             *err = B200ATTN_ERR_NO_DEVICE;
             return nullptr;
         }
-        void* dp = nullptr;
-        if (cudaGetSymbolAddress(&dp, g_decode_counters) != cudaSuccess) {
-            cudaGetLastError();
-            *err = B200ATTN_ERR_NO_DEVICE;
-            return nullptr;
-        }
-        g_decode_ptr[dev] = static_cast<int*>(dp);
         g_sched_ptr[dev] = static_cast<int*>(sp);
         g_status_ptr[dev] = static_cast<int*>(p);
     }
@@ -104,12 +107,6 @@ int* next_sched_pair(long long n_items, unsigned n_ctas) {
     int dev = 0;
     cudaGetDevice(&dev);
     return g_sched_ptr[dev] + 2 * (g_sched_seq.fetch_add(1, std::memory_order_relaxed) % kSchedSlots);
-}
-
-int* next_decode_counters() {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    return g_decode_ptr[dev] + kDecodeMaxCtas * (g_decode_seq.fetch_add(1, std::memory_order_relaxed) % kDecodeSlots);
 }
 
 // The static deal of the forward and the dQ pass (two CTAs per SM) as a table: items (ids are heaviest first;
@@ -869,7 +866,8 @@ inline int decode_max_ctas() { return std::min(2 * sm_count(), kDecodeMaxCtas); 
 
 struct DecodePlan {
     int G, n_chunks;
-    int splits;   // workspace slots per unit
+    int slots;    // workspace slots per unit for partial results
+    int splits;   // and with the room for the counters behind them
     int cluster;  // CTAs per unit, or 0: ranges of tiles
     bool whole;   // ranges of whole units
     int n_ctas, slot_mode;
@@ -903,17 +901,20 @@ DecodePlan decode_plan(int B, int L, int Hq, int Hkv, int D, int n_splits, bool 
     d.slot_mode = kDecodeSlotTile;
     if (n_splits > 0) {
         const int want = std::min(std::min(n_splits, n_128), 64), per = (n_128 + want - 1) / want;
-        d.splits = (n_128 + per - 1) / per;  // no split is empty
+        d.splits = d.slots = (n_128 + per - 1) / per;  // no split is empty
         while (d.cluster * 2 <= std::min(d.splits, kDecodeMaxCluster)) d.cluster *= 2;
     } else {
-        d.splits = (int)std::min<long long>(n_all, (2 * cap + units - 1) / units);
+        d.slots = (int)std::min<long long>(n_all, (2 * cap + units - 1) / units);
+        // a counter per CTA of the ranges, in units of a slot of every (batch, query head); a single tile is never shared
+        const long long slot_bytes = (long long)B * Hq * (D + 2) * 4, counter_bytes = n_all > 1 ? 8ll * std::min<long long>(tiles, cap) : 0;
+        d.splits = d.slots + (int)((counter_bytes + slot_bytes - 1) / slot_bytes);
         while (d.cluster < kDecodeMaxCluster && units * d.cluster * 2 <= sm_count() && n_all > 2 * d.cluster) d.cluster *= 2;
         const long long ctas = units * d.cluster, last = ctas % cap ? ctas % cap : cap;
         const long long idle = last < kSaturatingCtas ? unit_bytes / d.cluster * (kSaturatingCtas - last) : 0;
         if (tiles > d.cluster * units && (idle > kRangesBytes || (ragged && units * unit_bytes > kRangesBytes))) {
             d.cluster = 0;
             d.n_ctas = (int)std::min<long long>(tiles, cap);
-            d.slot_mode = d.splits == n_all ? kDecodeSlotTile : kDecodeSlotTwo;
+            d.slot_mode = d.slots == n_all ? kDecodeSlotTile : kDecodeSlotTwo;
             return d;
         }
     }
@@ -1010,11 +1011,12 @@ extern "C" int b200attn_decode_ragged(const void* q, const void* kcache, const v
     p.q = static_cast<const uint16_t*>(q);
     p.o = static_cast<uint16_t*>(o);
     p.lse = lse;
-    const size_t rows = (size_t)B * Hq * d.splits;  // slots x heads per slot
+    const size_t rows = (size_t)B * Hq * d.slots;  // slots x heads per slot
     p.part_o = static_cast<float*>(workspace);
     p.part_m = p.part_o + rows * D;
     p.part_l = p.part_m + rows;
-    p.counters = next_decode_counters();
+    p.counters = reinterpret_cast<unsigned long long*>(p.part_l + rows);  // (D + 2 is even: 8-byte aligned)
+    p.tag = next_decode_tag();
     p.status = status;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (D == 64) return d.G <= 8 ? launch_decode<64, 1>(tk, tv, p, d.n_ctas, st) : launch_decode<64, 2>(tk, tv, p, d.n_ctas, st);
@@ -1131,18 +1133,18 @@ extern "C" int b200attn_last_device_status(void* stream) {
         cudaGetLastError();
         return B200ATTN_ERR_CUDA;
     }
-    int host = 0;
-    if (cudaMemcpy(&host, status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return B200ATTN_ERR_CUDA;
-    if (host != 0) {
+    int host[2] = {0, 0};  // status word and epoch
+    if (cudaMemcpy(host, status, sizeof(host), cudaMemcpyDeviceToHost) != cudaSuccess) return B200ATTN_ERR_CUDA;
+    if (host[0] != 0) {
         // a kernel that gave up may have left its item counters behind: wait for everything else on the
         // device (kernels exit at once while the status word is set), then clear counters and status
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceSynchronize();
         cudaMemset(g_sched_ptr[dev], 0, sizeof(int) * 2 * kSchedSlots);
-        cudaMemset(g_decode_ptr[dev], 0, sizeof(int) * kDecodeSlots * kDecodeMaxCtas);
-        cudaMemset(status, 0, sizeof(int));
-        return host;
+        const int next[2] = {0, (host[1] + 1) & ((1 << kDecodeEpochBits) - 1)};
+        cudaMemcpy(status, next, sizeof(next), cudaMemcpyHostToDevice);
+        return host[0];
     }
     return B200ATTN_OK;
 }

@@ -107,3 +107,78 @@ def test_ranges_over_sequences_of_different_lengths(B, L, Hq, Hkv, D):
         wo, wl = ao.decode_c(np32(q[b:b + 1]), np32(kc[b:b + 1, :, :n]), np32(vc[b:b + 1, :, :n]))
         assert_close(f"O[{b}]", o[b:b + 1], wo)
         assert_close(f"LSE[{b}]", lse[b:b + 1], wl, max_abs=TOL_LSE, rel_l2=1.0)
+
+
+class _AbiDecode:
+    """A decode through the C ABI with a workspace of its own; two units shared by every CTA, some by two."""
+
+    def __init__(self, seed, fill=0):
+        self.dims = (2, 30001, 4, 2, 64)
+        B, L, Hq, Hkv, D = self.dims
+        self.q, self.kc, self.vc = randn_bf16((B, Hq, D), seed), randn_bf16((B, Hkv, L, D), seed + 1), randn_bf16((B, Hkv, L, D), seed + 2)
+        self.o, self.lse = torch.empty_like(self.q), torch.empty((B, Hq), device="cuda")
+        self.lib = m._lib.load()
+        self.ws = torch.full((self.lib.b200attn_decode_workspace_bytes(*self.dims, 0),), fill, dtype=torch.uint8, device="cuda")
+
+    def __call__(self):
+        m._lib.check(self.lib.b200attn_decode(
+            *(t.data_ptr() for t in (self.q, self.kc, self.vc, self.o, self.lse)), *self.dims, 0.0, 0, self.ws.data_ptr(), self.ws.numel(),
+            torch.cuda.current_stream().cuda_stream), "decode")
+
+    def poison(self):
+        self.o.fill_(float("nan"))
+        self.lse.fill_(float("nan"))
+
+
+def test_shared_units_do_not_depend_on_what_the_workspace_held():
+    d = _AbiDecode(31)
+    d()
+    m.device_status()
+    o, lse = d.o.clone(), d.lse.clone()
+    g = torch.Generator().manual_seed(0)
+    for fill in (0, 0xFF, 0x7F, 1, None, None, "its own"):
+        if fill is None:
+            d.ws.copy_(torch.randint(0, 256, d.ws.shape, generator=g, dtype=torch.uint8))
+        elif fill != "its own":
+            d.ws.fill_(fill)
+        d.poison()
+        d()
+        m.device_status()
+        assert torch.equal(d.o, o) and torch.equal(d.lse, lse), fill
+
+
+def test_captured_decodes_overlap_with_other_launches():
+    # Two graphs and direct launches on a third stream at the same time, each with its own workspace.  Counters taken in turn
+    # from a common pool of 64 would be shared: 64 launches lie between the captures.
+    ds = [_AbiDecode(41 + 3 * i) for i in range(3)]
+    want = []
+    for d in ds:
+        d()
+        m.device_status()
+        want.append((d.o.clone(), d.lse.clone()))
+    graphs = []
+    for d in ds[:2]:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            for _ in range(20):
+                d()
+        graphs.append(g)
+        for _ in range(64 - 20):
+            d()
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in ds]
+    for _ in range(10):
+        for d in ds:
+            d.poison()
+        torch.cuda.synchronize()
+        for g, s in zip(graphs, streams):
+            with torch.cuda.stream(s):
+                g.replay()
+        with torch.cuda.stream(streams[2]):
+            for _ in range(20):
+                ds[2]()
+        torch.cuda.synchronize()
+        m.device_status()
+        for d, (o, lse) in zip(ds, want):
+            assert torch.equal(d.o, o) and torch.equal(d.lse, lse)
+    del graphs
