@@ -17,9 +17,12 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstring>
 #include <list>
+#include <memory>
+#include <mutex>
 
 #include "../../include/b200attn.h"
 
@@ -141,40 +144,61 @@ struct Call {
     void* st() const { return stream.stream(); }
 };
 
+// The GIL is released for a scope (a full launch queue blocks in the driver) and taken again also when an exception leaves it.
+struct NoGil {
+    PyThreadState* state;
+    NoGil() : state(PyEval_SaveThread()) {}
+    NoGil(const NoGil&) = delete;
+    ~NoGil() { PyEval_RestoreThread(state); }
+};
+
 // Private temporaries of the operators (the reference allocates its D vector per call, llm/src/model/flash_attn.cu:463):
-// one buffer per (device, stream), so that calls issued on different streams never share scratch memory; calls on one
-// stream follow each other on the GPU and may.  A buffer grows when a call needs more and goes back to torch's
+// one buffer per (device, stream), so that calls issued on different streams never share scratch memory.  Calls on one
+// stream follow each other on the GPU and may, provided that a call's launches follow each other without another call's in
+// between (a backward is two launches with the row vectors alive between them): a call holds the buffer's lock from sizing
+// it to its last launch, without the GIL.  A buffer grows when a call needs more and goes back to torch's
 // allocator when it is replaced, when it is the least recently used of more than kMaxScratch (torch itself has 32
-// streams per device and priority) and when the interpreter ends.  Access is under the GIL.
+// streams per device and priority) and when the interpreter ends.  The list is accessed under the GIL; a call keeps its
+// entry alive.
 struct Scratch {
     int device;
     cudaStream_t stream;
+    std::mutex lock;  // of buf, and over the launches of the call that uses it
     at::Tensor buf;
+    Scratch(int d, cudaStream_t s) : device(d), stream(s) {}
 };
 constexpr size_t kMaxScratch = 128;
-std::list<Scratch>& scratch_list() {
-    static std::list<Scratch>* l = new std::list<Scratch>;  // emptied by release_scratch at exit, never destroyed
+std::list<std::shared_ptr<Scratch>>& scratch_list() {
+    static auto* l = new std::list<std::shared_ptr<Scratch>>;  // emptied by release_scratch at exit, never destroyed
     return *l;
 }
 
-const at::Tensor& scratch(const Call& c, size_t bytes) {
-    std::list<Scratch>& l = scratch_list();
+std::shared_ptr<Scratch> scratch_entry(const Call& c) {
+    std::list<std::shared_ptr<Scratch>>& l = scratch_list();
     const int dev = c.stream.device_index();
     auto it = l.begin();
-    while (it != l.end() && !(it->device == dev && it->stream == c.stream.stream())) ++it;
+    while (it != l.end() && !((*it)->device == dev && (*it)->stream == c.stream.stream())) ++it;
     if (it == l.end()) {
-        l.push_front({dev, c.stream.stream(), at::Tensor()});
+        l.push_front(std::make_shared<Scratch>(dev, c.stream.stream()));
         if (l.size() > kMaxScratch) l.pop_back();
     } else if (it != l.begin()) {
         l.splice(l.begin(), l, it);
     }
-    Scratch& s = l.front();
-    if (!s.buf.defined() || static_cast<size_t>(s.buf.numel()) < bytes) {
-        s.buf = at::Tensor();  // the smaller buffer first goes back to the allocator
-        s.buf = at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 4096))},
-                          at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(dev)));
+    return l.front();
+}
+
+// Runs `launch(workspace, its bytes)` with the stream's scratch buffer, at least `bytes` of it.
+template <typename Launch>
+int with_scratch(const Call& c, size_t bytes, Launch launch) {
+    const std::shared_ptr<Scratch> s = scratch_entry(c);
+    const NoGil no_gil;
+    const std::lock_guard<std::mutex> hold(s->lock);
+    if (!s->buf.defined() || static_cast<size_t>(s->buf.numel()) < bytes) {
+        s->buf = at::Tensor();  // the smaller buffer first goes back to the allocator
+        s->buf = at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 4096))},
+                           at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(s->device)));
     }
-    return s.buf;
+    return launch(s->buf.data_ptr(), static_cast<size_t>(s->buf.numel()));
 }
 
 PyObject* release_scratch(PyObject*, PyObject*) {
@@ -188,7 +212,7 @@ bool arg_count(Py_ssize_t got, Py_ssize_t want) {
     return false;
 }
 
-// Launches run without the GIL (a full launch queue blocks in the driver).  C++ exceptions (torch's) become RuntimeError.
+// C++ exceptions (torch's) become RuntimeError.
 #define B200ATTN_TRY try {
 #define B200ATTN_CATCH                                  \
     }                                                   \
@@ -221,9 +245,10 @@ PyObject* fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Call c(a[0]);
     void *q = ptr(a[0]), *k = ptr(a[1]), *v = ptr(a[2]), *o = ptr(a[3]), *lse = ptr(a[4]), *st = c.st();
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = b200attn_fwd(q, k, v, o, static_cast<float*>(lse), d[0], d[1], d[2], d[3], d[4], layout, scale, st);
-    Py_END_ALLOW_THREADS
+    {
+        const NoGil no_gil;
+        rc = b200attn_fwd(q, k, v, o, static_cast<float*>(lse), d[0], d[1], d[2], d[3], d[4], layout, scale, st);
+    }
     return finish(rc, fn);
     B200ATTN_CATCH
 }
@@ -257,16 +282,12 @@ PyObject* bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     float scale;
     if (!scale_of(a[15], &scale)) return nullptr;
     const Call c(a[0]);
-    const at::Tensor& ws = scratch(c, b200attn_bwd_workspace_bytes_mode(d[0], d[1], d[2], d[3], d[4], mode));
-    void* wp = ws.data_ptr();
-    const size_t wn = ws.numel();
     void *q = ptr(a[0]), *k = ptr(a[1]), *v = ptr(a[2]), *o = ptr(a[3]), *lse = ptr(a[4]), *dout = ptr(a[5]), *dq = ptr(a[6]),
          *dk = ptr(a[7]), *dv = ptr(a[8]), *st = c.st();
-    int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = b200attn_bwd_mode(q, k, v, o, static_cast<float*>(lse), dout, dq, dk, dv, d[0], d[1], d[2], d[3], d[4], layout, scale,
-                           mode, wp, wn, st);
-    Py_END_ALLOW_THREADS
+    const int rc = with_scratch(c, b200attn_bwd_workspace_bytes_mode(d[0], d[1], d[2], d[3], d[4], mode), [&](void* wp, size_t wn) {
+        return b200attn_bwd_mode(q, k, v, o, static_cast<float*>(lse), dout, dq, dk, dv, d[0], d[1], d[2], d[3], d[4], layout, scale,
+                                 mode, wp, wn, st);
+    });
     return finish(rc, fn);
     B200ATTN_CATCH
 }
@@ -289,14 +310,10 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     float scale;
     if (!scale_of(a[10], &scale)) return nullptr;
     const Call c(a[0]);
-    const at::Tensor& ws = scratch(c, b200attn_decode_workspace_bytes(d[0], d[1], d[2], d[3], d[4], splits));
-    void* wp = ws.data_ptr();
-    const size_t wn = ws.numel();
     void *q = ptr(a[0]), *k = ptr(a[1]), *v = ptr(a[2]), *o = ptr(a[3]), *lse = with_lse ? ptr(a[4]) : nullptr, *st = c.st();
-    int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = b200attn_decode(q, k, v, o, static_cast<float*>(lse), d[0], d[1], d[2], d[3], d[4], scale, splits, wp, wn, st);
-    Py_END_ALLOW_THREADS
+    const int rc = with_scratch(c, b200attn_decode_workspace_bytes(d[0], d[1], d[2], d[3], d[4], splits), [&](void* wp, size_t wn) {
+        return b200attn_decode(q, k, v, o, static_cast<float*>(lse), d[0], d[1], d[2], d[3], d[4], scale, splits, wp, wn, st);
+    });
     return finish(rc, fn);
     B200ATTN_CATCH
 }
@@ -398,12 +415,13 @@ PyObject* kv_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int* pos = ragged ? static_cast<int*>(pos_t.data_ptr()) : nullptr;
     void *pq = ptr(xq), *pk = ptr(xk), *pv = ptr(xv), *po = ptr(q_out), *st = call.st();
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = ragged ? b200attn_kv_append_at(pq, pk, pv, xd, po, l.k, l.v, gqp, gkp, cp, sp, pos, c.B, 1, c.L_cap, c.Hq, c.Hkv, c.D,
-                                        static_cast<float>(eps), st)
-                : b200attn_kv_append(pq, pk, pv, xd, po, l.k, l.v, gqp, gkp, cp, sp, c.B, int(n_new), c.length, c.L_cap, c.Hq,
-                                     c.Hkv, c.D, static_cast<float>(eps), st);
-    Py_END_ALLOW_THREADS
+    {
+        const NoGil no_gil;
+        rc = ragged ? b200attn_kv_append_at(pq, pk, pv, xd, po, l.k, l.v, gqp, gkp, cp, sp, pos, c.B, 1, c.L_cap, c.Hq, c.Hkv, c.D,
+                                            static_cast<float>(eps), st)
+                    : b200attn_kv_append(pq, pk, pv, xd, po, l.k, l.v, gqp, gkp, cp, sp, c.B, int(n_new), c.length, c.L_cap, c.Hq,
+                                         c.Hkv, c.D, static_cast<float>(eps), st);
+    }
     return finish(rc, fn);
     B200ATTN_CATCH
 }
@@ -437,22 +455,18 @@ PyObject* kv_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
     at::Tensor lens_t;
     if (!cache_layer(self, c, layer, &l) || (ragged && !cache_tensor(self, n_lens_next, &lens_t))) return nullptr;
     const Call call(l.kt.device());
-    void *pq = ptr(q), *po = ptr(ctx), *st = call.st(), *wp = nullptr;
+    void *pq = ptr(q), *po = ptr(ctx), *st = call.st();
     float* pl = with_lse ? static_cast<float*>(ptr(lse)) : nullptr;
     const int* lens = ragged ? static_cast<int*>(lens_t.data_ptr()) : nullptr;
-    size_t wn = 0;
-    if (n_new == 1) {
-        const at::Tensor& ws = scratch(call, b200attn_decode_workspace_bytes(c.B, c.length + 1, c.Hq, c.Hkv, c.D, 0));
-        wp = ws.data_ptr();
-        wn = ws.numel();
-    }
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = n_new == 1 ? b200attn_decode_ragged(pq, l.k, l.v, po, pl, lens, c.B, c.length + 1, c.L_cap, c.Hq, c.Hkv, c.D, scale, 0, wp,
-                                             wn, st)
-                    : b200attn_fwd_kvcache_at(pq, l.k, l.v, po, pl, c.B, n_new, c.length, c.L_cap, c.Hq, c.Hkv, c.D,
-                                              B200ATTN_LAYOUT_BHTD, scale, st);
-    Py_END_ALLOW_THREADS
+    if (n_new == 1) {
+        rc = with_scratch(call, b200attn_decode_workspace_bytes(c.B, c.length + 1, c.Hq, c.Hkv, c.D, 0), [&](void* wp, size_t wn) {
+            return b200attn_decode_ragged(pq, l.k, l.v, po, pl, lens, c.B, c.length + 1, c.L_cap, c.Hq, c.Hkv, c.D, scale, 0, wp, wn, st);
+        });
+    } else {
+        const NoGil no_gil;
+        rc = b200attn_fwd_kvcache_at(pq, l.k, l.v, po, pl, c.B, n_new, c.length, c.L_cap, c.Hq, c.Hkv, c.D, B200ATTN_LAYOUT_BHTD, scale, st);
+    }
     return finish(rc, fn);
     B200ATTN_CATCH
 }
@@ -513,10 +527,11 @@ PyObject* rope_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     void *x = ptr(a[0]), *y = ptr(a[5]), *st = c.st();
     float *gamma = static_cast<float*>(ptr(a[3])), *rstd = static_cast<float*>(ptr(a[6]));
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = b200attn_rope_norm_fwd(x, xd, p.x_layout, y, p.y_layout, rstd, gamma, p.cos_t, p.sin_t, d[0], d[1], d[2], d[3],
-                                static_cast<float>(eps), st);
-    Py_END_ALLOW_THREADS
+    {
+        const NoGil no_gil;
+        rc = b200attn_rope_norm_fwd(x, xd, p.x_layout, y, p.y_layout, rstd, gamma, p.cos_t, p.sin_t, d[0], d[1], d[2], d[3],
+                                    static_cast<float>(eps), st);
+    }
     return finish(rc, fn);
     B200ATTN_CATCH
 }
@@ -543,16 +558,12 @@ PyObject* rope_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (numel(a[0]) != rows * p.D || numel(a[6]) != rows * p.D || numel(a[7]) != p.D)
         return value_error("%s: shape mismatch (d_y/d_x/d_gamma)", fn);
     const Call c(a[1]);
-    const at::Tensor& ws = scratch(c, b200attn_rope_norm_bwd_workspace_bytes(p.D));
-    void* wp = ws.data_ptr();
-    const size_t wn = ws.numel();
     void *dy = ptr(a[0]), *x = ptr(a[1]), *dx = ptr(a[6]), *st = c.st();
     float *gamma = static_cast<float*>(ptr(a[4])), *rstd = static_cast<float*>(ptr(a[5])), *dg = static_cast<float*>(ptr(a[7]));
-    int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = b200attn_rope_norm_bwd(dy, p.y_layout, x, xd, p.x_layout, rstd, gamma, p.cos_t, p.sin_t, dx, dg, d[0], d[1], d[2], d[3], wp,
-                                wn, st);
-    Py_END_ALLOW_THREADS
+    const int rc = with_scratch(c, b200attn_rope_norm_bwd_workspace_bytes(p.D), [&](void* wp, size_t wn) {
+        return b200attn_rope_norm_bwd(dy, p.y_layout, x, xd, p.x_layout, rstd, gamma, p.cos_t, p.sin_t, dx, dg, d[0], d[1], d[2], d[3], wp,
+                                      wn, st);
+    });
     return finish(rc, fn);
     B200ATTN_CATCH
 }
@@ -587,10 +598,11 @@ PyObject* rope_fwd_qk(PyObject*, PyObject* const* a, Py_ssize_t n) {
     float *gq = static_cast<float*>(ptr(a[4])), *gk = static_cast<float*>(ptr(a[5])), *sq = static_cast<float*>(ptr(a[9])),
           *sk = static_cast<float*>(ptr(a[10]));
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = b200attn_rope_norm_fwd_qk(xq, xk, xd, p.x_layout, yq, yk, p.y_layout, sq, sk, gq, gk, p.cos_t, p.sin_t, d[0], d[1], d[2],
-                                   d[3], d[4], static_cast<float>(eps), st);
-    Py_END_ALLOW_THREADS
+    {
+        const NoGil no_gil;
+        rc = b200attn_rope_norm_fwd_qk(xq, xk, xd, p.x_layout, yq, yk, p.y_layout, sq, sk, gq, gk, p.cos_t, p.sin_t, d[0], d[1], d[2],
+                                       d[3], d[4], static_cast<float>(eps), st);
+    }
     return finish(rc, fn);
     B200ATTN_CATCH
 }
@@ -622,17 +634,13 @@ PyObject* rope_bwd_qk(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (numel(a[7]) != p.D || numel(a[9]) != rk || numel(a[12]) != p.D || numel(a[13]) != p.D)
         return value_error("%s: shape mismatch (gamma_k/rstd_k/d_gamma)", fn);
     const Call c(a[2]);
-    const at::Tensor& ws = scratch(c, b200attn_rope_norm_bwd_workspace_bytes(p.D));
-    void* wp = ws.data_ptr();
-    const size_t wn = ws.numel();
     void *dyq = ptr(a[0]), *dyk = ptr(a[1]), *xq = ptr(a[2]), *xk = ptr(a[3]), *dxq = ptr(a[10]), *dxk = ptr(a[11]), *st = c.st();
     float *gq = static_cast<float*>(ptr(a[6])), *gk = static_cast<float*>(ptr(a[7])), *sq = static_cast<float*>(ptr(a[8])),
           *sk = static_cast<float*>(ptr(a[9])), *dgq = static_cast<float*>(ptr(a[12])), *dgk = static_cast<float*>(ptr(a[13]));
-    int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = b200attn_rope_norm_bwd_qk(dyq, dyk, p.y_layout, xq, xk, xd, p.x_layout, sq, sk, gq, gk, p.cos_t, p.sin_t, dxq, dxk, dgq, dgk,
-                                   d[0], d[1], d[2], d[3], d[4], wp, wn, st);
-    Py_END_ALLOW_THREADS
+    const int rc = with_scratch(c, b200attn_rope_norm_bwd_workspace_bytes(p.D), [&](void* wp, size_t wn) {
+        return b200attn_rope_norm_bwd_qk(dyq, dyk, p.y_layout, xq, xk, xd, p.x_layout, sq, sk, gq, gk, p.cos_t, p.sin_t, dxq, dxk, dgq,
+                                         dgk, d[0], d[1], d[2], d[3], d[4], wp, wn, st);
+    });
     return finish(rc, fn);
     B200ATTN_CATCH
 }
