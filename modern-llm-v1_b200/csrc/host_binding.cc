@@ -13,16 +13,19 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdarg>
 #include <cstring>
 #include <list>
 #include <memory>
 #include <mutex>
+#include <vector>
 
 #include "../../include/b200attn.h"
 
@@ -158,13 +161,16 @@ struct NoGil {
 // between (a backward is two launches with the row vectors alive between them): a call holds the buffer's lock from sizing
 // it to its last launch, without the GIL.  A buffer grows when a call needs more and goes back to torch's
 // allocator when it is replaced, when it is the least recently used of more than kMaxScratch (torch itself has 32
-// streams per device and priority) and when the interpreter ends.  The list is accessed under the GIL; a call keeps its
-// entry alive.
+// streams per device and priority) and when the interpreter ends.  A captured launch keeps the address, so a buffer that one
+// has used is not given back before the end; it then grows at least by doubling, so what is kept that way is less than the
+// buffer itself.  The list is accessed under the GIL; a call keeps its entry alive.
 struct Scratch {
     int device;
     cudaStream_t stream;
     std::mutex lock;  // of buf, and over the launches of the call that uses it
     at::Tensor buf;
+    std::vector<at::Tensor> kept;        // outgrown buffers that captured launches may still use
+    std::atomic<bool> captured{false};  // a capture has used buf: the entry stays
     Scratch(int d, cudaStream_t s) : device(d), stream(s) {}
 };
 constexpr size_t kMaxScratch = 128;
@@ -180,7 +186,10 @@ std::shared_ptr<Scratch> scratch_entry(const Call& c) {
     while (it != l.end() && !((*it)->device == dev && (*it)->stream == c.stream.stream())) ++it;
     if (it == l.end()) {
         l.push_front(std::make_shared<Scratch>(dev, c.stream.stream()));
-        if (l.size() > kMaxScratch) l.pop_back();
+        if (l.size() > kMaxScratch) {
+            auto last = std::find_if(l.rbegin(), l.rend(), [](const auto& s) { return !s->captured; });
+            if (last != l.rend()) l.erase(std::next(last).base());
+        }
     } else if (it != l.begin()) {
         l.splice(l.begin(), l, it);
     }
@@ -194,10 +203,15 @@ int with_scratch(const Call& c, size_t bytes, Launch launch) {
     const NoGil no_gil;
     const std::lock_guard<std::mutex> hold(s->lock);
     if (!s->buf.defined() || static_cast<size_t>(s->buf.numel()) < bytes) {
+        if (s->captured && s->buf.defined()) {
+            bytes = std::max(bytes, 2 * static_cast<size_t>(s->buf.numel()));
+            s->kept.push_back(std::move(s->buf));
+        }
         s->buf = at::Tensor();  // the smaller buffer first goes back to the allocator
         s->buf = at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 4096))},
                            at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(s->device)));
     }
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) s->captured = true;
     return launch(s->buf.data_ptr(), static_cast<size_t>(s->buf.numel()));
 }
 

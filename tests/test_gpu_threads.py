@@ -1,5 +1,5 @@
-"""Operators called from several host threads, all on one CUDA stream (every thread's default): an operator's launches may not
-have another call's between them while they share scratch memory."""
+"""Scratch memory of the operators.  Operators called from several host threads, all on one CUDA stream (every thread's default): an operator's launches may not
+have another call's between them while they share scratch memory.  A captured backward keeps its scratch when the stream's buffer grows."""
 import threading
 
 import pytest
@@ -80,3 +80,37 @@ def test_backward_beside_other_operators_of_other_threads():
     m.device_status()
     wrong = sum(not torch.equal(a, b) for side in outs for got in side for a, b in zip(got, want))
     assert wrong == 0, f"{wrong} of {2 * 3 * n} gradients differ"
+
+
+def test_a_captured_backward_keeps_its_scratch():
+    B, T, Hq, Hkv, D = 1, 256, 2, 1, 64
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        q, k, v, do = (randn_bf16((B, h, T, D), s) for s, h in ((1, Hq), (2, Hkv), (3, Hkv), (4, Hq)))
+        o, lse = torch.empty_like(q), torch.empty((B, Hq, T), device="cuda")
+        m.flash_attn_forward_gqa(q, k, v, o, lse, B, T, Hq, Hkv, D)
+        grads = tuple(torch.empty_like(t) for t in (q, k, v))
+        run = lambda: m.flash_attn_backward_gqa(q, k, v, o, lse, do, *grads, B, T, Hq, Hkv, D)
+        run()
+        m.device_status()
+        want = tuple(t.clone() for t in grads)
+        graph = torch.cuda.CUDAGraph()
+        side.synchronize()
+        with torch.cuda.graph(graph, stream=side):
+            run()
+        # larger problems on the same stream outgrow the buffer the graph writes its row vectors to; whatever is allocated
+        # then may not lie in it
+        for n in (2, 8, 64):
+            big = [randn_bf16((n, h, T, D), s) for s, h in ((1, Hq), (2, Hkv), (3, Hkv), (4, Hq))]
+            bo, bl = torch.empty_like(big[0]), torch.empty((n, Hq, T), device="cuda")
+            m.flash_attn_forward_gqa(*big[:3], bo, bl, n, T, Hq, Hkv, D)
+            m.flash_attn_backward_gqa(*big[:3], bo, bl, big[3], *(torch.empty_like(t) for t in big[:3]), n, T, Hq, Hkv, D)
+            del big, bo, bl
+            others = [torch.full((size,), 7, dtype=torch.uint8, device="cuda") for size in (4096, 8192, 16384, 65536) for _ in range(50)]
+            for t in grads:
+                t.fill_(float("nan"))
+            graph.replay()
+            side.synchronize()
+            assert all((t == 7).all().item() for t in others)
+            assert all(torch.equal(a, b) for a, b in zip(grads, want))
+    m.device_status()
