@@ -140,16 +140,18 @@ int b200attn_bwd_static(const void* q, const void* k, const void* v, const void*
  * NULL.  Equals row L-1 of b200attn_fwd with T = L.  The reference has no such
  * path: infer_modern_gpt re-runs the full forward per token
  * (llm/apps/infer_modern_gpt.cu:253-255); this is the kernel its KV cache would call.
- * n_splits <= 0 lets the library choose how the cache is split over CTAs; n_splits > 0 asks for that many splits
- * per (batch, KV head) and gets the next power of two below, at most 8.  Results are bit-reproducible either
- * way.  workspace: at least b200attn_decode_workspace_bytes(...) bytes, 256-byte aligned; it needs no initialisation,
- * and calls that may overlap (other streams, concurrently replayed graphs) need workspaces of their own.
+ * n_splits <= 0 lets the library choose how the cache is split over CTAs; n_splits > 0 asks for that many even splits
+ * per (batch, KV head) of blocks of 128 keys, at most 64 and none of them empty.  Results are bit-reproducible either
+ * way.  workspace: at least b200attn_decode_workspace_bytes(...) bytes, 256-byte aligned, required also where the split
+ * chosen leaves nothing in it; it needs no initialisation, and calls that may overlap (other streams, concurrently
+ * replayed graphs) need workspaces of their own.
  */
 int b200attn_decode(const void* q, const void* kcache, const void* vcache, void* o, float* lse, int B, int L, int Hq,
                     int Hkv, int D, float softmax_scale, int n_splits, void* workspace, size_t workspace_bytes,
                     void* stream);
 size_t b200attn_decode_workspace_bytes(int B, int L, int Hq, int Hkv, int D, int n_splits);
-/* The workspace slots per (batch, KV head) that b200attn_decode needs for n_splits <= 0. */
+/* The slots of (D + 2) floats per (batch, query head) that the workspace has for n_splits <= 0.  Not the number of CTAs that
+ * share a cache: the library's own split is not even, and may need no slot at all. */
 int b200attn_decode_default_splits(int B, int L, int Hq, int Hkv, int D);
 
 /* Element type of a projection output handed to the RoPE / QK-Norm / KV-cache calls. */

@@ -7,8 +7,9 @@
 // (batch, KV head, chunk of at most 16 query heads of the group): all its query heads are served from the same K/V tile,
 // which is the bandwidth win of GQA.  One launch does everything; it deals the units' tiles in one of two ways
 // (decode_plan in b200attn_api.cu chooses):
-//  * clusters: a unit's tiles are split over the CTAs of a cluster (1, 2, 4 or 8), which exchange their partial results
-//    through distributed shared memory, each CTA finishing a slice of the outputs.
+//  * shares: a unit's tiles are split evenly over 1, 2, 4 or 8 CTAs, a cluster, which exchange their partial results
+//    through distributed shared memory, each CTA finishing a slice of the outputs.  (A caller may ask for any other number of
+//    shares; their partial results go through the workspace as in the next deal.)
 //  * ranges: the tiles of all units are numbered through and CTA c of n takes tiles [c total / n, (c + 1) total / n), the
 //    same number for every CTA (to one) whatever the units' lengths are.  A range falls into pieces at unit boundaries; a
 //    piece that is a whole unit is written at once, the pieces of a unit that several CTAs share are left un-normalised
@@ -41,8 +42,9 @@ struct DecodeParams {
     int G;         // query heads per unit (a divisor of group, <= 16)
     int n_chunks;  // group / G
     int units_per_seq;  // Hkv * n_chunks
-    FastDiv div_units, div_chunks, div_cluster, div_tiles, div_slice;  // by units_per_seq, n_chunks, cluster, tiles of L, output pairs per CTA of a cluster
-    int cluster;        // CTAs per unit (clusters), or 0: ranges
+    FastDiv div_units, div_chunks, div_shares, div_tiles, div_slice;  // by units_per_seq, n_chunks, shares, tiles of L, output pairs per CTA of a cluster
+    int shares;         // CTAs per unit, or 0: ranges
+    int cluster;        // CTAs per cluster: shares where they exchange through distributed shared memory, else 1
     int whole;          // ranges: they begin and end at unit boundaries (all sequences have length L)
     int slot_mode;      // where a shared unit's pieces lie in the workspace, see decode_slot
     float scale, scale_log2;
@@ -54,14 +56,14 @@ struct DecodeParams {
     float* part_m;      // [slot][G]     row maximum, raw score units
     float* part_l;      // [slot][G]     sum of exp2((s - m) * scale_log2)
     unsigned long long* counters;  // one per CTA, see decode_count: pieces finished of the shared unit that begins in that CTA
+                                   // (not where a cluster shares it)
     unsigned long long tag;        // of this launch
     int* status;                   // status word and epoch
 };
 
 constexpr int kDecodeMaxCtas = 320, kDecodeMaxCluster = 8, kDecodeThreads = 192;
-// Workspace slot of CTA c's piece of a shared unit.  The workspace has (units x splits) slots: one per tile when every
-// split is one tile (mode 0), one per CTA when the CTAs' ranges begin at unit boundaries (mode 1), else two per CTA
-// (mode 2: a range may end one shared unit and begin another).
+// Workspace slot of CTA c's piece of a shared unit: one per tile when there are as many slots (mode 0), one per CTA in the deal
+// by shares (mode 1), else two per CTA (mode 2: a range may end one shared unit and begin another).
 enum { kDecodeSlotTile = 0, kDecodeSlotCta = 1, kDecodeSlotTwo = 2 };
 
 template <int D>
@@ -116,7 +118,8 @@ struct DecodeWalk {
     int t, t_end;        // next tile and end of this CTA's range, in the numbering over all units
     int b, u, j0;        // unit at t: sequence, unit within the sequence, tile within the unit
     int len, n_tiles;    // length and tiles per unit of sequence b
-    int total, n_ctas;   // tiles of all units, CTAs that share them
+    int total, n_ctas;   // tiles of all units (shares: of the unit), CTAs that share them
+    int cta0;            // the first of those CTAs
 };
 
 __device__ __forceinline__ int decode_len(const DecodeParams& p, int b) {
@@ -134,18 +137,25 @@ __device__ __forceinline__ int decode_cta_of(const DecodeWalk& w, int t) {
 template <int KEYS>
 __device__ __forceinline__ DecodeWalk decode_walk_start(const DecodeParams& p, int cta, int n_ctas, int lane) {
     DecodeWalk w;
-    if (p.cluster) {  // one piece: this CTA's share of its unit's tiles, possibly none
-        const int unit = int(fastdiv(cta, p.div_cluster)), rank = cta - unit * p.cluster;
+    if (p.shares) {  // one piece: this CTA's share of its unit's tiles, possibly none
+        const int unit = int(fastdiv(cta, p.div_shares)), rank = cta - unit * p.shares;
         w.b = int(fastdiv(unit, p.div_units));
         w.u = unit - w.b * p.units_per_seq;
         w.len = decode_len(p, w.b);
         w.n_tiles = (w.len + KEYS - 1) / KEYS;
         w.total = w.n_tiles;
-        w.n_ctas = p.cluster;
-        w.t = w.j0 = int(fastdiv(w.n_tiles * rank, p.div_cluster));
-        w.t_end = int(fastdiv(w.n_tiles * (rank + 1), p.div_cluster));
+        w.cta0 = unit * p.shares;
+        w.n_ctas = p.shares;
+        w.t = w.j0 = int(fastdiv(w.n_tiles * rank, p.div_shares));
+        w.t_end = int(fastdiv(w.n_tiles * (rank + 1), p.div_shares));
+        if (p.cluster == 1 && w.n_tiles < p.shares) {  // a sequence shorter than that: the pieces are counted, none may be empty
+            w.n_ctas = w.n_tiles;
+            w.t = w.j0 = min(rank, w.n_tiles);
+            w.t_end = min(rank + 1, w.n_tiles);
+        }
         return w;
     }
+    w.cta0 = 0;
     if (!p.lens) {
         w.len = p.L;
         w.n_tiles = (p.L + KEYS - 1) / KEYS;
@@ -212,7 +222,7 @@ __device__ __forceinline__ void decode_walk_next(const DecodeParams& p, DecodeWa
 }
 __device__ __forceinline__ int decode_slot(const DecodeParams& p, const DecodeWalk& w, int c, int first_cta, int unit_start) {
     if (p.slot_mode == kDecodeSlotTile) return max(unit_start, decode_range(w, c));
-    if (p.slot_mode == kDecodeSlotCta) return c;
+    if (p.slot_mode == kDecodeSlotCta) return w.cta0 + c;
     return 2 * c + (c == first_cta ? 1 : 0);
 }
 
@@ -458,7 +468,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         grid_dep_wait();
         const DecodeWalk w = decode_walk_start<KEYS>(p, int(blockIdx.x), int(gridDim.x), lane);
         __syncthreads();
-        if (p.cluster || *fail_flag != 0 || w.t >= w.t_end) return;
+        if (p.shares || *fail_flag != 0 || w.t >= w.t_end) return;
         const int tiles = decode_piece(w);
         if (tiles == w.n_tiles || w.t + tiles == w.t_end) return;
         const int unit_start = w.t - w.j0;
@@ -644,16 +654,17 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         } else if (tiles == w.n_tiles) {
             decode_merge<D, NH>(st, sO, sMl, warp, lane, tid, G, p.scale_log2, write_rows);
         } else {
-            const int cta = int(blockIdx.x);
+            const int cta = int(blockIdx.x) - w.cta0;
             const int unit_start = w.t - w.j0;
             const int first = decode_cta_of(w, unit_start), last = decode_cta_of(w, unit_start + w.n_tiles - 1);
             const size_t slot = decode_slot(p, w, cta, first, unit_start);
             const bool ends_range = w.t + tiles == w.t_end;
             // At the range's end nothing is left to hide latency behind.  Usually all other pieces have been stored by then
             // (they lie at the beginning of their CTAs' ranges): one look at the counter instead of store, fence and count.
+            unsigned long long* const counter = p.counters + w.cta0 + first;
             const unsigned long long tag = p.tag + ((unsigned long long)*epoch << kDecodeCountBits);
             unsigned long long seen = 0;
-            if (tid == 0 && ends_range) seen = decode_ld_acquire(p.counters + first);
+            if (tid == 0 && ends_range) seen = decode_ld_acquire(counter);
             if (tid == 0) *last_flag = ends_range && seen == tag + (last - first);
             decode_merge<D, NH>(st, sO, sMl, warp, lane, tid, G, p.scale_log2, [&](int g, int d, float a0, float a1, float m, float l) {
                 if (*last_flag) {
@@ -669,13 +680,13 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
             if (!ends_range) {
                 mbar_arrive(bar_part);
             } else if (*last_flag) {
-                if (tid == 0) p.counters[first] = tag;
+                if (tid == 0) *counter = tag;
             } else {
                 __threadfence();
                 named_bar_sync(1, 128);
                 if (tid == 0) {
-                    const bool is_last = decode_count(p.counters + first, tag, seen) == last - first + 1;
-                    if (is_last) p.counters[first] = tag;
+                    const bool is_last = decode_count(counter, tag, seen) == last - first + 1;
+                    if (is_last) *counter = tag;
                     *last_flag = is_last;
                     __threadfence();
                 }

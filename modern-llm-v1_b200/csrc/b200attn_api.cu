@@ -868,7 +868,8 @@ struct DecodePlan {
     int G, n_chunks;
     int slots;    // workspace slots per unit for partial results
     int splits;   // and with the room for the counters behind them
-    int cluster;  // CTAs per unit, or 0: ranges of tiles
+    int shares;   // CTAs per unit, or 0: ranges of tiles
+    int cluster;  // CTAs per cluster
     bool whole;   // ranges of whole units
     int n_ctas, slot_mode;
 };
@@ -884,7 +885,7 @@ struct DecodePlan {
 // A cluster is the smallest that leaves a CTA at most two tiles, as far as that is one CTA per SM: more of them saturate
 // HBM by themselves.
 //
-// n_splits > 0 asks for that many splits per unit: clusters of the next power of two below.
+// n_splits > 0 asks for that many shares per unit (at most 64, none empty): a cluster where it can have that size.
 constexpr long long kRangesBytes = 16ll << 20;
 constexpr int kSaturatingCtas = 60;
 
@@ -896,31 +897,42 @@ DecodePlan decode_plan(int B, int L, int Hq, int Hkv, int D, int n_splits, bool 
     const long long units = (long long)B * Hkv * d.n_chunks;
     const int keys = decode_tile_keys(D), n_all = (L + keys - 1) / keys, n_128 = (L + 127) / 128;
     const long long unit_bytes = 4ll * L * D, tiles = units * n_all;
-    d.cluster = 1;
+    d.shares = d.cluster = 1;
     d.whole = false;
     d.slot_mode = kDecodeSlotTile;
+    long long counters = 0;
     if (n_splits > 0) {
         const int want = std::min(std::min(n_splits, n_128), 64), per = (n_128 + want - 1) / want;
-        d.splits = d.slots = (n_128 + per - 1) / per;  // no split is empty
-        while (d.cluster * 2 <= std::min(d.splits, kDecodeMaxCluster)) d.cluster *= 2;
+        d.slots = d.shares = (n_128 + per - 1) / per;
+        if (d.shares <= kDecodeMaxCluster && (d.shares & (d.shares - 1)) == 0) {
+            d.cluster = d.shares;
+        } else {
+            d.slot_mode = kDecodeSlotCta;
+            counters = units * d.shares;
+        }
     } else {
         d.slots = (int)std::min<long long>(n_all, (2 * cap + units - 1) / units);
-        // a counter per CTA of the ranges, in units of a slot of every (batch, query head); a single tile is never shared
-        const long long slot_bytes = (long long)B * Hq * (D + 2) * 4, counter_bytes = n_all > 1 ? 8ll * std::min<long long>(tiles, cap) : 0;
-        d.splits = d.slots + (int)((counter_bytes + slot_bytes - 1) / slot_bytes);
+        if (n_all > 1) counters = std::min<long long>(tiles, cap);  // (a single tile is never shared)
         while (d.cluster < kDecodeMaxCluster && units * d.cluster * 2 <= sm_count() && n_all > 2 * d.cluster) d.cluster *= 2;
+        d.shares = d.cluster;
         const long long ctas = units * d.cluster, last = ctas % cap ? ctas % cap : cap;
         const long long idle = last < kSaturatingCtas ? unit_bytes / d.cluster * (kSaturatingCtas - last) : 0;
         if (tiles > d.cluster * units && (idle > kRangesBytes || (ragged && units * unit_bytes > kRangesBytes))) {
-            d.cluster = 0;
-            d.n_ctas = (int)std::min<long long>(tiles, cap);
+            d.shares = 0;
+            d.cluster = 1;
             d.slot_mode = d.slots == n_all ? kDecodeSlotTile : kDecodeSlotTwo;
-            return d;
         }
     }
-    d.n_ctas = (int)std::min<long long>(units * d.cluster, 1ll << 30);
-    if (d.cluster == 1 && units > cap && !ragged) {  // the ring of a CTA then runs on from unit to unit
-        d.cluster = 0;
+    // the counters behind the slots, in units of a slot of every (batch, query head)
+    const long long slot_bytes = (long long)B * Hq * (D + 2) * 4;
+    d.splits = d.slots + (int)((8 * counters + slot_bytes - 1) / slot_bytes);
+    if (d.shares == 0) {
+        d.n_ctas = (int)std::min<long long>(tiles, cap);
+        return d;
+    }
+    d.n_ctas = (int)std::min<long long>(units * d.shares, 1ll << 30);
+    if (d.shares == 1 && units > cap && !ragged) {  // the ring of a CTA then runs on from unit to unit
+        d.shares = 0;
         d.whole = true;
         d.n_ctas = cap;
     }
@@ -999,9 +1011,10 @@ extern "C" int b200attn_decode_ragged(const void* q, const void* kcache, const v
     p.units_per_seq = Hkv * d.n_chunks;
     p.div_units = fastdiv_make((unsigned)p.units_per_seq);
     p.div_chunks = fastdiv_make((unsigned)d.n_chunks);
-    p.div_cluster = fastdiv_make((unsigned)std::max(d.cluster, 1));
+    p.div_shares = fastdiv_make((unsigned)std::max(d.shares, 1));
     p.div_tiles = fastdiv_make((unsigned)((L + decode_tile_keys(D) - 1) / decode_tile_keys(D)));
-    p.div_slice = fastdiv_make((unsigned)(d.G * (D / 2) / std::max(d.cluster, 1)));
+    p.div_slice = fastdiv_make((unsigned)(d.G * (D / 2) / d.cluster));
+    p.shares = d.shares;
     p.cluster = d.cluster;
     p.whole = d.whole;
     p.slot_mode = d.slot_mode;

@@ -82,6 +82,12 @@ def test_workspace_sizes(lib):
     assert lib.b200attn_decode_workspace_bytes(64, 4096, 16, 4, 64, 0) == 64 * 16 * s * (64 + 2) * 4
     assert lib.b200attn_decode_workspace_bytes(2, 100, 4, 2, 64, 9) == 2 * 4 * 1 * 66 * 4  # one tile -> one split
     assert lib.b200attn_decode_default_splits(1, 128, 6, 4, 64) == 0
+    # n_splits asks for that many splits: a slot each, and a counter each where a cluster cannot have that size
+    for splits in range(1, 70):
+        n = -(-17 // -(-17 // min(splits, 17)))  # of 17 blocks of 128 keys, none empty
+        slot = 2 * 6 * (64 + 2) * 4
+        extra = 0 if n in (1, 2, 4, 8) else -(-2 * 2 * n * 8 // slot)
+        assert lib.b200attn_decode_workspace_bytes(2, 2085, 6, 2, 64, splits) == slot * (n + extra), splits
 
 
 def test_check_maps_status_to_reference_exception_types(lib):

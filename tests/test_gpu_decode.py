@@ -182,3 +182,36 @@ def test_captured_decodes_overlap_with_other_launches():
         for d, (o, lse) in zip(ds, want):
             assert torch.equal(d.o, o) and torch.equal(d.lse, lse)
     del graphs
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("splits", [3, 5, 7, 11, 16, 40, 64])
+def test_any_number_of_splits_matches_the_oracle(splits, D):
+    # numbers a cluster cannot have: partial results through the workspace, added up by whoever finishes last
+    B, L, Hq, Hkv = 2, 2085, 12, 2
+    q, kc, vc = randn_bf16((B, Hq, D), 51), randn_bf16((B, Hkv, L, D), 52), randn_bf16((B, Hkv, L, D), 53)
+    o, lse = _decode(q, kc, vc, splits)
+    wo, wl = ao.decode_c(np32(q), np32(kc), np32(vc))
+    assert_close("O", o, wo)
+    assert_close("LSE", lse, wl, max_abs=TOL_LSE, rel_l2=1.0)
+    o2, lse2 = _decode(q, kc, vc, splits)
+    assert torch.equal(o, o2) and torch.equal(lse, lse2)
+
+
+@pytest.mark.parametrize("splits", [5, 12])
+def test_splits_over_sequences_shorter_than_them(splits):
+    # lengths of 1 .. 17 blocks: a sequence of fewer blocks than splits leaves the other CTAs without a piece
+    B, L, Hq, Hkv, D = 9, 2100, 6, 2, 64
+    lens = [1 + (L - 1) * b // (B - 1) for b in range(B)]
+    q, kc, vc = randn_bf16((B, Hq, D), 54), randn_bf16((B, Hkv, L, D), 55), randn_bf16((B, Hkv, L, D), 56)
+    lens_d = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    o, lse = torch.full_like(q, float("nan")), torch.full((B, Hq), float("nan"), device="cuda")
+    lib = m._lib.load()
+    ws = torch.empty(lib.b200attn_decode_workspace_bytes(B, L, Hq, Hkv, D, splits), dtype=torch.uint8, device="cuda")
+    m._lib.check(lib.b200attn_decode_ragged(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), o.data_ptr(), lse.data_ptr(), lens_d.data_ptr(), B, L,
+                                            L, Hq, Hkv, D, 0.0, splits, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream), "decode")
+    m.device_status()
+    for b, n in enumerate(lens):
+        wo, wl = ao.decode_c(np32(q[b:b + 1]), np32(kc[b:b + 1, :, :n]), np32(vc[b:b + 1, :, :n]))
+        assert_close(f"O[{b}]", o[b:b + 1], wo)
+        assert_close(f"LSE[{b}]", lse[b:b + 1], wl, max_abs=TOL_LSE, rel_l2=1.0)
