@@ -63,11 +63,6 @@ __device__ __forceinline__ uint32_t rn_pack_bf16x2(float lo, float hi) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
     return r;
 }
-__device__ __forceinline__ float rn_warp_sum(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 // sum over the LPR lanes that share a row (LPR a power of two, lanes of a row are adjacent)
 template <int LPR>
 __device__ __forceinline__ float rn_row_sum(float v) {
