@@ -448,9 +448,9 @@ int launch_bwd_onepass(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
     return B200ATTN_OK;
 }
 
+// own: what the dQ pass alone reads or writes through TMA.  D = 64: K and V in boxes of 64 rows, and O; D = 128: dQ.
 template <int D>
-int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk64, const CUtensorMap& tv64, const CUtensorMap& tk,
-               const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& to, const CUtensorMap& tdq,
+int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap (&own)[3],
                const BwdParams& p, cudaStream_t st) {
     static bool dq_set[kMaxDevices] = {false}, dkdv_set[kMaxDevices] = {false};
     // D = 64: 64-key tiles, two CTAs per SM.  D = 128: 128-key tiles, one CTA per SM (tensor-pipe bound).
@@ -466,13 +466,13 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk64, const CUtensorMap
     const unsigned dq_items = (unsigned)(p.n_tiles * p.Hq * p.B);
     cudaError_t e;
     if constexpr (kWide) {
-        e = launch_pdl(attn_bwd_dq_wide_kernel<D>, dq_items, DqWideCfg<D>::kThreads, DqWideCfg<D>::kSmemBytes, st, tq, tk, tv, tdo, tdq, p);
+        e = launch_pdl(attn_bwd_dq_wide_kernel<D>, dq_items, DqWideCfg<D>::kThreads, DqWideCfg<D>::kSmemBytes, st, tq, tk, tv, tdo, own[0], p);
     } else {
         // the D = 64 kernel is persistent: two CTAs per SM walk the item list
         const unsigned dq_grid = std::min(dq_items, 2u * (unsigned)sm_count());
         BwdParams pq = p;
         pq.sched = next_sched_pair(dq_items, dq_grid);
-        e = launch_pdl(attn_bwd_dq_kernel<D>, dq_grid, DqCfg<D>::kThreads, DqCfg<D>::kSmemBytes, st, tq, tk64, tv64, tdo, to, pq,
+        e = launch_pdl(attn_bwd_dq_kernel<D>, dq_grid, DqCfg<D>::kThreads, DqCfg<D>::kSmemBytes, st, tq, own[0], own[1], tdo, own[2], pq,
                        item_table_for(pq.sched ? -1 : (long long)dq_items, dq_grid, p.B * p.Hq, p.n_tiles, p.T, 4));
     }
     if (e != cudaSuccess) {
@@ -750,16 +750,18 @@ extern "C" int b200attn_bwd_mode(const void* q, const void* k, const void* v, co
     int* status = status_ptr(&rc);
     if (!status) return rc;
     const Strides sq = strides_for(layout, Hq, T, D), sk = strides_for(layout, Hkv, T, D);
-    CUtensorMap tq, tk, tv, tk64, tv64, tdo, to, tdq;
-    if (!make_tmap_bf16_4d(&tq, q, D, T, Hq, B, sq.t, sq.h, sq.b, 128) ||
-        !make_tmap_bf16_4d(&tk, k, D, T, Hkv, B, sk.t, sk.h, sk.b, 128) ||
-        !make_tmap_bf16_4d(&tv, v, D, T, Hkv, B, sk.t, sk.h, sk.b, 128) ||
-        !make_tmap_bf16_4d(&tk64, k, D, T, Hkv, B, sk.t, sk.h, sk.b, 64) ||
-        !make_tmap_bf16_4d(&tv64, v, D, T, Hkv, B, sk.t, sk.h, sk.b, 64) ||
-        !make_tmap_bf16_4d(&tdo, dout, D, T, Hq, B, sq.t, sq.h, sq.b, 128) ||
-        !make_tmap_bf16_4d(&to, o, D, T, Hq, B, sq.t, sq.h, sq.b, 128) ||
-        !make_tmap_bf16_4d(&tdq, dq, D, T, Hq, B, sq.t, sq.h, sq.b, 128))
-        return B200ATTN_ERR_TENSOR_MAP;
+    CUtensorMap tq, tk, tv, tdo, own[3];
+    bool maps = make_tmap_bf16_4d(&tq, q, D, T, Hq, B, sq.t, sq.h, sq.b, 128) &&
+                make_tmap_bf16_4d(&tk, k, D, T, Hkv, B, sk.t, sk.h, sk.b, 128) &&
+                make_tmap_bf16_4d(&tv, v, D, T, Hkv, B, sk.t, sk.h, sk.b, 128) &&
+                make_tmap_bf16_4d(&tdo, dout, D, T, Hq, B, sq.t, sq.h, sq.b, 128);
+    if (mode == B200ATTN_BWD_TWO_PASS && D == 64)
+        maps = maps && make_tmap_bf16_4d(&own[0], k, D, T, Hkv, B, sk.t, sk.h, sk.b, 64) &&
+               make_tmap_bf16_4d(&own[1], v, D, T, Hkv, B, sk.t, sk.h, sk.b, 64) &&
+               make_tmap_bf16_4d(&own[2], o, D, T, Hq, B, sq.t, sq.h, sq.b, 128);
+    else if (mode == B200ATTN_BWD_TWO_PASS)
+        maps = maps && make_tmap_bf16_4d(&own[0], dq, D, T, Hq, B, sq.t, sq.h, sq.b, 128);
+    if (!maps) return B200ATTN_ERR_TENSOR_MAP;
     float* ws = static_cast<float*>(workspace);
     const size_t nvec = bwd_vec_elems(B, T, Hq);
     BwdParams p;
@@ -801,8 +803,7 @@ extern "C" int b200attn_bwd_mode(const void* q, const void* k, const void* v, co
         float* dq_acc = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + bwd_vec_bytes_padded(B, T, Hq));
         return launch_bwd_onepass(tq, tk, tv, tdo, p, dq_acc, st);
     }
-    return D == 64 ? launch_bwd<64>(tq, tk64, tv64, tk, tv, tdo, to, tdq, p, st)
-                   : launch_bwd<128>(tq, tk64, tv64, tk, tv, tdo, to, tdq, p, st);
+    return D == 64 ? launch_bwd<64>(tq, tk, tv, tdo, own, p, st) : launch_bwd<128>(tq, tk, tv, tdo, own, p, st);
 }
 
 // ---------------------------------------------------------------------------------------
