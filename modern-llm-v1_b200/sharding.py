@@ -53,3 +53,26 @@ def gather_units(local, n_units: int, rank: int, world: int):
     parts = [torch.empty_like(pad) for _ in range(world)]
     dist.all_gather(parts, pad.contiguous())
     return torch.cat([p[:n] for p, n in zip(parts, sizes)])
+
+
+# Two runs of the same units may add the same FP32 terms in another grouping (CTAs of a cluster share an item when a GPU has
+# few), which flips the BF16 rounding of some elements by one step: 4e-4 of a tile's norm measured (dK, dV of 1/4 and 1/8 of the
+# training configurations), up to 2.6e-3 where a forward rounds P against another reference.  A step in every element is at
+# least 2^-8.  One wrong row of 128 is 2^-4 and more.
+TILE_REL_L2 = 2.0 ** -8
+
+
+def worst_tile_rel_l2(got, want, rows: int = 128) -> float:
+    """The largest relative L2 difference over the tiles of `rows` tokens of every unit and head; got, want [units, heads, T, D].
+    NaN when either side has one."""
+    import torch
+
+    worst = 0.0
+    for g, w in zip(got.split(rows, dim=2), want.split(rows, dim=2)):
+        g, w = g.double(), w.double()
+        diff, norm = (g - w).flatten(2).norm(dim=2), w.flatten(2).norm(dim=2)
+        rel = torch.where(diff == 0, diff, diff / norm)  # (a tile of zeros: inf unless it is met)
+        worst = max(worst, float(rel.max())) if not torch.isnan(rel).any() else float("nan")
+        if worst != worst:
+            break
+    return worst
