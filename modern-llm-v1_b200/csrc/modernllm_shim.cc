@@ -3,10 +3,12 @@
 
 #include <cuda_runtime.h>
 
+#include <cstdint>
+#include <list>
+#include <memory>
 #include <mutex>
 #include <stdexcept>
 #include <string>
-#include <vector>
 
 #include "b200attn.h"
 
@@ -33,28 +35,43 @@ void raise(int status, const char* fn) {
 }
 
 // A private temporary that is kept between calls: one per (device, stream, operator), grown when a larger problem
-// comes and never shrunk.  Growing frees the old buffer, and cudaFree waits for the work that still reads it.
-enum WsKind { kWsBackward = 0, kWsDecode = 1, kWsRopeNorm = 2 };
+// comes and never shrunk.  Growing frees the old buffer, and cudaFree waits for the work that still reads it.  A call holds
+// it from sizing to its last launch: a backward is two launches with live data between them, and another host thread on the
+// stream may not put its own in between.
+enum WsKind { kWsBackward = 0, kWsDecode = 1, kWsRopeNorm = 2, kWsStatic = 3 /* the library's fixed scratch: the lock alone */ };
 struct WsEntry {
     int device;
     void* stream;
     int kind;
-    Tensor buf;
+    std::mutex lock;
+    std::unique_ptr<Tensor> buf;
+    WsEntry(int d, void* s, int k) : device(d), stream(s), kind(k) {}
 };
-void* cached_workspace(int kind, size_t bytes, void* stream) {
+struct Workspace {
+    std::unique_lock<std::mutex> held;
+    void* data;
+    size_t bytes;
+};
+Workspace hold_workspace(int kind, size_t bytes, void* stream) {
     static std::mutex mu;
-    static std::vector<WsEntry> cache;
+    static std::list<WsEntry> entries;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) throw std::runtime_error("cached_workspace: no current CUDA device");
-    std::lock_guard<std::mutex> lock(mu);
-    for (WsEntry& e : cache) {
-        if (e.device == dev && e.stream == stream && e.kind == kind) {
-            if (e.buf.bytes() < bytes) e.buf = Tensor({static_cast<std::int64_t>((bytes + 3) / 4)}, DType::FP32, Device::Cuda);
-            return e.buf.data();
-        }
+    if (cudaGetDevice(&dev) != cudaSuccess) throw std::runtime_error("hold_workspace: no current CUDA device");
+    WsEntry* e = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        for (WsEntry& x : entries)
+            if (x.device == dev && x.stream == stream && x.kind == kind) e = &x;
+        if (!e) e = &entries.emplace_back(dev, stream, kind);
     }
-    cache.push_back(WsEntry{dev, stream, kind, Tensor({static_cast<std::int64_t>((bytes + 1023) / 4)}, DType::FP32, Device::Cuda)});
-    return cache.back().buf.data();
+    Workspace w{std::unique_lock<std::mutex>(e->lock), nullptr, bytes};
+    if (bytes == 0) return w;
+    if (!e->buf || e->buf->bytes() < bytes) {
+        e->buf.reset();
+        e->buf = std::make_unique<Tensor>(Tensor({static_cast<std::int64_t>((bytes + 1023) / 4)}, DType::FP32, Device::Cuda));
+    }
+    w.data = e->buf->data();
+    return w;
 }
 
 }  // namespace
@@ -97,15 +114,16 @@ void flash_attn_backward_gqa(const Tensor& q, const Tensor& k, const Tensor& v, 
     // scratch serves every problem that fits it; otherwise a workspace kept for this (device, stream).
     const long long rows = 1LL * B * Hq * ((T + 127) / 128 * 128);
     if (stream == nullptr && rows <= B200ATTN_BWD_STATIC_MAX_ROWS) {
+        const Workspace ws = hold_workspace(kWsStatic, 0, stream);
         raise(b200attn_bwd_static(q.data(), k.data(), v.data(), ctx.data(), L.data_as<float>(), d_ctx.data(), d_q.data(),
                                   d_k.data(), d_v.data(), B, T, Hq, Hkv, D, static_cast<int>(layout), 0.f, stream),
               fn);
         return;
     }
-    const size_t ws_bytes = b200attn_bwd_workspace_bytes_mode(B, T, Hq, Hkv, D, B200ATTN_BWD_TWO_PASS);
+    const Workspace ws = hold_workspace(kWsBackward, b200attn_bwd_workspace_bytes_mode(B, T, Hq, Hkv, D, B200ATTN_BWD_TWO_PASS), stream);
     raise(b200attn_bwd_mode(q.data(), k.data(), v.data(), ctx.data(), L.data_as<float>(), d_ctx.data(), d_q.data(),
                             d_k.data(), d_v.data(), B, T, Hq, Hkv, D, static_cast<int>(layout), 0.f, B200ATTN_BWD_TWO_PASS,
-                            cached_workspace(kWsBackward, ws_bytes, stream), ws_bytes, stream),
+                            ws.data, ws.bytes, stream),
           fn);
 }
 
@@ -131,9 +149,9 @@ void flash_attn_decode(const Tensor& q, const Tensor& kcache, const Tensor& vcac
     if (q.numel() != 1LL * B * Hq * D || o.numel() != q.numel() || kcache.numel() != 1LL * B * Hkv * Lcache * D ||
         vcache.numel() != kcache.numel())
         throw std::invalid_argument("flash_attn_decode: shape mismatch");
-    const size_t ws_bytes = b200attn_decode_workspace_bytes(B, Lcache, Hq, Hkv, D, 0);
+    const Workspace ws = hold_workspace(kWsDecode, b200attn_decode_workspace_bytes(B, Lcache, Hq, Hkv, D, 0), stream);
     raise(b200attn_decode(q.data(), kcache.data(), vcache.data(), o.data(), nullptr, B, Lcache, Hq, Hkv, D, 0.f, 0,
-                          cached_workspace(kWsDecode, ws_bytes, stream), ws_bytes, stream),
+                          ws.data, ws.bytes, stream),
           fn);
 }
 
@@ -180,12 +198,12 @@ void rope_qknorm_backward(const Tensor& d_y, const Tensor& x, const Tensor& cos,
         throw std::invalid_argument("rope: x numel mismatch");
     if (gamma.numel() != d_h || d_gamma.numel() != d_h || rstd.numel() != 1LL * B * H * T)
         throw std::invalid_argument("rope_qknorm_backward: shape mismatch (gamma/d_gamma/rstd)");
-    const size_t ws_bytes = b200attn_rope_norm_bwd_workspace_bytes(d_h);
+    const Workspace ws = hold_workspace(kWsRopeNorm, b200attn_rope_norm_bwd_workspace_bytes(d_h), stream);
     raise(b200attn_rope_norm_bwd(d_y.data(), static_cast<int>(y_layout), x.data(), xd, static_cast<int>(x_layout),
                                  static_cast<const float*>(rstd.data()), static_cast<const float*>(gamma.data()),
                                  static_cast<const float*>(cos.data()), static_cast<const float*>(sin.data()), d_x.data(),
                                  static_cast<float*>(d_gamma.data()), B, T, H, d_h,
-                                 cached_workspace(kWsRopeNorm, ws_bytes, stream), ws_bytes, stream),
+                                 ws.data, ws.bytes, stream),
           fn);
 }
 
@@ -225,9 +243,9 @@ void flash_attn_decode_cached(const Tensor& q, const Tensor& kcache, const Tenso
     if (q.numel() != 1LL * B * Hq * D || o.numel() != q.numel() || kcache.numel() != 1LL * B * Hkv * L_cap * D ||
         vcache.numel() != kcache.numel())
         throw std::invalid_argument("flash_attn_decode_cached: shape mismatch");
-    const size_t ws_bytes = b200attn_decode_workspace_bytes(B, L, Hq, Hkv, D, 0);
+    const Workspace ws = hold_workspace(kWsDecode, b200attn_decode_workspace_bytes(B, L, Hq, Hkv, D, 0), stream);
     raise(b200attn_decode_cached(q.data(), kcache.data(), vcache.data(), o.data(), nullptr, B, L, L_cap, Hq, Hkv, D, 0.f, 0,
-                                 cached_workspace(kWsDecode, ws_bytes, stream), ws_bytes, stream),
+                                 ws.data, ws.bytes, stream),
           fn);
 }
 

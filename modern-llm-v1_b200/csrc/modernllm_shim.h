@@ -17,7 +17,9 @@
 // Private temporaries: where the reference allocates per call (llm/src/model/flash_attn.cu:463,
 // llm/src/model/attention.cu:197,225), the backward here uses the library's fixed scratch (b200attn_bwd_static)
 // when the problem fits it, and otherwise - like decode and the RoPE/QK-Norm backward - a workspace kept per
-// (device, stream, operator) that only ever grows: in steady state no call allocates, frees or synchronises.
+// (device, stream, operator) that only ever grows: in steady state no call allocates, frees or synchronises.  A call
+// holds its workspace (or the fixed scratch) until its last launch, so several host threads may use one stream.
+// (A captured launch keeps its workspace's address: capture after the largest problem of the stream has run.)
 #pragma once
 
 #include "core/tensor.h"
