@@ -34,18 +34,17 @@ if ROOT not in sys.path:
 
 FALLBACK_PEAKS = {"bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0, "hbm_gbs": 6650.0}
 
-# DRAM traffic of the dominant kernel per launch at the default workload, from the committed ncu
-# summary (profiles/); None until a capture exists for the current kernel.
-# (dram read + write per launch of each kernel, profiles/attn_fwd_bwd_c2_50m_train.md)
-NCU_TRAFFIC_BYTES = {"c2_50m_train": {"attn_fwd_kernel": 21033728, "attn_bwd_dq_kernel": 46777088,
-                                      "attn_bwd_dkdv_kernel": 34416896},
-                     # profiles/attn_fwd_bwd_c3_300m_class.md
-                     "c3_300m_class": {"attn_fwd_kernel": 53215488, "attn_bwd_dq_kernel": 132836864,
-                                       "attn_bwd_dkdv_kernel": 96702208},
-                     # profiles/attn_fwd_bwd_c4_long_context.md (the dK/dV pass streams Q and dO once per key tile: the
-                     # re-reads hit L2 at 78 %, the rest comes from DRAM again)
-                     "c4_long_context": {"attn_fwd_kernel": 473484288, "attn_bwd_dq_kernel": 1000673280,
-                                         "attn_bwd_dkdv_kernel": 1197408512}}
+# DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum, one launch of each kernel of this library as it is now,
+# counted with `ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k regex:attn_ -s 9 -c 3 python
+# bench.py --config NAME --steps 3 --warmup 3 --no-cpu-baseline --no-graph`); to be counted again when a kernel changes what it
+# reads.  Writes still in L2 at a kernel's end are not among them.  In the long-context configuration the dQ and dK/dV passes
+# read K, V or Q, dO several times, mostly from L2.
+NCU_TRAFFIC_BYTES = {"c2_50m_train": {"attn_fwd_kernel": 21190912, "attn_bwd_dq_kernel": 46794240,
+                                      "attn_bwd_dkdv_kernel": 34414080},
+                     "c3_300m_class": {"attn_fwd_kernel": 52976384, "attn_bwd_dq_kernel": 134066944,
+                                       "attn_bwd_dkdv_kernel": 95216128},
+                     "c4_long_context": {"attn_fwd_kernel": 486543616, "attn_bwd_dq_kernel": 1004139776,
+                                         "attn_bwd_dkdv_kernel": 1173410560}}
 
 
 def load_peaks():
@@ -140,8 +139,8 @@ class ClockSampler:
 # CPU side: the oracle port timed on the host cores (cpu_baseline leg and --impl reference)
 # ------------------------------------------------------------------------------------------
 class StepGraphs:
-    """Runs exactly K steps from CUDA graphs.  A step is a few short launches (2-3 kernels of 25-45 us); issued one
-    by one from Python the host can set the pace (15-25 us per call on a slow host), so one round over the buffer
+    """Runs exactly K steps from CUDA graphs.  A step is a few short launches (three kernels of 20-30 us); issued one by
+    one a slow host can set the pace, so one round over the buffer
     sets is captured in a graph and replayed; a remainder of K % round steps comes from single-step graphs.  The
     launches inside a graph keep their programmatic-dependent-launch edges."""
 
@@ -332,7 +331,8 @@ def workload_config(cfg_full, world, scaling):
 
 
 def kernel_breakdown(m, cfg, sets, steps):
-    """Average device time of each kernel of a step, CUDA events on the launching stream."""
+    """Average device time of each kernel of a step, CUDA events on the launching stream.  An event between two kernels
+    keeps the second from setting itself up under the first, so these times add up to more than a step."""
     import torch
 
     lib = m._lib.load()
@@ -540,7 +540,7 @@ def run_decode(m, cfg, args, rank, world, device, peaks, warmup, steps, barrier)
                             "on the device, as it does between the tokens of a sampling loop"},
             "roofline": {"bound": "hbm", "kernel": "attn_decode_kernel", "achieved": gbs / world, "peak": peak,
                          "unit": "GB/s", "frac": gbs / world / peak,
-                         "traffic": 273341184 if cfg.name == "c5_decode" else None,  # profiles/attn_decode_c5_decode.md
+                         "traffic": 272321792 if cfg.name == "c5_decode" else None,  # as NCU_TRAFFIC_BYTES
                          "peak_source": f"hbm_gbs of {peaks['_source']}", "bytes_per_launch": nbytes,
                          "note": "1 launch per step"},
         }), flush=True)
@@ -582,8 +582,8 @@ def run_qkprep(m, cfg, args, rank, world, device, peaks, warmup, steps, barrier)
     for i in range(warmup):
         step(i)
     m.device_status()
-    # Three short launches per step: issued one by one from Python the host, not the GPU, sets the pace
-    # (about 20 us per call), so one round over the buffer sets is captured in a CUDA graph and replayed.
+    # Three short launches per step: issued one by one a slow host, not the GPU, could set the pace, so one round over the
+    # buffer sets is captured in a CUDA graph and replayed.
     side = torch.cuda.Stream()
     side.wait_stream(torch.cuda.current_stream())
     graph = torch.cuda.CUDAGraph()
@@ -652,7 +652,7 @@ def run_qkprep(m, cfg, args, rank, world, device, peaks, warmup, steps, barrier)
                 "note": "bound by the host link: every tensor crosses it once per step"},
         "roofline": {"bound": "hbm", "kernel": "rope_norm_fwd_kernel + rope_norm_bwd_kernel", "achieved": gbs / world,
                      "peak": peak, "unit": "GB/s", "frac": gbs / world / peak,
-                     "traffic": 794041344 if cfg.name == "c4_long_context" else None,  # profiles/rope_norm_c4_long_context.md
+                     "traffic": 740370944 if cfg.name == "c4_long_context" else None,  # as NCU_TRAFFIC_BYTES, the three launches
                      "peak_source": f"hbm_gbs of {peaks['_source']}", "bytes_per_step": nbytes,
                      "note": "3 launches per step: q and k together, forward, backward, d_gamma sums"},
     }
@@ -761,8 +761,7 @@ def run_decode_step(m, cfg, args, rank, world, device, peaks, warmup, steps, bar
                 "note": "the new token's rows from pinned host memory, o read back, a stream synchronise per step"},
         "roofline": {"bound": "hbm", "kernel": "attn_decode_kernel", "achieved": gbs / world, "peak": peak,
                      "unit": "GB/s", "frac": gbs / world / peak,
-                     # the kernels of a step, profiles/kv_append_decode_step_c5_decode.md
-                     "traffic": 272819456 if cfg.name == "c5_decode" else None,
+                     "traffic": 272920064 if cfg.name == "c5_decode" else None,  # as NCU_TRAFFIC_BYTES, both kernels
                      "peak_source": f"hbm_gbs of {peaks['_source']}", "bytes_per_step": nbytes,
                      "note": "2 launches per step: kv_append_kernel, attn_decode_kernel"},
     }
@@ -866,7 +865,7 @@ def main():
     barrier()
 
     # ONE launch protocol gives `value`: a round over the buffer sets captured in a CUDA graph and replayed (it does
-    # not depend on how fast the host's Python issues three 25-30 us launches); --no-graph makes it direct calls.
+    # not depend on how fast the host issues three launches of 20-30 us); --no-graph makes it direct calls.
     # The other way is timed too, over the same K steps, and only reported in config.ms_per_step_by_launch.
     graphs = None
     if not args.no_graph:
@@ -920,8 +919,10 @@ def main():
         dist.all_gather(parts, t)
         checksum = [float(p.item()) for p in parts]
 
-    # per-kernel device times (same loop, events between the kernels)
-    kt = kernel_breakdown(m, cfg, sets, steps)
+    # per-kernel device times (same loop, events between the kernels), and what of the measured step falls to each
+    kt_events = kernel_breakdown(m, cfg, sets, steps)
+    in_step = min(1.0, ms_step / sum(kt_events.values()))
+    kt = {k: v * in_step for k, v in kt_events.items()}
     # FLOPs per launch.  Credited (the metric's convention: forward 2 products over the causal half, backward 5):
     # the backward's 5 are split over its two kernels in the ratio of what they execute (dQ pass 3 products,
     # dK/dV pass 4: both recompute the scores), so the credited shares add up to the metric's FLOPs.
@@ -945,12 +946,13 @@ def main():
         "executed": {"flops_per_launch": executed[dom], "achieved": executed[dom] / (kt[dom] * 1e-3) / 1e12,
                      "frac_of_burst": executed[dom] / (kt[dom] * 1e-3) / 1e12 / burst,
                      "frac_of_sustained": executed[dom] / (kt[dom] * 1e-3) / 1e12 / sustained},
-        "kernels_ms": kt,
+        "kernels_ms": kt, "kernels_ms_with_events_between": kt_events,
+        "kernels_ms_what": "the measured step, divided in the ratio of the times with events between the kernels (which "
+                           "switch the overlap of consecutive kernels off and so add up to more than the step)",
         "fwd": {"ms": kt["attn_fwd_kernel"], "tflops": cfg.fwd_flops() / (kt["attn_fwd_kernel"] * 1e-3) / 1e12,
                 "frac_of_burst": cfg.fwd_flops() / (kt["attn_fwd_kernel"] * 1e-3) / 1e12 / burst},
         "bwd": {"ms": bwd_ms, "tflops": 2.5 * cfg.fwd_flops() / (bwd_ms * 1e-3) / 1e12,
-                "frac_of_burst": 2.5 * cfg.fwd_flops() / (bwd_ms * 1e-3) / 1e12 / burst,
-                "note": "kernels timed one by one with events between them; back to back they overlap a little"},
+                "frac_of_burst": 2.5 * cfg.fwd_flops() / (bwd_ms * 1e-3) / 1e12 / burst},
         "whole_step": {"achieved": value / world, "frac": value / world / burst, "frac_of_sustained": value / world / sustained,
                        "l2_warm_ms_per_step": ms_warm,
                        "l2_warm_tflops": flops_step / (ms_warm * 1e-3) / 1e12},

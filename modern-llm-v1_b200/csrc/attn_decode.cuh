@@ -394,8 +394,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = p.G;
 
-    // All CTAs of a launch are resident at once, so the next kernel of the stream may be brought in at once too: its
-    // set-up then runs under this kernel, and it waits for this kernel's end before it touches global memory.
+    // The next kernel of the stream may be brought in as soon as every CTA of this one has started (all at once where they fit
+    // the device, else with the last round): its set-up then runs under this kernel, and it waits for this kernel's end before
+    // it touches global memory.
     grid_dep_launch();
     if (p.cluster > 1) cluster_arrive();  // waited for in front of the first access to another CTA's shared memory
     if (warp == 4) {

@@ -255,8 +255,14 @@ int set_smem_once(K kernel, int bytes, bool* done) {
 
 // How many CTAs of a cluster share an item (forward: its key tiles, dK/dV pass: its units): the number with the smallest
 // estimate of the kernel's time, 1 unless another one is at least 5 % better.  Not only few items are split: 126 items of
-// 126 to 2 units on 148 SMs are bound by the longest one (dK/dV at B=1 T=8000 4/2 D=128: 229 -> 134 us).  The estimates were
-// held against measurements of some thirty shapes, most of which they meet within 15 %.
+// 126 to 2 units on 148 SMs are bound by the longest one (dK/dV at B=1 T=8000 4/2 D=128: 229 -> 134 us).  Held against every
+// number of shares at forty shapes from 2 to 2048 items, 15 to 8000 tokens, the pick was the fastest at each; some of them, us
+// for 1 / 2 / 4 / 8 shares: forward B=2 T=128 6/2 D=64 5.4 / 8.2 / 8.2 / 8.7, B=1 T=2000 6/2 D=64 22.5 / 18.2 / 23.9 / 36.6, 15 tokens
+// behind 6000 6/2 D=64 57.4 / 35.1 / 21.3 / 14.7, 500 behind 3000 B=2 16/4 D=128 43.6 / 36.2 / 50.6 / 86.5; dQ pass and dK/dV pass
+// B=1 T=2000 6/2 D=64 78.0 / 56.3 / 43.8 / 58.3, B=8 T=512 6/2 D=64 26.8 / 23.7 / 32.7 / 62.9, B=1 T=4096 8/2 D=128 264 / 162 / 121 /
+// 167, B=32 T=1001 1/1 D=128 44.2 / 77.9 / 136 / 262.  The order of the estimates is what counts: they are within some 12 % of the
+// time in one round of items, and up to half too low where shared items run in many rounds.  They do not see how items of
+// different lengths pack.
 struct SplitCosts {
     int per_sm;                // CTAs of the kernel that fit an SM
     float tile_one, tile_all;  // us per tile in a CTA that has the SM to itself, and with a second CTA beside it
