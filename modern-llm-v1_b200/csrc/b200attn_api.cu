@@ -9,9 +9,6 @@
 #include <atomic>
 #include <chrono>
 #include <functional>
-#include <queue>
-#include <utility>
-#include <vector>
 #include <math.h>
 #include <stdint.h>
 #include <stdlib.h>
@@ -140,35 +137,36 @@ const ItemTable& item_table_for(long long n_items, unsigned n_ctas, int n_groups
             return e.tab.per_cta >= 0 ? e.tab : none;
     Entry& e = cache[next++ % 4];
     e.n_items = n_items, e.n_ctas = n_ctas, e.n_groups = n_groups, e.n_qtiles = n_qtiles, e.T = T, e.cost = item_cost;
-    // longest processing time first; work in half tiles: an item costs its tiles plus half a tile
-    std::vector<std::vector<unsigned short>> lists(n_ctas);
-    std::vector<long long> load(n_ctas, 0);
-    using Slot = std::pair<long long, unsigned>;  // (work, list), least work first, then lowest index
-    std::priority_queue<Slot, std::vector<Slot>, std::greater<Slot>> heap;
-    for (unsigned c = 0; c < n_ctas; ++c) heap.push({0, c});
-    size_t longest = 0;
+    // longest processing time first; work in half tiles: an item costs its tiles plus half a tile.  (Fixed arrays: this runs
+    // under C entry points, which never throw.)
+    struct List {  // on the heap: least work first, then lowest index
+        long long work;
+        unsigned index;
+        bool operator>(const List& o) const { return work != o.work ? work > o.work : index > o.index; }
+    };
+    List heap[kItemTableCtas];
+    unsigned short ids[kItemTableCtas][kItemTableMaxPerCta];
+    int count[kItemTableCtas] = {}, longest = 0;
+    for (unsigned c = 0; c < n_ctas; ++c) heap[c] = {0, c};
     for (long long id = 0; id < n_items; ++id) {
         const int qt = n_qtiles - 1 - (int)(id / n_groups);
         const int rows = std::min(T, qt * 128 + 128);
-        const long long work = 2 * ((rows + 63) / 64) + item_cost;
-        const Slot s = heap.top();
-        heap.pop();
-        lists[s.second].push_back((unsigned short)id);
-        load[s.second] = s.first + work;
-        heap.push({load[s.second], s.second});
-        longest = std::max(longest, lists[s.second].size());
+        std::pop_heap(heap, heap + n_ctas, std::greater<List>());
+        List& l = heap[n_ctas - 1];
+        if (count[l.index] == kItemTableMaxPerCta) {
+            e.tab.per_cta = -1;  // remembered as "no table"
+            return none;
+        }
+        ids[l.index][count[l.index]++] = (unsigned short)id;
+        longest = std::max(longest, count[l.index]);
+        l.work += 2 * ((rows + 63) / 64) + item_cost;
+        std::push_heap(heap, heap + n_ctas, std::greater<List>());
     }
-    if (longest > (size_t)kItemTableMaxPerCta) {
-        e.tab.per_cta = -1;  // remembered as "no table"
-        return none;
-    }
-    std::vector<unsigned> order(n_ctas);
-    for (unsigned c = 0; c < n_ctas; ++c) order[c] = c;
-    std::stable_sort(order.begin(), order.end(), [&](unsigned a, unsigned b) { return load[a] > load[b]; });
-    e.tab.per_cta = (int)longest;
+    std::sort(heap, heap + n_ctas, [](const List& a, const List& b) { return a.work != b.work ? a.work > b.work : a.index < b.index; });
+    e.tab.per_cta = longest;
     for (unsigned c = 0; c < n_ctas; ++c)
-        for (size_t n = 0; n < longest; ++n)
-            e.tab.ids[c * longest + n] = n < lists[order[c]].size() ? lists[order[c]][n] : kItemTableEnd;
+        for (int n = 0; n < longest; ++n)
+            e.tab.ids[c * longest + n] = n < count[heap[c].index] ? ids[heap[c].index][n] : kItemTableEnd;
     return e.tab;
 }
 
