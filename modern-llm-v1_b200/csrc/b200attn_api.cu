@@ -30,7 +30,7 @@ namespace {
 __device__ int g_status_word[2];
 
 constexpr int kMaxDevices = 64;
-int* g_status_ptr[kMaxDevices] = {nullptr};
+std::atomic<int*> g_status_ptr[kMaxDevices] = {};  // (the words are zero at load)
 
 // Item counters of the persistent kernels (two words per launch, see ptx.cuh), also in the device
 // image (zero at load).  A kernel leaves its two words zero again when it ends, so one pair would do
@@ -42,7 +42,7 @@ int* g_status_ptr[kMaxDevices] = {nullptr};
 // then every kernel exits at once because the status word is set.
 constexpr int kSchedSlots = 64;
 __device__ int g_sched_words[2 * kSchedSlots];
-int* g_sched_ptr[kMaxDevices] = {nullptr};
+std::atomic<int*> g_sched_ptr[kMaxDevices] = {};
 std::atomic<unsigned> g_sched_seq{0};
 
 // What tells a decode launch's counters from those of every other launch (see decode_count).  The sequence starts anywhere, so
@@ -66,28 +66,19 @@ int* status_ptr(int* err) {
         *err = B200ATTN_ERR_NO_DEVICE;
         return nullptr;
     }
-    if (!g_status_ptr[dev]) {
-        void* p = nullptr;
-        if (cudaGetSymbolAddress(&p, g_status_word) != cudaSuccess) {
+    int* status = g_status_ptr[dev].load(std::memory_order_acquire);
+    if (!status) {  // several threads may come here at once: all find the same addresses
+        void *p = nullptr, *sp = nullptr;
+        if (cudaGetSymbolAddress(&p, g_status_word) != cudaSuccess || cudaGetSymbolAddress(&sp, g_sched_words) != cudaSuccess) {
             cudaGetLastError();
             *err = B200ATTN_ERR_NO_DEVICE;
             return nullptr;
         }
-        if (cudaMemset(p, 0, sizeof(g_status_word)) != cudaSuccess) {
-            cudaGetLastError();
-            *err = B200ATTN_ERR_CUDA;
-            return nullptr;
-        }
-        void* sp = nullptr;
-        if (cudaGetSymbolAddress(&sp, g_sched_words) != cudaSuccess) {
-            cudaGetLastError();
-            *err = B200ATTN_ERR_NO_DEVICE;
-            return nullptr;
-        }
-        g_sched_ptr[dev] = static_cast<int*>(sp);
-        g_status_ptr[dev] = static_cast<int*>(p);
+        status = static_cast<int*>(p);
+        g_sched_ptr[dev].store(static_cast<int*>(sp), std::memory_order_relaxed);
+        g_status_ptr[dev].store(status, std::memory_order_release);
     }
-    return g_status_ptr[dev];
+    return status;
 }
 
 // The counter pair for the next launch of a persistent kernel on the current device (status_ptr()
@@ -103,7 +94,7 @@ int* next_sched_pair(long long n_items, unsigned n_ctas) {
     if (forced == 1 || (forced == 0 && n_items < 4LL * n_ctas)) return nullptr;
     int dev = 0;
     cudaGetDevice(&dev);
-    return g_sched_ptr[dev] + 2 * (g_sched_seq.fetch_add(1, std::memory_order_relaxed) % kSchedSlots);
+    return g_sched_ptr[dev].load(std::memory_order_relaxed) + 2 * (g_sched_seq.fetch_add(1, std::memory_order_relaxed) % kSchedSlots);
 }
 
 // The static deal of the forward and the dQ pass (two CTAs per SM) as a table: items (ids are heaviest first;
@@ -819,7 +810,7 @@ namespace {
 // In host code this name is only a handle for cudaGetSymbolAddress, never a device pointer.
 static __device__ __align__(256) float g_bwd_static_scratch[2 * B200ATTN_BWD_STATIC_MAX_ROWS];
 
-float* g_bwd_static_ptr[kMaxDevices] = {nullptr};
+std::atomic<float*> g_bwd_static_ptr[kMaxDevices] = {};
 
 // Device address of the array on the current device, resolved once per device.
 float* bwd_static_scratch(int* err) {
@@ -1159,7 +1150,7 @@ extern "C" int b200attn_last_device_status(void* stream) {
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceSynchronize();
-        cudaMemset(g_sched_ptr[dev], 0, sizeof(int) * 2 * kSchedSlots);
+        cudaMemset(g_sched_ptr[dev].load(), 0, sizeof(int) * 2 * kSchedSlots);
         const int next[2] = {0, (host[1] + 1) & ((1 << kDecodeEpochBits) - 1)};
         cudaMemcpy(status, next, sizeof(next), cudaMemcpyHostToDevice);
         return host[0];
