@@ -136,20 +136,27 @@ __device__ __forceinline__ void stage_row_chunk(uint8_t* tile, int row, int col,
 // dQ pass (D = 64): persistent CTAs, two per SM.  A CTA walks a list of work items (item = one 128-row query tile
 // of one (batch, query head); items are ordered heaviest first), and every pipeline keeps running across item
 // boundaries.  The O tile travels with Q and dO, so the preprocess D = rowsum(O * dO)
-// (flash_attn_compute_D_kernel, llm/src/model/flash_attn.cu:150-172) is shared-memory work at the head of each
-// item; D and L * log2(e) are also left in the workspace for the dK/dV pass, which therefore has to run after this
-// kernel.
+// (flash_attn_compute_D_kernel, llm/src/model/flash_attn.cu:150-172) is shared-memory work once per item; D and L * log2(e)
+// are also left in the workspace for the dK/dV pass, which therefore has to run after this kernel.
 //
 // Q and dO in tensor memory.  Every D = 64 kernel here is bound by the shared-memory data path (a product M128 N64
 // K16 with both operands in shared memory fetches 4 KB of A and 2 KB of B for 32 clocks of math), and Q and dO are
-// the A operands of every S = Q K^T and dP = dO V^T product of an item.  The compute warps therefore copy the two
-// tiles once per item from shared memory into tensor memory (the 128 bytes of row r are the 32 BF16-pair columns
+// the A operands of every S = Q K^T and dP = dO V^T product of an item.  The two tiles are therefore copied
+// once per item from shared memory into tensor memory (the 128 bytes of row r are the 32 BF16-pair columns
 // of lane r as they stand), all three products of a key tile take their A operand from tensor memory, and the
 // shared-memory tiles are free for the NEXT item's loads while this item is still being worked on.
 //
-// Roles (320 threads): warps 0-7 compute (thread owns query row (warp % 4) * 32 + lane == TMEM lane and the 32 key
-// columns of its part warp / 4), warp 8 TMA producer, warp 9 TMEM allocation + MMA issue (converged warps, one
-// elected lane issues).
+// Row warps.  What happens once per item - the preprocess, the copy into tensor memory, the dQ rows on their way out - has
+// four warps of its own, beside the compute warps that go from one item's last tile to the next item's first.  Done by the
+// compute warps it kept them from 3400 clocks of tiles per item (1250 a tile); what is left of that is 1200, from the last dP
+// product over the copy to the next item's first scores.  Measured on B200, us for both passes of the backward: B=32 T=512 6/2
+// 47.0 -> 45.5, B=16 T=1024 16/4 159.1 -> 155.3, B=8 T=2000 16/4 279 -> 272, B=2 T=128 6/2 12.15 -> 12.21 (one item per CTA: nothing
+// to overlap).  dS through shared memory instead of over the dP block, so that the next dP need not wait for dQ, was slower
+// (B=16 T=1024: 168 against 162): the tiles of two CTAs cover that wait already.
+//
+// Roles (512 threads): warps 0-7 compute (thread owns query row (warp % 4) * 32 + lane == TMEM lane and the 32 key
+// columns of its part warp / 4), warps 8-11 rows, warp 12 TMA producer, warp 13 TMEM allocation + MMA issue (converged
+// warps, one elected lane issues), warps 14-15 idle (they complete a warpgroup, the unit in which registers are dealt).
 // TMEM (256 columns): S [0,64), dP [64,128) (dS as BF16 over the first 16 columns of each part's range), dQ
 // accumulator [128,192), Q [192,224), dO [224,256).  There is one S buffer: the compute warps read a tile's scores
 // into registers in one go and hand the buffer back at once, so the next tile's Q K^T runs under this tile's
@@ -164,8 +171,9 @@ struct DqCfg {
     static constexpr int kKVTileBytes = kKeys * D * 2;
     static constexpr int kKVBoxBytes = kKeys * 64 * 2;
     static constexpr int kBoxes = D / 64;
-    static constexpr int kOutBytes = 8 * kRowStageBytes;  // per compute warp: its output rows on their way to global memory
-    static constexpr int kSmemBytes = 3 * kQTileBytes + 2 * kStages * kKVTileBytes + kOutBytes + 512;  // Q, dO, O + ring + barriers
+    static constexpr int kOutBytes = 4 * kRowStageBytes;  // per row warp: its output rows on their way to global memory
+    static constexpr int kVecBytes = 2 * 128 * 8;         // (L * log2(e), D) of the rows of two items
+    static constexpr int kSmemBytes = 3 * kQTileBytes + 2 * kStages * kKVTileBytes + kOutBytes + kVecBytes + 512;  // Q, dO, O + ring + barriers
     static_assert(2 * (kSmemBytes + 1024) <= 228 * 1024, "two CTAs per SM");
     static constexpr int kTmemCols = 256;
     static constexpr int kCtasPerSm = 2;
@@ -173,8 +181,11 @@ struct DqCfg {
     static constexpr int kParts = 2;
     static constexpr int kPartCols = kKeys / kParts;  // 32
     static constexpr int kComputeThreads = 128 * kParts;
-    static constexpr int kThreads = kComputeThreads + 64;
-    static constexpr int kProducerWarp = 4 * kParts, kMmaWarp = 4 * kParts + 1;
+    static constexpr int kThreads = kComputeThreads + 256;
+    static constexpr int kRowWarp = 4 * kParts, kProducerWarp = kRowWarp + 4, kMmaWarp = kProducerWarp + 1;
+    // registers per thread of the compute warps, the row warps and the others: together the launch's kThreads x 64
+    static constexpr int kRegsCompute = 80, kRegsRow = 56, kRegsOther = 40;
+    static_assert(kRegsCompute * kComputeThreads + (kRegsRow + kRegsOther) * 128 <= 64 * kThreads, "more registers than the launch has");
 };
 
 template <int D>
@@ -191,11 +202,14 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     uint8_t* sO = sdO + Cfg::kQTileBytes;
     uint8_t* sK = sO + Cfg::kQTileBytes;         // [NST]
     uint8_t* sV = sK + NST * Cfg::kKVTileBytes;  // [NST]
-    uint8_t* sOut = sV + NST * Cfg::kKVTileBytes;  // [8 warps]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + Cfg::kOutBytes);
+    uint8_t* sOut = sV + NST * Cfg::kKVTileBytes;  // [4 row warps]
+    float2* sVec = reinterpret_cast<float2*>(sOut + Cfg::kOutBytes);  // [2][128], by item parity
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + Cfg::kOutBytes + Cfg::kVecBytes);
     uint64_t* bar_q = bars + 0;         // Q, dO, O of an item have landed in shared memory      (phase: item)
-    uint64_t* bar_qs_free = bars + 1;   // the compute warps have read those three tiles          (phase: item)
+    uint64_t* bar_qs_free = bars + 1;   // the row warps have read those three tiles              (phase: item)
     uint64_t* bar_qt_full = bars + 2;   // Q and dO of an item are in tensor memory               (phase: item)
+    uint64_t* bar_qt_free = bars + 7;   // every S and dP product of an item has run              (phase: item)
+    uint64_t* bar_vec = bars + 10;      // the item's row vectors are in sVec                     (phase: item)
     uint64_t* bar_s_full = bars + 3;    //                                                         (phase: tile)
     uint64_t* bar_s_loaded = bars + 4;  // S is in registers: the buffer may be overwritten       (phase: tile)
     uint64_t* bar_dp_full = bars + 5;   //                                                         (phase: tile)
@@ -228,14 +242,16 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tma_prefetch_desc(&tmdO);
         tma_prefetch_desc(&tmO);
         mbar_init(bar_q, 1);
-        mbar_init(bar_qs_free, Cfg::kComputeThreads);
-        mbar_init(bar_qt_full, Cfg::kComputeThreads);
+        mbar_init(bar_qs_free, 128);
+        mbar_init(bar_qt_full, 128);
+        mbar_init(bar_qt_free, 1);
+        mbar_init(bar_vec, 128);
         mbar_init(bar_s_full, 1);
         mbar_init(bar_s_loaded, Cfg::kComputeThreads);
         mbar_init(bar_dp_full, 1);
         mbar_init(bar_ds_full, Cfg::kComputeThreads);
         mbar_init(bar_acc, 1);
-        mbar_init(bar_acc_free, Cfg::kComputeThreads);
+        mbar_init(bar_acc_free, 128);
         for (int s = 0; s < NST; ++s) {
             mbar_init(&bar_kv_full[s], 1);
             mbar_init(&bar_kv_free[s], 1);
@@ -258,8 +274,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
     if (*abort_flag != 0) {
         // an earlier CTA already failed: fall through to the teardown
+    } else if (warp > Cfg::kMmaWarp) {
+        reg_dealloc<Cfg::kRegsOther>();  // idle warps
     } else if (warp == Cfg::kProducerWarp) {
         // ------------------------------------------------------------------ producer
+        reg_dealloc<Cfg::kRegsOther>();
         int g = 0;  // tiles issued so far by this CTA (ring position)
         bool ok = true;
         int id = sched_first(tab, p.sched, int(blockIdx.x));  // the first item needs no fetch
@@ -310,6 +329,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (ok && lane == 0) sched_finish(p.sched, int(gridDim.x));
     } else if (warp == Cfg::kMmaWarp) {
         // ------------------------------------------------------------------ MMA issuer
+        reg_dealloc<Cfg::kRegsOther>();
         constexpr uint32_t idesc_s = make_idesc_bf16(128, Cfg::kKeys, 0, 0);  // A in TMEM, B (K or V tile) K-major
         constexpr uint32_t idesc_acc = make_idesc_bf16(128, D, 0, 1);         // A in TMEM, B (K tile) MN-major
         // g numbers this CTA's key tiles across all its items: ring stage g % NST
@@ -331,7 +351,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         };
         // dP(g) = dO V^T; tile g's loads have landed (S(g) was issued), and the product that read dS(g - 1) out of
         // this block was issued before (the products execute in order)
-        auto issue_dp = [&](int g) {
+        auto issue_dp = [&](int g, bool last) {
             const int s = g % NST;
             const uint64_t v_desc = make_sdesc_sw128(smem_u32(sV + s * Cfg::kKVTileBytes), 16, 1024);
             if (elect_one()) {
@@ -339,32 +359,41 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 for (int ks = 0; ks < D / 16; ++ks)
                     umma_ts(tmem + Cfg::kColDP, tmem + Cfg::kColDO + ks * 8, v_desc + kmajor_step(ks, Cfg::kKVBoxBytes), idesc_s, ks > 0);
                 umma_commit(bar_dp_full);
+                if (last) umma_commit(bar_qt_free);  // no later product reads this item's Q and dO
             }
             __syncwarp();
         };
-        int g0 = 0, n = 0;
+        int g = 0, n = 0;
         bool ok = true;
-        for (int id; ok && (id = get_item(n)) >= 0; ++n) {
-            const int n_kv = item_nkv(id);
+        int id = get_item(0);
+        // S of the first tile of this CTA's n-th item
+        auto start_item = [&]() {
             B200ATTN_STAMP(lane == 0, 440 + 2 * n);
-            ok = mbar_wait_warp(bar_qt_full, n & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+            ok = mbar_wait_warp(bar_qt_full, uint32_t(n) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
             B200ATTN_STAMP(lane == 0, 441 + 2 * n);
-            if (ok) ok = issue_s(g0);
-            if (!ok) break;
-            issue_dp(g0);
-            for (int j = 0; j < n_kv && ok; ++j) {
-                const int g = g0 + j;
+            if (ok) ok = issue_s(g);
+        };
+        if (id >= 0) start_item();
+        while (ok && id >= 0) {
+            const int n_kv = item_nkv(id);
+            issue_dp(g, n_kv == 1);
+            int id_next = -1;
+            for (int j = 0; j < n_kv; ++j) {
                 const int s = g % NST;
+                ++g;
                 if (j + 1 < n_kv) {
-                    ok = issue_s(g + 1);  // as soon as S(g) is in registers
-                    if (!ok) break;
+                    ok = issue_s(g);  // as soon as the tile's scores are in registers
+                } else {
+                    id_next = get_item(n + 1);
+                    ++n;
+                    if (id_next >= 0) start_item();
                 }
-                ok = mbar_wait_warp(bar_ds_full, uint32_t(g) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
+                if (ok) ok = mbar_wait_warp(bar_ds_full, uint32_t(g - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
                 if (!ok) break;
-                B200ATTN_STAMP(lane == 0, 240 + 8 * g + 5);
+                B200ATTN_STAMP(lane == 0, 240 + 8 * (g - 1) + 5);
                 // the accumulator still belongs to the previous item's epilogue until it has been read
-                if (j == 0 && n > 0) {
-                    ok = mbar_wait_warp(bar_acc_free, (n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
+                if (j == 0 && n - (n_kv == 1) > 0) {
+                    ok = mbar_wait_warp(bar_acc_free, uint32_t(n - (n_kv == 1) - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
                     if (!ok) break;
                 }
                 tc_fence_after_sync();
@@ -381,83 +410,133 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                     if (j + 1 == n_kv) umma_commit(bar_acc);
                 }
                 __syncwarp();
-                B200ATTN_STAMP(lane == 0, 240 + 8 * g + 6);
-                if (j + 1 < n_kv) issue_dp(g + 1);
+                B200ATTN_STAMP(lane == 0, 240 + 8 * (g - 1) + 6);
+                if (j + 1 < n_kv) issue_dp(g, j + 2 == n_kv);
             }
-            g0 += n_kv;
+            id = id_next;
         }
         // drain: nothing may be in flight when TMEM is freed
         if (ok && n > 0) mbar_wait_warp(bar_acc, (n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
-    } else {
-        // ------------------------------------------------------------------ compute
-        const int w4 = warp & 3, part = warp >> 2;
+    } else if (warp >= Cfg::kRowWarp) {
+        // ------------------------------------------------------------------ rows: what happens once per item
+        reg_dealloc<Cfg::kRegsRow>();
+        const int w4 = warp & 3;
         const int row = w4 * 32 + lane;  // query row in the tile == TMEM lane
         const uint32_t lane_base = uint32_t(w4 * 32) << 16;
-        const int c0 = part * Cfg::kPartCols;  // first key column of this thread's part
+        const uint32_t sw = uint32_t(row & 7) << 4;  // the tiles' swizzle
         bool ok = true;
-        float dv = 0.f, lse2 = INFINITY;  // of the item whose Q and dO are in tensor memory
-        // Head of this CTA's n-th item: the preprocess of this row from the tiles in shared memory
-        // (D = rowsum(O * dO); L * log2(e)), and Q (part 0) / dO (part 1) into tensor memory.  All S and dP products
-        // of the previous item have completed when this runs (their results were waited for).
-        auto item_head = [&](int n_item, int id) -> bool {
-            const int q0 = item_qt(id) * 128, h = item_h(id), b = item_b(id);
+        // dQ rows of the CTA's n_item-th item (times scale) -> BF16 -> global memory
+        auto epilogue = [&](int n_item, int id) {
+            ok = mbar_wait_warp(bar_acc, uint32_t(n_item) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+            if (!ok) return;
+            B200ATTN_STAMP(tid == Cfg::kRowWarp * 32, 400 + 4 * n_item + 2);
+            tc_fence_after_sync();
+            const int q0 = item_qt(id) * 128;
+            uint16_t* out = p.dq + size_t(item_b(id)) * p.q_sb + size_t(item_h(id)) * p.q_sh + size_t(q0 + w4 * 32) * p.q_st;
+#pragma unroll
+            for (int c = 0; c < D / 32; ++c) {
+                uint32_t v[32], w[16];
+                tmem_ld_x32(tmem + lane_base + Cfg::kColAcc + c * 32, v);
+                tmem_wait_ld();
+                if (c + 1 == D / 32) {
+                    tc_fence_before_sync();
+                    mbar_arrive(bar_acc_free);  // the MMA warp may start the next item's accumulation
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(__uint_as_float(v[2 * i]) * p.scale, __uint_as_float(v[2 * i + 1]) * p.scale);
+                store_rows_64b(sOut + w4 * kRowStageBytes, w, lane, out + c * 32, p.q_st, p.T - (q0 + w4 * 32));
+            }
+            B200ATTN_STAMP(tid == Cfg::kRowWarp * 32, 400 + 4 * n_item + 3);
+        };
+        // 64 BF16 of this row: its 128 bytes are 32 BF16-pair columns of lane `row` as they stand
+        auto copy_row = [&](const uint8_t* tile, uint32_t col) {
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t tw[16];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const uint4 w = *reinterpret_cast<const uint4*>(tile + row * 128 + (((half * 4 + c) << 4) ^ sw));
+                    tw[4 * c] = w.x, tw[4 * c + 1] = w.y, tw[4 * c + 2] = w.z, tw[4 * c + 3] = w.w;
+                }
+                tmem_st_x16(tmem + lane_base + col + half * 16, tw);
+            }
+        };
+        int n = 0, id_prev = -1;
+        for (int id; ok && (id = get_item(n)) >= 0; ++n) {
+            const int q0 = item_qt(id) * 128;
+            const size_t bh = size_t(item_b(id)) * p.Hq + item_h(id);
             const bool in_range = q0 + row < p.T;
             // (issued here and first used after the wait below, so that its latency overlaps the wait)
-            const float lse_raw = in_range ? p.lse[(size_t(b) * p.Hq + h) * p.T + q0 + row] : 0.f;
-            B200ATTN_STAMP(tid == 0, 400 + 4 * n_item + 0);
-            if (!mbar_wait_warp(bar_q, n_item & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD)) return false;
-            B200ATTN_STAMP(tid == 0, 400 + 4 * n_item + 1);
-            tc_fence_after_sync();
-            float acc = 0.f;
-            uint32_t tw[32];  // this row of Q (part 0) or dO (part 1) as it goes into tensor memory
+            const float lse_raw = in_range ? p.lse[bh * p.T + q0 + row] : 0.f;
+            B200ATTN_STAMP(tid == Cfg::kRowWarp * 32, 400 + 4 * n + 0);
+            ok = mbar_wait_warp(bar_q, uint32_t(n) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+            if (!ok) break;
+            B200ATTN_STAMP(tid == Cfg::kRowWarp * 32, 400 + 4 * n + 1);
+            // The preprocess of this row, D = rowsum(O * dO) and L * log2(e), in front of the wait for the item before; of the CTA's
+            // first item behind the copy, which its first products wait for.
+            auto row_vectors = [&]() {
+                float acc = 0.f;
 #pragma unroll
-            for (int c = 0; c < D / 8; ++c) {
-                const uint32_t off = row * 128 + ((c ^ (row & 7)) << 4);
-                const uint4 a = *reinterpret_cast<const uint4*>(sO + off);
-                const uint4 gq = *reinterpret_cast<const uint4*>(sdO + off);
-                const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
-                const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w};
+                for (int c = 0; c < D / 8; ++c) {
+                    const uint32_t off = row * 128 + ((uint32_t(c) << 4) ^ sw);
+                    const uint4 a = *reinterpret_cast<const uint4*>(sO + off);
+                    const uint4 gq = *reinterpret_cast<const uint4*>(sdO + off);
+                    const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
+                    const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w};
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    acc = fmaf(__uint_as_float(aw[e] << 16), __uint_as_float(gw[e] << 16), acc);
-                    acc = fmaf(__uint_as_float(aw[e] & 0xffff0000u), __uint_as_float(gw[e] & 0xffff0000u), acc);
+                    for (int e = 0; e < 4; ++e) {
+                        acc = fmaf(__uint_as_float(aw[e] << 16), __uint_as_float(gw[e] << 16), acc);
+                        acc = fmaf(__uint_as_float(aw[e] & 0xffff0000u), __uint_as_float(gw[e] & 0xffff0000u), acc);
+                    }
                 }
-                if (part == 0) {
-                    const uint4 qv = *reinterpret_cast<const uint4*>(sQ + off);
-                    tw[4 * c] = qv.x, tw[4 * c + 1] = qv.y, tw[4 * c + 2] = qv.z, tw[4 * c + 3] = qv.w;
-                } else {
-                    tw[4 * c] = gq.x, tw[4 * c + 1] = gq.y, tw[4 * c + 2] = gq.z, tw[4 * c + 3] = gq.w;
-                }
+                // exp2(x - inf) = 0: padding query rows contribute nothing
+                const float2 vec = make_float2(in_range ? lse_raw * 1.4426950408889634f : INFINITY, in_range ? acc : 0.f);
+                // (the compute warps have read what the buffer held by the end of that item's epilogue below)
+                sVec[(n & 1) * 128 + row] = vec;
+                mbar_arrive(bar_vec);
+                const size_t vrow = bh * p.Tpad + q0 + row;
+                p.lse2_w[vrow] = vec.x;
+                p.dvec_w[vrow] = vec.y;
+            };
+            if (n > 0) {
+                row_vectors();
+                ok = mbar_wait_warp(bar_qt_free, uint32_t(n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+                if (!ok) break;
+                tc_fence_after_sync();
             }
+            copy_row(sQ, Cfg::kColQ);
+            copy_row(sdO, Cfg::kColDO);
+            tmem_wait_st();
+            tc_fence_before_sync();
+            mbar_arrive(bar_qt_full);
+            if (n == 0) row_vectors();
             // The tiles were read with ordinary loads and will be overwritten by TMA, which works through the async
             // proxy: without this fence the producer's next load, issued the moment the last thread has arrived, may
             // overtake reads that are still in flight (the producer is parked at the barrier whenever the item before
             // was short; dQ rows of whole warps, sometimes of single lanes, then came out wrong once in a few launches).
             fence_proxy_async_smem();
             mbar_arrive(bar_qs_free);  // the three tiles may be overwritten by the next item's loads
-            tmem_st_x32(tmem + lane_base + (part == 0 ? Cfg::kColQ : Cfg::kColDO), tw);
-            // exp2(x - inf) = 0: padding query rows contribute nothing
-            lse2 = in_range ? lse_raw * 1.4426950408889634f : INFINITY;
-            dv = in_range ? acc : 0.f;
-            if (part == 0) {
-                const size_t vrow = (size_t(b) * p.Hq + h) * p.Tpad + q0 + row;
-                p.lse2_w[vrow] = lse2;
-                p.dvec_w[vrow] = dv;
-            }
-            tmem_wait_st();
-            tc_fence_before_sync();
-            mbar_arrive(bar_qt_full);
-            return true;
-        };
+            if (n > 0) epilogue(n - 1, id_prev);
+            id_prev = id;
+        }
+        if (ok && n > 0) epilogue(n - 1, id_prev);
+    } else {
+        // ------------------------------------------------------------------ compute
+        reg_alloc<Cfg::kRegsCompute>();
+        const int w4 = warp & 3, part = warp >> 2;
+        const int row = w4 * 32 + lane;  // query row in the tile == TMEM lane
+        const uint32_t lane_base = uint32_t(w4 * 32) << 16;
+        const int c0 = part * Cfg::kPartCols;  // first key column of this thread's part
+        bool ok = true;
         const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2);
-        int g0 = 0, n = 0;
-        int id = get_item(0);
-        if (id >= 0) ok = item_head(0, id);
-        while (ok && id >= 0) {
-            const int qt = item_qt(id), h = item_h(id), b = item_b(id), n_kv = item_nkv(id);
-            const int q0 = qt * 128;
-            for (int j = 0; j < n_kv; ++j) {
-                const int g = g0 + j;
+        int g = 0, n = 0;
+        for (int id; ok && (id = get_item(n)) >= 0; ++n) {
+            const int q0 = item_qt(id) * 128, n_kv = item_nkv(id);
+            ok = mbar_wait_warp(bar_vec, uint32_t(n) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+            if (!ok) break;
+            const float2 vec = sVec[(n & 1) * 128 + row];
+            const float lse2 = vec.x, dv = vec.y;
+            for (int j = 0; j < n_kv; ++j, ++g) {
                 ok = mbar_wait_warp(bar_s_full, uint32_t(g) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
                 if (!ok) break;
                 B200ATTN_STAMP(tid == 0, 240 + 8 * g + 0);
@@ -510,35 +589,6 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 mbar_arrive(bar_ds_full);
                 B200ATTN_STAMP(tid == 0, 240 + 8 * g + 3);
             }
-            if (!ok) break;
-            g0 += n_kv;
-            // The next item's head before this item's epilogue: its first products then run while the dQ rows are
-            // written.  (dv and lse2 change here; the epilogue below needs neither.)
-            const int id_next = get_item(n + 1);
-            if (id_next >= 0) {
-                ok = item_head(n + 1, id_next);
-                if (!ok) break;
-            }
-            // epilogue of the item: dQ rows (times scale) -> BF16 -> global memory; each part writes D / 2 columns
-            ok = mbar_wait_warp(bar_acc, n & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
-            if (!ok) break;
-            B200ATTN_STAMP(tid == 0, 400 + 4 * n + 2);
-            tc_fence_after_sync();
-            constexpr int kCols = D / Cfg::kParts;
-            uint32_t v[kCols];
-            tmem_ld_x32(tmem + lane_base + Cfg::kColAcc + part * kCols, v);
-            tmem_wait_ld();
-            tc_fence_before_sync();
-            mbar_arrive(bar_acc_free);  // the MMA warp may start the next item's accumulation
-            uint32_t w[kCols / 2];
-#pragma unroll
-            for (int i = 0; i < kCols / 2; ++i) w[i] = pack_bf16x2(__uint_as_float(v[2 * i]) * p.scale, __uint_as_float(v[2 * i + 1]) * p.scale);
-            store_rows_64b(sOut + warp * kRowStageBytes, w, lane,
-                           p.dq + size_t(b) * p.q_sb + size_t(h) * p.q_sh + size_t(q0 + w4 * 32) * p.q_st + part * kCols, p.q_st,
-                           p.T - (q0 + w4 * 32));
-            B200ATTN_STAMP(tid == 0, 400 + 4 * n + 3);
-            id = id_next;
-            ++n;
         }
     }
 
