@@ -26,7 +26,11 @@
 // softmax warps (scores out of tensor memory, maximum, exponentials at 16 a clock, P back, three barriers of about 100 clocks
 // each), two such chains per scheduler.  Hence 128 keys a tile at D = 64, packed FP32 arithmetic, and no commit whose completion
 // another barrier implies.  Measured against 64-key tiles with P over S and Q in tensor memory, us: B=2 T=128 6/2 D=64
-// 6.0 -> 5.4, B=32 T=512 6/2 21.9 -> 20.6, B=16 T=1024 16/4 74.3 -> 69.2, B=8 T=2000 16/4 122.0 -> 115.1.
+// 6.0 -> 5.4, B=32 T=512 6/2 21.9 -> 20.6, B=16 T=1024 16/4 74.3 -> 69.2, B=8 T=2000 16/4 122.0 -> 115.1.  In the steady state two
+// CTAs take 2550 clocks for a tile each, of which the exponentials alone are 2048.  Four epilogue warps of their own, as the dQ
+// pass has, pay only on long rows (B=8 T=2000 121 -> 118, B=32 T=512 20.1 -> 20.8, B=2 T=128 5.0 -> 5.5, D=128 137 -> 145: the
+// softmax warps lose registers to them); exponentials against the reference of the tile before, with the maximum taken under
+// them, were 5 % slower, a warp of its own for Q K^T made no difference.
 #pragma once
 
 #include "ptx.cuh"
@@ -443,9 +447,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     // tile touches the diagonal: key kbase + c is visible to query q0 + row iff it is <= the query's
                     // own position kv_off + q0 + row
                     const int lim = p.kv_off + q0 + row - kbase;  // columns c <= lim are visible
+                    // 32 columns at a time: those that the whole warp sees (it does from its first row on) need no look.  The
+                    // comparisons of all columns cost such a tile 550 of 3600 clocks at D = 64.
 #pragma unroll
-                    for (int c = 0; c < KEYS; ++c)
-                        if (c > lim) sr[c] = 0xff800000u;  // -inf
+                    for (int c32 = 0; c32 < KEYS; c32 += 32)
+                        if (c32 + 31 > lim - lane) {
+#pragma unroll
+                            for (int c = c32; c < c32 + 32; ++c)
+                                if (c > lim) sr[c] = 0xff800000u;  // -inf
+                        }
                 }
                 float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -485,7 +495,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     if (!__all_sync(0xffffffffu, pv_seen)) ok = mbar_wait_warp(bar_pv, pv_par, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
                     if (ok) tc_fence_after_sync();
                 };
-                const bool rescale = j > 0 && __any_sync(0xffffffffu, alpha != 1.f);
                 const uint32_t t_p = Cfg::kSepP ? tmem + lane_base + Cfg::kColP : t_s;
                 {
                     uint32_t pk[16];
@@ -500,6 +509,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     chunk(c * 32, pk);
                     tmem_st_x16(t_p + c * 16, pk);
                 }
+                const bool rescale = j > 0 && __any_sync(0xffffffffu, alpha != 1.f);  // (in front of the exponentials the vote holds them up)
                 {
                     float s0, s1;
                     unpack_f32x2(add_f32x2(sum2[0], sum2[1]), s0, s1);
