@@ -320,28 +320,41 @@ rope_norm_bwd_kernel(const __grid_constant__ RopeNormParams p0, const __grid_con
 
 // d_gamma[d] += sum of the CTAs' partial sums, for one or two tensors.  A CTA takes 8 columns (one 32-byte sector of every
 // part): thread (r, c) adds parts r, r + 32, ... of column c in order, then the 32 sums of a column are added in order, so
-// the result is bit-reproducible and all loads are in flight at once.  (Done by the last CTA of the backward kernel
-// instead, the same sums took 25 us: one CTA cannot keep enough loads in flight.)
-constexpr int kDgammaThreads = 256;
+// the result is bit-reproducible.  The kernel is latency and nothing else: a thread's sixteen loads, enough for the 444 parts of
+// three CTAs per SM, and the old d_gamma are all issued before the first is used (in a loop unrolled by eight the last six parts
+// cost a round trip through L2 each): forward and backward FP32 B=16 T=1024 16/4 D=128 115.0 -> 113.4 us, BF16 B=32 T=512 6/2
+// D=64 29.0 -> 27.9.  With 128 threads and four columns a CTA it was 1.8 us slower, with 512 the same, with 1024 slower where the
+// backward kernel has filled the SMs.  (Done by the last CTA of the backward kernel instead, the same sums took 25 us: one CTA
+// cannot keep enough loads in flight.  Bringing this kernel or the next in early made no difference.)
+constexpr int kDgammaThreads = 256, kDgammaRows = kDgammaThreads / 8, kDgammaLoads = 16;
 template <int D>
 __global__ void __launch_bounds__(kDgammaThreads) rope_norm_dgamma_kernel(const float* __restrict__ partial0, float* __restrict__ d_gamma0,
                                                                           const float* __restrict__ partial1, float* __restrict__ d_gamma1,
                                                                           int n_parts) {
-    __shared__ float s_sum[32][9];
+    __shared__ float s_sum[kDgammaRows][9];
     const int ts = blockIdx.x / (D / 8), c = threadIdx.x & 7, r = threadIdx.x >> 3, d = (blockIdx.x % (D / 8)) * 8 + c;
     const float* partial = ts ? partial1 : partial0;
     float* d_gamma = ts ? d_gamma1 : d_gamma0;
     float acc = 0.f;
     grid_dep_wait();  // the partial sums come from the kernel before this one
-#pragma unroll 8
-    for (int i = r; i < n_parts; i += 32) acc += partial[static_cast<long long>(i) * D + d];
+    const float old = r == 0 ? d_gamma[d] : 0.f;
+    for (int i0 = r; i0 < n_parts; i0 += kDgammaLoads * kDgammaRows) {
+        float v[kDgammaLoads];
+#pragma unroll
+        for (int k = 0; k < kDgammaLoads; ++k) {
+            const int i = i0 + k * kDgammaRows;
+            v[k] = i < n_parts ? partial[static_cast<long long>(i) * D + d] : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < kDgammaLoads; ++k) acc += v[k];
+    }
     s_sum[r][c] = acc;
     __syncthreads();
     if (r == 0) {
         acc = 0.f;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) acc += s_sum[i][c];
-        d_gamma[d] += acc;
+        for (int i = 0; i < kDgammaRows; ++i) acc += s_sum[i][c];
+        d_gamma[d] = old + acc;
     }
 }
 
