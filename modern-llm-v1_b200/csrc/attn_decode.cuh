@@ -122,8 +122,10 @@ struct DecodeWalk {
     int cta0;            // the first of those CTAs
 };
 
+// EARLY: in front of the wait for the kernel that may write the lengths; read through L2, so that no stale copy stays in L1
+template <bool EARLY = false>
 __device__ __forceinline__ int decode_len(const DecodeParams& p, int b) {
-    return p.lens ? max(1, min(__ldg(p.lens + b), p.L)) : p.L;
+    return p.lens ? max(1, min(EARLY ? __ldcg(p.lens + b) : __ldg(p.lens + b), p.L)) : p.L;
 }
 // First tile of CTA c's range, and the CTA whose range holds tile t.
 __device__ __forceinline__ int decode_range(const DecodeWalk& w, int c) {
@@ -134,14 +136,14 @@ __device__ __forceinline__ int decode_cta_of(const DecodeWalk& w, int t) {
     return int(((unsigned long long)(unsigned)(t + 1) * (unsigned)w.n_ctas - 1) / (unsigned)w.total);
 }
 
-template <int KEYS>
+template <int KEYS, bool EARLY = false>
 __device__ __forceinline__ DecodeWalk decode_walk_start(const DecodeParams& p, int cta, int n_ctas, int lane) {
     DecodeWalk w;
     if (p.shares) {  // one piece: this CTA's share of its unit's tiles, possibly none
         const int unit = int(fastdiv(cta, p.div_shares)), rank = cta - unit * p.shares;
         w.b = int(fastdiv(unit, p.div_units));
         w.u = unit - w.b * p.units_per_seq;
-        w.len = decode_len(p, w.b);
+        w.len = decode_len<EARLY>(p, w.b);
         w.n_tiles = (w.len + KEYS - 1) / KEYS;
         w.total = w.n_tiles;
         w.cta0 = unit * p.shares;
@@ -162,7 +164,7 @@ __device__ __forceinline__ DecodeWalk decode_walk_start(const DecodeParams& p, i
         w.total = p.B * p.units_per_seq * w.n_tiles;
     } else {
         int sum = 0;
-        for (int b = lane; b < p.B; b += 32) sum += (decode_len(p, b) + KEYS - 1) / KEYS;
+        for (int b = lane; b < p.B; b += 32) sum += (decode_len<EARLY>(p, b) + KEYS - 1) / KEYS;
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         w.total = sum * p.units_per_seq;
     }
@@ -184,7 +186,7 @@ __device__ __forceinline__ DecodeWalk decode_walk_start(const DecodeParams& p, i
         int before = 0;
         w.b = p.B - 1, w.len = 1, w.n_tiles = 1, w.u = 0, w.j0 = 0;
         for (int b0 = 0; b0 < p.B; b0 += 32) {
-            const int len = b0 + lane < p.B ? decode_len(p, b0 + lane) : 0;
+            const int len = b0 + lane < p.B ? decode_len<EARLY>(p, b0 + lane) : 0;
             const int n = (len + KEYS - 1) / KEYS;
             int incl = n;
             for (int o = 1; o < 32; o <<= 1) {
@@ -209,14 +211,14 @@ __device__ __forceinline__ DecodeWalk decode_walk_start(const DecodeParams& p, i
 }
 // Tiles of the piece at w.t
 __device__ __forceinline__ int decode_piece(const DecodeWalk& w) { return min(w.t_end - w.t, w.n_tiles - w.j0); }
-template <int KEYS>
+template <int KEYS, bool EARLY = false>
 __device__ __forceinline__ void decode_walk_next(const DecodeParams& p, DecodeWalk& w, int n) {
     w.t += n;
     w.j0 = 0;  // the piece ended at its unit's end, or the range is over
     if (w.t < w.t_end && ++w.u == p.units_per_seq) {
         w.u = 0;
         ++w.b;
-        w.len = decode_len(p, w.b);
+        w.len = decode_len<EARLY>(p, w.b);
         w.n_tiles = (w.len + KEYS - 1) / KEYS;
     }
 }
@@ -363,7 +365,8 @@ __device__ __forceinline__ int decode_count(unsigned long long* word, unsigned l
     return int(atomicAdd(word, 1ull) - tag) + 1;
 }
 
-template <int D, int NH>
+// PF: tiles that a CTA brings into L2 while the kernel in front of this one ends
+template <int D, int NH, int PF>
 __global__ void __launch_bounds__(kDecodeThreads, 2)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                    const DecodeParams p) {
@@ -466,6 +469,24 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     };
     if (warp == 5) {
         // ------------------------------------------------------------------ counter of the range's first piece
+        // First, while the kernel in front is still at work: this CTA's first tiles into L2 (coherent: what that kernel still
+        // writes there is what the loads behind the wait find).
+        if constexpr (PF > 0) {
+            DecodeWalk w = decode_walk_start<KEYS, true>(p, int(blockIdx.x), int(gridDim.x), lane);
+            for (int left = PF; w.t < w.t_end && left > 0;) {
+                const int tiles = decode_piece(w), hk = int(fastdiv(w.u, p.div_chunks));
+                for (int i = 0; i < tiles && left > 0; ++i, --left)
+                    if (elect_one()) {
+#pragma unroll
+                        for (int bx = 0; bx < Cfg::kBoxes; ++bx) {
+                            tma_prefetch_4d(&tmK, bx * 64, (w.j0 + i) * KEYS, hk, w.b);
+                            tma_prefetch_4d(&tmV, bx * 64, (w.j0 + i) * KEYS, hk, w.b);
+                        }
+                    }
+                __syncwarp();
+                decode_walk_next<KEYS, true>(p, w, tiles);
+            }
+        }
         grid_dep_wait();
         const DecodeWalk w = decode_walk_start<KEYS>(p, int(blockIdx.x), int(gridDim.x), lane);
         __syncthreads();

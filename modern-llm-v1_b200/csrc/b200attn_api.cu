@@ -935,17 +935,27 @@ DecodePlan decode_plan(int B, int L, int Hq, int Hkv, int D, int n_splits, bool 
     return d;
 }
 
-template <int D, int NH>
-int launch_decode(const CUtensorMap& tk, const CUtensorMap& tv, const DecodeParams& p, int n_ctas, cudaStream_t st) {
+template <int D, int NH, int PF>
+int launch_decode_pf(const CUtensorMap& tk, const CUtensorMap& tv, const DecodeParams& p, int n_ctas, cudaStream_t st) {
     using Cfg = DecodeCfg<D>;
     static bool set[kMaxDevices] = {false};
-    int rc = set_smem_once(attn_decode_kernel<D, NH>, Cfg::kSmemBytes, set);
+    int rc = set_smem_once(attn_decode_kernel<D, NH, PF>, Cfg::kSmemBytes, set);
     if (rc) return rc;
-    if (launch_cluster(attn_decode_kernel<D, NH>, dim3(n_ctas), kDecodeThreads, Cfg::kSmemBytes, st, p.cluster, tk, tv, p) != cudaSuccess) {
+    if (launch_cluster(attn_decode_kernel<D, NH, PF>, dim3(n_ctas), kDecodeThreads, Cfg::kSmemBytes, st, p.cluster, tk, tv, p) != cudaSuccess) {
         cudaGetLastError();
         return B200ATTN_ERR_CUDA;
     }
     return B200ATTN_OK;
+}
+
+// Where the CTAs fill most of the device the launch is bound by HBM, and the first two tiles of each come into L2 while the kernel
+// in front ends (us per call, append + decode: B=48 L<=6000 16/4 D=64 35.4 -> 34.0, B=64 L=4096 43.4 -> 42.6; decode alone, B=300
+// L=200 8/8 23.6 -> 22.4, B=8 L=2000 8/8 D=128, 128 CTAs, 14.2 -> 13.8; with three tiles the gain is smaller, with six it is gone).
+// Fewer CTAs are bound by latency, of which this hides nothing: B=6 L<=3000 8/1 D=128 8.5 -> 8.6, B=1 L=1500 16/4 5.26 -> 5.30.
+constexpr int kPrefetchCtas = 128;
+template <int D, int NH>
+int launch_decode(const CUtensorMap& tk, const CUtensorMap& tv, const DecodeParams& p, int n_ctas, cudaStream_t st) {
+    return n_ctas >= kPrefetchCtas ? launch_decode_pf<D, NH, 2>(tk, tv, p, n_ctas, st) : launch_decode_pf<D, NH, 0>(tk, tv, p, n_ctas, st);
 }
 
 }  // namespace
