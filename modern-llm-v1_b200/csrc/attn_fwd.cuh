@@ -18,19 +18,26 @@
 //   warp  5    TMEM allocation and tcgen05.mma issue (converged warp, one elected lane issues)
 //   warps 6-7  idle (they only donate registers)
 // TMEM (256 columns):
-//   D = 64   S (128 FP32 columns), O (64), P (BF16 pairs, 64).  Tiles of 128 keys.  The softmax warps take a tile's scores
-//            into registers in one go and hand S back, so the next tile's Q K^T runs under this tile's exponentials; P V of a
-//            tile runs under the next tile's.
-//   D = 128  two S buffers of 64 columns, each re-used as P, and O (128).  Tiles of 64 keys; Q K^T runs two tiles ahead of P V.
-// What bounds it: at D = 128 the tensor pipe (Q K^T with both operands in shared memory); at D = 64 the chain of a tile in the
-// softmax warps (scores out of tensor memory, maximum, exponentials at 16 a clock, P back, three barriers of about 100 clocks
-// each), two such chains per scheduler.  Hence 128 keys a tile at D = 64, packed FP32 arithmetic, and no commit whose completion
-// another barrier implies.  Measured against 64-key tiles with P over S and Q in tensor memory, us: B=2 T=128 6/2 D=64
-// 6.0 -> 5.4, B=32 T=512 6/2 21.9 -> 20.6, B=16 T=1024 16/4 74.3 -> 69.2, B=8 T=2000 16/4 122.0 -> 115.1.  In the steady state two
-// CTAs take 2550 clocks for a tile each, of which the exponentials alone are 2048.  Four epilogue warps of their own, as the dQ
-// pass has, pay only on long rows (B=8 T=2000 121 -> 118, B=32 T=512 20.1 -> 20.8, B=2 T=128 5.0 -> 5.5, D=128 137 -> 145: the
-// softmax warps lose registers to them); exponentials against the reference of the tile before, with the maximum taken under
-// them, were 5 % slower, a warp of its own for Q K^T made no difference.
+//   D = 64   S (128 FP32 columns), O (64), P (BF16 pairs, 64).  Tiles of 128 keys.
+//   D = 128  S (64), P (32), columns 0-63 of Q (32), O (128).  Tiles of 64 keys.
+// The softmax warps take a tile's scores into registers in one go and hand S back, so the next tile's Q K^T runs under this
+// tile's exponentials; P V of a tile runs under the next tile's.
+// What bounds it: at D = 64 the chain of a tile in the softmax warps (scores out of tensor memory, maximum, exponentials at 16 a
+// clock, P back, three barriers of about 100 clocks each), two such chains per scheduler.  Hence 128 keys a tile, packed FP32
+// arithmetic, and no commit whose completion another barrier implies.  In the steady state two CTAs take 2350 clocks for a tile
+// each, of which the exponentials alone are 2048.  At D = 128 it is that chain and the tensor pipe alike: a Q K^T step of 64 keys
+// takes 64 clocks of it with both operands in shared memory, 37 with Q in tensor memory, where beside S, P and O half of Q has
+// room (copied there by the MMA warp, tcgen05.cp): 680 clocks a tile instead of 788, and a tile every 1450 to 1650 instead of
+// 1700.  (Two S buffers of 64 columns with P over them, as before, leave no room for Q.)
+// Measured on B200, us: against 64-key tiles with P over S and Q in tensor memory at D=64: B=2 T=128 6/2
+// 6.0 -> 5.4, B=32 T=512 6/2 21.9 -> 20.6, B=16 T=1024 16/4 74.3 -> 69.2; one code path for both head dimensions, without the
+// second S buffer: B=32 T=512 20.4 -> 19.4, B=16 T=1024 72.9 -> 68.8, B=8 T=2000 16/4 123.5 -> 115, B=1 T=2000 6/2 18.1 -> 16.5,
+// and with half of Q in tensor memory at D=128: B=4 T=8192 16/4 1080 -> 1025, B=8 T=1024 16/4 46.1 -> 44.4, B=32 T=1001 1/1
+// 20.0 -> 19.2, B=20 T=200 8/4 12.0 both.
+// Measured and dropped: four epilogue warps of their own, as the dQ pass has (B=8 T=2000 121 -> 118, but B=32 T=512 20.1 -> 20.8,
+// B=2 T=128 5.0 -> 5.5, D=128 137 -> 145: the softmax warps lose registers to them); exponentials against the reference of the
+// tile before with the maximum taken under them (5 % slower); a warp of its own for Q K^T (no difference); Q copied by the
+// softmax warps (D=128 T=200 12.0 -> 13.1).
 #pragma once
 
 #include "ptx.cuh"
@@ -56,24 +63,26 @@ struct FwdParams {
 
 template <int D>
 struct FwdCfg {
-    static constexpr bool kSepP = (D == 64);          // P has its own columns (else it overwrites S)
-    static constexpr int kKeys = kSepP ? 128 : 64;    // keys per K/V tile
+    static constexpr int kKeys = D == 64 ? 128 : 64;  // keys per K/V tile
     static constexpr int kStages = 2;
-    static constexpr int kQBufs = (D == 64) ? 2 : 1;  // Q tiles in shared memory (the next item's Q is prefetched)
+    static constexpr int kQBufs = 2;                  // the next item's Q is prefetched
+    static constexpr bool kQTmem = D == 128;          // the first 64 columns of Q are in tensor memory
     static constexpr int kQTileBytes = 128 * D * 2;
     static constexpr int kQBoxBytes = 128 * 64 * 2;   // Q TMA box: 128 rows x 64 bf16
+    static constexpr int kQStageBytes = kQTmem ? kQBoxBytes : 0;  // where those 64 columns land
+    static constexpr int kQBytes = kQStageBytes + kQBufs * kQBoxBytes;
     static constexpr int kKVTileBytes = kKeys * D * 2;
     static constexpr int kKVBoxBytes = kKeys * 64 * 2;  // K/V TMA box: kKeys rows x 64 bf16
     static constexpr int kBoxes = D / 64;
-    static constexpr int kBarBytes = 384;
-    static constexpr int kSmemBytes = kQBufs * kQTileBytes + 2 * kStages * kKVTileBytes + kBarBytes + 1024;
+    static constexpr int kBarBytes = 512;
+    static constexpr int kSmemBytes = kQBytes + 2 * kStages * kKVTileBytes + kBarBytes;
+    static_assert(2 * (kSmemBytes + 1024) <= 228 * 1024, "two CTAs per SM");
     static constexpr int kTmemCols = 256;
-    static constexpr int kSBufs = kSepP ? 1 : 2;
-    static constexpr int kColO = 128;
-    static constexpr int kColP = kColO + D;  // kSepP only
+    static constexpr int kColS = 0, kColO = 128;
+    static constexpr int kColP = D == 64 ? kColO + D : kKeys;
+    static constexpr int kColQ = 96;  // kQTmem
     // registers per thread of the softmax warpgroup and of the other one: together the launch's 256 x 128
-    static constexpr int kRegsSoftmax = kSepP ? 192 : 168, kRegsOther = 256 - kRegsSoftmax;
-    __host__ __device__ static constexpr int col_s(int buf) { return buf * 64; }
+    static constexpr int kRegsSoftmax = D == 64 ? 192 : 168, kRegsOther = 256 - kRegsSoftmax;
 };
 
 // log2 of the growth of the row maximum that is tolerated before O and the row
@@ -92,17 +101,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     using Cfg = FwdCfg<D>;
     constexpr int NST = Cfg::kStages;
     constexpr int NQB = Cfg::kQBufs;
-    constexpr int NSB = Cfg::kSBufs;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* sQ = smem;
-    uint8_t* sK = sQ + NQB * Cfg::kQTileBytes;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint8_t* sQ = smem;                         // kQTmem: columns 0-63 on their way to tensor memory
+    uint8_t* sQb = sQ + Cfg::kQStageBytes;      // [NQB] Q as the products read it (kQTmem: columns 64-127)
+    uint8_t* sK = sQb + NQB * Cfg::kQBoxBytes;
     uint8_t* sV = sK + NST * Cfg::kKVTileBytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(sV + NST * Cfg::kKVTileBytes);
     uint64_t* bar_q = bars + 0;        // [2] per Q buffer: Q of an item has landed              (phase: item / NQB)
     uint64_t* bar_q_free = bars + 2;   // [2] per Q buffer: every Q K^T product of the item done (phase: item / NQB)
-    uint64_t* bar_s_full = bars + 4;   // [NSB] per S buffer                                      (phase: tile / NSB)
-    uint64_t* bar_p_full = bars + 7;   // [NSB] per S buffer: P written, O rescaled               (phase: tile / NSB)
+    uint64_t* bar_s_full = bars + 4;   //                                                         (phase: tile)
+    uint64_t* bar_s_loaded = bars + 5; // S is in registers                                       (phase: tile)
+    uint64_t* bar_p_full = bars + 7;   // P written, O rescaled                                   (phase: tile)
+    uint64_t* bar_qt_full = bars + 8;  // kQTmem: columns 0-63 of an item's Q are in tensor memory, the staging box is free (phase: item)
     uint64_t* bar_o_done = bars + 11;  // O of an item is complete                                (phase: item)
     uint64_t* bar_o_free = bars + 12;  // O has been read by the epilogue                         (phase: item)
     uint64_t* bar_k_full = bars + 13;            // [NST]
@@ -111,7 +121,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     uint64_t* bar_v_free = bars + 13 + 3 * NST;  // [NST] P V of the tile is complete
     uint64_t* bar_item = bars + 32;    // [kItemRing] item ids handed out by the producer
     volatile int* item_ring = reinterpret_cast<volatile int*>(bars + 32 + kItemRing);
-    uint64_t* bar_s_loaded = bars + 44; // kSepP: S is in registers                              (phase: tile)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 30);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 31);
 
@@ -147,11 +156,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             mbar_init(&bar_q[i], 1);
             mbar_init(&bar_q_free[i], 1);
         }
-        for (int i = 0; i < NSB; ++i) {
-            mbar_init(&bar_s_full[i], 1);
-            mbar_init(&bar_p_full[i], 128);
-        }
+        mbar_init(bar_s_full, 1);
         mbar_init(bar_s_loaded, 128);
+        mbar_init(bar_p_full, 128);
+        mbar_init(bar_qt_full, 1);
         mbar_init(bar_o_done, 1);
         mbar_init(bar_o_free, 128);
         for (int s = 0; s < NST; ++s) {
@@ -190,12 +198,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             const int qb = n % NQB;
             if (n >= NQB)
                 ok = mbar_wait_warp(&bar_q_free[qb], uint32_t(n / NQB - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
+            if (Cfg::kQTmem && n > 0 && ok)  // the item before has left the staging box
+                ok = mbar_wait_warp(bar_qt_full, uint32_t(n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
             if (!ok) return;
             if (elect_one()) {
                 mbar_arrive_expect_tx(&bar_q[qb], Cfg::kQTileBytes);
 #pragma unroll
                 for (int bx = 0; bx < Cfg::kBoxes; ++bx)
-                    tma_load_4d(sQ + qb * Cfg::kQTileBytes + bx * Cfg::kQBoxBytes, &tmQ, &bar_q[qb], bx * 64,
+                    tma_load_4d(bx + 1 < Cfg::kBoxes ? sQ : sQb + qb * Cfg::kQBoxBytes, &tmQ, &bar_q[qb], bx * 64,
                                 item_qt(id) * 128, item_h(id), item_b(id));
             }
             __syncwarp();
@@ -213,8 +223,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             const int h = item_h(id), b = item_b(id), hk = int(fastdiv(unsigned(h), p.div_group)), n_kv = item_nkv(id);
             // The next item is taken, announced and its Q requested a few tiles before this item's loads end
             // (late, so that a CTA commits itself to little work ahead, but not before the ring has been
-            // filled for this item); with one Q buffer, after this item's last tile (it is free only then).
-            const int j_next = NQB > 1 ? max(min(n_kv, NST) - 1, n_kv - 3) : n_kv - 1;
+            // filled for this item).
+            const int j_next = max(min(n_kv, NST) - 1, n_kv - 3);
             int id_new = n_items;
             for (int j = 0; j < n_kv; ++j, ++g) {
                 const int s = g % NST;
@@ -260,9 +270,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         reg_dealloc<Cfg::kRegsOther>();
         constexpr uint32_t idesc_s = make_idesc_bf16(128, Cfg::kKeys, 0, 0);
         constexpr uint32_t idesc_o = make_idesc_bf16(128, D, 0, 1);
-        // This CTA's key tiles are numbered g = 0, 1, ... across all its items: ring stage g % NST,
-        // S buffer g % NSB.  The cursor `sc` walks that sequence for the products Q K^T, NSB tiles ahead
-        // of the loop below that issues the products P V, also across item boundaries.
+        // This CTA's key tiles are numbered g = 0, 1, ... across all its items: ring stage g % NST.  The cursor `sc`
+        // walks that sequence for the products Q K^T, one tile ahead of the loop below that issues the products P V, also
+        // across item boundaries.
         struct Cursor {
             int id, n, j, n_kv, g;  // item id, items before it on this CTA, tile in item, tiles of item, global tile
         };
@@ -278,13 +288,30 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 ok = mbar_wait_warp(&bar_q[qb], uint32_t(sc.n / NQB) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
             if (ok) ok = mbar_wait_warp(&bar_k_full[s], uint32_t(sc.g / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
         };
-        // one thread: S(cursor) = Q K^T
-        auto issue_s = [&](uint32_t s_col, uint64_t q_desc, uint64_t k_desc, int qb, uint64_t* full, bool last) {
+        const uint32_t sq_addr = smem_u32(sQb), sk_addr = smem_u32(sK), sv_addr = smem_u32(sV);
+        // S(cursor) = Q K^T
+        auto issue_s = [&]() {
+            tc_fence_after_sync();
+            const int qb = sc.n % NQB;
+            const uint64_t q_desc = make_sdesc_sw128(sq_addr + qb * Cfg::kQBoxBytes, 16, 1024);
+            const uint64_t k_desc = make_sdesc_sw128(sk_addr + (sc.g % NST) * Cfg::kKVTileBytes, 16, 1024);
+            if (elect_one()) {
+                if (Cfg::kQTmem && sc.j == 0) {  // (the products of the item before have been read out of the S buffer)
+                    const uint64_t stage_desc = make_sdesc_sw128(smem_u32(sQ), 16, 1024);
 #pragma unroll
-            for (int ks = 0; ks < D / 16; ++ks)
-                umma_ss(tmem + s_col, q_desc + kmajor_step(ks, Cfg::kQBoxBytes), k_desc + kmajor_step(ks, Cfg::kKVBoxBytes), idesc_s, ks > 0);
-            umma_commit(full);
-            if (last) umma_commit(&bar_q_free[qb]);  // no later product reads this item's Q
+                    for (int ks = 0; ks < 4; ++ks) tmem_copy_128x32b(tmem + Cfg::kColQ + ks * 8, stage_desc + kmajor_step(ks, 0));
+                    umma_commit(bar_qt_full);
+                }
+#pragma unroll
+                for (int ks = 0; ks < D / 16; ++ks) {
+                    const uint64_t b_desc = k_desc + kmajor_step(ks, Cfg::kKVBoxBytes);
+                    if (Cfg::kQTmem && ks < 4) umma_ts(tmem + Cfg::kColS, tmem + Cfg::kColQ + ks * 8, b_desc, idesc_s, ks > 0);
+                    else umma_ss(tmem + Cfg::kColS, q_desc + kmajor_step(ks % 4, 0), b_desc, idesc_s, ks > 0);
+                }
+                umma_commit(bar_s_full);
+                if (sc.j + 1 == sc.n_kv) umma_commit(&bar_q_free[qb]);  // no later product reads this item's Q
+            }
+            __syncwarp();
         };
         auto next_s = [&]() {
             ++sc.g;
@@ -294,17 +321,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 sc.n_kv = sc.id >= 0 ? item_nkv(sc.id) : 0;
             }
         };
-        const uint32_t sq_addr = smem_u32(sQ), sk_addr = smem_u32(sK), sv_addr = smem_u32(sV);
-        for (int i = 0; i < NSB && ok && sc.id >= 0; ++i) {
+        if (sc.id >= 0) {
             wait_s();
-            if (!ok) break;
-            tc_fence_after_sync();
-            if (elect_one())
-                issue_s(Cfg::col_s(sc.g % NSB), make_sdesc_sw128(sq_addr + (sc.n % NQB) * Cfg::kQTileBytes, 16, 1024),
-                        make_sdesc_sw128(sk_addr + (sc.g % NST) * Cfg::kKVTileBytes, 16, 1024), sc.n % NQB, &bar_s_full[sc.g % NSB],
-                        sc.j + 1 == sc.n_kv);
-            __syncwarp();
-            next_s();
+            if (ok) issue_s(), next_s();
         }
         int g = 0, n = 0;
         // (this warp has already waited for the ring entry of item n: the cursor above is never behind)
@@ -313,32 +332,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             for (int j = 0; j < n_kv; ++j, ++g) {
                 // What P V needs besides P is waited for first: a wait costs 100 clocks even when the barrier is complete.
                 const int s = g % NST;
-                if constexpr (Cfg::kSepP) {
-                    // S(g + 1) as soon as S(g) is in registers: it runs under the exponentials of tile g
-                    if (sc.id >= 0) {
-                        wait_s();
-                        if (ok) ok = mbar_wait_warp(bar_s_loaded, uint32_t(g) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
-                        if (!ok) break;
-                        tc_fence_after_sync();
-                        if (elect_one())
-                            issue_s(Cfg::col_s(0), make_sdesc_sw128(sq_addr + (sc.n % NQB) * Cfg::kQTileBytes, 16, 1024),
-                                    make_sdesc_sw128(sk_addr + (sc.g % NST) * Cfg::kKVTileBytes, 16, 1024), sc.n % NQB, &bar_s_full[0],
-                                    sc.j + 1 == sc.n_kv);
-                        __syncwarp();
-                        next_s();
-                    }
+                // S(g + 1) as soon as S(g) is in registers: it runs under the exponentials of tile g
+                if (sc.id >= 0) {
+                    wait_s();
+                    if (ok) ok = mbar_wait_warp(bar_s_loaded, uint32_t(g) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
+                    if (!ok) break;
+                    issue_s();
+                    next_s();
                 }
                 if (ok) ok = mbar_wait_warp(&bar_v_full[s], uint32_t(g / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
                 // the accumulator belongs to the previous item's epilogue until it has been read
                 if (ok && j == 0 && n > 0) ok = mbar_wait_warp(bar_o_free, uint32_t(n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
                 if (!ok) break;
-                const bool more = !Cfg::kSepP && sc.id >= 0, s_last = sc.j + 1 == sc.n_kv, o_last = j + 1 == n_kv;
-                const int qb = sc.n % NQB;
                 const uint64_t v_desc = make_sdesc_sw128(sv_addr + s * Cfg::kKVTileBytes, Cfg::kKVBoxBytes, 1024);
-                const uint64_t q_desc = make_sdesc_sw128(sq_addr + qb * Cfg::kQTileBytes, 16, 1024);
-                const uint64_t k_desc = make_sdesc_sw128(sk_addr + (sc.g % NST) * Cfg::kKVTileBytes, 16, 1024);
-                const uint32_t col = Cfg::kSepP ? Cfg::kColP : Cfg::col_s(g % NSB);  // of P(g), and without kSepP of S(g + NSB)
-                ok = mbar_wait_warp(&bar_p_full[g % NSB], uint32_t(g / NSB) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
+                ok = mbar_wait_warp(bar_p_full, uint32_t(g) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
                 if (!ok) break;
                 B200ATTN_STAMP(lane == 0, 16 + 8 * g + 4);
                 tc_fence_after_sync();
@@ -346,21 +353,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     // O += P V : 16 keys per K step, 8 columns of BF16 pairs each
 #pragma unroll
                     for (int ks = 0; ks < Cfg::kKeys / 16; ++ks)
-                        umma_ts(tmem + Cfg::kColO, tmem + col + ks * 8, v_desc + uint64_t(ks * 128), idesc_o, (j > 0) || (ks > 0));
+                        umma_ts(tmem + Cfg::kColO, tmem + Cfg::kColP + ks * 8, v_desc + uint64_t(ks * 128), idesc_o, (j > 0) || (ks > 0));
                     umma_commit(&bar_v_free[s]);
-                    if (o_last) umma_commit(bar_o_done);
+                    if (j + 1 == n_kv) umma_commit(bar_o_done);
                 }
                 __syncwarp();
-                if (more) {
-                    // S of tile g + NSB into the buffer that the products just issued read.  (With two K/V stages its K is
-                    // requested late: P V must not wait for it.)
-                    wait_s();
-                    if (!ok) break;
-                    if (elect_one()) issue_s(col, q_desc, k_desc, qb, &bar_s_full[g % NSB], s_last);
-                    __syncwarp();
-                }
                 B200ATTN_STAMP(lane == 0, 16 + 8 * g + 6);
-                if (more) next_s();
             }
         }
         // nothing may be in flight when TMEM is freed: the last commit covers every MMA issued above
@@ -427,8 +425,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             float m_ref = -INFINITY;  // exponent reference (a past row maximum), raw score units
             float l = 0.f;            // running sum of exp2((s - m_ref) * scale_log2)
             for (int j = 0; j < n_kv; ++j, ++g) {
-                const uint32_t t_s = tmem + lane_base + Cfg::col_s(g % NSB);
-                ok = mbar_wait_warp(&bar_s_full[g % NSB], uint32_t(g / NSB) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+                const uint32_t t_s = tmem + lane_base + Cfg::kColS;
+                ok = mbar_wait_warp(bar_s_full, uint32_t(g) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
                 if (!ok) break;
                 B200ATTN_STAMP(tid == 0, 16 + 8 * g + 0);
                 if (tid == 0) mbar_arrive(&bar_k_free[g % NST]);
@@ -438,10 +436,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
                 for (int c = 0; c < KEYS; c += 32) tmem_ld_x32(t_s + c, &sr[c]);
                 tmem_wait_ld();
-                if constexpr (Cfg::kSepP) {
-                    tc_fence_before_sync();
-                    mbar_arrive(bar_s_loaded);  // the buffer goes back to the MMA warp at once
-                }
+                tc_fence_before_sync();
+                mbar_arrive(bar_s_loaded);  // the buffer goes back to the MMA warp at once
                 const int kbase = (j_first + j) * KEYS;  // first key of this tile
                 if (kbase + KEYS - 1 > q0 + p.kv_off) {
                     // tile touches the diagonal: key kbase + c is visible to query q0 + row iff it is <= the query's
@@ -485,21 +481,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         pk[i] = pack_bf16x2(a0, a1);
                     }
                 };
-                // P V of the previous tile: it reads the columns P goes to (kSepP) and adds to O, which may have to be rescaled.
+                // P V of the previous tile: it reads the columns P goes to and adds to O, which may have to be rescaled.
                 // (At most one phase of this barrier is outstanding here: P V of this tile cannot start before this warp has
                 // arrived on bar_p_full below.)
                 uint64_t* bar_pv = &bar_v_free[(g - 1) % NST];
                 const uint32_t pv_par = uint32_t((g - 1) / NST) & 1;
-                const bool pv_seen = Cfg::kSepP && (g == 0 || mbar_try_wait(bar_pv, pv_par));  // (looked at again below)
+                const bool pv_seen = g == 0 || mbar_try_wait(bar_pv, pv_par);  // (looked at again below)
                 auto wait_pv = [&]() {
                     if (!__all_sync(0xffffffffu, pv_seen)) ok = mbar_wait_warp(bar_pv, pv_par, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
                     if (ok) tc_fence_after_sync();
                 };
-                const uint32_t t_p = Cfg::kSepP ? tmem + lane_base + Cfg::kColP : t_s;
+                const uint32_t t_p = tmem + lane_base + Cfg::kColP;
                 {
                     uint32_t pk[16];
                     chunk(0, pk);
-                    if (Cfg::kSepP) wait_pv();
+                    wait_pv();
                     if (!ok) break;
                     tmem_st_x16(t_p, pk);
                 }
@@ -517,8 +513,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 }
                 B200ATTN_STAMP(tid == 0, 16 + 8 * g + 1);
                 if (rescale) {
-                    if (!Cfg::kSepP) wait_pv();
-                    if (!ok) break;
 #pragma unroll
                     for (int c = 0; c < D / 32; ++c) {
                         uint32_t orr[32];
@@ -531,7 +525,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 }
                 tmem_wait_st();
                 tc_fence_before_sync();
-                mbar_arrive(&bar_p_full[g % NSB]);
+                mbar_arrive(bar_p_full);
                 B200ATTN_STAMP(tid == 0, 16 + 8 * g + 2);
                 if (j == 0 && pending) {
                     ok = epilogue(n - 1, pend_id, pend_m, pend_l);

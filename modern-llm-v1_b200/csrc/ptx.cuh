@@ -353,7 +353,13 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
         "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// Makes `bar` receive one arrival when all MMAs issued so far by this thread
+// Copies 32 bytes of each of 128 rows, described like one K step of an operand in shared memory, into 8 columns of tensor memory.
+// Issued by the thread that issues the products; a product issued behind it finds the values there, but it does not wait for
+// products in front of it that still read those columns.
+__device__ __forceinline__ void tmem_copy_128x32b(uint32_t d_tmem, uint64_t sdesc) {
+    asm volatile("tcgen05.cp.cta_group::1.128x256b [%0], %1;" ::"r"(d_tmem), "l"(sdesc) : "memory");
+}
+// Makes `bar` receive one arrival when all MMAs (and copies) issued so far by this thread
 // have completed (implies tcgen05.fence::before_thread_sync).
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
