@@ -142,16 +142,16 @@ __device__ __forceinline__ void stage_row_chunk(uint8_t* tile, int row, int col,
 // Q and dO in tensor memory.  Every D = 64 kernel here is bound by the shared-memory data path (a product M128 N64
 // K16 with both operands in shared memory fetches 4 KB of A and 2 KB of B for 32 clocks of math), and Q and dO are
 // the A operands of every S = Q K^T and dP = dO V^T product of an item.  The two tiles are therefore copied
-// once per item from shared memory into tensor memory (the 128 bytes of row r are the 32 BF16-pair columns
-// of lane r as they stand), all three products of a key tile take their A operand from tensor memory, and the
-// shared-memory tiles are free for the NEXT item's loads while this item is still being worked on.
+// once per item from shared memory into tensor memory (tcgen05.cp, issued by the MMA warp in front of the products that read
+// them), all three products of a key tile take their A operand from tensor memory, and the shared-memory tiles are free for
+// the NEXT item's loads while this item is still being worked on.
 //
-// Row warps.  What happens once per item - the preprocess, the copy into tensor memory, the dQ rows on their way out - has
-// four warps of its own, beside the compute warps that go from one item's last tile to the next item's first.  Done by the
-// compute warps it kept them from 3400 clocks of tiles per item (1250 a tile); what is left of that is 1200, from the last dP
-// product over the copy to the next item's first scores.  Measured on B200, us for both passes of the backward: B=32 T=512 6/2
-// 47.0 -> 45.5, B=16 T=1024 16/4 159.1 -> 155.3, B=8 T=2000 16/4 279 -> 272, B=2 T=128 6/2 12.15 -> 12.21 (one item per CTA: nothing
-// to overlap).  dS through shared memory instead of over the dP block, so that the next dP need not wait for dQ, was slower
+// Row warps.  What happens once per item - the preprocess, the dQ rows on their way out - has four warps of its own, beside the
+// compute warps that go from one item's last tile to the next item's first; the next item's first scores are computed under the
+// last tile.  Done by the compute warps, the copy into tensor memory too, it kept them from 3400 clocks of tiles per item (1250 a
+// tile).  Measured on B200, us for both passes of the backward, with the row warps and then with the copies as tcgen05.cp: B=32
+// T=512 6/2 47.0 -> 45.4 -> 44.7, B=16 T=1024 16/4 163.5 -> 161.0 -> 158.3, B=8 T=2000 16/4 279 -> 275.7 -> 274.5, B=2 T=128 6/2
+// 12.15 -> 12.26 -> 12.06.  dS through shared memory instead of over the dP block, so that the next dP need not wait for dQ, was slower
 // (B=16 T=1024: 168 against 162): the tiles of two CTAs cover that wait already.
 //
 // Roles (512 threads): warps 0-7 compute (thread owns query row (warp % 4) * 32 + lane == TMEM lane and the 32 key
@@ -206,9 +206,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     float2* sVec = reinterpret_cast<float2*>(sOut + Cfg::kOutBytes);  // [2][128], by item parity
     uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + Cfg::kOutBytes + Cfg::kVecBytes);
     uint64_t* bar_q = bars + 0;         // Q, dO, O of an item have landed in shared memory      (phase: item)
-    uint64_t* bar_qs_free = bars + 1;   // the row warps have read those three tiles              (phase: item)
-    uint64_t* bar_qt_full = bars + 2;   // Q and dO of an item are in tensor memory               (phase: item)
-    uint64_t* bar_qt_free = bars + 7;   // every S and dP product of an item has run              (phase: item)
+    uint64_t* bar_qs_free = bars + 1;   // those three tiles have been read                       (phase: item)
     uint64_t* bar_vec = bars + 10;      // the item's row vectors are in sVec                     (phase: item)
     uint64_t* bar_s_full = bars + 3;    //                                                         (phase: tile)
     uint64_t* bar_s_loaded = bars + 4;  // S is in registers: the buffer may be overwritten       (phase: tile)
@@ -242,9 +240,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tma_prefetch_desc(&tmdO);
         tma_prefetch_desc(&tmO);
         mbar_init(bar_q, 1);
-        mbar_init(bar_qs_free, 128);
-        mbar_init(bar_qt_full, 128);
-        mbar_init(bar_qt_free, 1);
+        mbar_init(bar_qs_free, 128 + 1);  // the row warps, and the MMA warp's copies
         mbar_init(bar_vec, 128);
         mbar_init(bar_s_full, 1);
         mbar_init(bar_s_loaded, Cfg::kComputeThreads);
@@ -333,14 +329,21 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         constexpr uint32_t idesc_s = make_idesc_bf16(128, Cfg::kKeys, 0, 0);  // A in TMEM, B (K or V tile) K-major
         constexpr uint32_t idesc_acc = make_idesc_bf16(128, D, 0, 1);         // A in TMEM, B (K tile) MN-major
         // g numbers this CTA's key tiles across all its items: ring stage g % NST
-        auto issue_s = [&](int g) -> bool {  // S(g) = Q K^T; the buffer still holds S(g - 1) until it has been read
+        // S(g) = Q K^T; the buffer still holds S(g - 1) until it has been read.  first: of an item, whose Q is copied into tensor
+        // memory in front (the products that read the Q before it are complete: their scores have been read)
+        auto issue_s = [&](int g, bool first) -> bool {
             const int s = g % NST;
             if (g > 0 && !mbar_wait_warp(bar_s_loaded, uint32_t(g - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX))
                 return false;
             if (!mbar_wait_warp(&bar_kv_full[s], (g / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD)) return false;
             tc_fence_after_sync();
             const uint64_t k_desc = make_sdesc_sw128(smem_u32(sK + s * Cfg::kKVTileBytes), 16, 1024);
+            const uint64_t q_desc = make_sdesc_sw128(smem_u32(sQ), 16, 1024);
             if (elect_one()) {
+                if (first) {
+#pragma unroll
+                    for (int ks = 0; ks < D / 16; ++ks) tmem_copy_128x32b(tmem + Cfg::kColQ + ks * 8, q_desc + kmajor_step(ks, 0));
+                }
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks)
                     umma_ts(tmem + Cfg::kColS, tmem + Cfg::kColQ + ks * 8, k_desc + kmajor_step(ks, Cfg::kKVBoxBytes), idesc_s, ks > 0);
@@ -350,16 +353,22 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             return true;
         };
         // dP(g) = dO V^T; tile g's loads have landed (S(g) was issued), and the product that read dS(g - 1) out of
-        // this block was issued before (the products execute in order)
-        auto issue_dp = [&](int g, bool last) {
+        // this block was issued before (the products execute in order).  first: of an item, whose dO is copied into tensor memory
+        // in front (the products that read the dO before it are complete: dS has been made of them)
+        auto issue_dp = [&](int g, bool first) {
             const int s = g % NST;
             const uint64_t v_desc = make_sdesc_sw128(smem_u32(sV + s * Cfg::kKVTileBytes), 16, 1024);
+            const uint64_t do_desc = make_sdesc_sw128(smem_u32(sdO), 16, 1024);
             if (elect_one()) {
+                if (first) {
+#pragma unroll
+                    for (int ks = 0; ks < D / 16; ++ks) tmem_copy_128x32b(tmem + Cfg::kColDO + ks * 8, do_desc + kmajor_step(ks, 0));
+                    umma_commit(bar_qs_free);
+                }
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks)
                     umma_ts(tmem + Cfg::kColDP, tmem + Cfg::kColDO + ks * 8, v_desc + kmajor_step(ks, Cfg::kKVBoxBytes), idesc_s, ks > 0);
                 umma_commit(bar_dp_full);
-                if (last) umma_commit(bar_qt_free);  // no later product reads this item's Q and dO
             }
             __syncwarp();
         };
@@ -369,20 +378,20 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         // S of the first tile of this CTA's n-th item
         auto start_item = [&]() {
             B200ATTN_STAMP(lane == 0, 440 + 2 * n);
-            ok = mbar_wait_warp(bar_qt_full, uint32_t(n) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+            ok = mbar_wait_warp(bar_q, uint32_t(n) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
             B200ATTN_STAMP(lane == 0, 441 + 2 * n);
-            if (ok) ok = issue_s(g);
+            if (ok) ok = issue_s(g, true);
         };
         if (id >= 0) start_item();
         while (ok && id >= 0) {
             const int n_kv = item_nkv(id);
-            issue_dp(g, n_kv == 1);
+            issue_dp(g, true);
             int id_next = -1;
             for (int j = 0; j < n_kv; ++j) {
                 const int s = g % NST;
                 ++g;
                 if (j + 1 < n_kv) {
-                    ok = issue_s(g);  // as soon as the tile's scores are in registers
+                    ok = issue_s(g, false);  // as soon as the tile's scores are in registers
                 } else {
                     id_next = get_item(n + 1);
                     ++n;
@@ -411,7 +420,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 }
                 __syncwarp();
                 B200ATTN_STAMP(lane == 0, 240 + 8 * (g - 1) + 6);
-                if (j + 1 < n_kv) issue_dp(g, j + 2 == n_kv);
+                if (j + 1 < n_kv) issue_dp(g, false);
             }
             id = id_next;
         }
@@ -448,19 +457,6 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             }
             B200ATTN_STAMP(tid == Cfg::kRowWarp * 32, 400 + 4 * n_item + 3);
         };
-        // 64 BF16 of this row: its 128 bytes are 32 BF16-pair columns of lane `row` as they stand
-        auto copy_row = [&](const uint8_t* tile, uint32_t col) {
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint32_t tw[16];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const uint4 w = *reinterpret_cast<const uint4*>(tile + row * 128 + (((half * 4 + c) << 4) ^ sw));
-                    tw[4 * c] = w.x, tw[4 * c + 1] = w.y, tw[4 * c + 2] = w.z, tw[4 * c + 3] = w.w;
-                }
-                tmem_st_x16(tmem + lane_base + col + half * 16, tw);
-            }
-        };
         int n = 0, id_prev = -1;
         for (int id; ok && (id = get_item(n)) >= 0; ++n) {
             const int q0 = item_qt(id) * 128;
@@ -472,44 +468,29 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             ok = mbar_wait_warp(bar_q, uint32_t(n) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
             if (!ok) break;
             B200ATTN_STAMP(tid == Cfg::kRowWarp * 32, 400 + 4 * n + 1);
-            // The preprocess of this row, D = rowsum(O * dO) and L * log2(e), in front of the wait for the item before; of the CTA's
-            // first item behind the copy, which its first products wait for.
-            auto row_vectors = [&]() {
-                float acc = 0.f;
+            // the preprocess of this row, D = rowsum(O * dO) and L * log2(e)
+            float acc = 0.f;
 #pragma unroll
-                for (int c = 0; c < D / 8; ++c) {
-                    const uint32_t off = row * 128 + ((uint32_t(c) << 4) ^ sw);
-                    const uint4 a = *reinterpret_cast<const uint4*>(sO + off);
-                    const uint4 gq = *reinterpret_cast<const uint4*>(sdO + off);
-                    const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
-                    const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w};
+            for (int c = 0; c < D / 8; ++c) {
+                const uint32_t off = row * 128 + ((uint32_t(c) << 4) ^ sw);
+                const uint4 a = *reinterpret_cast<const uint4*>(sO + off);
+                const uint4 gq = *reinterpret_cast<const uint4*>(sdO + off);
+                const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
+                const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w};
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        acc = fmaf(__uint_as_float(aw[e] << 16), __uint_as_float(gw[e] << 16), acc);
-                        acc = fmaf(__uint_as_float(aw[e] & 0xffff0000u), __uint_as_float(gw[e] & 0xffff0000u), acc);
-                    }
+                for (int e = 0; e < 4; ++e) {
+                    acc = fmaf(__uint_as_float(aw[e] << 16), __uint_as_float(gw[e] << 16), acc);
+                    acc = fmaf(__uint_as_float(aw[e] & 0xffff0000u), __uint_as_float(gw[e] & 0xffff0000u), acc);
                 }
-                // exp2(x - inf) = 0: padding query rows contribute nothing
-                const float2 vec = make_float2(in_range ? lse_raw * 1.4426950408889634f : INFINITY, in_range ? acc : 0.f);
-                // (the compute warps have read what the buffer held by the end of that item's epilogue below)
-                sVec[(n & 1) * 128 + row] = vec;
-                mbar_arrive(bar_vec);
-                const size_t vrow = bh * p.Tpad + q0 + row;
-                p.lse2_w[vrow] = vec.x;
-                p.dvec_w[vrow] = vec.y;
-            };
-            if (n > 0) {
-                row_vectors();
-                ok = mbar_wait_warp(bar_qt_free, uint32_t(n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
-                if (!ok) break;
-                tc_fence_after_sync();
             }
-            copy_row(sQ, Cfg::kColQ);
-            copy_row(sdO, Cfg::kColDO);
-            tmem_wait_st();
-            tc_fence_before_sync();
-            mbar_arrive(bar_qt_full);
-            if (n == 0) row_vectors();
+            // exp2(x - inf) = 0: padding query rows contribute nothing
+            const float2 vec = make_float2(in_range ? lse_raw * 1.4426950408889634f : INFINITY, in_range ? acc : 0.f);
+            // (the compute warps have read what the buffer held by the end of that item's epilogue below)
+            sVec[(n & 1) * 128 + row] = vec;
+            mbar_arrive(bar_vec);
+            const size_t vrow = bh * p.Tpad + q0 + row;
+            p.lse2_w[vrow] = vec.x;
+            p.dvec_w[vrow] = vec.y;
             // The tiles were read with ordinary loads and will be overwritten by TMA, which works through the async
             // proxy: without this fence the producer's next load, issued the moment the last thread has arrived, may
             // overtake reads that are still in flight (the producer is parked at the barrier whenever the item before
@@ -604,7 +585,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // ---------------------------------------------------------------------------------------
 // dQ pass for D = 128: one CTA per item (128-row query tile of one (batch, query head)), one CTA per SM, 128-key tiles loaded
 // by TMA and worked on as two halves of 64 keys.  As in the D = 64 kernel, Q and dO are copied once from shared memory into
-// tensor memory, so that S = Q K^T, dP = dO V^T and dQ += dS K all take their A operand from there (a 128-wide product with
+// tensor memory (by the MMA warps: copied by the compute warps behind the preprocess the backward took, us, at B=8 T=512 6/2 40.6
+// instead of 39.0, at B=20 T=200 8/4 43.6 instead of 41.2, at B=8 T=1024 16/4 169.5 instead of 165.7), so that S = Q K^T, dP = dO V^T and dQ += dS K all take their A operand from there (a 128-wide product with
 // A in shared memory fetches 4 KB of A and 4 KB of B per K step).
 // The halves are two streams with their own barriers: S of the next tile's half follows as soon as this one's scores are in
 // registers, and dP of the next tile's half as soon as dQ has read dS out of its block, so one half's products run under the
@@ -651,7 +633,7 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     float* sD = reinterpret_cast<float*>(sV01 + 2 * Cfg::kTileBytes);  // [128] rowsum(O * dO)
     uint64_t* bars = reinterpret_cast<uint64_t*>(sD + 128);
     uint64_t* bar_q = bars + 0;         // Q and dO have landed in shared memory
-    uint64_t* bar_qt_full = bars + 1;   // Q and dO are in tensor memory
+    uint64_t* bar_qt_full = bars + 1;   // Q and dO are in tensor memory (one arrival each)
     uint64_t* bar_acc = bars + 2;
     uint64_t* bar_s_full = bars + 3;    // [2] per half                                        (phase: tile)
     uint64_t* bar_s_loaded = bars + 5;  // [2] S is in registers: the half may be overwritten  (phase: tile)
@@ -680,7 +662,7 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         tma_prefetch_desc(&tmdO);
         tma_prefetch_desc(&tmdQ);
         mbar_init(bar_q, 1);
-        mbar_init(bar_qt_full, Cfg::kComputeThreads);
+        mbar_init(bar_qt_full, 2);
         mbar_init(bar_acc, 1);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bar_s_full[i], 1);
@@ -742,7 +724,18 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         // ------------------------------------------------------------------ MMA issuers (whole warps, one lane issues)
         constexpr uint32_t idesc_s = make_idesc_bf16(128, 64, 0, 0);    // A in TMEM, B (64 rows of the K or V tile) K-major
         constexpr uint32_t idesc_acc = make_idesc_bf16(128, D, 0, 1);   // A in TMEM, B (K tile) MN-major
-        bool ok = mbar_wait_warp(bar_qt_full, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+        bool ok = mbar_wait_warp(bar_q, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+        if (ok) {  // Q (the warp that issues S) and dO (the other) into tensor memory
+            tc_fence_after_sync();
+            const uint64_t desc = kmajor_desc<D>(warp == kMmaSWarp ? sQ : sdO);
+            const uint32_t col = warp == kMmaSWarp ? Cfg::kColQ : Cfg::kColDO;
+            if (elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < D / 16; ++ks) tmem_copy_128x32b(tmem + col + ks * 8, desc + kmajor_step(ks, Cfg::kBoxBytes));
+                umma_commit(bar_qt_full);
+            }
+            __syncwarp();
+        }
         // D[tmem, 64 columns] = A[tmem] * (rows 64 half .. + 64 of the tile)^T
         auto issue_half = [&](uint32_t d_col, uint32_t a_col, const uint8_t* tile, int half, uint64_t* full) {
             const uint64_t desc = kmajor_desc<D>(tile + half * 64 * 128);
@@ -839,25 +832,7 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
                 p.dvec_w[vrow] = dv;
             }
         }
-        // 64 elements (box `part`) of this row of Q (half 0) or dO (half 1) from the swizzled tile in shared memory into tensor
-        // memory: its 128 bytes are 32 BF16-pair columns of lane `row` as they stand
-        bool ok = mbar_wait_warp(bar_q, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
-        if (ok) {
-            const uint8_t* tile = (half == 0 ? sQ : sdO) + part * Cfg::kBoxBytes + row * 128;
-            uint32_t tw[32];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const uint4 w = *reinterpret_cast<const uint4*>(tile + ((c ^ (row & 7)) << 4));
-                tw[4 * c] = w.x, tw[4 * c + 1] = w.y, tw[4 * c + 2] = w.z, tw[4 * c + 3] = w.w;
-            }
-            tmem_st_x32(tmem + lane_base + (half == 0 ? Cfg::kColQ : Cfg::kColDO) + part * 32, tw);
-            tmem_wait_st();
-            tc_fence_before_sync();
-            // the producer re-uses the two tiles as a K/V stage once this barrier completes: the ordinary reads
-            // above are ordered before the async proxy's (TMA) writes
-            fence_proxy_async_smem();
-            mbar_arrive(bar_qt_full);
-        }
+        bool ok = true;
         const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), neg_l2 = pack_f32x2(-lse2, -lse2), neg_d2 = pack_f32x2(-dv, -dv);
         for (int j = 0; j < n_kv && ok; ++j) {
             ok = mbar_wait_warp(&bar_s_full[half], uint32_t(j) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
