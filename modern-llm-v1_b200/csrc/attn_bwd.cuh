@@ -207,7 +207,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + Cfg::kOutBytes + Cfg::kVecBytes);
     uint64_t* bar_q = bars + 0;         // Q, dO, O of an item have landed in shared memory      (phase: item)
     uint64_t* bar_qs_free = bars + 1;   // those three tiles have been read                       (phase: item)
-    uint64_t* bar_vec = bars + 10;      // the item's row vectors are in sVec                     (phase: item)
+    uint64_t* bar_vec = bars + 10;      // [2] by item parity: the item's row vectors are in sVec (phase: item / 2)
     uint64_t* bar_s_full = bars + 3;    //                                                         (phase: tile)
     uint64_t* bar_s_loaded = bars + 4;  // S is in registers: the buffer may be overwritten       (phase: tile)
     uint64_t* bar_dp_full = bars + 5;   //                                                         (phase: tile)
@@ -241,7 +241,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tma_prefetch_desc(&tmO);
         mbar_init(bar_q, 1);
         mbar_init(bar_qs_free, 128 + 1);  // the row warps, and the MMA warp's copies
-        mbar_init(bar_vec, 128);
+        mbar_init(&bar_vec[0], 128);
+        mbar_init(&bar_vec[1], 128);
         mbar_init(bar_s_full, 1);
         mbar_init(bar_s_loaded, Cfg::kComputeThreads);
         mbar_init(bar_dp_full, 1);
@@ -485,9 +486,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             }
             // exp2(x - inf) = 0: padding query rows contribute nothing
             const float2 vec = make_float2(in_range ? lse_raw * 1.4426950408889634f : INFINITY, in_range ? acc : 0.f);
-            // (the compute warps have read what the buffer held by the end of that item's epilogue below)
+            // (Every compute warp has passed the barrier and read what the buffer held by the end of that item's epilogue below.  With
+            // one barrier for all items a row warp could be an item ahead of another and arrive for both.)
             sVec[(n & 1) * 128 + row] = vec;
-            mbar_arrive(bar_vec);
+            mbar_arrive(&bar_vec[n & 1]);
             const size_t vrow = bh * p.Tpad + q0 + row;
             p.lse2_w[vrow] = vec.x;
             p.dvec_w[vrow] = vec.y;
@@ -513,7 +515,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         int g = 0, n = 0;
         for (int id; ok && (id = get_item(n)) >= 0; ++n) {
             const int q0 = item_qt(id) * 128, n_kv = item_nkv(id);
-            ok = mbar_wait_warp(bar_vec, uint32_t(n) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+            ok = mbar_wait_warp(&bar_vec[n & 1], uint32_t(n >> 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
             if (!ok) break;
             const float2 vec = sVec[(n & 1) * 128 + row];
             const float lse2 = vec.x, dv = vec.y;
