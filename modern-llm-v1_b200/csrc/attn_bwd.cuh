@@ -114,24 +114,6 @@ __device__ __forceinline__ uint64_t mnmajor_desc(const void* tile) {
     return make_sdesc_sw128(smem_u32(tile), BwdCfg<D>::kBoxBytes, 1024);
 }
 
-// Converts 32 FP32 accumulator columns [col, col+32) of this thread's row to BF16 (times
-// `mul`) and writes them into a 128-byte-swizzled [128 rows][64] box layout.
-template <int D>
-__device__ __forceinline__ void stage_row_chunk(uint8_t* tile, int row, int col, const uint32_t* v, float mul) {
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-        uint4 w;
-        w.x = pack_bf16x2(__uint_as_float(v[g * 8 + 0]) * mul, __uint_as_float(v[g * 8 + 1]) * mul);
-        w.y = pack_bf16x2(__uint_as_float(v[g * 8 + 2]) * mul, __uint_as_float(v[g * 8 + 3]) * mul);
-        w.z = pack_bf16x2(__uint_as_float(v[g * 8 + 4]) * mul, __uint_as_float(v[g * 8 + 5]) * mul);
-        w.w = pack_bf16x2(__uint_as_float(v[g * 8 + 6]) * mul, __uint_as_float(v[g * 8 + 7]) * mul);
-        const int c = col + g * 8;
-        const int bx = c >> 6;
-        const int cc = (c & 63) >> 3;
-        *reinterpret_cast<uint4*>(tile + bx * BwdCfg<D>::kBoxBytes + row * 128 + ((cc ^ (row & 7)) << 4)) = w;
-    }
-}
-
 // ---------------------------------------------------------------------------------------
 // dQ pass (D = 64): persistent CTAs, two per SM.  A CTA walks a list of work items (item = one 128-row query tile
 // of one (batch, query head); items are ordered heaviest first), and every pipeline keeps running across item
@@ -585,76 +567,116 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 }
 
 // ---------------------------------------------------------------------------------------
-// dQ pass for D = 128: one CTA per item (128-row query tile of one (batch, query head)), one CTA per SM, 128-key tiles loaded
-// by TMA and worked on as two halves of 64 keys.  As in the D = 64 kernel, Q and dO are copied once from shared memory into
-// tensor memory (by the MMA warps: copied by the compute warps behind the preprocess the backward took, us, at B=8 T=512 6/2 40.6
-// instead of 39.0, at B=20 T=200 8/4 43.6 instead of 41.2, at B=8 T=1024 16/4 169.5 instead of 165.7), so that S = Q K^T, dP = dO V^T and dQ += dS K all take their A operand from there (a 128-wide product with
+// dQ pass for D = 128: persistent CTAs, one per SM, that walk a list of the same items; 128-key tiles loaded by TMA and worked
+// on as two halves of 64 keys.  As in the D = 64 kernel, Q and dO are copied once per item from shared memory into tensor memory,
+// so that S = Q K^T, dP = dO V^T and dQ += dS K all take their A operand from there (a 128-wide product with
 // A in shared memory fetches 4 KB of A and 4 KB of B per K step).
 // The halves are two streams with their own barriers: S of the next tile's half follows as soon as this one's scores are in
 // registers, and dP of the next tile's half as soon as dQ has read dS out of its block, so one half's products run under the
 // other half's arithmetic.  (With whole tiles and one dP block, dS, dQ and the next dP followed one another: 3900 clocks per
-// 128 x 128 block for 1800 of tensor-pipe time.  There is no room for a second dP block beside S, dQ, Q and dO.)
+// 128 x 128 block for 1800 of tensor-pipe time, against 2020 now.  There is no room for a second dP block beside S, dQ, Q and dO.)
 // The halves' dQ products are issued by one warp in a fixed order, so dQ is bit-reproducible.
+// What bounds it: the tensor pipe inside an item.  Between two items a CTA of its own for each left the pipe idle for 3 us (its
+// start, the preprocess from global memory, Q and dO, K and V, the way out of dQ); now the ring of loads runs on into the next item,
+// whose Q and dO take one place in it, and row warps of their own do the preprocess and the dQ rows, as in the D = 64 kernel.
+// Measured on B200, us for both passes of the backward: B=8 T=512 6/2 39.0 -> 33.6, B=20 T=200 8/4 41.2 -> 33.4, B=8 T=1024 16/4
+// 168 -> 146, B=32 T=1001 1/1 48.2 -> 43.2, B=4 T=2048 16/4 267 -> 245, B=4 T=8192 16/4 3437 -> 3375; one item per CTA: B=2 T=128 6/2
+// 15.7 both, B=1 T=2000 6/2 53.2 -> 53.5.
 //
-// Roles (608 threads): warps 0-15 compute (thread owns row (warp % 4) * 32 + lane and 32 of the half's 64 columns: half
-// warp / 8, part (warp / 4) % 2), warp 16 TMA producer, warp 17 TMEM allocation and S, warp 18 dQ and dP.
-// Shared memory: the Q and dO staging tiles (64 KB; re-used as the third K/V ring stage once they have been copied
-// into tensor memory, and at the very end as the staging tile of the dQ store) and two more K/V stages.
+// Roles (736 threads): warps 0-15 compute (thread owns row (warp % 4) * 32 + lane and 32 of the half's 64 columns: half
+// warp / 8, part (warp / 4) % 2), warps 16-19 rows, warp 20 TMA producer, warp 21 TMEM allocation and S, warp 22 dQ and dP.
+// A CTA's first preprocess and its last dQ rows, which nothing hides, are the sixteen compute warps' instead.
+// Shared memory: three ring places of 64 KB, Q and dO of an item or K and V of a tile.
 // TMEM (512 columns): S [0,128), dP [128,256) (dS as BF16 over the first 16 columns of each part's range), dQ
 // accumulator [256,384), Q [384,448), dO [448,512).
 // ---------------------------------------------------------------------------------------
 template <int D>
 struct DqWideCfg {
-    static constexpr int kStages = 3;  // K/V tile pairs in flight; the third one lives where Q and dO were staged
+    static constexpr int kStages = 3;  // ring places
     static constexpr int kTileBytes = 128 * D * 2;
     static constexpr int kBoxBytes = 128 * 64 * 2;
     static constexpr int kBoxes = D / 64;
-    static constexpr int kComputeThreads = 512, kStreamThreads = 256, kThreads = kComputeThreads + 96;
-    static constexpr int kSmemBytes = 2 * kStages * kTileBytes + 512 + 256 + 1024;
+    static constexpr int kComputeThreads = 512, kStreamThreads = 256, kRowThreads = 128, kThreads = kComputeThreads + kRowThreads + 96;
+    static constexpr int kOutBytes = 4 * kRowStageBytes;  // per row warp: its output rows on their way to global memory
+    static constexpr int kVecBytes = 2 * 128 * 8 + 512;   // (L * log2(e), D) of the rows of two items; D of the first
+    static constexpr int kSmemBytes = 2 * kStages * kTileBytes + kOutBytes + kVecBytes + 512;
+    static_assert(kSmemBytes <= 232448, "shared memory of an SM");
     static constexpr int kTmemCols = 512;
     static constexpr int kColS = 0, kColDP = 128, kColAcc = 256, kColQ = 384, kColDO = 448;
 };
+
+// D of rows r0 .. r0 + 8 n of a tile from global memory, LPR lanes to a row; `use(r, D)` by the first of them
+template <int D, int PASSES, typename Use>
+__device__ __forceinline__ void dq_wide_row_sums(const BwdParams& p, size_t tile_off, int q0, int r0, int lane, Use use) {
+    constexpr int LPR = D / 8, RPP = 32 / LPR;
+    uint4 a[PASSES], g[PASSES];
+#pragma unroll
+    for (int i = 0; i < PASSES; ++i) {
+        const int r = r0 + i * RPP + lane / LPR;
+        a[i] = g[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (q0 + r < p.T) {
+            const size_t off = tile_off + size_t(q0 + r) * p.q_st + (lane % LPR) * 8;
+            a[i] = *reinterpret_cast<const uint4*>(p.o + off);
+            g[i] = *reinterpret_cast<const uint4*>(p.dout + off);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < PASSES; ++i) {
+        const uint32_t aw[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+        const uint32_t gw[4] = {g[i].x, g[i].y, g[i].z, g[i].w};
+        float acc = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            acc = fmaf(__uint_as_float(aw[e] << 16), __uint_as_float(gw[e] << 16), acc);
+            acc = fmaf(__uint_as_float(aw[e] & 0xffff0000u), __uint_as_float(gw[e] & 0xffff0000u), acc);
+        }
+#pragma unroll
+        for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane % LPR == 0) use(r0 + i * RPP + lane / LPR, acc);
+    }
+}
 
 template <int D>
 __global__ void __launch_bounds__(DqWideCfg<D>::kThreads, 1)
 attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
-                   const __grid_constant__ CUtensorMap tmdQ, const BwdParams p) {
+                   const BwdParams p, const __grid_constant__ ItemTable tab) {
     static_assert(D == 128, "Q and dO take 2 x 64 tensor-memory columns: D = 128 only");
     using Cfg = DqWideCfg<D>;
     constexpr int NST = Cfg::kStages;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* sQ = smem;
-    uint8_t* sdO = sQ + Cfg::kTileBytes;
-    uint8_t* sK01 = sdO + Cfg::kTileBytes;      // K of ring stages 0 and 1
-    uint8_t* sV01 = sK01 + 2 * Cfg::kTileBytes; // V of ring stages 0 and 1
-    // ring stage 2 re-uses the two tiles Q and dO were staged in (free once they are in tensor memory)
-    auto stage_k = [&](int st) { return st < 2 ? sK01 + st * Cfg::kTileBytes : sQ; };
-    auto stage_v = [&](int st) { return st < 2 ? sV01 + st * Cfg::kTileBytes : sdO; };
-    float* sD = reinterpret_cast<float*>(sV01 + 2 * Cfg::kTileBytes);  // [128] rowsum(O * dO)
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sD + 128);
-    uint64_t* bar_q = bars + 0;         // Q and dO have landed in shared memory
-    uint64_t* bar_qt_full = bars + 1;   // Q and dO are in tensor memory (one arrival each)
-    uint64_t* bar_acc = bars + 2;
-    uint64_t* bar_s_full = bars + 3;    // [2] per half                                        (phase: tile)
-    uint64_t* bar_s_loaded = bars + 5;  // [2] S is in registers: the half may be overwritten  (phase: tile)
-    uint64_t* bar_dp_full = bars + 7;   // [2]                                                 (phase: tile)
-    uint64_t* bar_ds_full = bars + 9;   // [2] dS written over dP                              (phase: tile)
-    uint64_t* bar_kv_full = bars + 11;          // [NST]
-    uint64_t* bar_kv_free = bars + 11 + NST;    // [NST]
+    extern __shared__ __align__(1024) uint8_t smem[];
+    auto place_a = [&](int e) { return smem + (e % NST) * 2 * Cfg::kTileBytes; };  // Q or K of ring entry e
+    auto place_b = [&](int e) { return smem + (e % NST) * 2 * Cfg::kTileBytes + Cfg::kTileBytes; };  // dO or V
+    uint8_t* sOut = smem + 2 * NST * Cfg::kTileBytes;                 // [4 row warps]
+    float2* sVec = reinterpret_cast<float2*>(sOut + Cfg::kOutBytes);  // [2][128], by item parity
+    float* sD = reinterpret_cast<float*>(sVec + 2 * 128);             // [128] rowsum(O * dO) of the CTA's first item
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + Cfg::kOutBytes + Cfg::kVecBytes);
+    uint64_t* bar_full = bars + 0;      // [NST] a ring entry has landed                       (phase: entry / NST)
+    uint64_t* bar_free = bars + 3;      // [NST] both MMA warps are through with it            (phase: entry / NST)
+    uint64_t* bar_s_full = bars + 6;    // [2] per half                                        (phase: tile)
+    uint64_t* bar_s_loaded = bars + 8;  // [2] S is in registers: the half may be overwritten  (phase: tile)
+    uint64_t* bar_dp_full = bars + 10;  // [2]                                                 (phase: tile)
+    uint64_t* bar_ds_full = bars + 12;  // [2] dS written over dP                              (phase: tile)
+    uint64_t* bar_vec = bars + 14;      // [2] by item parity: the row vectors are in sVec     (phase: (item - 1) / 2)
+    uint64_t* bar_acc = bars + 16;      // dQ accumulator of an item complete                  (phase: item)
+    uint64_t* bar_acc_free = bars + 17; // dQ accumulator read by the row warps                (phase: item)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 19);
+    uint64_t* bar_item = bars + 24;     // [kItemRing] item ids handed out by the producer
+    volatile int* item_ring = reinterpret_cast<volatile int*>(bars + 24 + kItemRing);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr int kProducerWarp = Cfg::kComputeThreads / 32, kMmaSWarp = kProducerWarp + 1;
+    constexpr int kRowWarp = Cfg::kComputeThreads / 32, kProducerWarp = kRowWarp + 4, kMmaSWarp = kProducerWarp + 1;
     const int n_bh = p.B * p.Hq;
-    const int item_hi = int(fastdiv(blockIdx.x, p.div_bhq));  // ids are ordered by work, heaviest query tile first
-    const int qt = p.n_tiles - 1 - item_hi, rest = int(blockIdx.x) - item_hi * n_bh;
-    const int b = int(fastdiv(unsigned(rest), p.div_hq)), h = rest - b * p.Hq;
-    const int hk = int(fastdiv(unsigned(h), p.div_group));
-    const int q0 = qt * 128;
-    const int n_kv = qt + 1;
+    const int n_items = p.n_tiles * n_bh;
+    // item id -> (query tile, head, batch); ids are ordered by work, heaviest query tile first
+    auto item_rest = [&](int id) { return id - int(fastdiv(unsigned(id), p.div_bhq)) * n_bh; };  // b * Hq + h
+    auto item_qt = [&](int id) { return p.n_tiles - 1 - int(fastdiv(unsigned(id), p.div_bhq)); };
+    auto item_b = [&](int id) { return int(fastdiv(unsigned(item_rest(id)), p.div_hq)); };
+    auto item_h = [&](int id) { return item_rest(id) - item_b(id) * p.Hq; };
+    auto item_nkv = [&](int id) { return item_qt(id) + 1; };
+    auto get_item = [&](int n) { return item_get(bar_item, item_ring, n, abort_flag, p.status); };
+    auto q_offset = [&](int id) { return size_t(item_b(id)) * p.q_sb + size_t(item_h(id)) * p.q_sh; };
 
     B200ATTN_TRACE_BEGIN(1);
     if (warp == kProducerWarp && lane == 0) {
@@ -662,20 +684,20 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         tma_prefetch_desc(&tmK);
         tma_prefetch_desc(&tmV);
         tma_prefetch_desc(&tmdO);
-        tma_prefetch_desc(&tmdQ);
-        mbar_init(bar_q, 1);
-        mbar_init(bar_qt_full, 2);
-        mbar_init(bar_acc, 1);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bar_s_full[i], 1);
             mbar_init(&bar_s_loaded[i], Cfg::kStreamThreads);
             mbar_init(&bar_dp_full[i], 1);
             mbar_init(&bar_ds_full[i], Cfg::kStreamThreads);
+            mbar_init(&bar_vec[i], Cfg::kRowThreads);
         }
+        mbar_init(bar_acc, 1);
+        mbar_init(bar_acc_free, Cfg::kRowThreads);
         for (int s = 0; s < NST; ++s) {
-            mbar_init(&bar_kv_full[s], 1);
-            mbar_init(&bar_kv_free[s], 1);
+            mbar_init(&bar_full[s], 1);
+            mbar_init(&bar_free[s], 2);
         }
+        for (int i = 0; i < kItemRing; ++i) mbar_init(&bar_item[i], 1);
         fence_mbar_init();
         // launched with programmatic stream serialization: wait for the previous kernel before any global access
         grid_dep_wait();
@@ -696,101 +718,186 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         // an earlier CTA already failed: fall through to the teardown
     } else if (warp == kProducerWarp) {
         // ------------------------------------------------------------------ producer (whole warp, one lane issues)
-        if (elect_one()) {
-            mbar_arrive_expect_tx(bar_q, 2 * Cfg::kTileBytes);
-#pragma unroll
-            for (int bx = 0; bx < Cfg::kBoxes; ++bx) {
-                tma_load_4d(sQ + bx * Cfg::kBoxBytes, &tmQ, bar_q, bx * 64, q0, h, b);
-                tma_load_4d(sdO + bx * Cfg::kBoxBytes, &tmdO, bar_q, bx * 64, q0, h, b);
-            }
+        int e = 0;  // ring entries issued so far by this CTA
+        bool ok = true;
+        int id = sched_first(tab, p.sched, int(blockIdx.x));  // the first item needs no fetch
+        int id_next = 0;  // lane 0: the id fetched for the next item
+        if (lane == 0) {
+            item_publish(bar_item, item_ring, 0, id);
+            id_next = sched_fetch(tab, p.sched, 1, int(blockIdx.x), int(gridDim.x));
         }
         __syncwarp();
-        for (int j = 0; j < n_kv; ++j) {
-            const int s = j % NST;
-            if (j >= NST &&
-                !mbar_wait_warp(&bar_kv_free[s], ((j / NST) - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE))
-                break;
-            // the first use of stage 2 overwrites Q and dO in shared memory: they must be in tensor memory by then
-            if (j == 2 && !mbar_wait_warp(bar_qt_full, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE)) break;
+        auto load = [&](const CUtensorMap* ma, const CUtensorMap* mb, int row, int head, int b) {
+            if (e >= NST) ok = mbar_wait_warp(&bar_free[e % NST], uint32_t(e / NST - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
+            if (!ok) return;
             if (elect_one()) {
-                mbar_arrive_expect_tx(&bar_kv_full[s], 2 * Cfg::kTileBytes);
+                uint64_t* full = &bar_full[e % NST];
+                mbar_arrive_expect_tx(full, 2 * Cfg::kTileBytes);
 #pragma unroll
                 for (int bx = 0; bx < Cfg::kBoxes; ++bx) {
-                    tma_load_4d(stage_k(s) + bx * Cfg::kBoxBytes, &tmK, &bar_kv_full[s], bx * 64, j * 128, hk, b);
-                    tma_load_4d(stage_v(s) + bx * Cfg::kBoxBytes, &tmV, &bar_kv_full[s], bx * 64, j * 128, hk, b);
+                    tma_load_4d(place_a(e) + bx * Cfg::kBoxBytes, ma, full, bx * 64, row, head, b);
+                    tma_load_4d(place_b(e) + bx * Cfg::kBoxBytes, mb, full, bx * 64, row, head, b);
                 }
             }
             __syncwarp();
+            ++e;
+        };
+        for (int n = 0; ok; ++n) {
+            const int h = item_h(id), b = item_b(id), hk = int(fastdiv(unsigned(h), p.div_group)), n_kv = item_nkv(id);
+            // the next item is taken and announced shortly before this item's loads end, but not before the
+            // ring has been filled for this item
+            const int j_next = max(min(n_kv, NST - 1) - 1, n_kv - 2);
+            int id_new = n_items;
+            load(&tmQ, &tmdO, item_qt(id) * 128, h, b);
+            for (int j = 0; j < n_kv && ok; ++j) {
+                load(&tmK, &tmV, j * 128, hk, b);
+                if (ok && j == j_next) {
+                    id_new = __shfl_sync(0xffffffffu, id_next, 0);
+                    if (lane == 0) {
+                        item_publish(bar_item, item_ring, n + 1, id_new < n_items ? id_new : -1);
+                        if (id_new < n_items) id_next = sched_fetch(tab, p.sched, n + 2, int(blockIdx.x), int(gridDim.x));
+                    }
+                    __syncwarp();
+                }
+            }
+            if (!ok || id_new >= n_items) break;
+            id = id_new;
         }
+        if (ok && lane == 0) sched_finish(p.sched, int(gridDim.x));
     } else if (warp >= kMmaSWarp) {
         // ------------------------------------------------------------------ MMA issuers (whole warps, one lane issues)
         constexpr uint32_t idesc_s = make_idesc_bf16(128, 64, 0, 0);    // A in TMEM, B (64 rows of the K or V tile) K-major
         constexpr uint32_t idesc_acc = make_idesc_bf16(128, D, 0, 1);   // A in TMEM, B (K tile) MN-major
-        bool ok = mbar_wait_warp(bar_q, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
-        if (ok) {  // Q (the warp that issues S) and dO (the other) into tensor memory
+        bool ok = true;
+        int e = 0, g = 0;  // ring entry, and tile across all items of the CTA
+        auto wait_entry = [&](int entry) {
+            ok = mbar_wait_warp(&bar_full[entry % NST], uint32_t(entry / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+        };
+        // an operand of the item from its ring entry into tensor memory
+        auto copy_operand = [&](const uint8_t* tile, uint32_t col) {
             tc_fence_after_sync();
-            const uint64_t desc = kmajor_desc<D>(warp == kMmaSWarp ? sQ : sdO);
-            const uint32_t col = warp == kMmaSWarp ? Cfg::kColQ : Cfg::kColDO;
+            const uint64_t desc = kmajor_desc<D>(tile);
             if (elect_one()) {
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks) tmem_copy_128x32b(tmem + col + ks * 8, desc + kmajor_step(ks, Cfg::kBoxBytes));
-                umma_commit(bar_qt_full);
+                umma_commit(&bar_free[e % NST]);
             }
             __syncwarp();
-        }
+        };
         // D[tmem, 64 columns] = A[tmem] * (rows 64 half .. + 64 of the tile)^T
-        auto issue_half = [&](uint32_t d_col, uint32_t a_col, const uint8_t* tile, int half, uint64_t* full) {
+        auto issue_half = [&](uint32_t d_col, uint32_t a_col, const uint8_t* tile, int half, uint64_t* full, uint64_t* free) {
             const uint64_t desc = kmajor_desc<D>(tile + half * 64 * 128);
             if (elect_one()) {
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks)
                     umma_ts(tmem + d_col + half * 64, tmem + a_col + ks * 8, desc + kmajor_step(ks, Cfg::kBoxBytes), idesc_s, ks > 0);
                 umma_commit(full);
+                if (free) umma_commit(free);
             }
             __syncwarp();
         };
         if (warp == kMmaSWarp) {
-            for (int j = 0; j < n_kv && ok; ++j) {
-                const int s = j % NST;
-                ok = mbar_wait_warp(&bar_kv_full[s], (j / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
-                for (int half = 0; half < 2 && ok; ++half) {
-                    if (j > 0) ok = mbar_wait_warp(&bar_s_loaded[half], uint32_t(j - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
-                    if (!ok) break;
-                    tc_fence_after_sync();
-                    issue_half(Cfg::kColS, Cfg::kColQ, stage_k(s), half, &bar_s_full[half]);
+            for (int n = 0, id; ok && (id = get_item(n)) >= 0; ++n) {
+                const int n_kv = item_nkv(id);
+                // (the products that read the Q before are complete when their scores have been read)
+                for (int half = 0; half < 2 && ok && g > 0; ++half)
+                    ok = mbar_wait_warp(&bar_s_loaded[half], uint32_t(g - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
+                if (ok) wait_entry(e);
+                if (!ok) break;
+                copy_operand(place_a(e), Cfg::kColQ);
+                ++e;
+                for (int j = 0; j < n_kv && ok; ++j, ++g, ++e) {
+                    wait_entry(e);
+                    for (int half = 0; half < 2 && ok; ++half) {
+                        if (j > 0) ok = mbar_wait_warp(&bar_s_loaded[half], uint32_t(g - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
+                        if (!ok) break;
+                        tc_fence_after_sync();
+                        issue_half(Cfg::kColS, Cfg::kColQ, place_a(e), half, &bar_s_full[half], half ? &bar_free[e % NST] : nullptr);
+                    }
                 }
             }
         } else {
-            if (ok) ok = mbar_wait_warp(&bar_kv_full[0], 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
-            if (ok) {
+            int n = 0;
+            for (int id; ok && (id = get_item(n)) >= 0; ++n) {
+                const int n_kv = item_nkv(id);
+                wait_entry(e);
+                if (!ok) break;
+                copy_operand(place_b(e), Cfg::kColDO);  // (dS of the item before has been made of all its dP)
+                ++e;
+                wait_entry(e);
+                if (!ok) break;
                 tc_fence_after_sync();
-                for (int half = 0; half < 2; ++half) issue_half(Cfg::kColDP, Cfg::kColDO, stage_v(0), half, &bar_dp_full[half]);
-            }
-            for (int j = 0; j < n_kv && ok; ++j) {
-                const int s = j % NST, s1 = (j + 1) % NST;
-                const uint64_t k_desc = mnmajor_desc<D>(stage_k(s));
-                if (j + 1 < n_kv) ok = mbar_wait_warp(&bar_kv_full[s1], ((j + 1) / NST) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
-                for (int half = 0; half < 2 && ok; ++half) {
-                    ok = mbar_wait_warp(&bar_ds_full[half], uint32_t(j) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
-                    if (!ok) break;
-                    tc_fence_after_sync();
-                    if (elect_one()) {
-                        // dQ += dS K over the half's 64 keys: 4 K steps, two per part
+                for (int half = 0; half < 2; ++half) issue_half(Cfg::kColDP, Cfg::kColDO, place_b(e), half, &bar_dp_full[half], nullptr);
+                for (int j = 0; j < n_kv && ok; ++j, ++g, ++e) {
+                    const bool more = j + 1 < n_kv;
+                    const uint64_t k_desc = mnmajor_desc<D>(place_a(e));
+                    if (more) wait_entry(e + 1);
+                    for (int half = 0; half < 2 && ok; ++half) {
+                        ok = mbar_wait_warp(&bar_ds_full[half], uint32_t(g) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
+                        // the accumulator belongs to the previous item's rows until they have been read
+                        if (ok && j == 0 && half == 0 && n > 0)
+                            ok = mbar_wait_warp(bar_acc_free, uint32_t(n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_SOFTMAX);
+                        if (!ok) break;
+                        tc_fence_after_sync();
+                        if (elect_one()) {
+                            // dQ += dS K over the half's 64 keys: 4 K steps, two per part
 #pragma unroll
-                        for (int ks = 0; ks < 4; ++ks)
-                            umma_ts(tmem + Cfg::kColAcc, tmem + Cfg::kColDP + half * 64 + (ks >> 1) * 32 + (ks & 1) * 8,
-                                    k_desc + uint64_t((half * 4 + ks) * 128), idesc_acc, j > 0 || half > 0 || ks > 0);
-                        if (half == 1) umma_commit(&bar_kv_free[s]);
+                            for (int ks = 0; ks < 4; ++ks)
+                                umma_ts(tmem + Cfg::kColAcc, tmem + Cfg::kColDP + half * 64 + (ks >> 1) * 32 + (ks & 1) * 8,
+                                        k_desc + uint64_t((half * 4 + ks) * 128), idesc_acc, j > 0 || half > 0 || ks > 0);
+                            if (half == 1) umma_commit(&bar_free[e % NST]);
+                            if (half == 1 && !more) umma_commit(bar_acc);
+                        }
+                        __syncwarp();
+                        // behind the product that reads dS out of the block
+                        if (more) issue_half(Cfg::kColDP, Cfg::kColDO, place_b(e + 1), half, &bar_dp_full[half], nullptr);
                     }
-                    __syncwarp();
-                    // behind the product that reads dS out of the block
-                    if (j + 1 < n_kv) issue_half(Cfg::kColDP, Cfg::kColDO, stage_v(s1), half, &bar_dp_full[half]);
                 }
             }
-            if (elect_one()) umma_commit(bar_acc);
-            __syncwarp();
             // nothing may be in flight when TMEM is freed (the compute warps have waited for the other warp's products)
-            if (ok) mbar_wait_warp(bar_acc, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+            if (ok && n > 0) mbar_wait_warp(bar_acc, uint32_t(n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+        }
+    } else if (warp >= kRowWarp) {
+        // ------------------------------------------------------------------ rows: what happens once per item
+        const int w4 = warp & 3, row = w4 * 32 + lane;  // query row in the tile == TMEM lane
+        bool ok = true;
+        int id_prev = get_item(0);
+        for (int n = 1, id; ok && (id = get_item(n)) >= 0; ++n) {
+            // preprocess of the next item
+            const int q0 = item_qt(id) * 128;
+            const size_t bh = size_t(item_b(id)) * p.Hq + item_h(id);
+            const float lse2 = q0 + row < p.T ? p.lse[bh * p.T + q0 + row] * 1.4426950408889634f : INFINITY;  // exp2(x - inf) = 0: padding
+            // (Every compute warp has passed the barrier and read what the buffer held by the end of that item's rows below.  With one
+            // barrier for all items a row warp could be an item ahead of another and arrive for both.)
+            float2* vec = sVec + (n & 1) * 128;
+#pragma unroll 1
+            for (int r = 0; r < 32; r += 8) dq_wide_row_sums<D, 4>(p, q_offset(id), q0, w4 * 32 + r, lane, [&](int r, float d) { vec[r].y = d; });
+            __syncwarp();
+            vec[row].x = lse2;
+            mbar_arrive(&bar_vec[n & 1]);
+            const size_t vrow = bh * p.Tpad + q0 + row;
+            p.lse2_w[vrow] = lse2;
+            p.dvec_w[vrow] = vec[row].y;
+            // dQ rows of the item before (times scale) -> BF16 -> global memory
+            ok = mbar_wait_warp(bar_acc, uint32_t(n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+            if (!ok) break;
+            tc_fence_after_sync();
+            const int q_prev = item_qt(id_prev) * 128 + w4 * 32;
+            uint16_t* out = p.dq + q_offset(id_prev) + size_t(q_prev) * p.q_st;
+#pragma unroll
+            for (int c = 0; c < D / 32; ++c) {
+                uint32_t v[32], w[16];
+                tmem_ld_x32(tmem + (uint32_t(w4 * 32) << 16) + Cfg::kColAcc + c * 32, v);
+                tmem_wait_ld();
+                if (c + 1 == D / 32) {
+                    tc_fence_before_sync();
+                    mbar_arrive(bar_acc_free);  // the MMA warp may start the next item's accumulation
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(__uint_as_float(v[2 * i]) * p.scale, __uint_as_float(v[2 * i + 1]) * p.scale);
+                store_rows_64b(sOut + w4 * kRowStageBytes, w, lane, out + c * 32, p.q_st, p.T - q_prev);
+            }
+            id_prev = id;
         }
     } else {
         // ------------------------------------------------------------------ compute
@@ -798,107 +905,93 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         const int row = w4 * 32 + lane;  // query row in the tile == TMEM lane
         const uint32_t lane_base = uint32_t(w4 * 32) << 16;
         const int c0 = half * 64 + part * 32;  // first key column of this thread
-        float lse2 = INFINITY, dv = 0.f;
-        {
-            // preprocess D = rowsum(O * dO): the four warps that share 32 rows take 8 each
-            constexpr int LPR = D / 8, RPP = 32 / LPR;
-            const size_t tile_off = size_t(b) * p.q_sb + size_t(h) * p.q_sh;
-            const int r0 = w4 * 32 + (warp >> 2) * 8;
-            const float lse_raw = q0 + row < p.T ? p.lse[(size_t(b) * p.Hq + h) * p.T + q0 + row] : INFINITY;
+        const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2);
+        bool ok = true;
+        int g = 0, n = 0, id_last = -1;
+        for (int id; ok && (id = get_item(n)) >= 0; ++n) {
+            const int qt = item_qt(id), n_kv = item_nkv(id), q0 = qt * 128;
+            float lse2, dv;
+            if (n == 0) {
+                // preprocess D = rowsum(O * dO) of the first item: the four warps that share 32 rows take 8 each
+                const size_t bh = size_t(item_b(id)) * p.Hq + item_h(id);
+                const float lse_raw = q0 + row < p.T ? p.lse[bh * p.T + q0 + row] : INFINITY;
+                dq_wide_row_sums<D, 4>(p, q_offset(id), q0, w4 * 32 + (warp >> 2) * 8, lane, [&](int r, float d) { sD[r] = d; });
+                lse2 = lse_raw * 1.4426950408889634f;
+                named_bar_sync(1, Cfg::kComputeThreads);
+                dv = sD[row];
+                if (warp < 4) {
+                    const size_t vrow = bh * p.Tpad + q0 + row;
+                    p.lse2_w[vrow] = lse2;
+                    p.dvec_w[vrow] = dv;
+                }
+            } else {
+                ok = mbar_wait_warp(&bar_vec[n & 1], uint32_t((n - 1) >> 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+                if (!ok) break;
+                const float2 vec = sVec[(n & 1) * 128 + row];
+                lse2 = vec.x, dv = vec.y;
+            }
+            const uint64_t neg_l2 = pack_f32x2(-lse2, -lse2), neg_d2 = pack_f32x2(-dv, -dv);
+            for (int j = 0; j < n_kv; ++j, ++g) {
+                ok = mbar_wait_warp(&bar_s_full[half], uint32_t(g) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+                if (!ok) break;
+                tc_fence_after_sync();
+                // phase A: P from S (the scores leave tensor memory in one go)
+                float pr[32];
+                {
+                    uint32_t sv[32];
+                    tmem_ld_x32(tmem + lane_base + Cfg::kColS + c0, sv);
+                    tmem_wait_ld();
+                    tc_fence_before_sync();
+                    mbar_arrive(&bar_s_loaded[half]);
 #pragma unroll
-            for (int i = 0; i < 8 / RPP; ++i) {
-                const int r = r0 + i * RPP + lane / LPR;
-                float acc = 0.f;
-                if (q0 + r < p.T) {
-                    const size_t off = tile_off + size_t(q0 + r) * p.q_st + (lane % LPR) * 8;
-                    const uint4 a = *reinterpret_cast<const uint4*>(p.o + off);
-                    const uint4 g = *reinterpret_cast<const uint4*>(p.dout + off);
-                    const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
-                    const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        acc = fmaf(__uint_as_float(aw[e] << 16), __uint_as_float(gw[e] << 16), acc);
-                        acc = fmaf(__uint_as_float(aw[e] & 0xffff0000u), __uint_as_float(gw[e] & 0xffff0000u), acc);
+                    for (int i = 0; i < 32; i += 2) {
+                        float x0, x1;
+                        unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), scale2, neg_l2), x0, x1);
+                        pr[i] = ex2_approx(x0);
+                        pr[i + 1] = ex2_approx(x1);
                     }
                 }
+                if (j == qt) {
 #pragma unroll
-                for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                if (lane % LPR == 0) sD[r] = acc;
-            }
-            lse2 = lse_raw * 1.4426950408889634f;
-            named_bar_sync(1, Cfg::kComputeThreads);
-            dv = sD[row];
-            if (warp < 4) {
-                const size_t vrow = (size_t(b) * p.Hq + h) * p.Tpad + q0 + row;
-                p.lse2_w[vrow] = lse2;
-                p.dvec_w[vrow] = dv;
-            }
-        }
-        bool ok = true;
-        const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), neg_l2 = pack_f32x2(-lse2, -lse2), neg_d2 = pack_f32x2(-dv, -dv);
-        for (int j = 0; j < n_kv && ok; ++j) {
-            ok = mbar_wait_warp(&bar_s_full[half], uint32_t(j) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
-            if (!ok) break;
-            tc_fence_after_sync();
-            // phase A: P from S (the scores leave tensor memory in one go)
-            float pr[32];
-            {
-                uint32_t sv[32];
-                tmem_ld_x32(tmem + lane_base + Cfg::kColS + c0, sv);
-                tmem_wait_ld();
+                    for (int i = 0; i < 32; ++i)
+                        if (c0 + i > row) pr[i] = 0.f;  // key above the diagonal
+                }
+                ok = mbar_wait_warp(&bar_dp_full[half], uint32_t(g) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+                if (!ok) break;
+                tc_fence_after_sync();
+                // phase B: dS = P (dP - D), written as BF16 over the first 16 of the thread's dP columns
+                {
+                    uint32_t dp[32], pk[16];
+                    const uint32_t t_dp = tmem + lane_base + Cfg::kColDP + c0;
+                    tmem_ld_x32(t_dp, dp);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2) {
+                        float y0, y1;
+                        unpack_f32x2(mul_f32x2(pack_f32x2(pr[i], pr[i + 1]),
+                                               add_f32x2(pack_f32x2(__uint_as_float(dp[i]), __uint_as_float(dp[i + 1])), neg_d2)), y0, y1);
+                        pk[i / 2] = pack_bf16x2(y0, y1);
+                    }
+                    tmem_st_x16(t_dp, pk);
+                }
+                tmem_wait_st();
                 tc_fence_before_sync();
-                mbar_arrive(&bar_s_loaded[half]);
-#pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    float x0, x1;
-                    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), scale2, neg_l2), x0, x1);
-                    pr[i] = ex2_approx(x0);
-                    pr[i + 1] = ex2_approx(x1);
-                }
+                mbar_arrive(&bar_ds_full[half]);
             }
-            if (j == qt) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    if (c0 + i > row) pr[i] = 0.f;  // key above the diagonal
-            }
-            ok = mbar_wait_warp(&bar_dp_full[half], uint32_t(j) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
-            if (!ok) break;
-            tc_fence_after_sync();
-            // phase B: dS = P (dP - D), written as BF16 over the first 16 of the thread's dP columns
-            {
-                uint32_t dp[32], pk[16];
-                const uint32_t t_dp = tmem + lane_base + Cfg::kColDP + c0;
-                tmem_ld_x32(t_dp, dp);
-                tmem_wait_ld();
-#pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    float y0, y1;
-                    unpack_f32x2(mul_f32x2(pack_f32x2(pr[i], pr[i + 1]),
-                                           add_f32x2(pack_f32x2(__uint_as_float(dp[i]), __uint_as_float(dp[i + 1])), neg_d2)), y0, y1);
-                    pk[i / 2] = pack_bf16x2(y0, y1);
-                }
-                tmem_st_x16(t_dp, pk);
-            }
-            tmem_wait_st();
-            tc_fence_before_sync();
-            mbar_arrive(&bar_ds_full[half]);
+            id_last = id;
         }
-        if (ok) ok = mbar_wait_warp(bar_acc, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
-        if (ok) {
+        if (ok && n > 0) ok = mbar_wait_warp(bar_acc, uint32_t(n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+        if (ok && n > 0) {
+            // dQ rows of the last item through the ring, which nothing reads or loads any more
             tc_fence_after_sync();
-            uint32_t v[32];
+            uint32_t v[32], w[16];
             tmem_ld_x32(tmem + lane_base + Cfg::kColAcc + c0, v);
             tmem_wait_ld();
-            stage_row_chunk<D>(sQ, row, c0, v, p.scale);
-            fence_proxy_async_smem();
-        }
-        tc_fence_before_sync();
-        named_bar_sync(1, Cfg::kComputeThreads);
-        if (ok && tid == 0) {
+            tc_fence_before_sync();
 #pragma unroll
-            for (int bx = 0; bx < Cfg::kBoxes; ++bx) tma_store_4d(&tmdQ, sQ + bx * Cfg::kBoxBytes, bx * 64, q0, h, b);
-            tma_store_commit();
-            tma_store_wait_read0();
+            for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(__uint_as_float(v[2 * i]) * p.scale, __uint_as_float(v[2 * i + 1]) * p.scale);
+            const int q0 = item_qt(id_last) * 128 + w4 * 32;
+            store_rows_64b(smem + warp * kRowStageBytes, w, lane, p.dq + q_offset(id_last) + size_t(q0) * p.q_st + c0, p.q_st, p.T - q0);
         }
     }
 

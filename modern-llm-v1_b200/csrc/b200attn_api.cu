@@ -443,12 +443,12 @@ int launch_bwd_onepass(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
     return B200ATTN_OK;
 }
 
-// own: what the dQ pass alone reads or writes through TMA.  D = 64: K and V in boxes of 64 rows, and O; D = 128: dQ.
+// own: what the dQ pass at D = 64 alone reads through TMA: K and V in boxes of 64 rows, and O.
 template <int D>
 int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap (&own)[3],
                const BwdParams& p, cudaStream_t st) {
     static bool dq_set[kMaxDevices] = {false}, dkdv_set[kMaxDevices] = {false};
-    // D = 64: 64-key tiles, two CTAs per SM.  D = 128: 128-key tiles, one CTA per SM (tensor-pipe bound).
+    // D = 64: 64-key tiles.  D = 128: 128-key tiles (tensor-pipe bound).
     constexpr bool kWide = (D == 128);
     int rc;
     if constexpr (kWide) rc = set_smem_once(attn_bwd_dq_wide_kernel<D>, DqWideCfg<D>::kSmemBytes, dq_set);
@@ -460,16 +460,16 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     // the dQ pass also writes the two per-row vectors the dK/dV pass reads
     const unsigned dq_items = (unsigned)(p.n_tiles * p.Hq * p.B);
     cudaError_t e;
-    if constexpr (kWide) {
-        e = launch_pdl(attn_bwd_dq_wide_kernel<D>, dq_items, DqWideCfg<D>::kThreads, DqWideCfg<D>::kSmemBytes, st, tq, tk, tv, tdo, own[0], p);
-    } else {
-        // the D = 64 kernel is persistent: two CTAs per SM walk the item list
-        const unsigned dq_grid = std::min(dq_items, 2u * (unsigned)sm_count());
-        BwdParams pq = p;
-        pq.sched = next_sched_pair(dq_items, dq_grid);
-        e = launch_pdl(attn_bwd_dq_kernel<D>, dq_grid, DqCfg<D>::kThreads, DqCfg<D>::kSmemBytes, st, tq, own[0], own[1], tdo, own[2], pq,
-                       item_table_for(pq.sched ? -1 : (long long)dq_items, dq_grid, p.B * p.Hq, p.n_tiles, p.T, 4));
-    }
+    // It is persistent: two CTAs per SM at D = 64, one at D = 128, walk the item list.
+    const unsigned dq_grid = std::min(dq_items, (kWide ? 1u : 2u) * (unsigned)sm_count());
+    BwdParams pq = p;
+    pq.sched = next_sched_pair(dq_items, dq_grid);
+    // (no table where every CTA has one item: one line of constants less in front of its first load)
+    const ItemTable& tab = item_table_for(pq.sched || dq_items <= dq_grid ? -1 : (long long)dq_items, dq_grid, p.B * p.Hq, p.n_tiles, p.T, 4);
+    if constexpr (kWide)
+        e = launch_pdl(attn_bwd_dq_wide_kernel<D>, dq_grid, DqWideCfg<D>::kThreads, DqWideCfg<D>::kSmemBytes, st, tq, tk, tv, tdo, pq, tab);
+    else
+        e = launch_pdl(attn_bwd_dq_kernel<D>, dq_grid, DqCfg<D>::kThreads, DqCfg<D>::kSmemBytes, st, tq, own[0], own[1], tdo, own[2], pq, tab);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return B200ATTN_ERR_CUDA;
@@ -754,8 +754,6 @@ extern "C" int b200attn_bwd_mode(const void* q, const void* k, const void* v, co
         maps = maps && make_tmap_bf16_4d(&own[0], k, D, T, Hkv, B, sk.t, sk.h, sk.b, 64) &&
                make_tmap_bf16_4d(&own[1], v, D, T, Hkv, B, sk.t, sk.h, sk.b, 64) &&
                make_tmap_bf16_4d(&own[2], o, D, T, Hq, B, sq.t, sq.h, sq.b, 128);
-    else if (mode == B200ATTN_BWD_TWO_PASS)
-        maps = maps && make_tmap_bf16_4d(&own[0], dq, D, T, Hq, B, sq.t, sq.h, sq.b, 128);
     if (!maps) return B200ATTN_ERR_TENSOR_MAP;
     float* ws = static_cast<float*>(workspace);
     const size_t nvec = bwd_vec_elems(B, T, Hq);

@@ -117,17 +117,6 @@ __device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_
                  "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
-__device__ __forceinline__ void tma_store_4d(const CUtensorMap* m, const void* src, int c0, int c1, int c2, int c3) {
-    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(
-                     reinterpret_cast<uint64_t>(m)),
-                 "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-                 : "memory");
-}
-__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// Waits until the bulk stores of this thread have finished READING shared memory.
-__device__ __forceinline__ void tma_store_wait_read0() {
-    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
 
 // ---------------------------------------------------------------------------
 // TMEM allocation (one warp, converged).
