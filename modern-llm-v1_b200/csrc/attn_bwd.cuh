@@ -215,6 +215,20 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     auto get_item = [&](int n) { return item_get(bar_item, item_ring, n, abort_flag, p.status); };
 
     B200ATTN_TRACE_BEGIN(1);
+    const int id_first = sched_first(tab, p.sched, int(blockIdx.x));  // the first item needs no fetch
+    // one thread: Q, dO and O of an item; a tile of K and V
+    auto load_rows = [&](int id) {
+        const int q0 = item_qt(id) * 128, h = item_h(id), b = item_b(id);
+        mbar_arrive_expect_tx(bar_q, 3 * Cfg::kQTileBytes);
+        tma_load_4d(sQ, &tmQ, bar_q, 0, q0, h, b);
+        tma_load_4d(sdO, &tmdO, bar_q, 0, q0, h, b);
+        tma_load_4d(sO, &tmO, bar_q, 0, q0, h, b);
+    };
+    auto load_kv = [&](int s, int j, int hk, int b) {
+        mbar_arrive_expect_tx(&bar_kv_full[s], 2 * Cfg::kKVTileBytes);
+        tma_load_4d(sK + s * Cfg::kKVTileBytes, &tmK, &bar_kv_full[s], 0, j * Cfg::kKeys, hk, b);
+        tma_load_4d(sV + s * Cfg::kKVTileBytes, &tmV, &bar_kv_full[s], 0, j * Cfg::kKeys, hk, b);
+    };
     if (warp == Cfg::kProducerWarp && lane == 0) {
         tma_prefetch_desc(&tmQ);
         tma_prefetch_desc(&tmK);
@@ -237,8 +251,25 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
         for (int i = 0; i < kItemRing; ++i) mbar_init(&bar_item[i], 1);
         fence_mbar_init();
+        *abort_flag = 0;
+        item_publish(bar_item, item_ring, 0, id_first);
+    }
+    if (warp == Cfg::kProducerWarp) {
+        __syncwarp();
         grid_dep_wait();  // first global access of this CTA comes next
-        *abort_flag = *reinterpret_cast<volatile int*>(p.status);
+        // The first loads: the status word, the barrier and the roles' start pass under their latency (both passes, us: B=32 T=512 6/2 44.9 -> 44.2,
+        // at D = 128 B=20 T=200 8/4 33.6 -> 32.6).
+        if (elect_one()) {
+            load_rows(id_first);
+            load_kv(0, 0, int(fastdiv(unsigned(item_h(id_first)), p.div_group)), item_b(id_first));
+            const int failed = *reinterpret_cast<volatile int*>(p.status);
+            if (failed != 0) {  // behind an earlier failure the CTA leaves, but not before its loads have landed
+                mbar_wait(bar_q, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+                mbar_wait(&bar_kv_full[0], 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+                *abort_flag = failed;
+            }
+        }
+        __syncwarp();
     }
     if (warp == Cfg::kMmaWarp) {
         tmem_alloc(tmem_slot, Cfg::kTmemCols);
@@ -260,15 +291,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         reg_dealloc<Cfg::kRegsOther>();
         int g = 0;  // tiles issued so far by this CTA (ring position)
         bool ok = true;
-        int id = sched_first(tab, p.sched, int(blockIdx.x));  // the first item needs no fetch
+        int id = id_first;
         int id_next = 0;      // lane 0: the id fetched for the next item
-        if (lane == 0) {
-            item_publish(bar_item, item_ring, 0, id);
-            id_next = sched_fetch(tab, p.sched, 1, int(blockIdx.x), int(gridDim.x));
-        }
+        if (lane == 0) id_next = sched_fetch(tab, p.sched, 1, int(blockIdx.x), int(gridDim.x));
         __syncwarp();
         for (int n = 0; ok; ++n) {
-            const int qt = item_qt(id), h = item_h(id), b = item_b(id), hk = int(fastdiv(unsigned(h), p.div_group)), n_kv = item_nkv(id);
+            const int h = item_h(id), b = item_b(id), hk = int(fastdiv(unsigned(h), p.div_group)), n_kv = item_nkv(id);
             // the next item is taken and announced shortly before this item's loads end, but not before the
             // ring has been filled for this item
             const int j_next = max(min(n_kv, NST) - 1, n_kv - 2);
@@ -276,22 +304,13 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             // the three tiles in shared memory are free as soon as the previous item has been copied out of them
             if (n > 0) ok = mbar_wait_warp(bar_qs_free, (n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
             if (!ok) break;
-            if (elect_one()) {
-                mbar_arrive_expect_tx(bar_q, 3 * Cfg::kQTileBytes);
-                tma_load_4d(sQ, &tmQ, bar_q, 0, qt * 128, h, b);
-                tma_load_4d(sdO, &tmdO, bar_q, 0, qt * 128, h, b);
-                tma_load_4d(sO, &tmO, bar_q, 0, qt * 128, h, b);
-            }
+            if (n > 0 && elect_one()) load_rows(id);
             __syncwarp();
             for (int j = 0; j < n_kv; ++j, ++g) {
                 const int s = g % NST;
                 if (g >= NST) ok = mbar_wait_warp(&bar_kv_free[s], ((g / NST) - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
                 if (!ok) break;
-                if (elect_one()) {
-                    mbar_arrive_expect_tx(&bar_kv_full[s], 2 * Cfg::kKVTileBytes);
-                    tma_load_4d(sK + s * Cfg::kKVTileBytes, &tmK, &bar_kv_full[s], 0, j * Cfg::kKeys, hk, b);
-                    tma_load_4d(sV + s * Cfg::kKVTileBytes, &tmV, &bar_kv_full[s], 0, j * Cfg::kKeys, hk, b);
-                }
+                if (g > 0 && elect_one()) load_kv(s, j, hk, b);
                 __syncwarp();
                 if (j == j_next) {
                     id_new = __shfl_sync(0xffffffffu, id_next, 0);
@@ -679,6 +698,17 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     auto q_offset = [&](int id) { return size_t(item_b(id)) * p.q_sb + size_t(item_h(id)) * p.q_sh; };
 
     B200ATTN_TRACE_BEGIN(1);
+    const int id_first = sched_first(tab, p.sched, int(blockIdx.x));  // the first item needs no fetch
+    // one thread: ring entry e
+    auto load = [&](int e, const CUtensorMap* ma, const CUtensorMap* mb, int row, int head, int b) {
+        uint64_t* full = &bar_full[e % NST];
+        mbar_arrive_expect_tx(full, 2 * Cfg::kTileBytes);
+#pragma unroll
+        for (int bx = 0; bx < Cfg::kBoxes; ++bx) {
+            tma_load_4d(place_a(e) + bx * Cfg::kBoxBytes, ma, full, bx * 64, row, head, b);
+            tma_load_4d(place_b(e) + bx * Cfg::kBoxBytes, mb, full, bx * 64, row, head, b);
+        }
+    };
     if (warp == kProducerWarp && lane == 0) {
         tma_prefetch_desc(&tmQ);
         tma_prefetch_desc(&tmK);
@@ -699,9 +729,24 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         }
         for (int i = 0; i < kItemRing; ++i) mbar_init(&bar_item[i], 1);
         fence_mbar_init();
+        *abort_flag = 0;
+        item_publish(bar_item, item_ring, 0, id_first);
+    }
+    if (warp == kProducerWarp) {
+        __syncwarp();
         // launched with programmatic stream serialization: wait for the previous kernel before any global access
         grid_dep_wait();
-        *abort_flag = *reinterpret_cast<volatile int*>(p.status);
+        if (elect_one()) {  // the first loads: the status word, the barrier and the roles' start pass under their latency
+            const int h = item_h(id_first), b = item_b(id_first);
+            load(0, &tmQ, &tmdO, item_qt(id_first) * 128, h, b);
+            load(1, &tmK, &tmV, 0, int(fastdiv(unsigned(h), p.div_group)), b);
+            const int failed = *reinterpret_cast<volatile int*>(p.status);
+            if (failed != 0) {  // behind an earlier failure the CTA leaves, but not before its loads have landed
+                for (int e = 0; e < 2; ++e) mbar_wait(&bar_full[e], 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+                *abort_flag = failed;
+            }
+        }
+        __syncwarp();
     }
     if (warp == kMmaSWarp) {
         tmem_alloc(tmem_slot, Cfg::kTmemCols);
@@ -720,25 +765,14 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         // ------------------------------------------------------------------ producer (whole warp, one lane issues)
         int e = 0;  // ring entries issued so far by this CTA
         bool ok = true;
-        int id = sched_first(tab, p.sched, int(blockIdx.x));  // the first item needs no fetch
+        int id = id_first;
         int id_next = 0;  // lane 0: the id fetched for the next item
-        if (lane == 0) {
-            item_publish(bar_item, item_ring, 0, id);
-            id_next = sched_fetch(tab, p.sched, 1, int(blockIdx.x), int(gridDim.x));
-        }
+        if (lane == 0) id_next = sched_fetch(tab, p.sched, 1, int(blockIdx.x), int(gridDim.x));
         __syncwarp();
-        auto load = [&](const CUtensorMap* ma, const CUtensorMap* mb, int row, int head, int b) {
+        auto next_entry = [&](const CUtensorMap* ma, const CUtensorMap* mb, int row, int head, int b) {
             if (e >= NST) ok = mbar_wait_warp(&bar_free[e % NST], uint32_t(e / NST - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
             if (!ok) return;
-            if (elect_one()) {
-                uint64_t* full = &bar_full[e % NST];
-                mbar_arrive_expect_tx(full, 2 * Cfg::kTileBytes);
-#pragma unroll
-                for (int bx = 0; bx < Cfg::kBoxes; ++bx) {
-                    tma_load_4d(place_a(e) + bx * Cfg::kBoxBytes, ma, full, bx * 64, row, head, b);
-                    tma_load_4d(place_b(e) + bx * Cfg::kBoxBytes, mb, full, bx * 64, row, head, b);
-                }
-            }
+            if (e >= 2 && elect_one()) load(e, ma, mb, row, head, b);  // (the first two are under way)
             __syncwarp();
             ++e;
         };
@@ -748,9 +782,9 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
             // ring has been filled for this item
             const int j_next = max(min(n_kv, NST - 1) - 1, n_kv - 2);
             int id_new = n_items;
-            load(&tmQ, &tmdO, item_qt(id) * 128, h, b);
+            next_entry(&tmQ, &tmdO, item_qt(id) * 128, h, b);
             for (int j = 0; j < n_kv && ok; ++j) {
-                load(&tmK, &tmV, j * 128, hk, b);
+                next_entry(&tmK, &tmV, j * 128, hk, b);
                 if (ok && j == j_next) {
                     id_new = __shfl_sync(0xffffffffu, id_next, 0);
                     if (lane == 0) {

@@ -147,7 +147,25 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
     B200ATTN_TRACE_BEGIN(0);
     // Set-up with one CTA-wide barrier: one lane of the producer warp initialises every mbarrier while
-    // the MMA warp allocates TMEM; nothing touches global memory before grid_dep_wait().
+    // the MMA warp allocates TMEM; nothing touches global memory before grid_dep_wait().  The first item's Q and its first K and V
+    // are requested at once then, so that the status word, the barrier and the roles' start pass under their latency (requested by
+    // the producer's role behind the barrier, us: B=2 T=128 6/2 D=64 5.07 instead of 4.75, B=32 T=512 6/2 19.4 instead of 18.4, B=2 T=128 D=128
+    // 6.1 instead of 5.8, B=32 T=1001 1/1 D=128 18.9 instead of 18.7).
+    const int id_first = SPLIT ? split_id : sched_first(tab, p.sched, int(blockIdx.x));  // the first item needs no fetch
+    const bool any = !SPLIT || item_nkv(id_first) > 0;
+    auto load_q = [&](int n, int id) {  // one thread: Q of this CTA's n-th item into Q buffer n % NQB
+        mbar_arrive_expect_tx(&bar_q[n % NQB], Cfg::kQTileBytes);
+#pragma unroll
+        for (int bx = 0; bx < Cfg::kBoxes; ++bx)
+            tma_load_4d(bx + 1 < Cfg::kBoxes ? sQ : sQb + (n % NQB) * Cfg::kQBoxBytes, &tmQ, &bar_q[n % NQB], bx * 64, item_qt(id) * 128,
+                        item_h(id), item_b(id));
+    };
+    auto load_kv = [&](uint8_t* tile, const CUtensorMap* map, uint64_t* full, int j, int hk, int b) {  // one thread
+        mbar_arrive_expect_tx(full, Cfg::kKVTileBytes);
+#pragma unroll
+        for (int bx = 0; bx < Cfg::kBoxes; ++bx)
+            tma_load_4d(tile + bx * Cfg::kKVBoxBytes, map, full, bx * 64, (j_first + j) * Cfg::kKeys, hk, b);
+    };
     if (warp == 4 && lane == 0) {
         tma_prefetch_desc(&tmQ);
         tma_prefetch_desc(&tmK);
@@ -170,8 +188,27 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         for (int i = 0; i < kItemRing; ++i) mbar_init(&bar_item[i], 1);
         fence_mbar_init();
+        *abort_flag = 0;
+        item_publish(bar_item, item_ring, 0, any ? id_first : -1);
+    }
+    if (warp == 4) {
+        __syncwarp();
         grid_dep_wait();  // first global access of this CTA comes next
-        *abort_flag = *reinterpret_cast<volatile int*>(p.status);
+        if (elect_one()) {
+            if (any) {
+                const int b = item_b(id_first), hk = int(fastdiv(unsigned(item_h(id_first)), p.div_group));
+                load_q(0, id_first);
+                load_kv(sK, &tmK, &bar_k_full[0], 0, hk, b);
+                load_kv(sV, &tmV, &bar_v_full[0], 0, hk, b);
+            }
+            const int failed = *reinterpret_cast<volatile int*>(p.status);
+            if (failed != 0) {  // behind an earlier failure the CTA leaves, but not before its loads have landed
+                for (uint64_t* bar : {bar_q, bar_k_full, bar_v_full})
+                    if (any) mbar_wait(bar, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
+                *abort_flag = failed;
+            }
+        }
+        __syncwarp();
     }
     if (warp == 5) {
         tmem_alloc(tmem_slot, Cfg::kTmemCols);
@@ -193,32 +230,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         int g = 0;  // key tiles issued so far by this CTA (ring position)
         bool ok = true;
         int id_next = 0;  // lane 0: the id fetched for the item after the next Q load
-        // Q of this CTA's n-th item (item id `id`) into Q buffer n % NQB
-        auto load_q = [&](int n, int id) {
-            const int qb = n % NQB;
+        // waits for Q buffer n % NQB and requests Q of the n-th item
+        auto next_q = [&](int n, int id) {
             if (n >= NQB)
-                ok = mbar_wait_warp(&bar_q_free[qb], uint32_t(n / NQB - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
-            if (Cfg::kQTmem && n > 0 && ok)  // the item before has left the staging box
+                ok = mbar_wait_warp(&bar_q_free[n % NQB], uint32_t(n / NQB - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
+            if (Cfg::kQTmem && ok)  // the item before has left the staging box
                 ok = mbar_wait_warp(bar_qt_full, uint32_t(n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
             if (!ok) return;
-            if (elect_one()) {
-                mbar_arrive_expect_tx(&bar_q[qb], Cfg::kQTileBytes);
-#pragma unroll
-                for (int bx = 0; bx < Cfg::kBoxes; ++bx)
-                    tma_load_4d(bx + 1 < Cfg::kBoxes ? sQ : sQb + qb * Cfg::kQBoxBytes, &tmQ, &bar_q[qb], bx * 64,
-                                item_qt(id) * 128, item_h(id), item_b(id));
-            }
+            if (elect_one()) load_q(n, id);
             __syncwarp();
         };
-        int id = SPLIT ? split_id : sched_first(tab, p.sched, int(blockIdx.x));  // the first item needs no fetch
-        const bool any = !SPLIT || item_nkv(id) > 0;
-        if (lane == 0) {
-            item_publish(bar_item, item_ring, 0, any ? id : -1);
-            id_next = SPLIT ? n_items : sched_fetch(tab, p.sched, 1, int(blockIdx.x), int(gridDim.x));
-        }
+        int id = id_first;
+        if (lane == 0) id_next = SPLIT ? n_items : sched_fetch(tab, p.sched, 1, int(blockIdx.x), int(gridDim.x));
         __syncwarp();
-        if (any) load_q(0, id);
-        else ok = false;
+        ok = any;
         for (int n = 0; ok; ++n) {
             const int h = item_h(id), b = item_b(id), hk = int(fastdiv(unsigned(h), p.div_group)), n_kv = item_nkv(id);
             // The next item is taken, announced and its Q requested a few tiles before this item's loads end
@@ -231,23 +256,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 const uint32_t use = uint32_t(g / NST);
                 if (g >= NST) ok = mbar_wait_warp(&bar_k_free[s], (use - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
                 if (!ok) break;
-                if (elect_one()) {
-                    mbar_arrive_expect_tx(&bar_k_full[s], Cfg::kKVTileBytes);
-#pragma unroll
-                    for (int bx = 0; bx < Cfg::kBoxes; ++bx)
-                        tma_load_4d(sK + s * Cfg::kKVTileBytes + bx * Cfg::kKVBoxBytes, &tmK, &bar_k_full[s], bx * 64,
-                                    (j_first + j) * Cfg::kKeys, hk, b);
-                }
+                if (g > 0 && elect_one()) load_kv(sK + s * Cfg::kKVTileBytes, &tmK, &bar_k_full[s], j, hk, b);
                 __syncwarp();
                 if (g >= NST) ok = mbar_wait_warp(&bar_v_free[s], (use - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
                 if (!ok) break;
-                if (elect_one()) {
-                    mbar_arrive_expect_tx(&bar_v_full[s], Cfg::kKVTileBytes);
-#pragma unroll
-                    for (int bx = 0; bx < Cfg::kBoxes; ++bx)
-                        tma_load_4d(sV + s * Cfg::kKVTileBytes + bx * Cfg::kKVBoxBytes, &tmV, &bar_v_full[s], bx * 64,
-                                    (j_first + j) * Cfg::kKeys, hk, b);
-                }
+                if (g > 0 && elect_one()) load_kv(sV + s * Cfg::kKVTileBytes, &tmV, &bar_v_full[s], j, hk, b);
                 __syncwarp();
                 if (j == j_next) {
                     id_new = __shfl_sync(0xffffffffu, id_next, 0);
@@ -257,7 +270,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         if (more) id_next = sched_fetch(tab, p.sched, n + 2, int(blockIdx.x), int(gridDim.x));
                     }
                     __syncwarp();
-                    if (more) load_q(n + 1, id_new);
+                    if (more) next_q(n + 1, id_new);
                     if (!ok) break;
                 }
             }
