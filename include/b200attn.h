@@ -93,7 +93,8 @@ size_t b200attn_bwd_workspace_bytes(int B, int T, int Hq, int Hkv, int D);
  *   (both are bound by shared-memory traffic, which is the same).  Workspace: the two row vectors plus
  *   B * Hq * ceil(T/128)*128 * D * 4 bytes.
  * B200ATTN_BWD_AUTO: TWO_PASS, unless the environment variable B200ATTN_BWD=two_pass|one_pass (read once) says
- *   otherwise.  If the workspace passed is too small for ONE_PASS but holds the two row vectors, AUTO runs TWO_PASS.
+ *   otherwise; sequences of at most 128 tokens may take one launch for all three gradients instead (bit-reproducible, too; it needs
+ *   no workspace but asks for the same).  If the workspace passed is too small for ONE_PASS but holds the two row vectors, AUTO runs TWO_PASS.
  * b200attn_bwd_workspace_bytes_mode gives the size for a mode (for AUTO: of the algorithm AUTO picks).
  */
 enum { B200ATTN_BWD_AUTO = 0, B200ATTN_BWD_TWO_PASS = 1, B200ATTN_BWD_ONE_PASS = 2 };

@@ -624,35 +624,46 @@ struct DqWideCfg {
     static constexpr int kColS = 0, kColDP = 128, kColAcc = 256, kColQ = 384, kColDO = 448;
 };
 
-// D of rows r0 .. r0 + 8 n of a tile from global memory, LPR lanes to a row; `use(r, D)` by the first of them
-template <int D, int PASSES, typename Use>
-__device__ __forceinline__ void dq_wide_row_sums(const BwdParams& p, size_t tile_off, int q0, int r0, int lane, Use use) {
-    constexpr int LPR = D / 8, RPP = 32 / LPR;
+// D = rowsum(O * dO) of PASSES * 256 / D rows of a tile from r0 on, by one warp from global memory, D / 8 lanes to a row
+template <int D, int PASSES>
+struct RowSums {
+    static constexpr int LPR = D / 8, RPP = 32 / LPR;
     uint4 a[PASSES], g[PASSES];
+    __device__ __forceinline__ void load(const BwdParams& p, size_t tile_off, int q0, int r0, int lane) {
 #pragma unroll
-    for (int i = 0; i < PASSES; ++i) {
-        const int r = r0 + i * RPP + lane / LPR;
-        a[i] = g[i] = make_uint4(0u, 0u, 0u, 0u);
-        if (q0 + r < p.T) {
-            const size_t off = tile_off + size_t(q0 + r) * p.q_st + (lane % LPR) * 8;
-            a[i] = *reinterpret_cast<const uint4*>(p.o + off);
-            g[i] = *reinterpret_cast<const uint4*>(p.dout + off);
+        for (int i = 0; i < PASSES; ++i) {
+            const int r = r0 + i * RPP + lane / LPR;
+            a[i] = g[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (q0 + r < p.T) {
+                const size_t off = tile_off + size_t(q0 + r) * p.q_st + (lane % LPR) * 8;
+                a[i] = *reinterpret_cast<const uint4*>(p.o + off);
+                g[i] = *reinterpret_cast<const uint4*>(p.dout + off);
+            }
         }
     }
+    template <typename Use>  // `use(r, D)` by the first lane of a row
+    __device__ __forceinline__ void sum(int r0, int lane, Use use) const {
 #pragma unroll
-    for (int i = 0; i < PASSES; ++i) {
-        const uint32_t aw[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
-        const uint32_t gw[4] = {g[i].x, g[i].y, g[i].z, g[i].w};
-        float acc = 0.f;
+        for (int i = 0; i < PASSES; ++i) {
+            const uint32_t aw[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+            const uint32_t gw[4] = {g[i].x, g[i].y, g[i].z, g[i].w};
+            float acc = 0.f;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            acc = fmaf(__uint_as_float(aw[e] << 16), __uint_as_float(gw[e] << 16), acc);
-            acc = fmaf(__uint_as_float(aw[e] & 0xffff0000u), __uint_as_float(gw[e] & 0xffff0000u), acc);
+            for (int e = 0; e < 4; ++e) {
+                acc = fmaf(__uint_as_float(aw[e] << 16), __uint_as_float(gw[e] << 16), acc);
+                acc = fmaf(__uint_as_float(aw[e] & 0xffff0000u), __uint_as_float(gw[e] & 0xffff0000u), acc);
+            }
+#pragma unroll
+            for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane % LPR == 0) use(r0 + i * RPP + lane / LPR, acc);
         }
-#pragma unroll
-        for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane % LPR == 0) use(r0 + i * RPP + lane / LPR, acc);
     }
+};
+template <int D, int PASSES, typename Use>
+__device__ __forceinline__ void row_sums(const BwdParams& p, size_t tile_off, int q0, int r0, int lane, Use use) {
+    RowSums<D, PASSES> s;
+    s.load(p, tile_off, q0, r0, lane);
+    s.sum(r0, lane, use);
 }
 
 template <int D>
@@ -905,7 +916,7 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
             // barrier for all items a row warp could be an item ahead of another and arrive for both.)
             float2* vec = sVec + (n & 1) * 128;
 #pragma unroll 1
-            for (int r = 0; r < 32; r += 8) dq_wide_row_sums<D, 4>(p, q_offset(id), q0, w4 * 32 + r, lane, [&](int r, float d) { vec[r].y = d; });
+            for (int r = 0; r < 32; r += 8) row_sums<D, 4>(p, q_offset(id), q0, w4 * 32 + r, lane, [&](int r, float d) { vec[r].y = d; });
             __syncwarp();
             vec[row].x = lse2;
             mbar_arrive(&bar_vec[n & 1]);
@@ -949,7 +960,7 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
                 // preprocess D = rowsum(O * dO) of the first item: the four warps that share 32 rows take 8 each
                 const size_t bh = size_t(item_b(id)) * p.Hq + item_h(id);
                 const float lse_raw = q0 + row < p.T ? p.lse[bh * p.T + q0 + row] : INFINITY;
-                dq_wide_row_sums<D, 4>(p, q_offset(id), q0, w4 * 32 + (warp >> 2) * 8, lane, [&](int r, float d) { sD[r] = d; });
+                row_sums<D, 4>(p, q_offset(id), q0, w4 * 32 + (warp >> 2) * 8, lane, [&](int r, float d) { sD[r] = d; });
                 lse2 = lse_raw * 1.4426950408889634f;
                 named_bar_sync(1, Cfg::kComputeThreads);
                 dv = sD[row];

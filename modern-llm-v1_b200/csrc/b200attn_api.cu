@@ -15,6 +15,7 @@
 
 #include "attn_bwd.cuh"
 #include "attn_bwd_onepass.cuh"
+#include "attn_bwd_tile.cuh"
 #include "attn_decode.cuh"
 #include "attn_fwd.cuh"
 #include "kv_cache.cuh"
@@ -398,17 +399,40 @@ inline void record_bwd_event(int i, cudaStream_t st) {
 inline size_t bwd_acc_bytes(int B, int T, int Hq, int D) { return bwd_vec_elems(B, T, Hq) * (size_t)D * sizeof(float); }
 inline size_t bwd_vec_bytes_padded(int B, int T, int Hq) { return (2 * bwd_vec_elems(B, T, Hq) * sizeof(float) + 255) & ~(size_t)255; }
 
-int bwd_resolve_mode(int mode, int B, int T, int Hq, int D) {
+int bwd_forced_mode() {
     static const int forced = [] {
         const char* e = getenv("B200ATTN_BWD");
         return !e ? 0 : (e[0] == 't' ? B200ATTN_BWD_TWO_PASS : (e[0] == 'o' ? B200ATTN_BWD_ONE_PASS : 0));
     }();
+    return forced;
+}
+int bwd_resolve_mode(int mode, int B, int T, int Hq, int D) {
+    const int forced = bwd_forced_mode();
     if (mode == B200ATTN_BWD_AUTO) {
         mode = forced ? forced : B200ATTN_BWD_TWO_PASS;
         if (D != 64) mode = B200ATTN_BWD_TWO_PASS;
         (void)B, (void)T, (void)Hq;
     }
     return mode;
+}
+
+// Whether AUTO takes the kernel for sequences of one tile (attn_bwd_tile.cuh): a CTA per query head, the group's CTAs in a
+// cluster, or a CTA per key/value head that goes through its group.  Measured at T = 128, us, two passes / group / head:
+//   heads without a group, always by head: 20 10.3 / 6.3 / 5.4, 300 21.2 / 20.5 / 18.5, 1500 75 / 72 / 65; D=128 1500 123 / 128 / 113
+//   by head while the clusters run in one round: 40 x 2 (B x group) 11.7 / 9.3 / 9.1, 20 x 4 13.9 / 15.0 / 10.0, 12 x 8 16.0 / 26.5 /
+//     10.8, D=128 30 x 2 14.7 / 14.8 / 12.9, 12 x 8 21.7 / 46 / 16; in two rounds no longer: 37 x 4 15.2 / 15.2 / 19.3, D=128 20.9 / 26 / 30
+//   by group from a tenth of the SMs per head of the group on (fewer CTAs are slower than the two passes' many: 40 x 8 21.3 / 27.3, D=128
+//     38 / 49): 120 x 2 15.8 / 10.5, 60 x 3 14.3 / 12.3, 100 x 4 19.8 / 17.1, 148 x 8 33.5 / 30.7; D=128 120 x 2 23.6 / 19.7, 100 x 4
+//     33.3 / 29.8, 444 x 4 117 / 91, 300 x 8 162 / 151; at D=64 in one round only: 444 x 4 48.6 / 51.0, 300 x 8 66 / 83
+enum BwdTile { kTileNo, kTileGroup, kTileHead };
+BwdTile bwd_tile(int B, int T, int Hq, int Hkv, int D) {
+    if (T > 128) return kTileNo;
+    const int sms = sm_count(), group = Hq / Hkv;
+    const long long items = (long long)B * Hkv, heads = (long long)B * Hq;
+    if (group == 1) return kTileHead;
+    // (clusters of three and more do not fill the last SMs of a GPC)
+    if (group <= BwdTileCfg<64>::kMaxCluster && heads <= sms * (group == 2 ? 1.0 : group <= 4 ? 0.89 : 0.81)) return kTileHead;
+    return items * 10 >= (long long)group * sms && (D == 128 || items <= sms) ? kTileGroup : kTileNo;
 }
 
 // One-pass backward (D = 64): row vectors + cleared accumulator, the fused kernel, accumulator -> dq.
@@ -440,6 +464,25 @@ int launch_bwd_onepass(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
         return B200ATTN_ERR_CUDA;
     }
     record_bwd_event(3, st);
+    return B200ATTN_OK;
+}
+
+// Sequences of one tile: one launch (attn_bwd_tile.cuh).
+template <int D, bool ONE>
+int launch_bwd_tile(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo, const BwdParams& p,
+                    cudaStream_t st) {
+    using Cfg = BwdTileCfg<D>;
+    static bool set[kMaxDevices] = {false};
+    if (int rc = set_smem_once(attn_bwd_tile_kernel<D, ONE>, Cfg::kSmemBytes, set)) return rc;
+    record_bwd_event(0, st);
+    const cudaError_t e = launch_cluster(attn_bwd_tile_kernel<D, ONE>, dim3((unsigned)(p.B * (ONE ? p.Hq : p.Hkv))), Cfg::kThreads, Cfg::kSmemBytes,
+                                         st, ONE ? p.group : 1, tk, tv, tq, tdo, p);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return B200ATTN_ERR_CUDA;
+    }
+    record_bwd_event(1, st);
+    record_bwd_event(2, st);
     return B200ATTN_OK;
 }
 
@@ -742,6 +785,7 @@ extern "C" int b200attn_bwd_mode(const void* q, const void* k, const void* v, co
         if (!auto_mode) return B200ATTN_ERR_WORKSPACE;
         mode = B200ATTN_BWD_TWO_PASS;
     }
+    const BwdTile tile = auto_mode && bwd_forced_mode() == 0 ? bwd_tile(B, T, Hq, Hkv, D) : kTileNo;
     int* status = status_ptr(&rc);
     if (!status) return rc;
     const Strides sq = strides_for(layout, Hq, T, D), sk = strides_for(layout, Hkv, T, D);
@@ -750,7 +794,7 @@ extern "C" int b200attn_bwd_mode(const void* q, const void* k, const void* v, co
                 make_tmap_bf16_4d(&tk, k, D, T, Hkv, B, sk.t, sk.h, sk.b, 128) &&
                 make_tmap_bf16_4d(&tv, v, D, T, Hkv, B, sk.t, sk.h, sk.b, 128) &&
                 make_tmap_bf16_4d(&tdo, dout, D, T, Hq, B, sq.t, sq.h, sq.b, 128);
-    if (mode == B200ATTN_BWD_TWO_PASS && D == 64)
+    if (mode == B200ATTN_BWD_TWO_PASS && D == 64 && tile == kTileNo)
         maps = maps && make_tmap_bf16_4d(&own[0], k, D, T, Hkv, B, sk.t, sk.h, sk.b, 64) &&
                make_tmap_bf16_4d(&own[1], v, D, T, Hkv, B, sk.t, sk.h, sk.b, 64) &&
                make_tmap_bf16_4d(&own[2], o, D, T, Hq, B, sq.t, sq.h, sq.b, 128);
@@ -792,6 +836,8 @@ extern "C" int b200attn_bwd_mode(const void* q, const void* k, const void* v, co
     p.div_hkv = fastdiv_make((unsigned)Hkv);
     p.div_group = fastdiv_make((unsigned)p.group);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (tile == kTileHead) return D == 64 ? launch_bwd_tile<64, true>(tq, tk, tv, tdo, p, st) : launch_bwd_tile<128, true>(tq, tk, tv, tdo, p, st);
+    if (tile == kTileGroup) return D == 64 ? launch_bwd_tile<64, false>(tq, tk, tv, tdo, p, st) : launch_bwd_tile<128, false>(tq, tk, tv, tdo, p, st);
     if (mode == B200ATTN_BWD_ONE_PASS) {
         float* dq_acc = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + bwd_vec_bytes_padded(B, T, Hq));
         return launch_bwd_onepass(tq, tk, tv, tdo, p, dq_acc, st);
