@@ -51,6 +51,7 @@ struct BwdParams {
     int split;    // dK/dV pass: CTAs (a cluster) that share an item's units; 1 except in the split kernel
     FastDiv div_split;
     FastDiv div_bhq, div_hq, div_bhkv, div_hkv, div_group;  // division by B * Hq, Hq, B * Hkv, Hkv and the group size
+    int early;    // whether the next kernel may start while this one's last items are worked on (see ptx.cuh)
 };
 
 template <int D>
@@ -1252,6 +1253,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             id = id_new;
         }
         if (!SPLIT && ok && lane == 0) sched_finish(p.sched2, int(gridDim.x));
+        if (p.early) grid_dep_launch();
     } else if (warp == kVecWarp) {
         // ------------------------------------------------------------------ row vectors
         // L and D are the same for a whole column of S^T and dP^T, so reading them costs the compute warps 32 shared-memory

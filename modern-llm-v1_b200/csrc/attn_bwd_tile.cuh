@@ -144,6 +144,7 @@ attn_bwd_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
                 prefetch_l2(p.o + size_t(b) * p.q_sb + size_t(h0 + u) * p.q_sh + size_t(i / (D / 64)) * p.q_st + (i % (D / 64)) * 64);
             __syncwarp();
         }
+        if (p.early) grid_dep_launch();
     } else if (warp == Cfg::kMmaWarp) {
         // ------------------------------------------------------------------ MMA issuer (whole warp, one lane issues)
         constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);   // S^T, dP^T: K-major operands

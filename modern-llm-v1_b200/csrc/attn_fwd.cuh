@@ -51,6 +51,7 @@ struct FwdParams {
                        // cover the same tokens; the cached tokens' count when a chunk of new tokens attends over a KV cache)
     int split;         // CTAs (a cluster) that share an item's key tiles; 1 except in the split kernel
     FastDiv div_split;
+    int early;         // whether the next kernel may start while this one's last items are worked on (see ptx.cuh)
     float scale;       // softmax scale
     float scale_log2;  // scale * log2(e)
     float* lse;        // [B, Hq, T]
@@ -278,6 +279,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             id = id_new;
         }
         if (!SPLIT && ok && lane == 0) sched_finish(p.sched, int(gridDim.x));
+        if (p.early) grid_dep_launch();
     } else if (warp == 5) {
         // ------------------------------------------------------------------ MMA issuer
         reg_dealloc<Cfg::kRegsOther>();

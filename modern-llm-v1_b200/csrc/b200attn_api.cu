@@ -243,6 +243,23 @@ int set_smem_once(K kernel, int bytes, bool* done) {
     return B200ATTN_OK;
 }
 
+// The SMs that clusters can have: those of four and eight do not fill the last SMs of a GPC and get 132 and 120 of 148.
+double cluster_slots(int cluster) { return sm_count() * (cluster <= 2 ? 1.0 : cluster <= 4 ? 0.89 : 0.81); }
+
+// Early launch of the next kernel (`early`): a kernel whose CTAs have one item each lets the next one start once their last loads are
+// issued, which hides the 1.3 us from the last CTA's end to the next kernel's first instruction.  The next kernel's CTAs then go to
+// whatever SMs are free, so kernels with room for two CTAs on an SM and no more CTAs than SMs ask for more shared memory than half
+// an SM has (spread_smem): without that they came to lie in pairs (forward and backward, us, released at the end / early / early and
+// spread: B=1 T=1500 8/8 D=64 49.4 / 51.1 / 47.4, B=8 T=128 16/4 D=128 23.0 / 23.3 / 21.8).  Both together: B=2 T=128 6/2 D=64 14.1 ->
+// 13.1, B=11 15.3 -> 14.1, B=36 19.7 -> 18.6, B=2 T=700 8/2 35.7 -> 33.6, D=128 B=1 T=500 6/2 35.3 -> 33.2, B=8 T=512 6/2 45.5 -> 43.7,
+// B=32 T=1001 1/1 60.5 -> 58.8.
+// Not early: kernels with several items per CTA (the next kernel's CTAs, dealt their work in pairs per SM, then share SMs as it happens:
+// forward of B=32 T=512 6/2 D=64 18.3 -> 18.7), clusters beyond one CTA per SM (forward of B=1 T=2000 4/4 D=128 18.0 -> 20.7), a dK/dV
+// pass whose forward has more CTAs than SMs (B=3 T=2000 6/2 D=64 83.3 -> 86.0), and heads in clusters on more than half the SMs
+// (the tile kernel: B=14 T=128 6/2 D=128 20.5 -> 21.2).
+constexpr int kAloneSmemBytes = 114 * 1024;
+inline size_t spread_smem(int bytes, bool one_per_sm) { return one_per_sm ? std::max(bytes, kAloneSmemBytes) : bytes; }
+
 // How many CTAs of a cluster share an item (forward: its key tiles, dK/dV pass: its units): the number with the smallest
 // estimate of the kernel's time, 1 unless another one is at least 5 % better.  Not only few items are split: 126 items of
 // 126 to 2 units on 148 SMs are bound by the longest one (dK/dV at B=1 T=8000 4/2 D=128: 229 -> 134 us).  Held against every
@@ -263,8 +280,7 @@ int pick_split(long long items, int longest, double total, const SplitCosts& c) 
     int best = 1;
     double best_us = 1e30;
     for (int split = 1; split <= 8; split *= 2) {
-        // clusters of four and eight do not fill the last SMs of a GPC: they get 132 and 120 of 148
-        const double slots = c.per_sm * (split <= 2 ? sms : split == 4 ? sms * 0.89 : sms * 0.81), ctas = (double)items * split;
+        const double slots = c.per_sm * cluster_slots(split), ctas = (double)items * split;
         const double shared = c.per_sm > 1 ? std::min(1.0, std::max(0.0, ctas / sms - 1)) : 0.0;  // SMs with two CTAs
         const double share = (longest + split - 1) / split * (c.tile_one + (c.tile_all - c.tile_one) * shared);
         const double all = total * c.tile_all / slots;
@@ -282,6 +298,14 @@ double fwd_total_tiles(int n_qtiles, int kv_off, int T, int keys) {
     return n_qtiles * (first + last) / 2;
 }
 
+// CTAs (a cluster) that share an item of the forward
+template <int D>
+int fwd_split(int B, int Hq, int T, int kv_off, int n_qtiles) {
+    constexpr int keys = FwdCfg<D>::kKeys;
+    constexpr SplitCosts kCosts = D == 64 ? SplitCosts{2, 1.25f, 1.95f, 2.f, 3.5f} : SplitCosts{2, 0.83f, 1.f, 3.5f, 3.5f};
+    return pick_split((long long)n_qtiles * Hq * B, (kv_off + T + keys - 1) / keys, (double)B * Hq * fwd_total_tiles(n_qtiles, kv_off, T, keys), kCosts);
+}
+
 template <int D>
 int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p,
                cudaStream_t st) {
@@ -291,24 +315,25 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     pl.div_bh = fastdiv_make((unsigned)(p.B * p.Hq));
     pl.div_h = fastdiv_make((unsigned)p.Hq);
     pl.div_group = fastdiv_make((unsigned)p.group);
-    constexpr SplitCosts kCosts = D == 64 ? SplitCosts{2, 1.25f, 1.95f, 2.f, 3.5f} : SplitCosts{2, 0.83f, 1.f, 3.5f, 3.5f};
-    pl.split = pick_split(items, (p.kv_off + p.T + Cfg::kKeys - 1) / Cfg::kKeys, (double)p.B * p.Hq * fwd_total_tiles(p.n_qtiles, p.kv_off, p.T, Cfg::kKeys), kCosts);
+    pl.split = fwd_split<D>(p.B, p.Hq, p.T, p.kv_off, p.n_qtiles);
     pl.div_split = fastdiv_make((unsigned)pl.split);
     cudaError_t e;
     if (pl.split > 1) {
         static bool set[kMaxDevices] = {false};
-        if (int rc = set_smem_once(attn_fwd_kernel<D, true>, Cfg::kSmemBytes, set)) return rc;
+        if (int rc = set_smem_once(attn_fwd_kernel<D, true>, std::max(Cfg::kSmemBytes, kAloneSmemBytes), set)) return rc;
         pl.sched = nullptr;
-        e = launch_cluster(attn_fwd_kernel<D, true>, dim3((unsigned)(items * pl.split)), 256, Cfg::kSmemBytes, st, pl.split, tq, tk, tv, pl,
+        pl.early = items * pl.split <= cluster_slots(pl.split);
+        e = launch_cluster(attn_fwd_kernel<D, true>, dim3((unsigned)(items * pl.split)), 256, spread_smem(Cfg::kSmemBytes, pl.early), st, pl.split, tq, tk, tv, pl,
                            item_table_for(-1, 1, 1, 1, 1, 1));
     } else {
         static bool set[kMaxDevices] = {false};
-        if (int rc = set_smem_once(attn_fwd_kernel<D, false>, Cfg::kSmemBytes, set)) return rc;
+        if (int rc = set_smem_once(attn_fwd_kernel<D, false>, std::max(Cfg::kSmemBytes, kAloneSmemBytes), set)) return rc;
         // persistent CTAs, two per SM, each walking a heaviest-first list of (query tile, head, batch) items
         const unsigned grid = (unsigned)std::min<long long>(items, 2LL * sm_count());
         pl.sched = next_sched_pair(items, grid);
+        pl.early = items <= grid;
         const ItemTable& tab = item_table_for(pl.sched ? -1 : items, grid, p.B * p.Hq, p.n_qtiles, p.T, 1);
-        e = launch_pdl(attn_fwd_kernel<D, false>, grid, 256, Cfg::kSmemBytes, st, tq, tk, tv, pl, tab);
+        e = launch_pdl(attn_fwd_kernel<D, false>, grid, 256, spread_smem(Cfg::kSmemBytes, grid <= (unsigned)sm_count()), st, tq, tk, tv, pl, tab);
     }
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -475,8 +500,11 @@ int launch_bwd_tile(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensor
     static bool set[kMaxDevices] = {false};
     if (int rc = set_smem_once(attn_bwd_tile_kernel<D, ONE>, Cfg::kSmemBytes, set)) return rc;
     record_bwd_event(0, st);
-    const cudaError_t e = launch_cluster(attn_bwd_tile_kernel<D, ONE>, dim3((unsigned)(p.B * (ONE ? p.Hq : p.Hkv))), Cfg::kThreads, Cfg::kSmemBytes,
-                                         st, ONE ? p.group : 1, tk, tv, tq, tdo, p);
+    const int ctas = p.B * (ONE ? p.Hq : p.Hkv);
+    BwdParams pt = p;
+    pt.early = !ONE || p.group == 1 || 2 * ctas <= sm_count();
+    const cudaError_t e = launch_cluster(attn_bwd_tile_kernel<D, ONE>, dim3((unsigned)ctas), Cfg::kThreads, Cfg::kSmemBytes, st, ONE ? p.group : 1,
+                                         tk, tv, tq, tdo, pt);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return B200ATTN_ERR_CUDA;
@@ -495,7 +523,7 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     constexpr bool kWide = (D == 128);
     int rc;
     if constexpr (kWide) rc = set_smem_once(attn_bwd_dq_wide_kernel<D>, DqWideCfg<D>::kSmemBytes, dq_set);
-    else rc = set_smem_once(attn_bwd_dq_kernel<D>, DqCfg<D>::kSmemBytes, dq_set);
+    else rc = set_smem_once(attn_bwd_dq_kernel<D>, std::max(DqCfg<D>::kSmemBytes, kAloneSmemBytes), dq_set);
     if (rc) return rc;
     rc = set_smem_once(attn_bwd_dkdv_kernel<D, false>, BwdCfg<D>::kSmemBytes, dkdv_set);
     if (rc) return rc;
@@ -512,7 +540,7 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     if constexpr (kWide)
         e = launch_pdl(attn_bwd_dq_wide_kernel<D>, dq_grid, DqWideCfg<D>::kThreads, DqWideCfg<D>::kSmemBytes, st, tq, tk, tv, tdo, pq, tab);
     else
-        e = launch_pdl(attn_bwd_dq_kernel<D>, dq_grid, DqCfg<D>::kThreads, DqCfg<D>::kSmemBytes, st, tq, own[0], own[1], tdo, own[2], pq, tab);
+        e = launch_pdl(attn_bwd_dq_kernel<D>, dq_grid, DqCfg<D>::kThreads, spread_smem(DqCfg<D>::kSmemBytes, dq_grid <= (unsigned)sm_count()), st, tq, own[0], own[1], tdo, own[2], pq, tab);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return B200ATTN_ERR_CUDA;
@@ -525,6 +553,8 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     constexpr SplitCosts kCosts = D == 64 ? SplitCosts{1, 1.4f, 1.4f, 3.f, 3.5f} : SplitCosts{1, 1.9f, 1.9f, 7.f, 3.5f};
     pk.split = pick_split(kv_items, p.group * p.n_tiles, (double)p.B * p.Hq * p.n_tiles * (p.n_tiles + 1) / 2, kCosts);
     pk.div_split = fastdiv_make((unsigned)pk.split);
+    const int fs = fwd_split<D>(p.B, p.Hq, p.T, 0, p.n_tiles);
+    pk.early = (pk.split > 1 || kv_items <= (unsigned)sm_count()) && (long long)dq_items * fs <= cluster_slots(fs);
     if (pk.split > 1) {
         static bool set[kMaxDevices] = {false};
         if ((rc = set_smem_once(attn_bwd_dkdv_kernel<D, true>, BwdCfg<D>::kSmemBytes, set))) return rc;

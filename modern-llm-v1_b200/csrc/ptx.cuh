@@ -188,11 +188,11 @@ __device__ __forceinline__ uint64_t make_sdesc_plain(uint32_t smem_addr, uint32_
 // a dQ pass that writes only dQ and the row vectors, loads K, V and the first Q and dO before
 // that.  grid_dep_launch() is called where the next kernel is short or known: in the dQ pass
 // (after its own wait, so everything older is complete), in the one-pass backward's row-vector
-// kernel, in the decode and in the append of one token.  The other persistent kernels do not call
-// it: all their CTAs start at once, so the call would release the next kernel at this one's very
-// beginning, and a dependent grid queued behind a kernel for its whole run time measured slower
-// (2 %; with grids smaller than the chip, B=2 T=128, 18.6 -> 21.6 us a pass) than one released as
-// the CTAs exit.
+// kernel, in the decode and in the append of one token.  The forward, the dK/dV pass and the
+// backward of one tile call it late, by their producer warps once their last loads are issued, and
+// only where the host says so (`early` in their parameters, see spread_smem in b200attn_api.cu).
+// From their very beginning a dependent grid would be queued behind a kernel for its whole run
+// time, which measured slower (2 %) than one released as the CTAs exit.
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
