@@ -255,8 +255,9 @@ double cluster_slots(int cluster) { return sm_count() * (cluster <= 2 ? 1.0 : cl
 // B=32 T=1001 1/1 60.5 -> 58.8.
 // Not early: kernels with several items per CTA (the next kernel's CTAs, dealt their work in pairs per SM, then share SMs as it happens:
 // forward of B=32 T=512 6/2 D=64 18.3 -> 18.7), clusters beyond one CTA per SM (forward of B=1 T=2000 4/4 D=128 18.0 -> 20.7), a dK/dV
-// pass whose forward has more CTAs than SMs (B=3 T=2000 6/2 D=64 83.3 -> 86.0), and heads in clusters on more than half the SMs
-// (the tile kernel: B=14 T=128 6/2 D=128 20.5 -> 21.2).
+// pass whose forward has more CTAs than SMs (B=3 T=2000 6/2 D=64 83.3 -> 86.0), heads in clusters on more than half the SMs (the tile kernel:
+// B=14 T=128 6/2 D=128 20.5 -> 21.2), and a forward at D = 64 of more than three query tiles and more CTAs than SMs, whose dQ pass shares SMs in
+// pairs of a heavy and a light CTA (B=8 T=512 6/2 34.5 -> 35.3, B=5 T=500 10/10 31.2 -> 32.0; of three, B=16 T=300 6/2, 33.8 -> 32.7).
 constexpr int kAloneSmemBytes = 114 * 1024;
 inline size_t spread_smem(int bytes, bool one_per_sm) { return one_per_sm ? std::max(bytes, kAloneSmemBytes) : bytes; }
 
@@ -331,7 +332,7 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
         // persistent CTAs, two per SM, each walking a heaviest-first list of (query tile, head, batch) items
         const unsigned grid = (unsigned)std::min<long long>(items, 2LL * sm_count());
         pl.sched = next_sched_pair(items, grid);
-        pl.early = items <= grid;
+        pl.early = items <= sm_count() || (items <= grid && (D == 128 || p.n_qtiles <= 3));
         const ItemTable& tab = item_table_for(pl.sched ? -1 : items, grid, p.B * p.Hq, p.n_qtiles, p.T, 1);
         e = launch_pdl(attn_fwd_kernel<D, false>, grid, 256, spread_smem(Cfg::kSmemBytes, grid <= (unsigned)sm_count()), st, tq, tk, tv, pl, tab);
     }
