@@ -48,7 +48,7 @@ struct BwdParams {
     long long k_st, k_sh, k_sb;  // element strides of the k layout: token, head, batch
     int* sched;   // two words of the device-wide item counter of the persistent dQ pass (see ptx.cuh), or nullptr
     int* sched2;  // the same for the dK/dV pass
-    int split;    // dK/dV pass: CTAs (a cluster) that share an item's units; 1 except in the split kernel
+    int split;    // CTAs (a cluster) that share an item's key tiles (dQ pass) or units (dK/dV pass); 1 except in the split kernels
     FastDiv div_split;
     FastDiv div_bhq, div_hq, div_bhkv, div_hkv, div_group;  // division by B * Hq, Hq, B * Hkv, Hkv and the group size
     int early;    // whether the next kernel may start while this one's last items are worked on (see ptx.cuh)
@@ -115,6 +115,79 @@ __device__ __forceinline__ uint64_t mnmajor_desc(const void* tile) {
     return make_sdesc_sw128(smem_u32(tile), BwdCfg<D>::kBoxBytes, 1024);
 }
 
+// The end of an item that a cluster shares (SPLIT): every CTA holds the dQ sums of its key tiles in tensor memory (32 columns from t_acc on
+// per part of the compute warps).  Query row r of the tile is finished by CTA r / rows, which adds the shares up in their order.  The
+// compute warps come here, also after a wait that gave up, and all other warps of the cluster to dq_exchange_idle; the tiles in shared
+// memory make room for the arrivals, so all CTAs must be through with theirs first.  Nobody writes an item of which a CTA has failed.
+__device__ __forceinline__ void dq_exchange_idle(const BwdParams& p, volatile uint32_t* fail, int rank) {
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    if (int(threadIdx.x) < p.split) cluster_store_1(const_cast<uint32_t*>(fail) + rank, threadIdx.x, 1u);  // the CTA left at its start
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+}
+template <int D, typename Begin>
+__device__ __forceinline__ void dq_exchange(const BwdParams& p, uint8_t* smem, volatile uint32_t* fail, const volatile int* abort_flag, uint32_t t_acc,
+                                            int id, int rank, bool any, Begin share_begin) {
+    constexpr int kThreads = 4 * D;  // the compute warps: 128 rows x D / 32 parts
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rows = 128 / p.split;
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    const bool failed = *abort_flag != 0;  // (final: every warp of the CTA has passed the barrier)
+    if (tid < p.split) cluster_store_1(const_cast<uint32_t*>(fail) + rank, tid, failed);
+    __syncwarp();
+    if (tid < kThreads && !failed && any) {
+        tc_fence_after_sync();
+        const int row = (warp & 3) * 32 + lane, part = warp >> 2, to = (row * p.split) >> 7, r = row - to * rows;
+        // [source CTA][row][D] FP32, 16-byte pieces swizzled by the row: the rows of a warp would share a bank
+        uint8_t* own = smem + (rank * rows + r) * D * 4;
+        const uint32_t dst = cluster_addr(own, to);
+        uint32_t v[32];
+        tmem_ld_x32(t_acc + (uint32_t((warp & 3) * 32) << 16) + part * 32, v);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int at = ((part * 8 + i) ^ (r & 7)) << 4;
+            if (to == rank)
+                *reinterpret_cast<uint4*>(own + at) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            else
+                cluster_store_4(dst + at, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        }
+        tc_fence_before_sync();
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    bool good = true;
+    for (int k = 0; k < p.split; ++k) good = good && fail[k] == 0;
+    if (tid < kThreads && good) {
+        const int n_bh = p.B * p.Hq, qt = int(fastdiv(unsigned(id), p.div_bhq)), bh = id - qt * n_bh, b = int(fastdiv(unsigned(bh), p.div_hq));
+        const int q0 = (p.n_tiles - 1 - qt) * 128 + rank * rows;
+        uint16_t* out = p.dq + size_t(b) * p.q_sb + size_t(bh - b * p.Hq) * p.q_sh + size_t(q0) * p.q_st;
+        for (int i = tid; i < rows * (D / 8); i += kThreads) {  // eight columns each
+            const int r = i / (D / 8), c8 = i % (D / 8);
+            if (q0 + r >= p.T) break;
+            float acc[8] = {};
+#pragma unroll 2
+            for (int k = 0; k < p.split; ++k) {
+                if (share_begin(k + 1) == share_begin(k)) continue;  // nothing was sent
+                const uint8_t* src = smem + (k * rows + r) * D * 4;
+                const float4 v0 = *reinterpret_cast<const float4*>(src + (((c8 * 2) ^ (r & 7)) << 4));
+                const float4 v1 = *reinterpret_cast<const float4*>(src + (((c8 * 2 + 1) ^ (r & 7)) << 4));
+                acc[0] += v0.x, acc[1] += v0.y, acc[2] += v0.z, acc[3] += v0.w;
+                acc[4] += v1.x, acc[5] += v1.y, acc[6] += v1.z, acc[7] += v1.w;
+            }
+            *reinterpret_cast<uint4*>(out + size_t(r) * p.q_st + c8 * 8) =
+                make_uint4(pack_bf16x2(acc[0] * p.scale, acc[1] * p.scale), pack_bf16x2(acc[2] * p.scale, acc[3] * p.scale),
+                           pack_bf16x2(acc[4] * p.scale, acc[5] * p.scale), pack_bf16x2(acc[6] * p.scale, acc[7] * p.scale));
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------------------
 // dQ pass (D = 64): persistent CTAs, two per SM.  A CTA walks a list of work items (item = one 128-row query tile
 // of one (batch, query head); items are ordered heaviest first), and every pipeline keeps running across item
@@ -136,6 +209,11 @@ __device__ __forceinline__ uint64_t mnmajor_desc(const void* tile) {
 // T=512 6/2 47.0 -> 45.4 -> 44.7, B=16 T=1024 16/4 163.5 -> 161.0 -> 158.3, B=8 T=2000 16/4 279 -> 275.7 -> 274.5, B=2 T=128 6/2
 // 12.15 -> 12.26 -> 12.06.  dS through shared memory instead of over the dP block, so that the next dP need not wait for dQ, was slower
 // (B=16 T=1024: 168 against 162): the tiles of two CTAs cover that wait already.
+//
+// SPLIT: few, long items (few sequences and heads).  A CTA works on a share of ONE item's key tiles, and the CTAs of a cluster that share it
+// exchange their dQ sums through distributed shared memory at the end (dq_exchange); the sums are in a fixed order, so dQ is
+// bit-reproducible.  What bounds it: the chain of the longest share's tiles, 0.43 us each, and 2 us for the exchange.  At B=1 T=4000 2/1 both
+// passes took 61 us with an item per CTA and take 44.
 //
 // Roles (512 threads): warps 0-7 compute (thread owns query row (warp % 4) * 32 + lane == TMEM lane and the 32 key
 // columns of its part warp / 4), warps 8-11 rows, warp 12 TMA producer, warp 13 TMEM allocation + MMA issue (converged
@@ -171,7 +249,7 @@ struct DqCfg {
     static_assert(kRegsCompute * kComputeThreads + (kRegsRow + kRegsOther) * 128 <= 64 * kThreads, "more registers than the launch has");
 };
 
-template <int D>
+template <int D, bool SPLIT>
 __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -212,11 +290,17 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     auto item_qt = [&](int id) { return p.n_tiles - 1 - int(fastdiv(unsigned(id), p.div_bhq)); };
     auto item_b = [&](int id) { return int(fastdiv(unsigned(item_rest(id)), p.div_hq)); };
     auto item_h = [&](int id) { return item_rest(id) - item_b(id) * p.Hq; };
-    auto item_nkv = [&](int id) { return (min(p.T, item_qt(id) * 128 + 128) + Cfg::kKeys - 1) / Cfg::kKeys; };
+    auto item_all = [&](int id) { return (min(p.T, item_qt(id) * 128 + 128) + Cfg::kKeys - 1) / Cfg::kKeys; };
+    // SPLIT: a CTA's tiles of an item, of cluster CTA r [tiles r / split, tiles (r + 1) / split)
+    const int split_id = SPLIT ? int(fastdiv(blockIdx.x, p.div_split)) : 0, rank = SPLIT ? int(blockIdx.x) - split_id * p.split : 0;
+    auto share_begin = [&](int r) { return int(fastdiv(unsigned(item_all(split_id) * r), p.div_split)); };
+    const int j_first = SPLIT ? share_begin(rank) : 0;
+    auto item_nkv = [&](int id) { return SPLIT ? share_begin(rank + 1) - j_first : item_all(id); };
     auto get_item = [&](int n) { return item_get(bar_item, item_ring, n, abort_flag, p.status); };
 
     B200ATTN_TRACE_BEGIN(1);
-    const int id_first = sched_first(tab, p.sched, int(blockIdx.x));  // the first item needs no fetch
+    const int id_first = SPLIT ? split_id : sched_first(tab, p.sched, int(blockIdx.x));  // the first item needs no fetch
+    const bool any = !SPLIT || item_nkv(id_first) > 0;
     // one thread: Q, dO and O of an item; a tile of K and V
     auto load_rows = [&](int id) {
         const int q0 = item_qt(id) * 128, h = item_h(id), b = item_b(id);
@@ -253,16 +337,16 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         for (int i = 0; i < kItemRing; ++i) mbar_init(&bar_item[i], 1);
         fence_mbar_init();
         *abort_flag = 0;
-        item_publish(bar_item, item_ring, 0, id_first);
+        item_publish(bar_item, item_ring, 0, any ? id_first : -1);
     }
     if (warp == Cfg::kProducerWarp) {
         __syncwarp();
         grid_dep_wait();  // first global access of this CTA comes next
         // The first loads: the status word, the barrier and the roles' start pass under their latency (both passes, us: B=32 T=512 6/2 44.9 -> 44.2,
         // at D = 128 B=20 T=200 8/4 33.6 -> 32.6).
-        if (elect_one()) {
+        if (any && elect_one()) {
             load_rows(id_first);
-            load_kv(0, 0, int(fastdiv(unsigned(item_h(id_first)), p.div_group)), item_b(id_first));
+            load_kv(0, j_first, int(fastdiv(unsigned(item_h(id_first)), p.div_group)), item_b(id_first));
             const int failed = *reinterpret_cast<volatile int*>(p.status);
             if (failed != 0) {  // behind an earlier failure the CTA leaves, but not before its loads have landed
                 mbar_wait(bar_q, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
@@ -283,7 +367,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
 
-    if (*abort_flag != 0) {
+    const bool left = *abort_flag != 0;
+    if (left) {
         // an earlier CTA already failed: fall through to the teardown
     } else if (warp > Cfg::kMmaWarp) {
         reg_dealloc<Cfg::kRegsOther>();  // idle warps
@@ -291,10 +376,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         // ------------------------------------------------------------------ producer
         reg_dealloc<Cfg::kRegsOther>();
         int g = 0;  // tiles issued so far by this CTA (ring position)
-        bool ok = true;
+        bool ok = any;
         int id = id_first;
         int id_next = 0;      // lane 0: the id fetched for the next item
-        if (lane == 0) id_next = sched_fetch(tab, p.sched, 1, int(blockIdx.x), int(gridDim.x));
+        if (lane == 0) id_next = SPLIT ? n_items : sched_fetch(tab, p.sched, 1, int(blockIdx.x), int(gridDim.x));
         __syncwarp();
         for (int n = 0; ok; ++n) {
             const int h = item_h(id), b = item_b(id), hk = int(fastdiv(unsigned(h), p.div_group)), n_kv = item_nkv(id);
@@ -311,7 +396,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 const int s = g % NST;
                 if (g >= NST) ok = mbar_wait_warp(&bar_kv_free[s], ((g / NST) - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
                 if (!ok) break;
-                if (g > 0 && elect_one()) load_kv(s, j, hk, b);
+                if (g > 0 && elect_one()) load_kv(s, j_first + j, hk, b);
                 __syncwarp();
                 if (j == j_next) {
                     id_new = __shfl_sync(0xffffffffu, id_next, 0);
@@ -325,7 +410,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             if (!ok || id_new >= n_items) break;
             id = id_new;
         }
-        if (ok && lane == 0) sched_finish(p.sched, int(gridDim.x));
+        if (!SPLIT && ok && lane == 0) sched_finish(p.sched, int(gridDim.x));
     } else if (warp == Cfg::kMmaWarp) {
         // ------------------------------------------------------------------ MMA issuer
         reg_dealloc<Cfg::kRegsOther>();
@@ -493,8 +578,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             sVec[(n & 1) * 128 + row] = vec;
             mbar_arrive(&bar_vec[n & 1]);
             const size_t vrow = bh * p.Tpad + q0 + row;
-            p.lse2_w[vrow] = vec.x;
-            p.dvec_w[vrow] = vec.y;
+            if (!SPLIT || rank == p.split - 1) {  // (the last share is never empty)
+                p.lse2_w[vrow] = vec.x;
+                p.dvec_w[vrow] = vec.y;
+            }
             // The tiles were read with ordinary loads and will be overwritten by TMA, which works through the async
             // proxy: without this fence the producer's next load, issued the moment the last thread has arrived, may
             // overtake reads that are still in flight (the producer is parked at the barrier whenever the item before
@@ -504,7 +591,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             if (n > 0) epilogue(n - 1, id_prev);
             id_prev = id;
         }
-        if (ok && n > 0) epilogue(n - 1, id_prev);
+        if (!SPLIT && ok && n > 0) epilogue(n - 1, id_prev);
     } else {
         // ------------------------------------------------------------------ compute
         reg_alloc<Cfg::kRegsCompute>();
@@ -542,7 +629,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                         pr[i + 1] = ex2_approx(x1);
                     }
                 }
-                const int kbase = j * Cfg::kKeys;
+                const int kbase = (j_first + j) * Cfg::kKeys;
                 if (kbase + Cfg::kKeys - 1 > q0) {
                     const int lim = q0 + row - kbase - c0;  // columns i <= lim of this part are visible
 #pragma unroll
@@ -575,8 +662,13 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 B200ATTN_STAMP(tid == 0, 240 + 8 * g + 3);
             }
         }
+        if constexpr (SPLIT) {
+            if (ok && n > 0) mbar_wait_warp(bar_acc, 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
+            dq_exchange<D>(p, smem, reinterpret_cast<volatile uint32_t*>(sVec), abort_flag, tmem + Cfg::kColAcc, split_id, rank, any, share_begin);
+        }
     }
 
+    if (SPLIT && (warp >= Cfg::kRowWarp || left)) dq_exchange_idle(p, reinterpret_cast<volatile uint32_t*>(sVec), rank);
     tc_fence_before_sync();
     __syncthreads();
     if (warp == Cfg::kMmaWarp) {
@@ -599,6 +691,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // What bounds it: the tensor pipe inside an item.  Between two items a CTA of its own for each left the pipe idle for 3 us (its
 // start, the preprocess from global memory, Q and dO, K and V, the way out of dQ); now the ring of loads runs on into the next item,
 // whose Q and dO take one place in it, and row warps of their own do the preprocess and the dQ rows, as in the D = 64 kernel.
+// SPLIT as in the D = 64 kernel: the exchange is 64 KB of every CTA, 5.6 us (B=1 T=4000 2/1 77 -> 65 us for both passes).
 // Measured on B200, us for both passes of the backward: B=8 T=512 6/2 39.0 -> 33.6, B=20 T=200 8/4 41.2 -> 33.4, B=8 T=1024 16/4
 // 168 -> 146, B=32 T=1001 1/1 48.2 -> 43.2, B=4 T=2048 16/4 267 -> 245, B=4 T=8192 16/4 3437 -> 3375; one item per CTA: B=2 T=128 6/2
 // 15.7 both, B=1 T=2000 6/2 53.2 -> 53.5.
@@ -667,7 +760,7 @@ __device__ __forceinline__ void row_sums(const BwdParams& p, size_t tile_off, in
     s.sum(r0, lane, use);
 }
 
-template <int D>
+template <int D, bool SPLIT>
 __global__ void __launch_bounds__(DqWideCfg<D>::kThreads, 1)
 attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -705,12 +798,18 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     auto item_qt = [&](int id) { return p.n_tiles - 1 - int(fastdiv(unsigned(id), p.div_bhq)); };
     auto item_b = [&](int id) { return int(fastdiv(unsigned(item_rest(id)), p.div_hq)); };
     auto item_h = [&](int id) { return item_rest(id) - item_b(id) * p.Hq; };
-    auto item_nkv = [&](int id) { return item_qt(id) + 1; };
+    auto item_all = [&](int id) { return item_qt(id) + 1; };
+    // SPLIT: a CTA's tiles of an item, of cluster CTA r [tiles r / split, tiles (r + 1) / split)
+    const int split_id = SPLIT ? int(fastdiv(blockIdx.x, p.div_split)) : 0, rank = SPLIT ? int(blockIdx.x) - split_id * p.split : 0;
+    auto share_begin = [&](int r) { return int(fastdiv(unsigned(item_all(split_id) * r), p.div_split)); };
+    const int j_first = SPLIT ? share_begin(rank) : 0;
+    auto item_nkv = [&](int id) { return SPLIT ? share_begin(rank + 1) - j_first : item_all(id); };
     auto get_item = [&](int n) { return item_get(bar_item, item_ring, n, abort_flag, p.status); };
     auto q_offset = [&](int id) { return size_t(item_b(id)) * p.q_sb + size_t(item_h(id)) * p.q_sh; };
 
     B200ATTN_TRACE_BEGIN(1);
-    const int id_first = sched_first(tab, p.sched, int(blockIdx.x));  // the first item needs no fetch
+    const int id_first = SPLIT ? split_id : sched_first(tab, p.sched, int(blockIdx.x));  // the first item needs no fetch
+    const bool any = !SPLIT || item_nkv(id_first) > 0;
     // one thread: ring entry e
     auto load = [&](int e, const CUtensorMap* ma, const CUtensorMap* mb, int row, int head, int b) {
         uint64_t* full = &bar_full[e % NST];
@@ -742,16 +841,16 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         for (int i = 0; i < kItemRing; ++i) mbar_init(&bar_item[i], 1);
         fence_mbar_init();
         *abort_flag = 0;
-        item_publish(bar_item, item_ring, 0, id_first);
+        item_publish(bar_item, item_ring, 0, any ? id_first : -1);
     }
     if (warp == kProducerWarp) {
         __syncwarp();
         // launched with programmatic stream serialization: wait for the previous kernel before any global access
         grid_dep_wait();
-        if (elect_one()) {  // the first loads: the status word, the barrier and the roles' start pass under their latency
+        if (any && elect_one()) {  // the first loads: the status word, the barrier and the roles' start pass under their latency
             const int h = item_h(id_first), b = item_b(id_first);
             load(0, &tmQ, &tmdO, item_qt(id_first) * 128, h, b);
-            load(1, &tmK, &tmV, 0, int(fastdiv(unsigned(h), p.div_group)), b);
+            load(1, &tmK, &tmV, j_first * 128, int(fastdiv(unsigned(h), p.div_group)), b);
             const int failed = *reinterpret_cast<volatile int*>(p.status);
             if (failed != 0) {  // behind an earlier failure the CTA leaves, but not before its loads have landed
                 for (int e = 0; e < 2; ++e) mbar_wait(&bar_full[e], 0, abort_flag, p.status, DEV_WAIT_TIMEOUT_LOAD);
@@ -771,15 +870,16 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
 
-    if (*abort_flag != 0) {
+    const bool left = *abort_flag != 0;
+    if (left) {
         // an earlier CTA already failed: fall through to the teardown
     } else if (warp == kProducerWarp) {
         // ------------------------------------------------------------------ producer (whole warp, one lane issues)
         int e = 0;  // ring entries issued so far by this CTA
-        bool ok = true;
+        bool ok = any;
         int id = id_first;
         int id_next = 0;  // lane 0: the id fetched for the next item
-        if (lane == 0) id_next = sched_fetch(tab, p.sched, 1, int(blockIdx.x), int(gridDim.x));
+        if (lane == 0) id_next = SPLIT ? n_items : sched_fetch(tab, p.sched, 1, int(blockIdx.x), int(gridDim.x));
         __syncwarp();
         auto next_entry = [&](const CUtensorMap* ma, const CUtensorMap* mb, int row, int head, int b) {
             if (e >= NST) ok = mbar_wait_warp(&bar_free[e % NST], uint32_t(e / NST - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_FREE);
@@ -796,7 +896,7 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
             int id_new = n_items;
             next_entry(&tmQ, &tmdO, item_qt(id) * 128, h, b);
             for (int j = 0; j < n_kv && ok; ++j) {
-                next_entry(&tmK, &tmV, j * 128, hk, b);
+                next_entry(&tmK, &tmV, (j_first + j) * 128, hk, b);
                 if (ok && j == j_next) {
                     id_new = __shfl_sync(0xffffffffu, id_next, 0);
                     if (lane == 0) {
@@ -809,7 +909,7 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
             if (!ok || id_new >= n_items) break;
             id = id_new;
         }
-        if (ok && lane == 0) sched_finish(p.sched, int(gridDim.x));
+        if (!SPLIT && ok && lane == 0) sched_finish(p.sched, int(gridDim.x));
     } else if (warp >= kMmaSWarp) {
         // ------------------------------------------------------------------ MMA issuers (whole warps, one lane issues)
         constexpr uint32_t idesc_s = make_idesc_bf16(128, 64, 0, 0);    // A in TMEM, B (64 rows of the K or V tile) K-major
@@ -908,7 +1008,7 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         const int w4 = warp & 3, row = w4 * 32 + lane;  // query row in the tile == TMEM lane
         bool ok = true;
         int id_prev = get_item(0);
-        for (int n = 1, id; ok && (id = get_item(n)) >= 0; ++n) {
+        for (int n = 1, id; ok && id_prev >= 0 && (id = get_item(n)) >= 0; ++n) {
             // preprocess of the next item
             const int q0 = item_qt(id) * 128;
             const size_t bh = size_t(item_b(id)) * p.Hq + item_h(id);
@@ -965,7 +1065,7 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
                 lse2 = lse_raw * 1.4426950408889634f;
                 named_bar_sync(1, Cfg::kComputeThreads);
                 dv = sD[row];
-                if (warp < 4) {
+                if (warp < 4 && (!SPLIT || rank == p.split - 1)) {  // (the last share is never empty)
                     const size_t vrow = bh * p.Tpad + q0 + row;
                     p.lse2_w[vrow] = lse2;
                     p.dvec_w[vrow] = dv;
@@ -997,7 +1097,7 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
                         pr[i + 1] = ex2_approx(x1);
                     }
                 }
-                if (j == qt) {
+                if (j_first + j == qt) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i)
                         if (c0 + i > row) pr[i] = 0.f;  // key above the diagonal
@@ -1027,7 +1127,7 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
             id_last = id;
         }
         if (ok && n > 0) ok = mbar_wait_warp(bar_acc, uint32_t(n - 1) & 1, abort_flag, p.status, DEV_WAIT_TIMEOUT_MMA);
-        if (ok && n > 0) {
+        if (!SPLIT && ok && n > 0) {
             // dQ rows of the last item through the ring, which nothing reads or loads any more
             tc_fence_after_sync();
             uint32_t v[32], w[16];
@@ -1039,8 +1139,11 @@ attn_bwd_dq_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
             const int q0 = item_qt(id_last) * 128 + w4 * 32;
             store_rows_64b(smem + warp * kRowStageBytes, w, lane, p.dq + q_offset(id_last) + size_t(q0) * p.q_st + c0, p.q_st, p.T - q0);
         }
+        if constexpr (SPLIT)
+            dq_exchange<D>(p, smem, reinterpret_cast<volatile uint32_t*>(sVec), abort_flag, tmem + Cfg::kColAcc, split_id, rank, any, share_begin);
     }
 
+    if (SPLIT && (warp >= kRowWarp || left)) dq_exchange_idle(p, reinterpret_cast<volatile uint32_t*>(sVec), rank);
     tc_fence_before_sync();
     __syncthreads();
     if (warp == kMmaSWarp) {

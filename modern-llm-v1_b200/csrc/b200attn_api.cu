@@ -519,13 +519,10 @@ int launch_bwd_tile(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensor
 template <int D>
 int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap (&own)[3],
                const BwdParams& p, cudaStream_t st) {
-    static bool dq_set[kMaxDevices] = {false}, dkdv_set[kMaxDevices] = {false};
+    static bool dq_set[kMaxDevices] = {false}, dq_split_set[kMaxDevices] = {false}, dkdv_set[kMaxDevices] = {false};
     // D = 64: 64-key tiles.  D = 128: 128-key tiles (tensor-pipe bound).
     constexpr bool kWide = (D == 128);
     int rc;
-    if constexpr (kWide) rc = set_smem_once(attn_bwd_dq_wide_kernel<D>, DqWideCfg<D>::kSmemBytes, dq_set);
-    else rc = set_smem_once(attn_bwd_dq_kernel<D>, std::max(DqCfg<D>::kSmemBytes, kAloneSmemBytes), dq_set);
-    if (rc) return rc;
     rc = set_smem_once(attn_bwd_dkdv_kernel<D, false>, BwdCfg<D>::kSmemBytes, dkdv_set);
     if (rc) return rc;
     record_bwd_event(0, st);
@@ -535,13 +532,32 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     // It is persistent: two CTAs per SM at D = 64, one at D = 128, walk the item list.
     const unsigned dq_grid = std::min(dq_items, (kWide ? 1u : 2u) * (unsigned)sm_count());
     BwdParams pq = p;
-    pq.sched = next_sched_pair(dq_items, dq_grid);
+    // Few, long items are shared by clusters (both passes of the backward, us for 1 / 2 / 4 / 8 CTAs of the dQ pass: B=1 T=4000 2/1 D=64 61.3 / 51.0 /
+    // 44.1 / 52.2, D=128 76.9 / 65.2 / 68.4 / 102; T=2000 6/2 D=64 41.7 / 37.9 / 43.1 / 54.3, D=128 54.1 / 56.0 / 70.1 / 115; T=1000 8/8 D=64 23.4 / 22.6 /
+    // 24.1 / 33.1; T=500 6/2 D=64 18.6 / 19.0 / 18.4 / 19.9, B=2 T=700 8/2 D=64 23.9 / 26.0 / 31.9 / 44.3).
+    constexpr SplitCosts kDqCosts = D == 64 ? SplitCosts{2, 0.43f, 0.6f, 2.f, 4.f} : SplitCosts{1, 1.06f, 1.06f, 5.6f, 4.f};
+    constexpr int kDqKeys = D == 64 ? 64 : 128;
+    pq.split = pick_split(dq_items, (p.T + kDqKeys - 1) / kDqKeys, (double)p.B * p.Hq * fwd_total_tiles(p.n_tiles, 0, p.T, kDqKeys), kDqCosts);
+    pq.div_split = fastdiv_make((unsigned)pq.split);
+    pq.sched = pq.split > 1 ? nullptr : next_sched_pair(dq_items, dq_grid);
     // (no table where every CTA has one item: one line of constants less in front of its first load)
-    const ItemTable& tab = item_table_for(pq.sched || dq_items <= dq_grid ? -1 : (long long)dq_items, dq_grid, p.B * p.Hq, p.n_tiles, p.T, 4);
-    if constexpr (kWide)
-        e = launch_pdl(attn_bwd_dq_wide_kernel<D>, dq_grid, DqWideCfg<D>::kThreads, DqWideCfg<D>::kSmemBytes, st, tq, tk, tv, tdo, pq, tab);
-    else
-        e = launch_pdl(attn_bwd_dq_kernel<D>, dq_grid, DqCfg<D>::kThreads, spread_smem(DqCfg<D>::kSmemBytes, dq_grid <= (unsigned)sm_count()), st, tq, own[0], own[1], tdo, own[2], pq, tab);
+    const ItemTable& tab = item_table_for(pq.split > 1 || pq.sched || dq_items <= dq_grid ? -1 : (long long)dq_items, dq_grid, p.B * p.Hq, p.n_tiles, p.T, 4);
+    auto launch_dq = [&](auto kernel, bool* set, int bytes, int threads, bool one_per_sm, auto&&... maps) {
+        if ((rc = set_smem_once(kernel, std::max(bytes, kAloneSmemBytes), set))) return cudaErrorInvalidValue;
+        return launch_cluster(kernel, dim3(pq.split > 1 ? dq_items * (unsigned)pq.split : dq_grid), threads, spread_smem(bytes, one_per_sm), st, pq.split,
+                              maps..., pq, tab);
+    };
+    const bool dq_spread = pq.split > 1 ? (double)dq_items * pq.split <= cluster_slots(pq.split) : dq_grid <= (unsigned)sm_count();
+    if constexpr (kWide) {
+        using Cfg = DqWideCfg<D>;
+        e = pq.split > 1 ? launch_dq(attn_bwd_dq_wide_kernel<D, true>, dq_split_set, Cfg::kSmemBytes, Cfg::kThreads, false, tq, tk, tv, tdo)
+                         : launch_dq(attn_bwd_dq_wide_kernel<D, false>, dq_set, Cfg::kSmemBytes, Cfg::kThreads, false, tq, tk, tv, tdo);
+    } else {
+        using Cfg = DqCfg<D>;
+        e = pq.split > 1 ? launch_dq(attn_bwd_dq_kernel<D, true>, dq_split_set, Cfg::kSmemBytes, Cfg::kThreads, dq_spread, tq, own[0], own[1], tdo, own[2])
+                         : launch_dq(attn_bwd_dq_kernel<D, false>, dq_set, Cfg::kSmemBytes, Cfg::kThreads, dq_spread, tq, own[0], own[1], tdo, own[2]);
+    }
+    if (rc) return rc;
     if (e != cudaSuccess) {
         cudaGetLastError();
         return B200ATTN_ERR_CUDA;
