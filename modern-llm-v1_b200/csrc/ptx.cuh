@@ -1,5 +1,5 @@
 // Inline-PTX building blocks for the sm_100a attention kernels: mbarriers with
-// bounded waits, TMA tiled loads/stores, TMEM allocation, tcgen05 MMA issue,
+// bounded waits, TMA tiled loads, TMEM allocation, tcgen05 MMA issue,
 // commit and TMEM load/store, plus the shared-memory and instruction
 // descriptors those MMAs consume.
 //
@@ -41,7 +41,7 @@ __device__ __forceinline__ void fence_mbar_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 // Makes generic-proxy writes to shared memory visible to the async proxy
-// (TMA stores, tcgen05.mma operand reads).
+// (tcgen05.mma operand reads).
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
