@@ -39,10 +39,10 @@ FALLBACK_PEAKS = {"bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0, "hbm_g
 # bench.py --config NAME --steps 3 --warmup 3 --no-cpu-baseline --no-graph`); to be counted again when a kernel changes what it
 # reads.  Writes still in L2 at a kernel's end are not among them.  In the long-context configuration the dQ and dK/dV passes
 # read K, V or Q, dO several times, mostly from L2.
-NCU_TRAFFIC_BYTES = {"c2_50m_train": {"attn_fwd_kernel": 21190912, "attn_bwd_dq_kernel": 46794240,
-                                      "attn_bwd_dkdv_kernel": 34414080},
-                     "c3_300m_class": {"attn_fwd_kernel": 52976384, "attn_bwd_dq_kernel": 134066944,
-                                       "attn_bwd_dkdv_kernel": 95216128},
+NCU_TRAFFIC_BYTES = {"c2_50m_train": {"attn_fwd_kernel": 21029120, "attn_bwd_dq_kernel": 47025152,
+                                      "attn_bwd_dkdv_kernel": 34439680},
+                     "c3_300m_class": {"attn_fwd_kernel": 54776832, "attn_bwd_dq_kernel": 136037632,
+                                       "attn_bwd_dkdv_kernel": 94533632},
                      "c4_long_context": {"attn_fwd_kernel": 486543616, "attn_bwd_dq_kernel": 1004139776,
                                          "attn_bwd_dkdv_kernel": 1173410560}}
 
