@@ -43,8 +43,8 @@ NCU_TRAFFIC_BYTES = {"c2_50m_train": {"attn_fwd_kernel": 21029120, "attn_bwd_dq_
                                       "attn_bwd_dkdv_kernel": 34439680},
                      "c3_300m_class": {"attn_fwd_kernel": 54776832, "attn_bwd_dq_kernel": 136037632,
                                        "attn_bwd_dkdv_kernel": 94533632},
-                     "c4_long_context": {"attn_fwd_kernel": 486543616, "attn_bwd_dq_kernel": 1004139776,
-                                         "attn_bwd_dkdv_kernel": 1173410560}}
+                     "c4_long_context": {"attn_fwd_kernel": 454878720, "attn_bwd_dq_kernel": 907771136,
+                                         "attn_bwd_dkdv_kernel": 1184512768}}
 
 
 def load_peaks():
