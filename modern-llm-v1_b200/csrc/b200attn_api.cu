@@ -244,7 +244,7 @@ int set_smem_once(K kernel, int bytes, bool* done) {
 }
 
 // The SMs that clusters can have: those of four and eight do not fill the last SMs of a GPC and get 132 and 120 of 148.
-double cluster_slots(int cluster) { return sm_count() * (cluster <= 2 ? 1.0 : cluster <= 4 ? 0.89 : 0.81); }
+double cluster_slots(int cluster) { return sm_count() * (cluster <= 2 ? 1.0 : cluster <= 4 ? 0.892 : 0.811); }
 
 // Early launch of the next kernel (`early`): a kernel whose CTAs have one item each lets the next one start once their last loads are
 // issued, which hides the 1.3 us from the last CTA's end to the next kernel's first instruction.  The next kernel's CTAs then go to
@@ -268,7 +268,10 @@ inline size_t spread_smem(int bytes, bool one_per_sm) { return one_per_sm ? std:
 // for 1 / 2 / 4 / 8 shares: forward B=2 T=128 6/2 D=64 5.4 / 8.2 / 8.2 / 8.7, B=1 T=2000 6/2 D=64 22.5 / 18.2 / 23.9 / 36.6, 15 tokens
 // behind 6000 6/2 D=64 57.4 / 35.1 / 21.3 / 14.7, 500 behind 3000 B=2 16/4 D=128 43.6 / 36.2 / 50.6 / 86.5; dQ pass and dK/dV pass
 // B=1 T=2000 6/2 D=64 78.0 / 56.3 / 43.8 / 58.3, B=8 T=512 6/2 D=64 26.8 / 23.7 / 32.7 / 62.9, B=1 T=4096 8/2 D=128 264 / 162 / 121 /
-// 167, B=32 T=1001 1/1 D=128 44.2 / 77.9 / 136 / 262.  The order of the estimates is what counts: they are within some 12 % of the
+// 167, B=32 T=1001 1/1 D=128 44.2 / 77.9 / 136 / 262.  The costs of the forward and of the dK/dV pass at D=128 are those of the kernels with one
+// S buffer and copies by tcgen05.cp, fitted at 32 shapes with every number of shares and 95 whose pick they change; with the costs of the
+// kernels before, us: forward B=1 T=3870 6/2 D=64 37.7 instead of 28.6, T=5151 2/1 28.7 instead of 22.6, B=2 T=512 8/1 8.7 instead of 7.5, B=2 T=906 6/2
+// D=128 14.9 instead of 13.2; both passes of the backward B=5 T=4257 2/1 D=128 181 instead of 163.  The order of the estimates is what counts: they are within some 12 % of the
 // time in one round of items, and up to half too low where shared items run in many rounds.  They do not see how items of
 // different lengths pack.
 struct SplitCosts {
@@ -303,7 +306,7 @@ double fwd_total_tiles(int n_qtiles, int kv_off, int T, int keys) {
 template <int D>
 int fwd_split(int B, int Hq, int T, int kv_off, int n_qtiles) {
     constexpr int keys = FwdCfg<D>::kKeys;
-    constexpr SplitCosts kCosts = D == 64 ? SplitCosts{2, 1.25f, 1.95f, 2.f, 3.5f} : SplitCosts{2, 0.83f, 1.f, 3.5f, 3.5f};
+    constexpr SplitCosts kCosts = D == 64 ? SplitCosts{2, 1.35f, 1.6f, 2.8f, 3.5f} : SplitCosts{2, 0.9f, 1.05f, 4.f, 3.5f};
     return pick_split((long long)n_qtiles * Hq * B, (kv_off + T + keys - 1) / keys, (double)B * Hq * fwd_total_tiles(n_qtiles, kv_off, T, keys), kCosts);
 }
 
@@ -567,7 +570,7 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     const unsigned kv_items = (unsigned)(p.n_tiles * p.Hkv * p.B);
     BwdParams pk = p;
     // (the exchange is 64 KB in and out of every CTA at D = 128, at the 13 bytes a clock of distributed shared memory)
-    constexpr SplitCosts kCosts = D == 64 ? SplitCosts{1, 1.4f, 1.4f, 3.f, 3.5f} : SplitCosts{1, 1.9f, 1.9f, 7.f, 3.5f};
+    constexpr SplitCosts kCosts = D == 64 ? SplitCosts{1, 1.4f, 1.4f, 3.f, 3.5f} : SplitCosts{1, 1.8f, 1.8f, 5.6f, 3.5f};
     pk.split = pick_split(kv_items, p.group * p.n_tiles, (double)p.B * p.Hq * p.n_tiles * (p.n_tiles + 1) / 2, kCosts);
     pk.div_split = fastdiv_make((unsigned)pk.split);
     const int fs = fwd_split<D>(p.B, p.Hq, p.T, 0, p.n_tiles);
