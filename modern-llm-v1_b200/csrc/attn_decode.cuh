@@ -33,6 +33,8 @@
 // Eight compute warps in one CTA per SM, taking tiles in two groups, were slower at every piece's end (B=300: 42.8).
 #pragma once
 
+#include <algorithm>
+
 #include "ptx.cuh"
 
 namespace b200attn {
@@ -124,11 +126,15 @@ struct DecodeWalk {
 
 // EARLY: in front of the wait for the kernel that may write the lengths; read through L2, so that no stale copy stays in L1
 template <bool EARLY = false>
-__device__ __forceinline__ int decode_len(const DecodeParams& p, int b) {
+__host__ __device__ __forceinline__ int decode_len(const DecodeParams& p, int b) {
+#ifdef __CUDA_ARCH__
     return p.lens ? max(1, min(EARLY ? __ldcg(p.lens + b) : __ldg(p.lens + b), p.L)) : p.L;
+#else
+    return p.lens ? std::max(1, std::min(p.lens[b], p.L)) : p.L;
+#endif
 }
 // First tile of CTA c's range, and the CTA whose range holds tile t.
-__device__ __forceinline__ int decode_range(const DecodeWalk& w, int c) {
+__host__ __device__ __forceinline__ int decode_range(const DecodeWalk& w, int c) {
     const unsigned n = unsigned(w.n_ctas), q = unsigned(w.total) / n;
     return int(unsigned(c) * q + unsigned(c) * (unsigned(w.total) - q * n) / n);
 }
@@ -210,16 +216,36 @@ __device__ __forceinline__ DecodeWalk decode_walk_start(const DecodeParams& p, i
     return w;
 }
 // Tiles of the piece at w.t
-__device__ __forceinline__ int decode_piece(const DecodeWalk& w) { return min(w.t_end - w.t, w.n_tiles - w.j0); }
+__host__ __device__ __forceinline__ int decode_piece(const DecodeWalk& w) {
+    const int range = w.t_end - w.t, unit = w.n_tiles - w.j0;
+    return range < unit ? range : unit;
+}
 template <int KEYS, bool EARLY = false>
-__device__ __forceinline__ void decode_walk_next(const DecodeParams& p, DecodeWalk& w, int n) {
+__host__ __device__ __forceinline__ void decode_walk_next(const DecodeParams& p, DecodeWalk& w, int n) {
     w.t += n;
     w.j0 = 0;  // the piece ended at its unit's end, or the range is over
     if (w.t < w.t_end && ++w.u == p.units_per_seq) {
         w.u = 0;
         ++w.b;
+        // (the range's end and this sequence may come from different lengths, see decode_first_tiles)
+        if (EARLY && w.b == p.B) {
+            w.t = w.t_end;
+            return;
+        }
         w.len = decode_len<EARLY>(p, w.b);
         w.n_tiles = (w.len + KEYS - 1) / KEYS;
+    }
+}
+// The range's first `left` tiles, for a look at them in front of the wait: visit(sequence, unit within it, tile).  The kernel in
+// front may write the lengths meanwhile, so w.t_end, w.b and what is read here need not fit together: the tiles are a guess, all
+// inside the cache, and the walk ends at the last sequence at the latest.
+#pragma nv_exec_check_disable
+template <int KEYS, typename Visit>
+__host__ __device__ __forceinline__ void decode_first_tiles(const DecodeParams& p, DecodeWalk w, int left, Visit visit) {
+    while (w.t < w.t_end && left > 0) {
+        const int tiles = decode_piece(w);
+        for (int i = 0; i < tiles && left > 0; ++i, --left) visit(w.b, w.u, w.j0 + i);
+        decode_walk_next<KEYS, true>(p, w, tiles);
     }
 }
 __device__ __forceinline__ int decode_slot(const DecodeParams& p, const DecodeWalk& w, int c, int first_cta, int unit_start) {
@@ -472,20 +498,18 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         // First, while the kernel in front is still at work: this CTA's first tiles into L2 (coherent: what that kernel still
         // writes there is what the loads behind the wait find).
         if constexpr (PF > 0) {
-            DecodeWalk w = decode_walk_start<KEYS, true>(p, int(blockIdx.x), int(gridDim.x), lane);
-            for (int left = PF; w.t < w.t_end && left > 0;) {
-                const int tiles = decode_piece(w), hk = int(fastdiv(w.u, p.div_chunks));
-                for (int i = 0; i < tiles && left > 0; ++i, --left)
-                    if (elect_one()) {
+            const DecodeWalk w = decode_walk_start<KEYS, true>(p, int(blockIdx.x), int(gridDim.x), lane);
+            decode_first_tiles<KEYS>(p, w, PF, [&](int b, int u, int tile) {
+                const int hk = int(fastdiv(u, p.div_chunks));
+                if (elect_one()) {
 #pragma unroll
-                        for (int bx = 0; bx < Cfg::kBoxes; ++bx) {
-                            tma_prefetch_4d(&tmK, bx * 64, (w.j0 + i) * KEYS, hk, w.b);
-                            tma_prefetch_4d(&tmV, bx * 64, (w.j0 + i) * KEYS, hk, w.b);
-                        }
+                    for (int bx = 0; bx < Cfg::kBoxes; ++bx) {
+                        tma_prefetch_4d(&tmK, bx * 64, tile * KEYS, hk, b);
+                        tma_prefetch_4d(&tmV, bx * 64, tile * KEYS, hk, b);
                     }
+                }
                 __syncwarp();
-                decode_walk_next<KEYS, true>(p, w, tiles);
-            }
+            });
         }
         grid_dep_wait();
         const DecodeWalk w = decode_walk_start<KEYS>(p, int(blockIdx.x), int(gridDim.x), lane);
