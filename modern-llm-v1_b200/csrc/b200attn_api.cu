@@ -1043,8 +1043,13 @@ int launch_decode_pf(const CUtensorMap& tk, const CUtensorMap& tv, const DecodeP
 }
 
 // Where the CTAs fill most of the device the launch is bound by HBM, and the first two tiles of each come into L2 while the kernel
-// in front ends (us per call, append + decode: B=48 L<=6000 16/4 D=64 35.4 -> 34.0, B=64 L=4096 43.4 -> 42.6; decode alone, B=300
-// L=200 8/8 23.6 -> 22.4, B=8 L=2000 8/8 D=128, 128 CTAs, 14.2 -> 13.8; with three tiles the gain is smaller, with six it is gone).
+// in front ends, provided that it lets this one start early, as the append of one token and the decode itself do (us per call over
+// caches larger than L2 in turn, without / with: append + decode B=48 L<=6000 16/4 D=64 35.6 / 34.3, B=64 L<=4096 33.5 / 31.8, B=20 L<=1500
+// D=128 19.3 / 18.0; decode behind decode B=64 L=4096 16/4 D=64 41.9 / 41.3, B=300 L=200 8/8 24.0 / 22.8, B=64 L=1000 6/2 9.0 / 8.5, B=8
+// L=2000 8/8 D=128, 128 CTAs, 14.3 / 14.1).  With a matrix product in front of each append + decode, the product included: 40.6 / 39.9,
+// 38.3 / 37.5, 23.4 / 23.0.  Behind a kernel that does not release this one early the tiles are asked for twice: product and decode
+// 46.1 / 46.0, 29.8 / 29.5, 13.3 / 13.4, 19.1 / 19.3; a first pass on new buffers on an idle device gains nothing (host's time of a call,
+// B=300 41.8 / 42.1, append + decode B=48 67.3 / 67.0).  With three tiles the gain is smaller, with six it is gone.
 // Fewer CTAs are bound by latency, of which this hides nothing: B=6 L<=3000 8/1 D=128 8.5 -> 8.6, B=1 L=1500 16/4 5.26 -> 5.30.
 constexpr int kPrefetchCtas = 128;
 template <int D, int NH>
