@@ -32,6 +32,34 @@ def test_groups_and_numbers_of_ctas(B, Hq, Hkv, D):
         assert (a.float() - b.float()).norm() <= 2.0 ** -9 * b.float().norm()
 
 
+@pytest.mark.parametrize("B,Hq,Hkv", [(3, 4, 4), (60, 6, 2), (50, 16, 4)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_heads_where_the_projection_left_them(B, Hq, Hkv, D):
+    check_against_oracle(*_case(B, 77, Hq, Hkv, D), layout="BTHD")
+
+
+# by head in a cluster, by head without a group, by group
+@pytest.mark.parametrize("B,Hq,Hkv", [(2, 6, 2), (3, 4, 4), (60, 6, 2)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("T", [100, 128])
+@pytest.mark.parametrize("where", ["key", "query", "value", "gradient"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_nan_and_infinity_go_where_the_two_passes_take_them(B, Hq, Hkv, D, T, where, bad):
+    q, k, v, do = _case(B, T, Hq, Hkv, D)
+    b, hk, group, row = B - 1, Hkv - 1, Hq // Hkv, 70
+    x, h = {"key": (k, hk), "query": (q, hk * group), "value": (v, hk), "gradient": (do, hk * group)}[where]
+    x[b, h, row, 5] = bad
+    got = [y.float() for y in run_fwd_bwd(q, k, v, do)]
+    want = [y.float() for y in run_fwd_bwd(q, k, v, do, mode="two_pass")]
+    for a, w in zip(got, want):
+        assert torch.equal(torch.isfinite(a), torch.isfinite(w)) and torch.equal(torch.isnan(a), torch.isnan(w))
+    assert not torch.isfinite(got[3 if where == "value" else 4][b, hk]).all()  # it reached dK or dV of its head
+    for i, own in enumerate((slice(hk * group, None),) * 3 + (slice(hk, None),) * 2):
+        rest = got[i].clone()
+        rest[b, own] = 0.0
+        assert torch.isfinite(rest).all()
+
+
 @pytest.mark.parametrize("B,Hq,Hkv", [(2, 6, 2), (3, 4, 4), (60, 6, 2)])
 @pytest.mark.parametrize("D", [64, 128])
 def test_a_set_status_word_leaves_the_gradients_alone(B, Hq, Hkv, D):

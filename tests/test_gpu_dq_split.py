@@ -22,6 +22,23 @@ def test_split_dq(B, T, Hq, Hkv, D):
     assert all(torch.equal(a, b) for a, b in zip(got, again)), "a call does not repeat bit for bit"
 
 
+@pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 1900, 4, 2), (1, 3011, 1, 1)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("where", ["key", "query", "value", "gradient"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_nan_and_infinity_go_where_an_unshared_item_takes_them(B, T, Hq, Hkv, D, where, bad):
+    # the same sequence sixteen times: too many items to share any
+    q, k, v, do = _case(B, T, Hq, Hkv, D)
+    x = {"key": k, "query": q, "value": v, "gradient": do}[where]
+    x[0, 0, T // 2, 5] = bad
+    got = [y.float() for y in run_fwd_bwd(q, k, v, do)]
+    want = [y[:1].float() for y in run_fwd_bwd(*(y.repeat(16, 1, 1, 1) for y in (q, k, v, do)))]
+    for a, w in zip(got, want):
+        assert torch.equal(torch.isfinite(a), torch.isfinite(w)) and torch.equal(torch.isnan(a), torch.isnan(w))
+    assert not torch.isfinite(got[2][0, 0]).all()  # it reached dQ of its head
+    assert Hkv == 1 or torch.isfinite(got[2][0, Hq // Hkv :]).all()
+
+
 @pytest.mark.parametrize("D", [64, 128])
 def test_a_set_status_word_leaves_dq_alone(D):
     B, T, Hq, Hkv = 1, 3000, 2, 1
