@@ -279,11 +279,11 @@ struct SplitCosts {
     float tile_one, tile_all;  // us per tile in a CTA that has the SM to itself, and with a second CTA beside it
     float exchange, start;     // us: the exchange in a cluster of two, a CTA's start
 };
-int pick_split(long long items, int longest, double total, const SplitCosts& c) {
+int pick_split(long long items, int longest, double total, const SplitCosts& c, int most = 8) {
     const int sms = sm_count();
     int best = 1;
     double best_us = 1e30;
-    for (int split = 1; split <= 8; split *= 2) {
+    for (int split = 1; split <= most; split *= 2) {
         const double slots = c.per_sm * cluster_slots(split), ctas = (double)items * split;
         const double shared = c.per_sm > 1 ? std::min(1.0, std::max(0.0, ctas / sms - 1)) : 0.0;  // SMs with two CTAs
         const double share = (longest + split - 1) / split * (c.tile_one + (c.tile_all - c.tile_one) * shared);
@@ -537,10 +537,11 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     BwdParams pq = p;
     // Few, long items are shared by clusters (both passes of the backward, us for 1 / 2 / 4 / 8 CTAs of the dQ pass: B=1 T=4000 2/1 D=64 61.3 / 51.0 /
     // 44.1 / 52.2, D=128 76.9 / 65.2 / 68.4 / 102; T=2000 6/2 D=64 41.7 / 37.9 / 43.1 / 54.3, D=128 54.1 / 56.0 / 70.1 / 115; T=1000 8/8 D=64 23.4 / 22.6 /
-    // 24.1 / 33.1; T=500 6/2 D=64 18.6 / 19.0 / 18.4 / 19.9, B=2 T=700 8/2 D=64 23.9 / 26.0 / 31.9 / 44.3).
+    // 24.1 / 33.1; T=500 6/2 D=64 18.6 / 19.0 / 18.4 / 19.9, B=2 T=700 8/2 D=64 23.9 / 26.0 / 31.9 / 44.3).  Four at most: the costs
+    // never ask for eight (1 to 296 heads of up to 38400 tokens), which was the slowest wherever it was measured but at T=4000 D=64.
     constexpr SplitCosts kDqCosts = D == 64 ? SplitCosts{2, 0.43f, 0.6f, 2.f, 4.f} : SplitCosts{1, 1.06f, 1.06f, 5.6f, 4.f};
     constexpr int kDqKeys = D == 64 ? 64 : 128;
-    pq.split = pick_split(dq_items, (p.T + kDqKeys - 1) / kDqKeys, (double)p.B * p.Hq * fwd_total_tiles(p.n_tiles, 0, p.T, kDqKeys), kDqCosts);
+    pq.split = pick_split(dq_items, (p.T + kDqKeys - 1) / kDqKeys, (double)p.B * p.Hq * fwd_total_tiles(p.n_tiles, 0, p.T, kDqKeys), kDqCosts, 4);
     pq.div_split = fastdiv_make((unsigned)pq.split);
     pq.sched = pq.split > 1 ? nullptr : next_sched_pair(dq_items, dq_grid);
     // (no table where every CTA has one item: one line of constants less in front of its first load)

@@ -10,7 +10,7 @@ from test_gpu_status_word import _full_cache, _nan_like, _overflow, _take_status
 
 pytestmark = pytest.mark.gpu
 
-# clusters of two, four and eight at D = 64, of two at D = 128; the first query tiles have fewer key tiles than the cluster CTAs
+# CTAs per item 2, 2, 4, 4, 2 at D = 64 and 1, 2, 2, 4, 2 at D = 128; the first query tiles have fewer key tiles than the cluster CTAs
 SHAPES = [(1, 1025, 8, 4), (1, 1900, 4, 2), (1, 2049, 2, 1), (1, 3011, 1, 1), (2, 2000, 2, 2)]
 
 
