@@ -936,8 +936,9 @@ extern "C" int b200attn_bwd_static(const void* q, const void* k, const void* v, 
     if (bwd_vec_elems(B, T, Hq) > (size_t)B200ATTN_BWD_STATIC_MAX_ROWS) return B200ATTN_ERR_TOO_LARGE;
     float* scratch = bwd_static_scratch(&rc);
     if (!scratch) return rc;
-    // Same kernels as b200attn_bwd; the preprocess kernel rewrites every row (padding included) that
-    // the two passes read, so stale contents of an earlier call are never seen.
+    // Always the two passes; the dQ pass rewrites every row of the row vectors (padding included) that the dK/dV pass reads, so
+    // stale contents of an earlier call are never seen.  b200attn_bwd may take the one-tile kernel for T <= 128 (bwd_tile), whose
+    // sums are grouped in another way: the two may differ there by roundings.
     return b200attn_bwd_mode(q, k, v, o, lse, dout, dq, dk, dv, B, T, Hq, Hkv, D, layout, softmax_scale,
                              B200ATTN_BWD_TWO_PASS, scratch, 2 * sizeof(float) * (size_t)B200ATTN_BWD_STATIC_MAX_ROWS, stream);
 }

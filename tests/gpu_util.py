@@ -72,3 +72,13 @@ def check_against_oracle(q, k, v, do, layout="BHTD", mode="auto"):
 def randn_bf16(shape, seed, std=1.0, device="cuda"):
     g = torch.Generator().manual_seed(seed)
     return (torch.randn(shape, generator=g) * std).bfloat16().to(device)
+
+
+def kernels_of(call):
+    """Names of the CUDA kernels that `call` launches, template arguments included."""
+    call()
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    return [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]

@@ -5,14 +5,17 @@ import torch
 
 import modern_llm_v1_b200 as m
 
-from gpu_util import check_against_oracle, randn_bf16, run_fwd_bwd
+from gpu_util import check_against_oracle, kernels_of, randn_bf16, run_fwd_bwd
 from test_gpu_parity import _case
 from test_gpu_status_word import _full_cache, _nan_like, _overflow, _take_status, _untouched
 
 pytestmark = pytest.mark.gpu
 
-# clusters of 1, 2, 3, 5, 6 and 8 query heads; by group: one and several rounds of CTAs; a group larger than a cluster
-GROUPS = [(3, 4, 4), (2, 4, 2), (2, 6, 2), (1, 5, 1), (2, 6, 1), (1, 16, 2), (60, 6, 2), (50, 16, 4), (24, 12, 1)]
+# clusters of 1, 2, 3, 5, 6 and 8 query heads; by group at both D or at D = 128 only (several rounds of CTAs, a group larger than a
+# cluster), where Q and dO of five heads and more go through two places; too few CTAs by group
+GROUPS = {(3, 4, 4): "head head", (2, 4, 2): "head head", (2, 6, 2): "head head", (1, 5, 1): "head head", (2, 6, 1): "head head",
+          (1, 16, 2): "head head", (60, 6, 2): "group group", (130, 8, 1): "group group", (50, 16, 4): "passes group",
+          (180, 12, 1): "passes group", (24, 12, 1): "passes passes"}
 
 
 @pytest.mark.parametrize("T", [1, 2, 33, 64, 127, 128])
@@ -30,6 +33,15 @@ def test_groups_and_numbers_of_ctas(B, Hq, Hkv, D):
     # the same products in another grouping: a few roundings to BF16 (2^-9 each) of the outputs
     for a, b in zip(got[2:], run_fwd_bwd(*_case(B, 100, Hq, Hkv, D), mode="two_pass")[2:]):
         assert (a.float() - b.float()).norm() <= 2.0 ** -9 * b.float().norm()
+
+
+@pytest.mark.parametrize("B,Hq,Hkv", GROUPS)
+@pytest.mark.parametrize("D", [64, 128])
+def test_which_kernel(B, Hq, Hkv, D):
+    names = " ".join(n for n in kernels_of(lambda: run_fwd_bwd(*_case(B, 100, Hq, Hkv, D))) if "attn_bwd" in n)
+    took = "head" if f"attn_bwd_tile_kernel<{D}, true>" in names else "group" if f"attn_bwd_tile_kernel<{D}, false>" in names else "passes"
+    assert took == GROUPS[B, Hq, Hkv].split()[D == 128], names
+    assert ("attn_bwd_dq" in names and "attn_bwd_dkdv" in names) == (took == "passes"), names
 
 
 @pytest.mark.parametrize("B,Hq,Hkv", [(3, 4, 4), (60, 6, 2), (50, 16, 4)])

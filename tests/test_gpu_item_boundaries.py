@@ -9,8 +9,10 @@ from test_gpu_parity import _case
 pytestmark = pytest.mark.gpu
 
 
-# items: 960 of one 64-key tile; 960 of two (the second a single key); 720 of two or three; counter-based lists with 1920
+# items of the dQ pass: 960 of one 64-key tile; 960 of two (the second a single key); 720 of two or three; counter-based lists with 1920.
+# "auto" takes the first two shapes at D = 128 to the kernel for sequences of one tile.
 @pytest.mark.parametrize("B,T,Hq,Hkv", [(80, 40, 12, 4), (160, 65, 6, 2), (60, 130, 6, 3), (160, 129, 6, 6)])
 @pytest.mark.parametrize("D", [64, 128])
-def test_short_items_in_a_row(B, T, Hq, Hkv, D):
-    check_against_oracle(*_case(B, T, Hq, Hkv, D), layout="BTHD" if T == 65 else "BHTD")
+@pytest.mark.parametrize("mode", ["auto", "two_pass"])
+def test_short_items_in_a_row(B, T, Hq, Hkv, D, mode):
+    check_against_oracle(*_case(B, T, Hq, Hkv, D), layout="BTHD" if T == 65 else "BHTD", mode=mode)
