@@ -260,16 +260,14 @@ double cluster_slots(int cluster) { return sm_count() * (cluster <= 2 ? 1.0 : cl
 // backward 22.0 / 22.8, D=128 34.6 / 36.0, RoPE + QK-Norm, forward and backward and back 37.7 / 37.9, D=128 58.0 / 59.2; B=100 T=100 16/4 D=128
 // 156.4 / 159.6; only backwards in a row gain, 14.4 / 14.1), and a forward at D = 64 of more than three query tiles and more CTAs than SMs, whose dQ pass shares SMs in
 // pairs of a heavy and a light CTA (B=8 T=512 6/2 34.5 -> 35.3, B=5 T=500 10/10 31.2 -> 32.0; of three, B=16 T=300 6/2, 33.8 -> 32.7).
-// What follows matters little to the release of the dK/dV pass and of the tile kernel by head, and not always for the good.  Released at the end /
-// early by this rule / wherever the items run in one round, us, with the forward behind (and a backward behind that), with the RoPE + QK-Norm
-// backward behind (in the chain of RoPE + QK-Norm, forward, backward and back), with a backward behind: B=2 T=700 8/2 35.2 / 34.9 / 34.9, 43.15 / 43.2 /
-// 43.2, 24.9 / 24.5 / 24.5; B=8 T=300 6/2 28.3 / 28.1 / 28.1, 37.4 / 38.05 / 38.05, 20.2 / 19.8 / 19.8; B=1 T=500 6/2 D=128 34.5 / 34.4 / 34.4, 41.5 / 41.8 /
-// 41.8, 24.9 / 24.4 / 24.4; B=2 T=128 6/2 13.9 to 14.1 / 13.9 / 13.9, 19.8 / 20.0 / 20.0, 9.6 / 9.5 / 9.5; where the rule says no: B=3 T=2000 6/2 82.8 /
-// 82.7 / 86.5, 97.3 / 97.4 / 98.1, 59.1 / 59.1 / 64.5; B=8 T=512 6/2 34.5 / 34.5 / 35.3, 46.0 / 46.0 / 47.1, 24.0 / 23.9 / 26.3; B=4 T=1024 16/4 75.2 / 75.1 / 75.1,
-// 93.0 / 93.1 / 95.0, 55.9 / 55.9 / 56.0.  A matrix product of a library waits for the end anyway.  So with attention behind the rule gains up to
-// 2 %, with RoPE + QK-Norm it costs up to 2 %, whose CTAs spread over the SMs by their shared memory do no better.  The forward's release, with
-// the backward behind, B=32 T=1001 1/1 D=128 60.6 / 58.6 and in the chain 92.7 / 87.6, B=4 T=1024 8/2 D=128 75.1 / 73.4 and 92.6 / 89.8, B=2 T=700 8/2
-// 35.5 / 34.8 and 43.0 / 42.8; with the RoPE + QK-Norm forward of the next call behind it costs 0.1 to 0.5 us (B=8 T=300 6/2 10.7 / 11.2).
+// For the release of the dK/dV pass and of the tile kernel by head it matters what follows: with attention behind it gains up to 2 %, with the RoPE +
+// QK-Norm backward behind it costs up to 2 % (spreading that kernel over the SMs, too, does not help), a matrix product of a library waits
+// for the end anyway.  us, released at the end / early, forward and backward; RoPE + QK-Norm, forward, backward and back; backwards in a row:
+//   B=2 T=700 8/2 35.2 / 34.9; 43.15 / 43.2; 24.9 / 24.5      B=8 T=300 6/2 28.3 / 28.1; 37.4 / 38.05; 20.2 / 19.8
+//   B=1 T=500 6/2 D=128 34.5 / 34.4; 41.5 / 41.8; 24.9 / 24.4  B=2 T=128 6/2 14.1 / 13.9; 19.8 / 20.0; 9.6 / 9.5
+//   and where the rule says no: B=3 T=2000 6/2 82.8 / 86.5; 97.3 / 98.1; 59.1 / 64.5   B=8 T=512 6/2 34.5 / 35.3; 46.0 / 47.1; 23.9 / 26.3
+// The forward's release, with the backward behind, alone and in that chain: B=32 T=1001 1/1 D=128 60.6 / 58.6; 92.7 / 87.6, B=2 T=700 8/2 35.5 / 34.8;
+// 43.0 / 42.8; with the RoPE + QK-Norm forward of another call behind it costs 0.1 to 0.5 us (B=8 T=300 6/2 10.7 / 11.2).
 constexpr int kAloneSmemBytes = 114 * 1024;
 inline size_t spread_smem(int bytes, bool one_per_sm) { return one_per_sm ? std::max(bytes, kAloneSmemBytes) : bytes; }
 
