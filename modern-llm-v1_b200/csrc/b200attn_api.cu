@@ -256,9 +256,9 @@ double cluster_slots(int cluster) { return sm_count() * (cluster <= 2 ? 1.0 : cl
 // Not early: kernels with several items per CTA (the next kernel's CTAs, dealt their work in pairs per SM, then share SMs as it happens:
 // forward of B=32 T=512 6/2 D=64 18.3 -> 18.7), clusters beyond one CTA per SM (forward of B=1 T=2000 4/4 D=128 18.0 -> 20.7), a dK/dV
 // pass whose forward has more CTAs than SMs (B=3 T=2000 6/2 D=64 83.3 -> 86.0; also with other kernels behind, below), the tile kernel by head in
-// clusters on more than half the SMs (B=14 T=128 6/2 D=128 20.5 -> 21.2) and by group (B=60 T=128 6/2, released at the end / early: forward and
-// backward 22.0 / 22.8, D=128 34.6 / 36.0, RoPE + QK-Norm, forward and backward and back 37.7 / 37.9, D=128 58.0 / 59.2; B=100 T=100 16/4 D=128
-// 156.4 / 159.6; only backwards in a row gain, 14.4 / 14.1), and a forward at D = 64 of more than three query tiles and more CTAs than SMs, whose dQ pass shares SMs in
+// clusters on more than half the SMs (B=14 T=128 6/2 D=128 20.5 -> 21.2), by group on more than half the SMs or at D = 128 (T=128 6/2, released at
+// the end / early, forward and backward; RoPE + QK-Norm, forward, backward and back: B=27 T=100 18.0 / 17.2; 28.1 / 28.25, B=36 19.5 / 19.1; 31.6 /
+// 31.85, B=48 20.15 / 19.95; 33.9 / 34.9, B=60 22.0 / 22.8; 37.7 / 37.9, D=128 B=36 30.1 / 30.75; 46.6 / 46.7, B=60 34.6 / 36.0; 58.0 / 59.2), and a forward at D = 64 of more than three query tiles and more CTAs than SMs, whose dQ pass shares SMs in
 // pairs of a heavy and a light CTA (B=8 T=512 6/2 34.5 -> 35.3, B=5 T=500 10/10 31.2 -> 32.0; of three, B=16 T=300 6/2, 33.8 -> 32.7).
 // For the release of the dK/dV pass and of the tile kernel by head it matters what follows: with attention behind it gains up to 2 %, with the RoPE +
 // QK-Norm backward behind it costs up to 2 % (spreading that kernel over the SMs, too, does not help), a matrix product of a library waits
@@ -516,7 +516,7 @@ int launch_bwd_tile(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensor
     record_bwd_event(0, st);
     const int ctas = p.B * (ONE ? p.Hq : p.Hkv);
     BwdParams pt = p;
-    pt.early = ONE && (p.group == 1 || 2 * ctas <= sm_count());
+    pt.early = (ONE && p.group == 1) || ((ONE || D == 64) && 2 * ctas <= sm_count());
     const cudaError_t e = launch_cluster(attn_bwd_tile_kernel<D, ONE>, dim3((unsigned)ctas), Cfg::kThreads, Cfg::kSmemBytes, st, ONE ? p.group : 1,
                                          tk, tv, tq, tdo, pt);
     if (e != cudaSuccess) {

@@ -189,7 +189,7 @@ __device__ __forceinline__ uint64_t make_sdesc_plain(uint32_t smem_addr, uint32_
 // that.  grid_dep_launch() is called where the next kernel is short or known: in the dQ pass
 // (after its own wait, so everything older is complete), in the one-pass backward's row-vector
 // kernel, in the decode and in the append of one token.  The forward, the dK/dV pass and the
-// backward of one tile by head call it late, by their producer warps once their last loads are issued, and
+// backward of one tile call it late, by their producer warps once their last loads are issued, and
 // only where the host says so (`early` in their parameters, see spread_smem in b200attn_api.cu).
 // From their very beginning a dependent grid would be queued behind a kernel for its whole run
 // time, which measured slower (2 %) than one released as the CTAs exit.
